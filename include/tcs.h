@@ -232,16 +232,18 @@ const char *tcs_timer_name(int timer);
 int tcs_bounds_checked(void);
 int tcs_bounds_violations(tcs_ctx *ctx, double *count);
 int tcs_set_use_graph(tcs_ctx *ctx, int on);
-/* launch-shape knobs (powers of two): lines per thread block of the strided
- * (y, z), contiguous (x) and modal line solvers and of the x and z FFTs, and
- * the most lanes (partitions) a tridiagonal line is split over.  A line-solver
+/* launch-shape knobs (powers of two): lines per thread block of the y lines,
+ * the contiguous (x) and the modal line solvers and of the x and z FFTs, and
+ * the most lanes (partitions) a tridiagonal line is split over (32: no bound for
+ * the z sweeps, whose segments also follow the line's length).  A line-solver
  * value is an upper bound: each launch runs the largest power of two up to it
  * whose blocks fit the SM's shared memory at the family's blocks per SM; a
- * value no single block could hold is refused (TCS_ERR_ARG).
- * TCS_TUNE_LONG_LINES picks where long strided lines run as one block per SM
- * (the same warps, lines fitted to 132 KiB of shared memory so that L1 keeps
- * 124 KiB) when the usual blocks would leave under 60 KiB of L1 or halve
- * their lines: 1 never, 2 the z sweeps (default), 4 the z and y sweeps.
+ * value no single block could hold is refused (TCS_ERR_ARG).  The z sweeps
+ * choose their own lines per block.
+ * TCS_TUNE_LONG_LINES: 4 runs long y lines as one block per SM (the same
+ * warps, lines fitted to 132 KiB of shared memory so that L1 keeps 124 KiB)
+ * when the usual blocks would leave under 60 KiB of L1 or halve their lines; 1
+ * and 2 (default) do not.
  * TCS_TUNE_Y_SOLVER picks the tridiagonal solver of the non-cyclic strided
  * lines: 1 the partitioned solver that every sweep uses (default: modified
  * Thomas per lane with a parallel reduced-system solve, pascal_tdma.f90:
@@ -259,16 +261,13 @@ int tcs_set_use_graph(tcs_ctx *ctx, int on);
  * (TCS_TUNE_FFT_LINES_X sets those of the pressure right-hand side and its
  * forward x transform).
  * TCS_TUNE_MIXED_ROWS (FP32-mixed form; no effect in the FP64 form): 1 the x
- * and z sweeps eliminate their FP32 rows in FP32 with one FP64-residual
- * refinement pass (default); 2 the x sweeps eliminate their FP32-built rows
- * in FP64 instead (no refinement pass; the solution is rounded once to FP32);
- * 4 the x and z sweeps; 8 the same with the z sweeps at three blocks per SM
- * (shared-memory elimination; faster at 256^3, slower at 512^3).
- * TCS_TUNE_Z_STAGING (FP64 form): 1 the z sweep of solvedW reads its stencil
- * inputs from global memory (default); 2 it stages them into shared memory with
- * tensor-memory-accelerator (TMA) box copies one pass of 64 k-planes ahead
- * (same arithmetic, same results; refused, TCS_ERR_ARG, unless the form is
- * FP64, N3 a multiple of 64 and N1 even). */
+ * sweeps eliminate their FP32 rows in FP32 with one FP64-residual refinement
+ * pass (default); 2, 4 and 8 they eliminate their FP32-built rows in FP64
+ * instead (no refinement pass; the solution is rounded once to FP32).  The z
+ * sweeps always eliminate in FP64.
+ * TCS_TUNE_Z_STAGING: 1 or 2; kept for programs that set it, without effect
+ * since the z sweeps have one staged form (2 is refused, TCS_ERR_ARG, unless the form is FP64, N3 a multiple of
+ * 64 and N1 even). */
 enum { TCS_TUNE_TL_STRIDED = 0, TCS_TUNE_TL_CONTIG, TCS_TUNE_TL_MODAL, TCS_TUNE_FFT_LINES_X, TCS_TUNE_FFT_LINES_Z,
        TCS_TUNE_LANES, TCS_TUNE_LONG_LINES, TCS_TUNE_Y_SOLVER, TCS_TUNE_IFFT_LINES_X, TCS_TUNE_MIXED_ROWS,
        TCS_TUNE_Z_STAGING, TCS_TUNE_COUNT };

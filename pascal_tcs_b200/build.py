@@ -22,7 +22,7 @@ LIB = os.path.join(HERE, "libtcs.so")
 LIB_BC = os.path.join(HERE, "libtcs_bc.so")
 SOURCES = ["tcs_thermal.cu", "tcs_momentum.cu", "tcs_pressure.cu", "tcs_post.cu",
            "tcs_tdma.cu", "tcs_capi.cu", "tcs_peak.cu"]
-HEADERS = ["tcs_device.cuh", "tcs_fields.cuh", "tcs_kernels.h"]
+HEADERS = ["tcs_device.cuh", "tcs_fields.cuh", "tcs_march.cuh", "tcs_tma.cuh", "tcs_kernels.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
          "--expt-relaxed-constexpr", "-I", CSRC, "-I", os.path.join(ROOT, "include")]

@@ -492,6 +492,8 @@ int tcs_create(const tcs_config *cfg, tcs_ctx **out)
         for (R **p : fl) if (!r) r = dalloc(c, p, NP);
         if (!r) r = dalloc(c, &F.Mu2, (size_t)(N2 + 2) * (N3 + 2));
         if (!r) r = dalloc(c, &F.iR2, (size_t)(N2 + 2) * (N3 + 2));
+        if (!r) r = dalloc(c, &F.MuT, (size_t)4 * (N2 + 2) * (N3 + 2));
+        if (!r) r = dalloc(c, &F.iRT, (size_t)4 * (N2 + 2) * (N3 + 2));
         if (HasLo<R>::on) {
             if (!r) r = dalloc(c, &F.iR2d, (size_t)(N2 + 2) * (N3 + 2));
         } else {
@@ -984,18 +986,18 @@ int tcs_set_tuning(tcs_ctx *c, int knob, int value)
         if (!ifftx_form(x.fp1u, value)) return set_err(TCS_ERR_ARG, "too many lines for shared memory");
         x.ifft_lines_x = value; break;
     case TCS_TUNE_MIXED_ROWS:
-        if (value > 8) return set_err(TCS_ERR_ARG, "mixed rows: 1 FP32 elimination, 2 FP64 rows in the x sweeps, 4 x and z sweeps, 8 z at 3 blocks per SM");
+        if (value > 8) return set_err(TCS_ERR_ARG, "mixed rows: 1 FP32 elimination in the x sweeps, 2, 4, 8 FP64 rows");
         x.mixed_rows = value; break;
     case TCS_TUNE_Z_STAGING:
-        if (value > 2) return set_err(TCS_ERR_ARG, "z staging: 1 global loads, 2 TMA-staged inputs for dw_z");
-        if (value == 2 && (c->fp32 || !dwz_staging_possible(x)))
+        if (value > 2) return set_err(TCS_ERR_ARG, "z staging: 1 or 2");
+        if (value == 2 && (c->fp32 || g.N3 % 64 || (g.P1 * 8) % 16))
             return set_err(TCS_ERR_ARG, "z staging needs the FP64 form, N3 a multiple of 64 and an even N1");
         x.z_staging = value; break;
     case TCS_TUNE_LANES:
         if (value < 2 || value > 32) return set_err(TCS_ERR_ARG, "lanes per line must be 2..32");
         x.lanes = value; break;
     case TCS_TUNE_LONG_LINES:
-        if (value > 4) return set_err(TCS_ERR_ARG, "long-line form: 1 never, 2 z sweeps, 4 z and y sweeps");
+        if (value > 4) return set_err(TCS_ERR_ARG, "long-line form: 1, 2 never, 4 the y sweeps");
         x.long_lines = value; break;
     case TCS_TUNE_Y_SOLVER: {
         if (value > 4) return set_err(TCS_ERR_ARG, "y solver: 1 partitioned, 2 one line per thread (y sweeps), 4 also the modal solves");

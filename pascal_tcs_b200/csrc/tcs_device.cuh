@@ -705,31 +705,26 @@ struct Refine { static constexpr bool on = std::is_same<R, float>::value; };
 
 // Blocks per SM a line-solver family is compiled for (each Prob's MINB; the
 // register budget is 65536 / (NT MINB), and fit_tl sizes the lines per block
-// to the matching shared-memory share).  Measured on B200 at 256^3: the FP64
-// z-sweep stencils need 128 registers and spill below that; the FP64 x and y
-// sweeps run fastest at 4 blocks (64 registers, no spills); the refined FP32
-// rows need 28 B each, so the FP32 z and y sweeps and the modal solves run best
-// at 3 blocks of 256 threads and the FP32 x sweeps at 6 blocks of 128.
+// to the matching shared-memory share).  Measured on B200 at 256^3: the FP64 x
+// and y sweeps run fastest at 4 blocks (64 registers, no spills); the refined FP32
+// rows need 28 B each, so the FP32 y sweeps and the modal solves run best at 3
+// blocks of 256 threads and the FP32 x sweeps at 6 blocks of 128.
 template <class R>
 struct LineOcc {
     static constexpr bool f32 = std::is_same<R, float>::value;
-    static constexpr int z = f32 ? 3 : 2;
     static constexpr int x = f32 ? 6 : 4;
     static constexpr int y = f32 ? 3 : 4;
     static constexpr int modal = 3;
     // rows per lane solved in registers (0: in shared memory), per family:
     // wherever the registers allow it without spills (not the FP64 x/y sweeps
     // at 64 registers, nor the two-right-hand-side modal solves at 80)
-    static constexpr int reg_z = 8;
     static constexpr int reg_x = f32 ? 8 : 0;
     static constexpr int reg_y = f32 ? 8 : 0;
     static constexpr int reg_modal = 0;
     // threads per block, per family (the FP32 x sweeps run best as 128-thread
     // blocks of 4 lines: the refined rows fill shared memory, and smaller
     // blocks wait less at their barriers)
-    static constexpr int nt_z = 256, nt_x = f32 ? 128 : 256, nt_y = 256, nt_modal = 256;
-    // the FP64 z sweeps build row-adjacent cells in pairs (PairRows)
-    static constexpr bool pair_z = !f32;
+    static constexpr int nt_x = f32 ? 128 : 256, nt_y = 256, nt_modal = 256;
     // the x sweeps' wide shape, for lines too long to fit 4 per 128-thread block
     static constexpr int xw = f32 ? 3 : 4, nt_xw = 256, reg_xw = reg_x;
 };
@@ -757,16 +752,10 @@ struct FastRcp { static constexpr bool on = false; };
 template <class P>
 struct FastRcp<P, std::void_t<decltype(P::FAST_RCP)>> { static constexpr bool on = P::FAST_RCP; };
 
-// Problems whose build takes row-adjacent cells in pairs (Prob::PAIR).
-template <class P, class = void>
-struct PairRows { static constexpr bool on = false; };
-template <class P>
-struct PairRows<P, std::void_t<decltype(P::PAIR)>> { static constexpr bool on = P::PAIR; };
-
-// Unpaired strided builds that keep one line per thread and step its rows by
+// Strided builds that keep one line per thread and step its rows by
 // NT / TL (Prob::LINE_PER_THREAD; default: FP32 rows).  Measured at 256^3: the
 // FP32 sweeps and the modal solves faster (modal -3% in FP64, -10% in FP32;
-// FP32 thermal_y -4%), the FP64 y sweeps and the FP32 dw_z slower (+4-8%, +3%).
+// FP32 thermal_y -4%), the FP64 y sweeps slower (+4-8%).
 template <class P, class = void>
 struct LinePerThread { static constexpr bool on = std::is_same<typename P::Real, float>::value; };
 template <class P>
@@ -828,26 +817,8 @@ __device__ __forceinline__ void line_block(const Prob &prob, const LinePlan &lp)
         for (; l < TL; l++)
             for (int r = threadIdx.x; r < n; r += blockDim.x) put(l, r);
     } else {
-        if constexpr (PairRows<Prob>::on) {
-            // two row-adjacent cells per thread: their loads are in flight together and
-            // the loads their stencils share are issued once (measured on the FP64 z
-            // sweeps: dw_z -8%, thermal_z -3%; slower on the y sweeps and in FP32).
-            // Pair t = threadIdx.x + m NT of the block's TL x nh pairs is (line t mod TL,
-            // pair t / TL); NT is a multiple of TL, so a thread keeps one line and steps
-            // its pairs by NT / TL: the same cells in the same order, with less index
-            // arithmetic per cell (dw_z -2%, dv_z -1%).
-            const int nh = (n + 1) >> 1, l = threadIdx.x & (TL - 1), hstep = Prob::NT >> lgTL;
-            for (int h = threadIdx.x >> lgTL; h < nh; h += hstep) {
-                const int r = h << 1;
-                if (r + 1 < n) {   // both cells in one block, so their loads can be merged and interleaved
-                    put(l, r);
-                    put(l, r + 1);
-                } else {
-                    put(l, r);
-                }
-            }
-        } else if constexpr (LinePerThread<Prob>::on) {
-            // the same cells and order as below, one line per thread
+        if constexpr (LinePerThread<Prob>::on) {
+            // one line per thread
             const int l = threadIdx.x & (TL - 1), rstep = Prob::NT >> lgTL;
 #pragma unroll 2
             for (int r = threadIdx.x >> lgTL; r < n; r += rstep) put(l, r);
@@ -901,7 +872,7 @@ __device__ __forceinline__ void line_block(const Prob &prob, const LinePlan &lp)
     if (Prob::CONTIG) {
         for (int l = 0; l < TL; l++)
             for (int r = threadIdx.x; r < n; r += blockDim.x) out(l, r);
-    } else if constexpr (PairRows<Prob>::on || LinePerThread<Prob>::on) {
+    } else if constexpr (LinePerThread<Prob>::on) {
         // one line per thread, as in the build
         const int l = threadIdx.x & (TL - 1);
         for (int r = threadIdx.x >> lgTL; r < n; r += Prob::NT >> lgTL) out(l, r);

@@ -36,6 +36,9 @@ struct FieldsT {
     // (3-8e-6 with the FP64 table).
     R *Mu2, *iR2;
     double *iR2d;
+    // the same properties with their face averages, four words per (j,k) entry
+    // (momentum_coeffi): Mu, Mu_y, Mu_z, Mu_yz and invRho, invRho_y, invRho_z, 0
+    R *MuT, *iRT;
     // Poisson spectral work array: (h1p, N2, N3) complex, kx fastest
     cplx_t<R> *S;
     // modified wavenumbers and y coefficients of the modal solves (FP64 in both forms)
@@ -55,6 +58,10 @@ __device__ __forceinline__ bool blown(const GridT<R> &g) { return g.scal[S_BLOWU
 
 // The FP32 form keeps low words of the velocity.
 template <class R> struct HasLo { static constexpr bool on = std::is_same<R, float>::value; };
+
+// Two adjacent words of a table (16-byte aligned in FP64, 8-byte in FP32).
+__device__ __forceinline__ double2 ld2(const double *p) { return __ldg(reinterpret_cast<const double2 *>(p)); }
+__device__ __forceinline__ float2 ld2(const float *p) { return __ldg(reinterpret_cast<const float2 *>(p)); }
 
 // v = hi + lo in FP64, and its split back into an FP32 pair.
 __device__ __forceinline__ double join(float hi, float lo) { return (double)hi + (double)lo; }

@@ -2,7 +2,7 @@
 // the launch helpers shared by the stage files.
 #pragma once
 
-#include "tcs_fields.cuh"
+#include "tcs_march.cuh"
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -77,11 +77,11 @@ struct Shapes {
     int fft_lines_x, fft_lines_z;
     int ifft_lines_x;                            // lines per block of the inverse x transform
     int lanes;                                   // at most this many partitions (lanes) per line
-    int long_lines;                              // one-block-per-SM form of long lines: 1 never, 2 z sweeps, 4 z and y sweeps
+    int long_lines;                              // one-block-per-SM form of long y lines: 4; 1, 2 never
     int y_solver;                                // y lines: 1 partitioned (line_block), 2 one line per thread for the y sweeps, 4 also the modal solves
     double *thomas_scr;                          // c', d' of the one-line-per-thread solver (null unless y_solver asks for it)
-    int mixed_rows;                              // FP32-mixed form: 1 FP32 elimination + refinement, 2 FP64 rows in the x sweeps, 4 x and z sweeps, 8 z at 3 blocks/SM
-    int z_staging;                               // FP64 dw_z: 1 loads from global memory, 2 inputs staged by TMA
+    int mixed_rows;                              // FP32-mixed form: 1 FP32 elimination + refinement in the x sweeps, 2, 4, 8 FP64 rows there
+    int z_staging;                               // 1 or 2 (FP64, N3 a multiple of 64, even N1): accepted, no effect
     FFTPlan fp1, fp3;
     FFTPlan fp1u;                                // N1 with radices up to 8 (the inverse x transform's one-radix form)
     int h1p;
@@ -110,23 +110,18 @@ inline size_t line_smem(const LinePlan &lp)
 }
 
 // The plan of a line problem: make_line_plan's partitions, and for the
-// unpaired, non-cyclic strided problems (the y sweeps and the modal solves) a
+// non-cyclic strided problems (the y sweeps and the modal solves) a
 // line stride LS chosen for the build and the emission, where one warp
 // touches TL lines x 32/TL rows: LS = banks/TL (mod banks), banks = 32
 // four-byte words (FP32 rows) or 16 eight-byte words per half-warp (FP64
 // rows), puts those accesses on distinct banks.  The solve (one line per
 // warp) only uses the odd partition stride PS.  Measured at 256^3: the y
-// sweeps 2-5% and the modal solves 3-4% faster in both forms.  The unpaired
-// cyclic (FP32 z) sweeps keep the odd LS: the longer stride takes three of
-// their blocks past the 196 KB shared-memory configuration into the 228 KB
-// one, whose 28 KB of L1 (against 60 KB) cost their stencil loads 11-43%.
-// The paired builds step rows by 2, where no LS avoids 2-way conflicts; they
-// keep the odd LS too.
+// sweeps 2-5% and the modal solves 3-4% faster in both forms.
 template <class Prob>
 inline LinePlan plan_for(int n, bool cyclic, int tl, int pmax)
 {
     LinePlan lp = make_line_plan(n, cyclic, tl, pmax);
-    if (!Prob::CONTIG && !PairRows<Prob>::on && !cyclic && tl > 1) {
+    if (!Prob::CONTIG && !cyclic && tl > 1) {
         const int banks = sizeof(typename Prob::Real) == 4 ? 32 : 16;
         const int want = tl < banks ? banks / tl : 1;
         const int ls = lp.P * lp.PS;
@@ -194,12 +189,7 @@ inline int smem_config_kib(size_t per_sm_bytes)
 
 // A line family in one block per SM: the same warps per SM (NT x MINB threads
 // in one block, so the same registers per thread) with its lines per block
-// fitted to 132 KiB of shared memory, which leaves the SM 124 KiB of L1.  The
-// z-sweep builds read every input through L1 about three times (their x and z
-// neighbours come from other threads' cells): measured on B200, forcing their
-// 256^3 blocks into the 228 KiB configuration (28 KiB of L1) made them 1.8x
-// slower, and 512-row lines put them there by themselves (two blocks of 8
-// lines x 512 rows need 213 KiB).
+// fitted to 132 KiB of shared memory, which leaves the SM 124 KiB of L1.
 template <class P>
 struct LongLines : P {
     static constexpr int NT = P::NT * P::MINB;
@@ -207,8 +197,7 @@ struct LongLines : P {
     static constexpr int SMEM_KIB = 132;
 };
 
-// A strided line sweep (z or y lines: TL consecutive i per block, gy block
-// rows).  With allow_long, the one-block-per-SM form runs instead where the
+// A strided line sweep (y lines: TL consecutive i per block, gy block rows).  With allow_long, the one-block-per-SM form runs instead where the
 // usual form would leave less than 60 KiB of L1 or would have to halve its
 // lines per block.  make(tl) builds the problem for tl lines per block.
 template <class P, class Make>
@@ -229,21 +218,17 @@ inline void launch_strided(const Shapes &cx, int n, bool cyclic, int nlines, int
     launch_lines(make(a.TL), a, dim3((nlines + a.TL - 1) / a.TL, gy), s, kid, cx);
 }
 
-// An FP32 line problem whose rows are eliminated in FP64 (Shapes::mixed_rows):
-// the problem's own build in the field type, its coefficients widened to FP64
-// in shared memory, the partitioned solve in FP64 without the refinement pass
+// An FP32 x sweep whose rows are eliminated in FP64 (Shapes::mixed_rows): the
+// problem's own build in the field type, its coefficients widened to FP64 in
+// shared memory, the partitioned solve in FP64 without the refinement pass
 // (Refine<double> is off), and the solution rounded once to the field type when
-// the problem emits it.  Launch shape of the FP64 family of the same axis
-// (AX: 0 the z sweeps, 1 the x sweeps), or for the z sweeps with Z3 three
-// blocks per SM and the shared-memory elimination (their FP32 builds need
-// fewer registers than FP64 ones: measured at 256^3 9% faster than the FP64
-// shape, at 512^3 3% slower).
-template <class P, int AX, int Z3 = 0>
+// the problem emits it.  Launch shape of the FP64 x sweeps.
+template <class P>
 struct FP64Rows : P {
     using Real = double;
-    static constexpr int MINB = AX ? LineOcc<double>::x : (Z3 ? 3 : LineOcc<double>::z);
-    static constexpr int MREG = AX ? LineOcc<double>::reg_x : (Z3 ? 0 : LineOcc<double>::reg_z);
-    static constexpr int NT = AX ? LineOcc<double>::nt_x : LineOcc<double>::nt_z;
+    static constexpr int MINB = LineOcc<double>::x;
+    static constexpr int MREG = LineOcc<double>::reg_x;
+    static constexpr int NT = LineOcc<double>::nt_x;
     __device__ Coef<double, P::NRHS> build(int l, int r, const typename P::State &st) const
     {
         const auto c = P::build(l, r, st);
@@ -281,25 +266,83 @@ inline void launch_thomas(const Shapes &cx, int n, int nlines, int gy, Make make
     record_launch_error(kernel_name(kid));
 }
 
-// A z sweep (cyclic strided lines, nlines x gy of n rows): in the FP32-mixed
-// form with mixed_rows 4 (8: three blocks per SM) its FP32-built rows are
-// eliminated in FP64.
-template <class P, class Make>
-inline void launch_z(const Shapes &cx, int n, int nlines, int gy, Make make, cudaStream_t s, int kid)
+// The shape of a marching sweep (march_block) of `lines` lines in all: TI lines
+// and NS segments of every line per block.  Rows per segment, m = n / NS: at
+// most 12, because the parked rows (24 B each, 512 threads per SM) then leave L1
+// room for the stencil's x neighbours and tables (measured in FP64, ps per cell
+// of dw_z: m = 16 at 256^3 36, m = 8 24; m = 12 at 192^3 24, m = 6 28), and at least
+// 4, because every segment loads its first plane twice; with few lines, short
+// segments fill the SMs.  Lines too long for 16 of them at 12 rows a segment keep
+// 512 threads and take more rows.
+inline MarchPlan march_plan(int n, bool cyclic, int nrhs, int lanes, long long lines)
 {
-    if constexpr (std::is_same<typename P::Real, float>::value) {
-        if (cx.mixed_rows >= 8) {
-            using Q = FP64Rows<P, 0, 1>;
-            launch_strided<Q>(cx, n, true, nlines, gy, [&](int tl) { return Q{make(tl)}; }, s, kid, cx.long_lines >= 2);
-            return;
-        }
-        if (cx.mixed_rows >= 4) {
-            using Q = FP64Rows<P, 0>;
-            launch_strided<Q>(cx, n, true, nlines, gy, [&](int tl) { return Q{make(tl)}; }, s, kid, cx.long_lines >= 2);
-            return;
-        }
+    MarchPlan mp;
+    mp.n = n; mp.cyclic = cyclic ? 1 : 0;
+    mp.lgNS = 1;
+    const int cap = lanes < 32 ? lanes : 256;
+    auto more = [&]() { return (2 << mp.lgNS) <= cap && (n >> (mp.lgNS + 1)) >= 4; };
+    while (more() && mp.lgNS < 5 && (n > (12 << mp.lgNS) || (lines << mp.lgNS) < 131072)) mp.lgNS++;
+    mp.lgTI = 4;
+    auto words = [&]() { return march_words(n, 1 << mp.lgNS, 1 << mp.lgTI, nrhs) * sizeof(double); };
+    while (mp.lgTI > 0 && words() > 227 * 1024) {
+        mp.lgTI--;
+        if (more() && mp.lgNS + mp.lgTI < 9) mp.lgNS++;
     }
-    launch_strided<P>(cx, n, true, nlines, gy, make, s, kid, cx.long_lines >= 2);
+    while (words() > 227 * 1024 || mp.lgTI + mp.lgNS < 5) {   // fits, in whole warps
+        if (words() > 227 * 1024) mp.lgTI--;
+        else mp.lgNS++;
+    }
+    mp.m0 = n >> mp.lgNS; mp.rem = n & ((1 << mp.lgNS) - 1);
+    return mp;
+}
+
+template <int NT, class P>
+inline void launch_march_nt(const Shapes &cx, const P &prob, const MarchPlan &mp, int nlines, int gy, cudaStream_t s, int kid)
+{
+    const int TI = 1 << mp.lgTI;
+    const size_t smem = march_words(mp.n, 1 << mp.lgNS, TI, P::NRHS) * sizeof(double);
+    static size_t conf[64] = {};
+    smem_opt_in((const void *)march_kernel<P, NT>, smem, conf);
+    probe_begin(cx, kid, s);
+    march_kernel<P, NT><<<dim3((nlines + TI - 1) / TI, gy), TI << mp.lgNS, smem, s>>>(prob, mp);
+    probe_end(cx, kid, s);
+    record_launch_error(kernel_name(kid));
+}
+
+// The column form of a z sweep (column_kernel), in two segments per line: FP64
+// lines of more than 384 rows, with rows of i that start on 16 bytes.  Measured
+// at 512^3 (ms, thermal_z, du_z, dv_z, dw_z): 3.17, 2.54, 2.81, 3.02 against 4.64,
+// 3.80, 4.85, 5.06 for march_kernel, whose parked rows then fill the shared
+// memory; at 384 rows the two are level, and below it march_kernel leads.
+template <class P>
+inline bool launch_column(const Shapes &cx, const P &prob, int n, int nlines, int gy, cudaStream_t s, int kid)
+{
+    constexpr int lgNS = 1;
+    if (n <= 384 || (prob.g.P1 & 1)) return false;
+    int w = 0, best = 1 << 30;
+    for (int c = 32; c <= (128 >> lgNS); c += 32) {       // the widest of the block widths that waste least
+        const int waste = (nlines + c - 1) / c * c;
+        if (waste <= best) { best = waste; w = c; }
+    }
+    const size_t smem = col_smem<P>(w, 1 << lgNS);
+    static size_t conf[64] = {};
+    smem_opt_in((const void *)column_kernel<P>, smem, conf);
+    probe_begin(cx, kid, s);
+    column_kernel<P><<<dim3((nlines + w - 1) / w, gy), w << lgNS, smem, s>>>(prob, n, w, lgNS, reinterpret_cast<double *>(prob.f.S), 2 * cx.h1p);
+    probe_end(cx, kid, s);
+    record_launch_error(kernel_name(kid));
+    return true;
+}
+
+// A strided line sweep: nlines x gy lines of n rows.
+template <class P>
+inline void launch_march(const Shapes &cx, const P &prob, int n, bool cyclic, int nlines, int gy, cudaStream_t s, int kid)
+{
+    if constexpr (std::is_same<typename P::Real, double>::value)
+        if (cyclic && launch_column(cx, prob, n, nlines, gy, s, kid)) return;
+    const MarchPlan mp = march_plan(n, cyclic, P::NRHS, cx.lanes, (long long)nlines * gy);
+    if (mp.lgTI + mp.lgNS > 8) launch_march_nt<512>(cx, prob, mp, nlines, gy, s, kid);
+    else launch_march_nt<256>(cx, prob, mp, nlines, gy, s, kid);
 }
 
 // A y sweep (non-cyclic strided lines, nlines x gy of n rows): the
@@ -419,6 +462,24 @@ inline void multi_stage(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStre
     }
 }
 
+// A marching sweep for a group of cases: one launch per case, side by side on
+// the aux streams.  (A persistent multi-case form of march_block was a second
+// compilation of the same source, whose multiply-adds the compiler fused
+// differently: the ensemble's results left its members' by one bit.)
+template <class R, class Launch>
+inline void march_stage(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s, Launch launch)
+{
+    if (A.planning || cs.empty()) return;
+    const size_t side = std::min(A.aux.size(), cs.size());
+    if (side) cudaEventRecord(A.fork, s);
+    for (size_t i = 0; i < side; i++) cudaStreamWaitEvent(A.aux[i], A.fork, 0);
+    for (size_t i = 0; i < cs.size(); i++) launch(*cs[i], side ? A.aux[i % side] : s);
+    for (size_t i = 0; i < side; i++) {
+        cudaEventRecord(A.join[i], A.aux[i]);
+        cudaStreamWaitEvent(s, A.join[i], 0);
+    }
+}
+
 // Whether a case runs its x sweeps in the wide shape (the rule of launch_x).
 template <template <class, int, int> class X, class R>
 inline bool x_is_wide(const Ctx<R> &cx)
@@ -448,7 +509,7 @@ inline void launch_x(const Ctx<R> &cx, int nlines, cudaStream_t s, int kid)
     const GridT<R> &g = cx.g;
     if constexpr (LineOcc<R>::f32) {
         if (cx.mixed_rows >= 2) {   // FP32-built rows eliminated in FP64
-            using P = FP64Rows<X<R, 0, 0>, 1>;
+            using P = FP64Rows<X<R, 0, 0>>;
             const LinePlan p = make_line_plan(g.N1, true, fit_tl<P>(g.N1, true, cx.tl_contig, cx.lanes), cx.lanes);
             launch_lines(P{X<R, 0, 0>{g, cx.f, p.TL}}, p, dim3((nlines + p.TL - 1) / p.TL, g.N3), s, kid, cx);
             return;
@@ -473,7 +534,6 @@ template <class R> void launch_momentum_coeffi(const Ctx<R> &cx, cudaStream_t s)
 template <class R> void launch_solve_du(const Ctx<R> &cx, cudaStream_t s);
 template <class R> void launch_solve_dv(const Ctx<R> &cx, cudaStream_t s);
 template <class R> void launch_solve_dw(const Ctx<R> &cx, cudaStream_t s);
-bool dwz_staging_possible(const Ctx<double> &cx);   // the TMA-staged dw_z can run this case
 template <class R> void launch_blockld_v(const Ctx<R> &cx, cudaStream_t s);
 template <class R> void launch_blockld_u(const Ctx<R> &cx, cudaStream_t s);
 template <class R> void launch_pseudo_update(const Ctx<R> &cx, cudaStream_t s);   // standalone (Un = U + dU, ...)

@@ -1,0 +1,409 @@
+// tcs_march.cuh -- the strided line sweeps (lines along z or y, i fastest in
+// memory): a marching, segmented tridiagonal solver.
+//
+// A block owns TI consecutive i (one line each) and cuts every line into NS
+// segments; thread (line l, segment s) marches along its segment row by row.
+// It keeps what the next row's stencil shares with this one in registers (the
+// problem's March object: the values and fluxes of the face between two rows are
+// loaded and computed once), eliminates the row as soon as it is built, and
+// parks the eliminated row in shared memory:
+//
+//     x_r + c_r x_{r+1} + e_r X_{s-1} = d_r
+//
+// where X_{s-1} is the last unknown of the segment before it.  The last rows of
+// the segments form a (cyclic) tridiagonal system in the X_s, closed by the
+// first unknown of each segment as a combination of X_{s-1} and X_s (sd, se, p,
+// accumulated on the way down); it is solved by parallel cyclic reduction
+// across the lanes, one line per group of NS lanes.  Each thread then
+// substitutes back through its rows and emits them.  It is the partitioned
+// solve of pascal_tdma.f90:487-578 with one partition per thread.
+//
+// Elimination, rows and solution are FP64 in both numerical forms; the
+// FP32-mixed form builds its rows in FP32 and rounds the solution once.
+#pragma once
+
+#include "tcs_fields.cuh"
+#include "tcs_tma.cuh"
+
+namespace tcs {
+
+struct MarchPlan {
+    int n;        // rows per line
+    int lgNS;     // log2 of the segments per line
+    int lgTI;     // log2 of the lines per block
+    int m0, rem;  // segment s has m0 + (s < rem) rows
+    int cyclic;
+};
+
+__host__ __device__ __forceinline__ size_t march_words(int n, int NS, int TI, int nrhs)
+{
+    // eliminated rows c, e, d[nrhs] of every line, then the reduced systems (padded lines)
+    return (size_t)n * TI * (2 + nrhs) + (size_t)(4 + 2 * nrhs) * NS * (TI + 1);
+}
+
+// The reduced systems of a block: words e, c, se, p, d[NR], sd[NR] of the last
+// row of segment s of line L at q NS TP + s TP + L of red, NS a power of two, NS
+// lines = the block's threads.  Parallel cyclic reduction, one row per thread:
+// across the lanes of a group of NS (row t mod NS of line t / NS in thread t),
+// or, for more than 32 segments, through shared memory (row t / lines of line
+// t mod lines).  Leaves X in words 0 .. NR-1.  Ends with a barrier; the caller
+// has put one before it.
+template <int NR>
+__device__ void march_reduce_wide(double *red, int lgNS, int TP, bool cyc)
+{
+    const int NS = 1 << lgNS, RS = NS * TP, TI = TP - 1;
+    const int g = threadIdx.x / TI, L = threadIdx.x - g * TI;
+    double *const own = red + g * TP + L;
+    const double *const nxt = red + ((g + 1) & (NS - 1)) * TP + L;
+    const double cp = (cyc || g < NS - 1) ? own[RS] : 0.0;
+    double al = own[0], be = 1.0, ga = 0.0, de[NR];
+#pragma unroll
+    for (int q = 0; q < NR; q++) de[q] = own[(4 + q) * RS];
+    if (cyc || g < NS - 1) {
+        be = 1.0 - cp * nxt[2 * RS];
+        ga = cp * nxt[3 * RS];
+#pragma unroll
+        for (int q = 0; q < NR; q++) de[q] -= cp * nxt[(4 + NR + q) * RS];
+    }
+    for (int h = 1; h < NS; h <<= 1) {
+        __syncthreads();                           // the words of the step before have been read
+        own[0] = al; own[RS] = qrcp(be); own[2 * RS] = ga;
+#pragma unroll
+        for (int q = 0; q < NR; q++) own[(3 + q) * RS] = de[q];
+        __syncthreads();
+        const bool lok = cyc || g >= h, hok = cyc || g + h < NS;
+        const double *const lo = red + ((g - h) & (NS - 1)) * TP + L, *const hi = red + ((g + h) & (NS - 1)) * TP + L;
+        const double k1 = lok ? al * lo[RS] : 0.0, k2 = hok ? ga * hi[RS] : 0.0;
+#pragma unroll
+        for (int q = 0; q < NR; q++) {
+            if (lok) de[q] = fma(-k1, lo[(3 + q) * RS], de[q]);
+            if (hok) de[q] = fma(-k2, hi[(3 + q) * RS], de[q]);
+        }
+        if (lok) be = fma(-k1, lo[2 * RS], be);
+        if (hok) be = fma(-k2, hi[0], be);
+        al = lok ? -k1 * lo[0] : 0.0;
+        ga = hok ? -k2 * hi[2 * RS] : 0.0;
+    }
+    const double den = qrcp(al + be + ga);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NR; q++) own[q * RS] = de[q] * den;
+    __syncthreads();
+}
+
+template <int NR>
+__device__ __forceinline__ void march_reduce(double *red, int lgNS, int TP, bool cyc)
+{
+    if (lgNS > 5) {
+        march_reduce_wide<NR>(red, lgNS, TP, cyc);
+        return;
+    }
+    const int NS = 1 << lgNS, RS = NS * TP;
+    const int g = threadIdx.x & (NS - 1), L = threadIdx.x >> lgNS;
+    const int gn = (g + 1) & (NS - 1);
+    const double *const own = red + g * TP + L, *const nxt = red + gn * TP + L;
+    const double cp = own[RS];
+    double al = own[0], be = 1.0 - cp * nxt[2 * RS], ga = cp * nxt[3 * RS], de[NR];
+#pragma unroll
+    for (int q = 0; q < NR; q++) de[q] = own[(4 + q) * RS] - cp * nxt[(4 + NR + q) * RS];
+    if (!cyc && g == NS - 1) {
+        be = 1.0; ga = 0.0;
+#pragma unroll
+        for (int q = 0; q < NR; q++) de[q] = own[(4 + q) * RS];
+    }
+    for (int h = 1; h < NS; h <<= 1) {
+        const int lo = (g - h) & (NS - 1), hi = (g + h) & (NS - 1);
+        const bool lok = cyc || g >= h, hok = cyc || g + h < NS;
+        const double rb = qrcp(be);
+        const double alm = __shfl_sync(0xffffffffu, al, lo, NS), gam = __shfl_sync(0xffffffffu, ga, lo, NS);
+        const double alp = __shfl_sync(0xffffffffu, al, hi, NS), gap = __shfl_sync(0xffffffffu, ga, hi, NS);
+        const double rbm = __shfl_sync(0xffffffffu, rb, lo, NS), rbp = __shfl_sync(0xffffffffu, rb, hi, NS);
+        const double k1 = lok ? al * rbm : 0.0, k2 = hok ? ga * rbp : 0.0;
+#pragma unroll
+        for (int q = 0; q < NR; q++) {
+            const double dm = __shfl_sync(0xffffffffu, de[q], lo, NS), dq = __shfl_sync(0xffffffffu, de[q], hi, NS);
+            if (lok) de[q] = fma(-k1, dm, de[q]);
+            if (hok) de[q] = fma(-k2, dq, de[q]);
+        }
+        if (lok) be = fma(-k1, gam, be);
+        if (hok) be = fma(-k2, alp, be);
+        al = lok ? -k1 * alm : 0.0;
+        ga = hok ? -k2 * gap : 0.0;
+    }
+    const double den = qrcp(al + be + ga);
+    __syncthreads();                               // every lane has read its rows: X takes the place of the first words
+#pragma unroll
+    for (int q = 0; q < NR; q++) red[q * RS + g * TP + L] = de[q] * den;
+    __syncthreads();
+}
+
+// The problem supplies
+//   static constexpr int NRHS;  static constexpr bool AHEAD (load a row ahead)
+//   skip(), lines() (count of lines along i of the block row)
+//   struct March { March(const Prob &, int line, int by, int r0);               // line: clamped to a valid one
+//                  struct In;  void load(const Prob &, int r, In &);             // the inputs of row r, rows in order from r0
+//                  void row(const Prob &, int r, const In &, double &a, double &b, double &c, double d[NRHS]); }
+//   emit(int line, int by, int r, const double x[NRHS])
+template <class Prob>
+__device__ __forceinline__ void march_block(const Prob &prob, const MarchPlan &mp, int bx, int by)
+{
+    constexpr int NR = Prob::NRHS, W = 2 + NR;
+    extern __shared__ __align__(16) double msm[];
+    if (prob.skip()) return;
+    const int TI = 1 << mp.lgTI, NS = 1 << mp.lgNS, TP = TI + 1;
+    const int l = threadIdx.x & (TI - 1), s = threadIdx.x >> mp.lgTI;
+    const int line = (bx << mp.lgTI) + l, nl = prob.lines();
+    const int m = mp.m0 + (s < mp.rem ? 1 : 0), r0 = s * mp.m0 + min(s, mp.rem);
+    double *const row0 = msm + (size_t)r0 * W * TI + l;
+    double *const red = msm + (size_t)mp.n * W * TI;   // e, c, d[NR], se, p, sd[NR] of the last rows: word q of (s, l) at q NS TP + s TP + l
+    const int RS = NS * TP;
+    {
+        typename Prob::March st(prob, min(line, nl - 1), by, r0);
+        double cp = 0.0, e = -1.0, p = 1.0, se = 0.0, dp[NR], sd[NR];
+#pragma unroll
+        for (int q = 0; q < NR; q++) { dp[q] = 0.0; sd[q] = 0.0; }
+        double *w = row0;
+        auto eliminate = [&](int r, const typename Prob::March::In &in) {
+            double a, b, c, d[NR];
+            st.row(prob, r, in, a, b, c, d);
+            const double rr = qrcp(fma(-a, cp, b));
+            e = -(a * rr) * e;
+#pragma unroll
+            for (int q = 0; q < NR; q++) dp[q] = fma(-a, dp[q], d[q]) * rr;
+            cp = c * rr;
+            if (!mp.cyclic) {                          // no unknown before the first row, none after the last
+                if (r == 0) e = 0.0;
+                if (r == mp.n - 1) cp = 0.0;
+            }
+        };
+        auto park = [&]() {
+            w[0] = cp; w[TI] = e;
+#pragma unroll
+            for (int q = 0; q < NR; q++) { w[(2 + q) * TI] = dp[q]; sd[q] = fma(p, dp[q], sd[q]); }
+            se = fma(p, e, se);
+            p = -p * cp;
+            w += W * TI;
+        };
+        const int last = r0 + m - 1;
+        int r = r0;
+        typename Prob::March::In in0;
+        st.load(prob, r, in0);
+        if constexpr (Prob::AHEAD) {                   // the next row's inputs are on their way while this one is worked on
+            typename Prob::March::In in1;
+            for (; r + 1 < last; r += 2) {
+                st.load(prob, r + 1, in1);
+                eliminate(r, in0);
+                park();
+                st.load(prob, r + 2, in0);
+                eliminate(r + 1, in1);
+                park();
+            }
+            if (r < last) {
+                st.load(prob, r + 1, in1);
+                eliminate(r, in0);
+                park();
+                in0 = in1;
+            }
+        } else {
+            while (r < last) {
+                eliminate(r, in0);
+                park();
+                st.load(prob, ++r, in0);
+            }
+        }
+        eliminate(last, in0);
+        double *const o = red + s * TP + l;
+        o[0] = e; o[RS] = cp; o[2 * RS] = se; o[3 * RS] = p;
+#pragma unroll
+        for (int q = 0; q < NR; q++) { o[(4 + q) * RS] = dp[q]; o[(4 + NR + q) * RS] = sd[q]; }
+    }
+    __syncthreads();
+    march_reduce<NR>(red, mp.lgNS, TP, mp.cyclic != 0);
+    if (line < nl) {
+        double x[NR], xp[NR];
+        const int sp = (s - 1) & (NS - 1);
+#pragma unroll
+        for (int q = 0; q < NR; q++) { x[q] = red[q * RS + s * TP + l]; xp[q] = red[q * RS + sp * TP + l]; }
+        prob.emit(line, by, r0 + m - 1, x);
+        const double *w = row0 + (m - 2) * W * TI;
+        for (int r = r0 + m - 2; r >= r0; r--, w -= W * TI) {
+            const double c = w[0], e = w[TI];
+#pragma unroll
+            for (int q = 0; q < NR; q++) x[q] = fma(-c, x[q], fma(-e, xp[q], w[(2 + q) * TI]));
+            prob.emit(line, by, r, x);
+        }
+    }
+}
+
+// NT: the most threads per block; 512 threads per SM (128 registers).
+template <class Prob, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) march_kernel(const __grid_constant__ Prob prob, MarchPlan mp)
+{
+    march_block(prob, mp, blockIdx.x, blockIdx.y);
+}
+
+// ---------------------------------------------------------------------------
+// The column form (FP64, z lines): a block of w consecutive i marches up NS
+// segments of the lines together (w NS threads; NS = 1 where there are lines
+// enough).  The rows of i that a plane needs (the problem's stream: its arrays
+// at j-1, j, j+1) come one bulk copy each into a ring of COL_SLOTS planes, up
+// to three planes ahead of the one being worked on, so no load latency is left
+// on the march; c and d of the eliminated rows go to global scratch
+// (consecutive i: coalesced) and the second march substitutes back.  The
+// segment's coupling e_r to the unknown before it is not stored: it dies out
+// within a few rows of a diagonally dominant line, so the rows up to the last
+// one with |e_r| above COL_TINY are built once more (their coefficients alone)
+// and d_r -= e_r X is applied to them.
+// ---------------------------------------------------------------------------
+constexpr int COL_SLOTS = 4;
+constexpr double COL_TINY = 7.8886090522101181e-31;   // 2^-100
+constexpr int COL_WAIT = 1 << 22;                     // polls of a bounded wait
+
+// Words of one segment's plane: NROW rows of w + 2, then the table words of rows
+// j-1, j, j+1 (Mu) and j (iR).
+template <class Prob>
+__host__ __device__ constexpr int col_slot_words(int w) { return Prob::NROW * (w + 2) + 16; }
+template <class Prob>
+__host__ __device__ constexpr size_t col_smem(int w, int NS) { return ((size_t)COL_SLOTS * NS * col_slot_words<Prob>(w) + COL_SLOTS) * sizeof(double); }
+
+template <class Prob>
+__global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ Prob prob, int n, int w, int lgNS, double *cscr, int cpitch)
+{
+    using March = typename Prob::March;
+    extern __shared__ __align__(16) double csm[];
+    if (prob.skip()) return;
+    const GridT<double> &g = prob.g;
+    const int NS = 1 << lgNS, s = threadIdx.x / w, l = threadIdx.x - s * w, by = blockIdx.y, x0 = w * blockIdx.x;
+    const int SW = col_slot_words<Prob>(w) * NS;                     // words of a ring slot
+    uint64_t *const bar = reinterpret_cast<uint64_t *>(csm + COL_SLOTS * SW);
+    double *const mine = csm + s * col_slot_words<Prob>(w);
+    const int nl = prob.lines(), line = x0 + l, sline = min(line, nl - 1);
+    const int i = 1 + sline, j = Prob::J0 + by;
+    const int m0 = n >> lgNS, rem = n & (NS - 1), m = m0 + (s < rem), r0 = s * m0 + min(s, rem), mmax = m0 + (rem > 0);
+    const long long sk = (long long)g.P1 * g.P2;
+    const uint32_t rowb = (uint32_t)min(w + 2, g.P1 - x0) * 8u;
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < COL_SLOTS; q++) mbar_init(&bar[q], NS);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    // one thread of each segment: plane k of the segment's row r (k = r0 + r + 1) into
+    // slot (r + 1) mod COL_SLOTS (r = -1: what the first row needs of the plane below)
+    auto issue = [&](int r) {
+        const int sl = (r + 1) % COL_SLOTS, k = r0 + r + 1;
+        if (r >= m) {                                                // a shorter segment has no such row
+            mbar_arrive_expect_tx(&bar[sl], 0);
+            return;
+        }
+        double *const dst = mine + sl * SW;
+        mbar_arrive_expect_tx(&bar[sl], Prob::NROW * rowb + (Prob::TABLES ? 128u : 0u));
+#pragma unroll
+        for (int q = 0; q < Prob::NROW; q++) {
+            const int jq = j + Prob::row_dj(q), kq = k + Prob::row_dk(q);
+            bulk_load(dst + q * (w + 2), prob.row_src(q) + (x0 + (long long)g.P1 * (jq + (long long)g.P2 * kq)), rowb, &bar[sl]);
+        }
+        if (Prob::TABLES) {
+            double *const t = dst + Prob::NROW * (w + 2);
+            bulk_load(t, prob.f.MuT + 4 * (j - 1 + g.P2 * (k + 1)), 96, &bar[sl]);
+            bulk_load(t + 12, prob.f.iRT + 4 * (j + g.P2 * (k + 1)), 32, &bar[sl]);
+        }
+    };
+    if (l == 0)
+        for (int r = -1; r < COL_SLOTS - 1 && r < mmax; r++) issue(r);
+    const long long ck = (long long)cpitch * g.N2;
+    double *const sc = cscr + (i - 1) + (long long)cpitch * (j - 1) + r0 * ck;
+    double *const sd_ = prob.f.scr + ix(g, i, j, 1 + r0);
+    double cp = 0.0, dp = 0.0, e = -1.0, p = 1.0, se = 0.0, sd = 0.0;
+    int K = -1;
+    {
+        March st(prob, sline, by, r0);
+        double a, b, c, d;
+        int r = 0;
+        bool ok = true, got = mbar_wait(&bar[0], 0, COL_WAIT);
+        for (; r < mmax; r++) {
+            got = mbar_wait(&bar[(r + 1) % COL_SLOTS], ((r + 1) / COL_SLOTS) & 1, COL_WAIT) && got;
+            if (got && r < m) {
+                typename March::In in;
+                st.fill(prob, r0 + r, in, mine + ((r + 1) % COL_SLOTS) * SW, mine + (r % COL_SLOTS) * SW, w, sline - x0);
+                st.row(prob, r0 + r, in, a, b, c, &d);
+                const double rr = qrcp(fma(-a, cp, b));
+                e = -(a * rr) * e;
+                dp = fma(-a, dp, d) * rr;
+                cp = c * rr;
+                if (r < m - 1) {
+                    if (line < nl) {
+                        sc[r * ck] = cp;
+                        sd_[r * sk] = dp;
+                    }
+                    sd = fma(p, dp, sd);
+                    se = fma(p, e, se);
+                    p = -p * cp;
+                    if (!(fabs(e) <= COL_TINY)) K = r;
+                }
+            }
+            if (__syncthreads_or(!got)) { ok = false; break; }     // every thread is done with the slot below
+            if (l == 0 && r + COL_SLOTS - 1 < mmax) {
+                fence_proxy_async();
+                issue(r + COL_SLOTS - 1);
+            }
+        }
+        if (!ok) {
+            // a copy did not arrive in time: record it, stop the step, and wait
+            // (bounded) for this block's copies still in flight before leaving
+            if (threadIdx.x == 0) {
+                atomicAdd(g.scal + S_TIMEOUT, 1.0);
+                g.scal[S_BLOWUP] = 1.0;
+                for (int q = r + 1; q < r + COL_SLOTS && q <= mmax; q++) mbar_wait(&bar[q % COL_SLOTS], (q / COL_SLOTS) & 1, COL_WAIT);
+            }
+            __syncthreads();
+            return;
+        }
+    }
+    double X, Xp;
+    if (NS == 1) {
+        X = Xp = (dp - cp * sd) * qrcp((1.0 - cp * se) + (e + cp * p));
+    } else {
+        // the ring is idle now: it holds the reduced systems
+        const int TP = w + 1, RS = NS * TP;
+        double *const o = csm + s * TP + l;
+        o[0] = e; o[RS] = cp; o[2 * RS] = se; o[3 * RS] = p; o[4 * RS] = dp; o[5 * RS] = sd;
+        __syncthreads();
+        march_reduce<1>(csm, lgNS, TP, true);
+        X = o[0];
+        Xp = csm[((s - 1) & (NS - 1)) * TP + l];
+    }
+    K = __reduce_max_sync(0xffffffffu, K);
+    {
+        March st(prob, sline, by, r0);
+        double c2 = 0.0, e2 = -1.0, a, b, c, d;
+        for (int r = 0; r <= K; r++) {
+            typename March::In in;
+            st.load(prob, r0 + r, in);
+            st.row(prob, r0 + r, in, a, b, c, &d);
+            const double rr = qrcp(fma(-a, c2, b));
+            e2 = -(a * rr) * e2;
+            c2 = c * rr;
+            if (line < nl) sd_[r * sk] = fma(-e2, Xp, sd_[r * sk]);
+        }
+    }
+    if (line >= nl) return;
+    double x = X;
+    sd_[(m - 1) * sk] = x;
+    int r = m - 2;
+    for (; r >= 7; r -= 8) {
+        double cc[8], dd[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) { cc[q] = sc[(r - q) * ck]; dd[q] = sd_[(r - q) * sk]; }
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            x = fma(-cc[q], x, dd[q]);
+            sd_[(r - q) * sk] = x;
+        }
+    }
+    for (; r >= 0; r--) {
+        x = fma(-sc[r * ck], x, sd_[r * sk]);
+        sd_[r * sk] = x;
+    }
+}
+
+} // namespace tcs

@@ -9,7 +9,6 @@
 // reference assigns whole rows Mu(:,j,k) inside its i loop (:156-171), so every
 // value along i equals the one computed from T(n1sub,j,k).
 #include "tcs_kernels.h"
-#include "tcs_tma.cuh"
 
 namespace tcs {
 
@@ -27,13 +26,37 @@ __global__ void momentum_coeffi_kernel(GridT<R> g, FieldsT<R> f)
     const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (j > g.N2 + 1 || blown(g)) return;
     const Phys &p = g.phd;
-    const double t1 = p.DeltaT * (double)f.T[ix(g, g.N1 + 1, j, k)];
-    const double t2 = t1 * t1, t3 = t2 * t1, t4 = t3 * t1, t5 = t4 * t1;
-    const double ra = (p.a10 + p.a10 * (p.a11 * t1 + p.a12 * t2 + p.a13 * t3 + p.a14 * t4 + p.a15 * t5));
-    const double ir = p.Rho0 / ra;
-    f.Mu2[ix2(g, j, k)] = (R)(ra * (p.d10 + p.d10 * (p.d11 * t1 + p.d12 * t2 + p.d13 * t3 + p.d14 * t4 + p.d15 * t5)) / p.Mu0);
-    f.iR2[ix2(g, j, k)] = (R)ir;
-    if constexpr (HasLo<R>::on) f.iR2d[ix2(g, j, k)] = ir;
+    auto props = [&](int jj, int kk, double &mu, double &ir) {
+        const double t1 = p.DeltaT * (double)f.T[ix(g, g.N1 + 1, jj, kk)];
+        const double t2 = t1 * t1, t3 = t2 * t1, t4 = t3 * t1, t5 = t4 * t1;
+        const double ra = (p.a10 + p.a10 * (p.a11 * t1 + p.a12 * t2 + p.a13 * t3 + p.a14 * t4 + p.a15 * t5));
+        ir = p.Rho0 / ra;
+        mu = ra * (p.d10 + p.d10 * (p.d11 * t1 + p.d12 * t2 + p.d13 * t3 + p.d14 * t4 + p.d15 * t5)) / p.Mu0;
+    };
+    double mu, ir;
+    props(j, k, mu, ir);
+    const int c = ix2(g, j, k);
+    f.Mu2[c] = (R)mu;
+    f.iR2[c] = (R)ir;
+    if constexpr (HasLo<R>::on) f.iR2d[c] = ir;
+    // the averages at the faces between row j-1 and j (y), plane k-1 and k (z)
+    // and at the edge between them (yz), which the sweeps read instead of
+    // forming them again at every i: Mu, Mu_y, Mu_z, Mu_yz and iR, iR_y, iR_z
+    double mj, rj, mk, rk, mjk, rjk;
+    props(max(j - 1, 0), k, mj, rj);
+    props(j, max(k - 1, 0), mk, rk);
+    props(max(j - 1, 0), max(k - 1, 0), mjk, rjk);
+    const double y0 = j ? 0.5 * g.d2.dx[j - 1] * g.d2.rdmx[j] : 0.0, y1 = j ? 0.5 * g.d2.dx[j] * g.d2.rdmx[j] : 0.0;
+    const double z0 = k ? 0.5 * g.d3.dx[k - 1] * g.d3.rdmx[k] : 0.0, z1 = k ? 0.5 * g.d3.dx[k] * g.d3.rdmx[k] : 0.0;
+    R *const mt = f.MuT + 4 * c, *const rt = f.iRT + 4 * c;
+    mt[0] = (R)mu;
+    mt[1] = (R)(y0 * mu + y1 * mj);
+    mt[2] = (R)(z0 * mu + z1 * mk);
+    mt[3] = (R)(z0 * (y0 * mu + y1 * mj) + z1 * (y0 * mk + y1 * mjk));
+    rt[0] = (R)ir;
+    rt[1] = (R)(y0 * ir + y1 * rj);
+    rt[2] = (R)(z0 * ir + z1 * rk);
+    rt[3] = R(0);
 }
 
 template <class R>
@@ -49,96 +72,135 @@ void launch_momentum_coeffi(const Ctx<R> &cx, cudaStream_t s)
 // ---------------------------------------------------------------------------
 // solvedU (:225-563)
 // ---------------------------------------------------------------------------
-template <class R, int ITEM = 0>
+template <class R>
 struct DUZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr int MINB = LineOcc<R>::z;
-    static constexpr int MREG = LineOcc<Real>::reg_z;
-    static constexpr int NT = LineOcc<Real>::nt_z;
-    static constexpr bool CONTIG = false;
-    static constexpr bool PAIR = LineOcc<Real>::pair_z;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr bool AHEAD = std::is_same<R, float>::value;   // FP64 inputs of two rows do not fit the registers
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt; };
-    __device__ State prepare() const { return State{R(g.scal[S_DT])}; }
-    __device__ int li(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return li(l) <= g.N1; }
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
+    __device__ int lines() const { return g.N1; }
+    // the rows of i that a plane needs in the column form
+    static constexpr int NROW = 8, J0 = 1;
+    static constexpr bool TABLES = true;
+    __device__ static constexpr int row_dj(int q) { constexpr int v[] = {0, -1, 1, 0, 1, 0, 0, 0}; return v[q]; }
+    __device__ static constexpr int row_dk(int q) { constexpr int v[] = {1, 0, 0, 0, 0, 1, 0, 0}; return v[q]; }
+    __device__ __forceinline__ const R *row_src(int q) const
     {
-        const int i = li(l), j = 1 + vby<ITEM>(), k = r + 1;
-        const int im = i - 1, jm = j - 1, jp = j + 1, km = k - 1, kp = k + 1;
-        const PhysT<R> &p = g.ph;
-        const R *dx1 = g.m1.dx, *dx2 = g.m2.dx, *dx3 = g.m3.dx;
-        const R *rdx1 = g.m1.rdx, *rdx2 = g.m2.rdx, *rdx3 = g.m3.rdx;
-        const R *rdmx1 = g.m1.rdmx, *rdmx2 = g.m2.rdmx, *rdmx3 = g.m3.rdmx;
-        const long long c = ix(g, i, j, k), sj = g.P1, sk = (long long)g.P1 * g.P2;
-        const R *U = f.U, *V = f.V, *W = f.W;
-        const R jum = (j == 1) ? R(0.0) : R(1.0), jup = (j == g.N2) ? R(0.0) : R(1.0);
-        const R Uc = ld(U + c), Uxm = ld(U + c - 1), Uxp = ld(U + c + 1), Uym = ld(U + c - sj), Uyp = ld(U + c + sj);
-        const R Uzm = ld(U + c - sk), Uzp = ld(U + c + sk);
-        const R Vc = ld(V + c), Vxm = ld(V + c - 1), Vyp = ld(V + c + sj), Vxmyp = ld(V + c - 1 + sj);
-        const R Wc = ld(W + c), Wxm = ld(W + c - 1), Wzp = ld(W + c + sk), Wxmzp = ld(W + c - 1 + sk);
-        const R Mjk = MU(j, k), Mjmk = MU(jm, k), Mjpk = MU(jp, k), Mjkm = MU(j, km), Mjkp = MU(j, kp);
-        const R iRjk = IR(j, k);
-        const R u1 = R(0.5) * (Uxm + Uc), u2 = R(0.5) * (Uxp + Uc);
-        const R v3 = R(0.5) * (dx1[im] * Vc + dx1[i] * Vxm) * rdmx1[i];
-        const R v4 = R(0.5) * (dx1[im] * Vyp + dx1[i] * Vxmyp) * rdmx1[i];
-        const R w5 = R(0.5) * (dx1[im] * Wc + dx1[i] * Wxm) * rdmx1[i];
-        const R w6 = R(0.5) * (dx1[im] * Wzp + dx1[i] * Wxmzp) * rdmx1[i];
-        const R dudx1 = (Uc - Uxm) * rdx1[im], dudx2 = (Uxp - Uc) * rdx1[i];
-        const R dudy3 = (Uc - Uym) * rdmx2[j], dudy4 = (Uyp - Uc) * rdmx2[jp];
-        const R dudz5 = (Uc - Uzm) * rdmx3[k], dudz6 = (Uzp - Uc) * rdmx3[kp];
-        const R dvdx3 = (Vc - Vxm) * rdmx1[i], dvdx4 = (Vyp - Vxmyp) * rdmx1[i];
-        const R dwdx5 = (Wc - Wxm) * rdmx1[i], dwdx6 = (Wzp - Wxmzp) * rdmx1[i];
-        R mua = R(0.5) * (dx1[im] * Mjmk + dx1[i] * Mjmk) * rdmx1[i];
-        const R muc = R(0.5) * (dx1[im] * Mjk + dx1[i] * Mjk) * rdmx1[i];
-        R mub = R(0.5) * (dx1[im] * Mjpk + dx1[i] * Mjpk) * rdmx1[i];
-        const R mu3 = R(0.5) * (dx2[jm] * muc + dx2[j] * mua) * rdmx2[j];
-        const R mu4 = R(0.5) * (dx2[jp] * muc + dx2[j] * mub) * rdmx2[jp];
-        mua = R(0.5) * (dx1[im] * Mjkm + dx1[i] * Mjkm) * rdmx1[i];
-        mub = R(0.5) * (dx1[im] * Mjkp + dx1[i] * Mjkp) * rdmx1[i];
-        const R mu5 = R(0.5) * (dx3[km] * muc + dx3[k] * mua) * rdmx3[k];
-        const R mu6 = R(0.5) * (dx3[kp] * muc + dx3[k] * mub) * rdmx3[kp];
-        const R invRhoc = R(0.5) * (dx1[im] * iRjk + dx1[i] * iRjk) * rdmx1[i];
-        const R ih = R(0.5) * p.Cmu * invRhoc;
-        const R vu1 = (Mjk * dudx2 - Mjk * dudx1) * rdmx1[i];
-        const R vu2 = (mu4 * dudy4 - mu3 * dudy3) * rdx2[j];
-        const R vu3 = (mu6 * dudz6 - mu5 * dudz5) * rdx3[k];
-        const R vu12 = (mu4 * dvdx4 - mu3 * dvdx3) * rdx2[j];
-        const R vu13 = (mu6 * dwdx6 - mu5 * dwdx5) * rdx3[k];
-        // The reduced right-hand side (see the thermal z sweep): the explicit
-        // operator minus the implicit ones applied to U, with the x and z parts
-        // collapsed (their coefficient terms cancel in exact arithmetic) and the
-        // y part in the reference's form on the wall-adjacent planes only.
-        R rhs = R(4.0) * ih * vu1 + R(2.0) * ih * (vu3 + vu13) - R(0.5) * (u1 * dudx1 + u2 * dudx2) - R(0.5) * (w5 * dudz5 + w6 * dudz6);
-        rhs = rhs - p.Cmp * invRhoc * (ld(f.P + c) - ld(f.P + c - 1)) * rdmx1[i];
-        const R Tc = R(0.5) * (dx1[im] * ld(f.T + c) + dx1[i] * ld(f.T + c - 1)) * rdmx1[i];
-        rhs = rhs + p.Cmt * (Tc + p.a12pera11 * (Tc * Tc) * p.DeltaT) * invRhoc;
-        if (j != 1 && j != g.N2) {
-            rhs = rhs + R(2.0) * ih * (vu2 + vu12) - R(0.5) * (v3 * dudy3 + v4 * dudy4);
-        } else {
-            R ubc_dn = R(0.25) * v3 * rdmx2[j] * p.Ubt - R(0.25) * dudy3 * (dx1[i] * p.Vbt + dx1[im] * p.Vbt) * rdmx1[i] * R(0.5);
-            R ubc_up = -R(0.25) * v4 * rdmx2[jp] * p.Uup - R(0.25) * dudy4 * (dx1[i] * p.Vup + dx1[im] * p.Vup) * rdmx1[i] * R(0.5);
-            ubc_dn = ubc_dn + ih * rdx2[j] * mu3 * rdmx2[j] * p.Ubt;
-            ubc_dn = ubc_dn - ih * rdx2[j] * mu3 * rdmx1[i] * (p.Vbt - p.Vbt);
-            ubc_up = ubc_up + ih * rdx2[j] * mu4 * rdmx2[jp] * p.Uup;
-            ubc_up = ubc_up + ih * rdx2[j] * mu4 * rdmx1[i] * (p.Vup - p.Vup);
-            const R mACJ = ih * rdx2[j] * (mu4 * rdmx2[jp] + mu3 * rdmx2[j]) + R(0.25) * (-v4 * rdmx2[jp] + v3 * rdmx2[j]);
-            const R mAPJ = (-ih * rdx2[j] * mu4 * rdmx2[jp] + R(0.25) * (v4 * rdmx2[jp])) * jup;
-            const R mAMJ = (-ih * rdx2[j] * mu3 * rdmx2[j] + R(0.25) * (-v3 * rdmx2[j])) * jum;
-            rhs = rhs + ih * (vu2 + vu12) + (R(1.0) - jum) * ubc_dn + (R(1.0) - jup) * ubc_up - (mAPJ * Uyp + mACJ * Uc + mAMJ * Uym)
-                  - (R(0.25) * (v4 * jup * dudy4 + v3 * jum * dudy3) - ih * rdx2[j] * (mu4 * dvdx4 * jup - mu3 * dvdx3 * jum));
+        switch (q) {
+        case 0: return f.U;
+        case 1: return f.U;
+        case 2: return f.U;
+        case 3: return f.V;
+        case 4: return f.V;
+        case 5: return f.W;
+        case 6: return f.P;
+        default: return f.T;
         }
-        const R mACK = ih * rdx3[k] * (mu6 * rdmx3[kp] + mu5 * rdmx3[k]) + R(0.25) * (-w6 * rdmx3[kp] + w5 * rdmx3[k]);
-        const R mAPK = -ih * rdx3[k] * mu6 * rdmx3[kp] + R(0.25) * (w6 * rdmx3[kp]);
-        const R mAMK = -ih * rdx3[k] * mu5 * rdmx3[k] + R(0.25) * (-w5 * rdmx3[k]);
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = mACK * dt + R(1.0); cf.c = mAPK * dt; cf.a = mAMK * dt; cf.d[0] = rhs * dt;
-        return cf;
     }
-    __device__ void emit(int l, int r, const R *x, const State &st) const { f.scr[ix(g, li(l), 1 + vby<ITEM>(), r + 1)] = x[0]; }
+    // Averages over a face weigh the two cells by w and 1 - w (dmx is the mean
+    // of the two dx on every mesh), and Mu and invRho are constant along i.
+    // The reduced right-hand side: the explicit operator minus the implicit
+    // ones applied to U.  Per direction the coefficient terms of the two
+    // cancel in exact arithmetic; on the wall-adjacent planes (j = 1, N2), where
+    // the jC_BC masks and the wall terms break that, the difference is added.
+    struct March {
+        R cu, rdx1, rdx1m, rdmx1, rdx2, rdmx2, rdmx2p, dt;   // fixed along the line; cu: weight of cell i at x face i (cell i-1: 1 - cu)
+        R Uc, F, G, ma, wa;                                  // the face below the row
+        long long c;
+        int t4, j;
+        __device__ __forceinline__ March(const DUZ &q, int line, int by, int r0)
+        {
+            const GridT<R> &g = q.g;
+            const FieldsT<R> &f = q.f;
+            const int i = 1 + line, im = i - 1, k = r0 + 1;
+            j = 1 + by;
+            rdmx1 = ld(g.m1.rdmx + i); rdx1 = ld(g.m1.rdx + i); rdx1m = ld(g.m1.rdx + im);
+            cu = R(0.5) * ld(g.m1.dx + im) * rdmx1;
+            rdx2 = ld(g.m2.rdx + j); rdmx2 = ld(g.m2.rdmx + j); rdmx2p = ld(g.m2.rdmx + j + 1);
+            dt = R(g.scal[S_DT]);
+            c = ix(g, i, j, k);
+            t4 = 4 * ix2(g, j, k);
+            Uc = ld(f.U + c);
+            face(ld(f.U + c - (long long)g.P1 * g.P2), Uc, ld(f.W + c), ld(f.W + c - 1), ld(f.MuT + t4 + 2), ld(g.m3.rdmx + k));
+        }
+        // the z face between planes k-1 and k: stress, convection and matrix terms
+        __device__ __forceinline__ void face(R Um, R Up, R W0, R Wxm, R mu, R rdmx3)
+        {
+            const R dw = W0 - Wxm, w = Wxm + cu * dw, du = (Up - Um) * rdmx3;
+            F = mu * (du + dw * rdmx1);
+            G = w * du;
+            ma = mu * rdmx3;
+            wa = R(0.25) * w * rdmx3;
+        }
+        struct In { R Uxm, Uxp, Uym, Uyp, Uzp, Vc, Vxm, Vyp, Vxmyp, Wzp, Wxmzp, Pc, Pxm, T0, Txm, muy4, muz6, iR, rdx3, rdmx3; cplx_t<R> mt; };
+        __device__ __forceinline__ void load(const DUZ &q, int r, In &n)
+        {
+            const GridT<R> &g = q.g;
+            const FieldsT<R> &f = q.f;
+            const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
+            n.Uxm = ld(f.U + c - 1); n.Uxp = ld(f.U + c + 1); n.Uym = ld(f.U + c - sj); n.Uyp = ld(f.U + c + sj); n.Uzp = ld(f.U + c + sk);
+            n.Vc = ld(f.V + c); n.Vxm = ld(f.V + c - 1); n.Vyp = ld(f.V + c + sj); n.Vxmyp = ld(f.V + c - 1 + sj);
+            n.Wzp = ld(f.W + c + sk); n.Wxmzp = ld(f.W + c - 1 + sk);
+            n.Pc = ld(f.P + c); n.Pxm = ld(f.P + c - 1); n.T0 = ld(f.T + c); n.Txm = ld(f.T + c - 1);
+            n.mt = ld2(f.MuT + t4);                        // Mu, Mu at the lower y face
+            n.muy4 = ld(f.MuT + t4 + 5); n.muz6 = ld(f.MuT + t4 + 4 * g.P2 + 2); n.iR = ld(f.iRT + t4);
+            n.rdx3 = ld(g.m3.rdx + r + 1); n.rdmx3 = ld(g.m3.rdmx + r + 2);
+            c += sk;
+            t4 += 4 * g.P2;
+        }
+        // the same values from the ring: slot a holds plane k's rows, b the plane below's
+        __device__ __forceinline__ void fill(const DUZ &q, int r, In &n, const double *a, const double *b, int w, int l)
+        {
+            const GridT<R> &g = q.g;
+            const int s = w + 2;
+            a += l + 1; b += l + 1;
+            const double *const ta = a - (l + 1) + NROW * s, *const tb = b - (l + 1) + NROW * s;   // table words of planes k + 1 and k
+            n.Uxm = b[-1]; n.Uxp = b[1]; n.Uzp = a[0]; n.Uym = a[s]; n.Uyp = a[2 * s];
+            n.Vc = a[3 * s]; n.Vxm = a[3 * s - 1]; n.Vyp = a[4 * s]; n.Vxmyp = a[4 * s - 1];
+            n.Wzp = a[5 * s]; n.Wxmzp = a[5 * s - 1];
+            n.Pc = a[6 * s]; n.Pxm = a[6 * s - 1]; n.T0 = a[7 * s]; n.Txm = a[7 * s - 1];
+            n.mt.x = tb[4]; n.mt.y = tb[5]; n.muy4 = tb[9]; n.muz6 = ta[6]; n.iR = tb[12];
+            n.rdx3 = ld(g.m3.rdx + r + 1); n.rdmx3 = ld(g.m3.rdmx + r + 2);
+        }
+        __device__ __forceinline__ void row(const DUZ &q, int r, const In &n, double &a, double &b, double &cc, double *d)
+        {
+            const GridT<R> &g = q.g;
+            const PhysT<R> &p = g.ph;
+            const R Uxm = n.Uxm, Uxp = n.Uxp, Uym = n.Uym, Uyp = n.Uyp, Uzp = n.Uzp, Vc = n.Vc, Vxm = n.Vxm, Vyp = n.Vyp, Vxmyp = n.Vxmyp;
+            const R Wzp = n.Wzp, Wxmzp = n.Wxmzp, Pc = n.Pc, Pxm = n.Pxm, T0 = n.T0, Txm = n.Txm, muy4 = n.muy4, muz6 = n.muz6, iR = n.iR;
+            const cplx_t<R> mt = n.mt;
+            const R rdx3 = n.rdx3;
+            const R ih = R(0.5) * p.Cmu * iR;
+            const R u1 = R(0.5) * (Uxm + Uc), u2 = R(0.5) * (Uxp + Uc);
+            const R dx1 = (Uc - Uxm) * rdx1m, dx2 = (Uxp - Uc) * rdx1;
+            const R dv3 = Vc - Vxm, dv4 = Vyp - Vxmyp;
+            const R v3 = Vxm + cu * dv3, v4 = Vxmyp + cu * dv4;
+            const R dy3 = (Uc - Uym) * rdmx2, dy4 = (Uyp - Uc) * rdmx2p;
+            const R vx3 = dv3 * rdmx1, vx4 = dv4 * rdmx1;
+            const R mu3 = mt.y, mu4 = muy4;
+            const R F5 = F, G5 = G, ma5 = ma, wa5 = wa, U0 = Uc;
+            Uc = Uzp;
+            face(U0, Uzp, Wzp, Wxmzp, muz6, n.rdmx3);
+            const R vs = R(2) * mt.x * ((dx2 - dx1) * rdmx1) + (F - F5) * rdx3 + (mu4 * (dy4 + vx4) - mu3 * (dy3 + vx3)) * rdx2;
+            R rhs = R(2) * ih * vs - R(0.5) * ((u1 * dx1 + u2 * dx2) + (G5 + G) + (v3 * dy3 + v4 * dy4));
+            const R Tc = Txm + cu * (T0 - Txm);
+            rhs = rhs + iR * (p.Cmt * (Tc + p.a12pera11 * (Tc * Tc) * p.DeltaT) - p.Cmp * ((Pc - Pxm) * rdmx1));
+            if (j == 1) {
+                const R am = -(ih * rdx2 * mu3 + R(0.25) * v3) * rdmx2;
+                rhs = rhs + am * (Uym - p.Ubt) + R(0.25) * dy3 * (v3 - p.Vbt) + ih * rdx2 * mu3 * vx3;
+            }
+            if (j == g.N2) {
+                const R ap = (R(0.25) * v4 - ih * rdx2 * mu4) * rdmx2p;
+                rhs = rhs + ap * (Uyp - p.Uup) + R(0.25) * dy4 * (v4 - p.Vup) - ih * rdx2 * mu4 * vx4;
+            }
+            const R h3 = ih * rdx3;
+            const R am = -(h3 * ma5 + wa5) * dt, ap = (wa - h3 * ma) * dt;
+            a = am; cc = ap; b = 1.0 - ((double)am + (double)ap);
+            d[0] = rhs * dt;
+        }
+    };
+    __device__ __forceinline__ void emit(int line, int by, int r, const double *x) const { f.scr[ix(g, 1 + line, 1 + by, r + 1)] = R(x[0]); }
 };
 
 template <class R, int WIDE = 0, int ITEM = 0>
@@ -228,95 +290,136 @@ struct DUY {
 // by the last stage-1 iteration (i=N1, j=N2, k=N3); the y stage scales the
 // upper coefficient by jvp = jS_BC(j-1) and the lower one by jvm = jS_BC(j+1).
 // ---------------------------------------------------------------------------
-template <class R, int ITEM = 0>
+template <class R>
 struct DVZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = std::is_same<R, float>::value;   // measured faster in FP32 only
-    static constexpr int MINB = LineOcc<R>::z;
-    static constexpr int MREG = LineOcc<Real>::reg_z;
-    static constexpr int NT = LineOcc<Real>::nt_z;
-    static constexpr bool CONTIG = false;
-    static constexpr bool PAIR = LineOcc<Real>::pair_z;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr bool AHEAD = std::is_same<R, float>::value;   // FP64 inputs of two rows do not fit the registers
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt; };
-    __device__ State prepare() const { return State{R(g.scal[S_DT])}; }
-    __device__ int li(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return li(l) <= g.N1; }
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
+    __device__ int lines() const { return g.N1; }
+    // the rows of i that a plane needs in the column form
+    static constexpr int NROW = 11, J0 = 2;
+    static constexpr bool TABLES = true;
+    __device__ static constexpr int row_dj(int q) { constexpr int v[] = {0, -1, 1, 0, -1, 0, -1, 0, -1, 0, -1}; return v[q]; }
+    __device__ static constexpr int row_dk(int q) { constexpr int v[] = {1, 0, 0, 0, 0, 0, 0, 1, 1, 0, 0}; return v[q]; }
+    __device__ __forceinline__ const R *row_src(int q) const
     {
-        const int i = li(l), j = 2 + vby<ITEM>(), k = r + 1;
-        const int im = i - 1, ip = i + 1, jm = j - 1, jp = j + 1, km = k - 1, kp = k + 1;
-        const PhysT<R> &p = g.ph;
-        const R *dx1 = g.m1.dx, *dx2 = g.m2.dx, *dx3 = g.m3.dx;
-        const R *rdx1 = g.m1.rdx, *rdx2 = g.m2.rdx, *rdx3 = g.m3.rdx;
-        const R *rdmx1 = g.m1.rdmx, *rdmx2 = g.m2.rdmx, *rdmx3 = g.m3.rdmx;
-        const long long c = ix(g, i, j, k), sj = g.P1, sk = (long long)g.P1 * g.P2;
-        const R *U = f.U, *V = f.V, *W = f.W, *dU = f.dU;
-        const R jvp = (jm >= 2) ? R(1.0) : R(0.0);               // jS_BC(jm)
-        const R jvm = (jp <= g.N2) ? R(1.0) : R(0.0);            // jS_BC(jp)
-        const R Vc = ld(V + c), Vym = ld(V + c - sj), Vyp = ld(V + c + sj), Vxm = ld(V + c - 1), Vxp = ld(V + c + 1);
-        const R Vzm = ld(V + c - sk), Vzp = ld(V + c + sk);
-        const R Uc = ld(U + c), Uym = ld(U + c - sj), Uxp = ld(U + c + 1), Uxpym = ld(U + c + 1 - sj);
-        const R Wc = ld(W + c), Wym = ld(W + c - sj), Wzp = ld(W + c + sk), Wzpym = ld(W + c + sk - sj);
-        const R dUc = ld(dU + c), dUym = ld(dU + c - sj), dUxp = ld(dU + c + 1), dUxpym = ld(dU + c + 1 - sj);
-        const R Mjk = MU(j, k), Mjmk = MU(jm, k), Mjkm = MU(j, km), Mjmkm = MU(jm, km), Mjkp = MU(j, kp), Mjmkp = MU(jm, kp);
-        const R iRjk = IR(j, k), iRjmk = IR(jm, k);
-        const R v3 = R(0.5) * (Vym + Vc), v4 = R(0.5) * (Vc + Vyp);
-        const R u1 = (dx2[jm] * Uc + dx2[j] * Uym) * rdmx2[j] * R(0.5);
-        const R u2 = (dx2[jm] * Uxp + dx2[j] * Uxpym) * rdmx2[j] * R(0.5);
-        const R w5 = (dx2[jm] * Wc + dx2[j] * Wym) * rdmx2[j] * R(0.5);
-        const R w6 = (dx2[jm] * Wzp + dx2[j] * Wzpym) * rdmx2[j] * R(0.5);
-        const R ddu1 = (dx2[jm] * dUc + dx2[j] * dUym) * rdmx2[j] * R(0.5);
-        const R ddu2 = (dx2[jm] * dUxp + dx2[j] * dUxpym) * rdmx2[j] * R(0.5);
-        const R dvdx1 = (Vc - Vxm) * rdmx1[i], dvdx2 = (Vxp - Vc) * rdmx1[ip];
-        const R dvdy3 = (Vc - Vym) * rdx2[jm], dvdy4 = (Vyp - Vc) * rdx2[j];
-        const R dvdz5 = (Vc - Vzm) * rdmx3[k], dvdz6 = (Vzp - Vc) * rdmx3[kp];
-        const R dudy1 = (Uc - Uym) * rdmx2[j], dudy2 = (Uxp - Uxpym) * rdmx2[j];
-        const R dwdy5 = (Wc - Wym) * rdmx2[j], dwdy6 = (Wzp - Wzpym) * rdmx2[j];
-        const R ddudy1 = (dUc - dUym) * rdmx2[j], ddudy2 = (dUxp - dUxpym) * rdmx2[j];
-        // Mu(im,..) = Mu(i,..) = Mu(ip,..): the three x-neighbour averages coincide
-        const R mxy = R(0.5) * (dx2[jm] * Mjk + dx2[j] * Mjmk) * rdmx2[j];
-        const R mu1 = R(0.5) * (dx1[im] * mxy + dx1[i] * mxy) * rdmx1[i];
-        const R mu2 = R(0.5) * (dx1[ip] * mxy + dx1[i] * mxy) * rdmx1[ip];
-        const R mua = R(0.5) * (dx2[jm] * Mjkm + dx2[j] * Mjmkm) * rdmx2[j];
-        const R mub = R(0.5) * (dx2[jm] * Mjkp + dx2[j] * Mjmkp) * rdmx2[j];
-        const R mu5 = R(0.5) * (dx3[km] * mxy + dx3[k] * mua) * rdmx3[k];
-        const R mu6 = R(0.5) * (dx3[kp] * mxy + dx3[k] * mub) * rdmx3[kp];
-        const R invRhoc = R(0.5) * (dx2[jm] * iRjk + dx2[j] * iRjmk) * rdmx2[j];
-        const R ih = R(0.5) * p.Cmu * invRhoc;
-        const R vv1 = (mu2 * dvdx2 - mu1 * dvdx1) * rdx1[i];
-        const R vv2 = (Mjk * dvdy4 - Mjmk * dvdy3) * rdmx2[j];
-        const R vv3 = (mu6 * dvdz6 - mu5 * dvdz5) * rdx3[k];
-        const R vv21 = (mu2 * dudy2 - mu1 * dudy1) * rdx1[i];
-        const R vv23 = (mu6 * dwdy6 - mu5 * dwdy5) * rdx3[k];
-        // The reduced right-hand side (see DUZ); the y part keeps the
-        // reference's form on the planes next to the walls (j = 2, N2).
-        R rhs = R(2.0) * ih * (vv1 + vv21 + vv3 + vv23) - R(0.5) * (u1 * dvdx1 + u2 * dvdx2) - R(0.5) * (w5 * dvdz5 + w6 * dvdz6)
-                - R(0.25) * (ddu1 * dvdx1 + ddu2 * dvdx2) + ih * rdx1[i] * (mu2 * ddudy2 - mu1 * ddudy1);
-        rhs = rhs - p.Cmp * invRhoc * (ld(f.P + c) - ld(f.P + c - sj)) * rdmx2[j];
-        if (jvp != R(0.0) && jvm != R(0.0)) {
-            rhs = rhs + R(4.0) * ih * vv2 - R(0.5) * (v3 * dvdy3 + v4 * dvdy4);
-        } else {
-            R vbc_dn = (R(0.25) * rdx2[jm] * v3 * p.Vbt - R(0.25) * R(0.5) * dvdy3 * p.Vbt);
-            R vbc_up = (-R(0.25) * rdx2[j] * v4 * p.Vup - R(0.25) * R(0.5) * dvdy4 * p.Vup);
-            vbc_dn = vbc_dn + ih * rdmx2[j] * Mjmk * rdx2[jm] * p.Vbt * R(2.0);
-            vbc_up = vbc_up + ih * rdmx2[j] * Mjk * rdx2[j] * p.Vup * R(2.0);
-            const R mACJ = ih * rdmx2[j] * (Mjk * rdx2[j] + Mjmk * rdx2[jm]) * R(2.0) + R(0.25) * (dvdy4 * R(0.5) + dvdy3 * R(0.5) - v4 * rdx2[j] + v3 * rdx2[jm]);
-            const R mAPJ = (-ih * rdmx2[j] * Mjk * rdx2[j] * R(2.0) + R(0.25) * (v4 * rdx2[j] + dvdy4 * R(0.5))) * jvp;
-            const R mAMJ = (-ih * rdmx2[j] * Mjmk * rdx2[jm] * R(2.0) + R(0.25) * (-v3 * rdx2[jm] + dvdy3 * R(0.5))) * jvm;
-            rhs = rhs + R(2.0) * ih * vv2 + (R(1.0) - jvm) * vbc_dn + (R(1.0) - jvp) * vbc_up - (mAPJ * Vyp + mACJ * Vc + mAMJ * Vym);
+        switch (q) {
+        case 0: return f.V;
+        case 1: return f.V;
+        case 2: return f.V;
+        case 3: return f.U;
+        case 4: return f.U;
+        case 5: return f.dU;
+        case 6: return f.dU;
+        case 7: return f.W;
+        case 8: return f.W;
+        case 9: return f.P;
+        default: return f.P;
         }
-        const R mACK = ih * rdx3[k] * (mu6 * rdmx3[kp] + mu5 * rdmx3[k]) + R(0.25) * (-w6 * rdmx3[kp] + w5 * rdmx3[k]);
-        const R mAPK = -ih * rdx3[k] * mu6 * rdmx3[kp] + R(0.25) * (w6 * rdmx3[kp]);
-        const R mAMK = -ih * rdx3[k] * mu5 * rdmx3[k] + R(0.25) * (-w5 * rdmx3[k]);
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = mACK * dt + R(1.0); cf.c = mAPK * dt; cf.a = mAMK * dt; cf.d[0] = rhs * dt;
-        return cf;
     }
-    __device__ void emit(int l, int r, const R *x, const State &st) const { f.scr[ix(g, li(l), 2 + vby<ITEM>(), r + 1)] = x[0]; }
+    // The reduced right-hand side (see DUZ), with solvedU's increment beside U in
+    // every term (U + dU/2); on the planes next to the walls (j = 2, N2) the
+    // reference masks the upper coefficient by jS_BC(j-1) and the lower one by
+    // jS_BC(j+1).
+    struct March {
+        R cy, rdx1, rdmx1, rdmx1p, rdx2, rdx2m, rdmx2, dt;     // cy: weight of row j at y face j (row j-1: 1 - cy)
+        R Vc, F, G, ma, wa;
+        long long c;
+        int t4, j;
+        __device__ __forceinline__ March(const DVZ &q, int line, int by, int r0)
+        {
+            const GridT<R> &g = q.g;
+            const FieldsT<R> &f = q.f;
+            const int i = 1 + line, k = r0 + 1;
+            j = 2 + by;
+            rdx1 = ld(g.m1.rdx + i); rdmx1 = ld(g.m1.rdmx + i); rdmx1p = ld(g.m1.rdmx + i + 1);
+            rdx2 = ld(g.m2.rdx + j); rdx2m = ld(g.m2.rdx + j - 1); rdmx2 = ld(g.m2.rdmx + j);
+            cy = R(0.5) * ld(g.m2.dx + j - 1) * rdmx2;
+            dt = R(g.scal[S_DT]);
+            c = ix(g, i, j, k);
+            t4 = 4 * ix2(g, j, k);
+            Vc = ld(f.V + c);
+            face(ld(f.V + c - (long long)g.P1 * g.P2), Vc, ld(f.W + c), ld(f.W + c - g.P1), ld(f.MuT + t4 + 3), ld(g.m3.rdmx + k));
+        }
+        __device__ __forceinline__ void face(R Vm, R Vp, R W0, R Wym, R mu, R rdmx3)
+        {
+            const R dw = W0 - Wym, w = Wym + cy * dw, dv = (Vp - Vm) * rdmx3;
+            F = mu * (dv + dw * rdmx2);
+            G = w * dv;
+            ma = mu * rdmx3;
+            wa = R(0.25) * w * rdmx3;
+        }
+        struct In { R Vxm, Vxp, Vym, Vyp, Vzp, U0, Uym, Uxp, Uxpym, D0, Dym, Dxp, Dxpym, Wzp, Wzpym, Pc, Pym, Mm, muz6, iR, rdx3, rdmx3; cplx_t<R> mt; };
+        __device__ __forceinline__ void load(const DVZ &q, int r, In &n)
+        {
+            const GridT<R> &g = q.g;
+            const FieldsT<R> &f = q.f;
+            const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
+            n.Vxm = ld(f.V + c - 1); n.Vxp = ld(f.V + c + 1); n.Vym = ld(f.V + c - sj); n.Vyp = ld(f.V + c + sj); n.Vzp = ld(f.V + c + sk);
+            n.U0 = ld(f.U + c); n.Uym = ld(f.U + c - sj); n.Uxp = ld(f.U + c + 1); n.Uxpym = ld(f.U + c + 1 - sj);
+            n.D0 = ld(f.dU + c); n.Dym = ld(f.dU + c - sj); n.Dxp = ld(f.dU + c + 1); n.Dxpym = ld(f.dU + c + 1 - sj);
+            n.Wzp = ld(f.W + c + sk); n.Wzpym = ld(f.W + c + sk - sj);
+            n.Pc = ld(f.P + c); n.Pym = ld(f.P + c - sj);
+            n.mt = ld2(f.MuT + t4);
+            n.Mm = ld(f.MuT + t4 - 4); n.muz6 = ld(f.MuT + t4 + 4 * g.P2 + 3); n.iR = ld(f.iRT + t4 + 1);
+            n.rdx3 = ld(g.m3.rdx + r + 1); n.rdmx3 = ld(g.m3.rdmx + r + 2);
+            c += sk;
+            t4 += 4 * g.P2;
+        }
+        // the same values from the ring: slot a holds plane k's rows, b the plane below's
+        __device__ __forceinline__ void fill(const DVZ &q, int r, In &n, const double *a, const double *b, int w, int l)
+        {
+            const GridT<R> &g = q.g;
+            const int s = w + 2;
+            a += l + 1; b += l + 1;
+            const double *const ta = a - (l + 1) + NROW * s, *const tb = b - (l + 1) + NROW * s;   // table words of planes k + 1 and k
+            n.Vxm = b[-1]; n.Vxp = b[1]; n.Vzp = a[0]; n.Vym = a[s]; n.Vyp = a[2 * s];
+            n.U0 = a[3 * s]; n.Uxp = a[3 * s + 1]; n.Uym = a[4 * s]; n.Uxpym = a[4 * s + 1];
+            n.D0 = a[5 * s]; n.Dxp = a[5 * s + 1]; n.Dym = a[6 * s]; n.Dxpym = a[6 * s + 1];
+            n.Wzp = a[7 * s]; n.Wzpym = a[8 * s];
+            n.Pc = a[9 * s]; n.Pym = a[10 * s];
+            n.mt.x = tb[4]; n.mt.y = tb[5]; n.Mm = tb[0]; n.muz6 = ta[7]; n.iR = tb[13];
+            n.rdx3 = ld(g.m3.rdx + r + 1); n.rdmx3 = ld(g.m3.rdmx + r + 2);
+        }
+        __device__ __forceinline__ void row(const DVZ &q, int r, const In &n, double &a, double &b, double &cc, double *d)
+        {
+            const GridT<R> &g = q.g;
+            const PhysT<R> &p = g.ph;
+            const R Vxm = n.Vxm, Vxp = n.Vxp, Vym = n.Vym, Vyp = n.Vyp, Vzp = n.Vzp, U0 = n.U0, Uym = n.Uym, Uxp = n.Uxp, Uxpym = n.Uxpym;
+            const R D0 = n.D0, Dym = n.Dym, Dxp = n.Dxp, Dxpym = n.Dxpym, Wzp = n.Wzp, Wzpym = n.Wzpym, Pc = n.Pc, Pym = n.Pym;
+            const R Mm = n.Mm, muz6 = n.muz6, iR = n.iR;
+            const cplx_t<R> mt = n.mt;
+            const R rdx3 = n.rdx3;
+            const R ih = R(0.5) * p.Cmu * iR;
+            const R dx1 = (Vc - Vxm) * rdmx1, dx2 = (Vxp - Vc) * rdmx1p;
+            const R v3 = R(0.5) * (Vym + Vc), v4 = R(0.5) * (Vc + Vyp);
+            const R dy3 = (Vc - Vym) * rdx2m, dy4 = (Vyp - Vc) * rdx2;
+            // differences of U and dU apart: U is the larger by orders of magnitude
+            const R ds1 = (U0 - Uym) + R(0.5) * (D0 - Dym), ds2 = (Uxp - Uxpym) + R(0.5) * (Dxp - Dxpym);
+            const R s1 = (Uym + R(0.5) * Dym) + cy * ds1, s2 = (Uxpym + R(0.5) * Dxpym) + cy * ds2;
+            const R F5 = F, G5 = G, ma5 = ma, wa5 = wa, V0 = Vc;
+            Vc = Vzp;
+            face(V0, Vzp, Wzp, Wzpym, muz6, n.rdmx3);
+            const R vs = mt.y * (((dx2 - dx1) + (ds2 - ds1) * rdmx2) * rdx1) + (F - F5) * rdx3 + R(2) * (mt.x * dy4 - Mm * dy3) * rdmx2;
+            R rhs = R(2) * ih * vs - R(0.5) * ((s1 * dx1 + s2 * dx2) + (G5 + G) + (v3 * dy3 + v4 * dy4));
+            rhs = rhs - p.Cmp * iR * (Pc - Pym) * rdmx2;
+            if (j == 2) {
+                const R ap = -R(2) * ih * rdmx2 * mt.x * rdx2 + R(0.25) * (v4 * rdx2 + R(0.5) * dy4);
+                rhs = rhs + ap * (Vyp - p.Vup);
+            }
+            if (j == g.N2) {
+                const R am = -R(2) * ih * rdmx2 * Mm * rdx2m + R(0.25) * (R(0.5) * dy3 - v3 * rdx2m);
+                rhs = rhs + am * (Vym - p.Vbt);
+            }
+            const R h3 = ih * rdx3;
+            const R am = -(h3 * ma5 + wa5) * dt, ap = (wa - h3 * ma) * dt;
+            a = am; cc = ap; b = 1.0 - ((double)am + (double)ap);
+            d[0] = rhs * dt;
+        }
+    };
+    __device__ __forceinline__ void emit(int line, int by, int r, const double *x) const { f.scr[ix(g, 1 + line, 2 + by, r + 1)] = R(x[0]); }
 };
 
 // mu1, mu2 of solvedV's last stage-1 iteration (i = N1, j = N2, k = N3).
@@ -416,112 +519,146 @@ struct DVY {
 // solvedW (:930-1272).  Stage 2 uses stale mu1, mu2 and stage 3 stale mu3,
 // mu4 (last stage-1 iteration) and a stale km = N3-1 (last stage-2 iteration).
 // ---------------------------------------------------------------------------
-template <class R, int ITEM = 0>
+template <class R>
 struct DWZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = std::is_same<R, float>::value;   // measured faster in FP32 only
-    static constexpr int MINB = LineOcc<R>::z;
-    static constexpr int MREG = LineOcc<Real>::reg_z;
-    static constexpr int NT = LineOcc<Real>::nt_z;
-    static constexpr bool CONTIG = false;
-    static constexpr bool PAIR = LineOcc<Real>::pair_z;
-    static constexpr bool LINE_PER_THREAD = false;   // the unpaired FP32 build: measured slower
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr bool AHEAD = std::is_same<R, float>::value;   // FP64 inputs of two rows do not fit the registers
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt; };
-    __device__ State prepare() const { return State{R(g.scal[S_DT])}; }
-    __device__ int li(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return li(l) <= g.N1; }
-    // The stencil inputs of a cell, read through val(array, di, dj, dk): from
-    // global memory (build) or from the staged tiles (dwz_staged_kernel), with
-    // the same arithmetic after them.
-    enum : int { A_W = 0, A_U, A_V, A_DU, A_DV, A_P };
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
+    __device__ int lines() const { return g.N1; }
+    // the rows of i that a plane needs in the column form
+    static constexpr int NROW = 10, J0 = 1;
+    static constexpr bool TABLES = true;
+    __device__ static constexpr int row_dj(int q) { constexpr int v[] = {0, -1, 1, 0, 0, 0, 1, 0, 1, 0}; return v[q]; }
+    __device__ static constexpr int row_dk(int q) { constexpr int v[] = {1, 0, 0, 0, 0, 0, 0, 0, 0, 0}; return v[q]; }
+    __device__ __forceinline__ const R *row_src(int q) const
     {
-        const long long c = ix(g, li(l), 1 + vby<ITEM>(), r + 1), sj = g.P1, sk = (long long)g.P1 * g.P2;
-        const R *const arr[6] = {f.W, f.U, f.V, f.dU, f.dV, f.P};
-        return build_with([&](int a, int di, int dj, int dk) { return ld(arr[a] + (c + di + dj * sj + dk * sk)); }, l, r, st);
-    }
-    template <class Val>
-    __device__ __forceinline__ Coef<R, 1> build_with(const Val &val, int l, int r, const State &st) const
-    {
-        const int i = li(l), j = 1 + vby<ITEM>(), k = r + 1;
-        const int im = i - 1, ip = i + 1, jm = j - 1, jp = j + 1, km = k - 1;
-        const PhysT<R> &p = g.ph;
-        const R *dx1 = g.m1.dx, *dx2 = g.m2.dx, *dx3 = g.m3.dx;
-        const R *rdx1 = g.m1.rdx, *rdx2 = g.m2.rdx, *rdx3 = g.m3.rdx;
-        const R *rdmx1 = g.m1.rdmx, *rdmx2 = g.m2.rdmx, *rdmx3 = g.m3.rdmx;
-        const R jwm = (j == 1) ? R(0.0) : R(1.0), jwp = (j == g.N2) ? R(0.0) : R(1.0);
-        const R Wc = val(A_W, 0, 0, 0), Wzm = val(A_W, 0, 0, -1), Wzp = val(A_W, 0, 0, 1), Wxm = val(A_W, -1, 0, 0), Wxp = val(A_W, 1, 0, 0);
-        const R Wym = val(A_W, 0, -1, 0), Wyp = val(A_W, 0, 1, 0);
-        const R Uc = val(A_U, 0, 0, 0), Uzm = val(A_U, 0, 0, -1), Uxp = val(A_U, 1, 0, 0), Uxpzm = val(A_U, 1, 0, -1);
-        const R Vc = val(A_V, 0, 0, 0), Vzm = val(A_V, 0, 0, -1), Vyp = val(A_V, 0, 1, 0), Vypzm = val(A_V, 0, 1, -1);
-        const R dUc = val(A_DU, 0, 0, 0), dUzm = val(A_DU, 0, 0, -1), dUxp = val(A_DU, 1, 0, 0), dUxpzm = val(A_DU, 1, 0, -1);
-        const R dVc = val(A_DV, 0, 0, 0), dVzm = val(A_DV, 0, 0, -1), dVyp = val(A_DV, 0, 1, 0), dVypzm = val(A_DV, 0, 1, -1);
-        const R Mjk = MU(j, k), Mjkm = MU(j, km), Mjmk = MU(jm, k), Mjmkm = MU(jm, km), Mjpk = MU(jp, k), Mjpkm = MU(jp, km);
-        const R iRjk = IR(j, k), iRjkm = IR(j, km);
-        const R w5 = R(0.5) * (Wc + Wzm), w6 = R(0.5) * (Wc + Wzp);
-        const R u1 = (dx3[km] * Uc + dx3[k] * Uzm) * rdmx3[k] * R(0.5);
-        const R u2 = (dx3[km] * Uxp + dx3[k] * Uxpzm) * rdmx3[k] * R(0.5);
-        const R v3 = (dx3[km] * Vc + dx3[k] * Vzm) * rdmx3[k] * R(0.5);
-        const R v4 = (dx3[km] * Vyp + dx3[k] * Vypzm) * rdmx3[k] * R(0.5);
-        const R dwdx1 = (Wc - Wxm) * rdmx1[i], dwdx2 = (Wxp - Wc) * rdmx1[ip];
-        const R dwdy3 = (Wc - Wym) * rdmx2[j], dwdy4 = (Wyp - Wc) * rdmx2[jp];
-        const R dwdz5 = (Wc - Wzm) * rdx3[km], dwdz6 = (Wzp - Wc) * rdx3[k];
-        const R dudz1 = (Uc - Uzm) * rdmx3[k], dudz2 = (Uxp - Uxpzm) * rdmx3[k];
-        const R dvdz3 = (Vc - Vzm) * rdmx3[k], dvdz4 = (Vyp - Vypzm) * rdmx3[k];
-        const R ddudz1 = (dUc - dUzm) * rdmx3[k], ddudz2 = (dUxp - dUxpzm) * rdmx3[k];
-        const R ddvdz3 = (dVc - dVzm) * rdmx3[k], ddvdz4 = (dVyp - dVypzm) * rdmx3[k];
-        const R ddu1 = (dx3[km] * dUc + dx3[k] * dUzm) * rdmx3[k] * R(0.5);
-        const R ddu2 = (dx3[km] * dUxp + dx3[k] * dUxpzm) * rdmx3[k] * R(0.5);
-        const R ddv3 = (dx3[km] * dVc + dx3[k] * dVzm) * rdmx3[k] * R(0.5) * jwm;
-        const R ddv4 = (dx3[km] * dVyp + dx3[k] * dVypzm) * rdmx3[k] * R(0.5) * jwp;
-        const R mxz = R(0.5) * (dx3[km] * Mjk + dx3[k] * Mjkm) * rdmx3[k];   // mua = muc = mub (x)
-        const R mu1 = R(0.5) * (dx1[im] * mxz + dx1[i] * mxz) * rdmx1[i];
-        const R mu2 = R(0.5) * (dx1[ip] * mxz + dx1[i] * mxz) * rdmx1[ip];
-        const R mua = R(0.5) * (dx3[km] * Mjmk + dx3[k] * Mjmkm) * rdmx3[k];
-        const R mub = R(0.5) * (dx3[km] * Mjpk + dx3[k] * Mjpkm) * rdmx3[k];
-        const R mu3 = R(0.5) * (dx2[jm] * mxz + dx2[j] * mua) * rdmx2[j];
-        const R mu4 = R(0.5) * (dx2[jp] * mxz + dx2[j] * mub) * rdmx2[jp];
-        const R invRhoc = R(0.5) * (dx3[km] * iRjk + dx3[k] * iRjkm) * rdmx3[k];
-        const R ih = R(0.5) * p.Cmu * invRhoc;
-        const R vw1 = (mu2 * dwdx2 - mu1 * dwdx1) * rdx1[i];
-        const R vw2 = (mu4 * dwdy4 - mu3 * dwdy3) * rdx2[j];
-        const R vw3 = (Mjk * dwdz6 - Mjkm * dwdz5) * rdmx3[k];
-        const R vw31 = (mu2 * dudz2 - mu1 * dudz1) * rdx1[i];
-        const R vw32 = (mu4 * dvdz4 - mu3 * dvdz3) * rdx2[j];
-        // The reduced right-hand side (see DUZ); the y part keeps the
-        // reference's form on the wall-adjacent planes (j = 1, N2).
-        R rhs = R(2.0) * ih * (vw1 + vw31) + R(4.0) * ih * vw3 - R(0.5) * (u1 * dwdx1 + u2 * dwdx2) - R(0.5) * (w5 * dwdz5 + w6 * dwdz6)
-                - R(0.25) * (ddu1 * dwdx1 + ddu2 * dwdx2) + ih * rdx1[i] * (mu2 * ddudz2 - mu1 * ddudz1);
-        rhs = rhs - p.Cmp * invRhoc * (val(A_P, 0, 0, 0) - val(A_P, 0, 0, -1)) * rdmx3[k];
-        if (j != 1 && j != g.N2) {
-            rhs = rhs + R(2.0) * ih * (vw2 + vw32) - R(0.5) * (v3 * dwdy3 + v4 * dwdy4)
-                  - R(0.25) * (ddv3 * dwdy3 + ddv4 * dwdy4) + ih * rdx2[j] * (mu4 * ddvdz4 - mu3 * ddvdz3);
-        } else {
-            R zbc_dn = R(0.25) * v3 * rdmx2[j] * p.Wbt - R(0.25) * dwdy3 * (dx3[km] * p.Vbt + dx3[k] * p.Vbt) * rdmx3[k] * R(0.5);
-            R zbc_up = -R(0.25) * v4 * rdmx2[jp] * p.Wup - R(0.25) * dwdy4 * (dx3[km] * p.Vup + dx3[k] * p.Vup) * rdmx3[k] * R(0.5);
-            zbc_dn = zbc_dn + ih * rdx2[j] * mu3 * rdmx2[jp] * p.Wbt;
-            zbc_up = zbc_up + ih * rdx2[j] * mu4 * rdmx2[j] * p.Wup;
-            zbc_dn = zbc_dn - ih * rdx2[j] * mu3 * rdmx3[k] * (p.Vbt - p.Vbt);
-            zbc_up = zbc_up + ih * rdx2[j] * mu4 * rdmx3[k] * (p.Vup - p.Vup);
-            const R mACJ = ih * rdx2[j] * (mu4 * rdmx2[jp] + mu3 * rdmx2[j]) + R(0.25) * (-v4 * rdmx2[jp] + v3 * rdmx2[j]);
-            const R mAPJ = (-ih * rdx2[j] * mu4 * rdmx2[jp] + R(0.25) * (v4 * rdmx2[jp])) * jwp;
-            const R mAMJ = (-ih * rdx2[j] * mu3 * rdmx2[j] + R(0.25) * (-v3 * rdmx2[j])) * jwm;
-            rhs = rhs + ih * (vw2 + vw32) + (R(1.0) - jwm) * zbc_dn + (R(1.0) - jwp) * zbc_up - (mAPJ * Wyp + mACJ * Wc + mAMJ * Wym)
-                  - (R(0.25) * (v3 * jwm * dwdy3 + v4 * jwp * dwdy4) - ih * rdx2[j] * (mu4 * dvdz4 * jwp - mu3 * dvdz3 * jwm))
-                  - (R(0.25) * (ddv3 * jwm * dwdy3 + ddv4 * jwp * dwdy4) - ih * rdx2[j] * (mu4 * ddvdz4 * jwp - mu3 * ddvdz3 * jwm));
+        switch (q) {
+        case 0: return f.W;
+        case 1: return f.W;
+        case 2: return f.W;
+        case 3: return f.U;
+        case 4: return f.dU;
+        case 5: return f.V;
+        case 6: return f.V;
+        case 7: return f.dV;
+        case 8: return f.dV;
+        default: return f.P;
         }
-        const R mACK = ih * rdmx3[k] * (Mjk * rdx3[k] + Mjkm * rdx3[km]) * R(2.0) + R(0.25) * (-w6 * rdx3[k] + w5 * rdx3[km] + R(0.5) * dwdz6 + R(0.5) * dwdz5);
-        const R mAPK = -ih * rdmx3[k] * Mjk * rdx3[k] * R(2.0) + R(0.25) * (w6 * rdx3[k] + R(0.5) * dwdz6);
-        const R mAMK = -ih * rdmx3[k] * Mjkm * rdx3[km] * R(2.0) + R(0.25) * (-w5 * rdx3[km] + R(0.5) * dwdz5);
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = mACK * dt + R(1.0); cf.c = mAPK * dt; cf.a = mAMK * dt; cf.d[0] = rhs * dt;
-        return cf;
     }
-    __device__ void emit(int l, int r, const R *x, const State &st) const { f.scr[ix(g, li(l), 1 + vby<ITEM>(), r + 1)] = x[0]; }
+    // The reduced right-hand side (see DUZ), with the increments of solvedU and
+    // solvedV beside U and V.
+    struct March {
+        R rdx1, rdmx1, rdmx1p, rdx2, rdmx2, rdmx2p, dt;
+        R U0, Uxp, D0, Dxp, V0, Vyp, E0, Eyp, P0;       // the plane below: U, dU at i, i+1; V, dV at j, j+1; P
+        R Wc, G, H, A, B, C, dx3;                       // the cell below (between W rows k-1 and k)
+        long long c;
+        int t4, j;
+        __device__ __forceinline__ March(const DWZ &q, int line, int by, int r0)
+        {
+            const GridT<R> &g = q.g;
+            const FieldsT<R> &f = q.f;
+            const int i = 1 + line, k = r0 + 1;
+            const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
+            j = 1 + by;
+            rdx1 = ld(g.m1.rdx + i); rdmx1 = ld(g.m1.rdmx + i); rdmx1p = ld(g.m1.rdmx + i + 1);
+            rdx2 = ld(g.m2.rdx + j); rdmx2 = ld(g.m2.rdmx + j); rdmx2p = ld(g.m2.rdmx + j + 1);
+            dt = R(g.scal[S_DT]);
+            c = ix(g, i, j, k);
+            t4 = 4 * ix2(g, j, k);
+            const long long cm = c - sk;
+            U0 = ld(f.U + cm); Uxp = ld(f.U + cm + 1); D0 = ld(f.dU + cm); Dxp = ld(f.dU + cm + 1);
+            V0 = ld(f.V + cm); Vyp = ld(f.V + cm + sj); E0 = ld(f.dV + cm); Eyp = ld(f.dV + cm + sj);
+            P0 = ld(f.P + cm);
+            Wc = ld(f.W + c);
+            cell(ld(f.W + cm), Wc, ld(f.MuT + t4 - 4 * g.P2), ld(g.m3.dx + k - 1), ld(g.m3.rdx + k - 1));
+        }
+        // the cell between W rows k and k + 1
+        __device__ __forceinline__ void cell(R Wm, R Wp, R mu, R dz, R rdx3)
+        {
+            dx3 = dz;
+            const R w = R(0.5) * (Wm + Wp), dw = (Wp - Wm) * rdx3;
+            G = w * dw;
+            H = mu * dw;
+            A = mu * rdx3;
+            B = R(0.25) * w * rdx3;
+            C = R(0.125) * dw;
+        }
+        struct In { R Wxm, Wxp, Wym, Wyp, Wzp, U, Ux, D, Dx, V, Vy, E, Ey, P, Mc, muyz4, iR, dx3, rdx3, rdmx3; cplx_t<R> mt; };
+        __device__ __forceinline__ void load(const DWZ &q, int r, In &n)
+        {
+            const GridT<R> &g = q.g;
+            const FieldsT<R> &f = q.f;
+            const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
+            n.Wxm = ld(f.W + c - 1); n.Wxp = ld(f.W + c + 1); n.Wym = ld(f.W + c - sj); n.Wyp = ld(f.W + c + sj); n.Wzp = ld(f.W + c + sk);
+            n.U = ld(f.U + c); n.Ux = ld(f.U + c + 1); n.D = ld(f.dU + c); n.Dx = ld(f.dU + c + 1);
+            n.V = ld(f.V + c); n.Vy = ld(f.V + c + sj); n.E = ld(f.dV + c); n.Ey = ld(f.dV + c + sj);
+            n.P = ld(f.P + c);
+            n.Mc = ld(f.MuT + t4);
+            n.mt = ld2(f.MuT + t4 + 2);                    // Mu at the lower z face, at the lower yz edge
+            n.muyz4 = ld(f.MuT + t4 + 7); n.iR = ld(f.iRT + t4 + 2);
+            n.dx3 = ld(g.m3.dx + r + 1); n.rdx3 = ld(g.m3.rdx + r + 1); n.rdmx3 = ld(g.m3.rdmx + r + 1);
+            c += sk;
+            t4 += 4 * g.P2;
+        }
+        // the same values from the ring: slot a holds plane k's rows, b the plane below's
+        __device__ __forceinline__ void fill(const DWZ &q, int r, In &n, const double *a, const double *b, int w, int l)
+        {
+            const GridT<R> &g = q.g;
+            const int s = w + 2;
+            a += l + 1; b += l + 1;
+            const double *const ta = a - (l + 1) + NROW * s, *const tb = b - (l + 1) + NROW * s;   // table words of planes k + 1 and k
+            n.Wxm = b[-1]; n.Wxp = b[1]; n.Wzp = a[0]; n.Wym = a[s]; n.Wyp = a[2 * s];
+            n.U = a[3 * s]; n.Ux = a[3 * s + 1]; n.D = a[4 * s]; n.Dx = a[4 * s + 1];
+            n.V = a[5 * s]; n.Vy = a[6 * s]; n.E = a[7 * s]; n.Ey = a[8 * s];
+            n.P = a[9 * s];
+            n.Mc = tb[4]; n.mt.x = tb[6]; n.mt.y = tb[7]; n.muyz4 = tb[11]; n.iR = tb[14];
+            n.dx3 = ld(g.m3.dx + r + 1); n.rdx3 = ld(g.m3.rdx + r + 1); n.rdmx3 = ld(g.m3.rdmx + r + 1);
+            (void)ta;
+        }
+        __device__ __forceinline__ void row(const DWZ &q, int r, const In &n, double &a, double &b, double &cc, double *d)
+        {
+            const GridT<R> &g = q.g;
+            const PhysT<R> &p = g.ph;
+            const R Wxm = n.Wxm, Wxp = n.Wxp, Wym = n.Wym, Wyp = n.Wyp, Wzp = n.Wzp, nU = n.U, nUx = n.Ux, nD = n.D, nDx = n.Dx;
+            const R nV = n.V, nVy = n.Vy, nE = n.E, nEy = n.Ey, nP = n.P, Mc = n.Mc, muyz4 = n.muyz4, iR = n.iR;
+            const cplx_t<R> mt = n.mt;
+            const R rdmx3 = n.rdmx3;
+            const R dx3m = dx3, G5 = G, H5 = H, A5 = A, B5 = B, C5 = C, W0 = Wc;
+            Wc = Wzp;
+            cell(W0, Wzp, Mc, n.dx3, n.rdx3);
+            const R cz = R(0.5) * dx3m * rdmx3;                            // weight of plane k at z face k (plane k-1: 1 - cz)
+            const R ih = R(0.5) * p.Cmu * iR;
+            const R dx1 = (W0 - Wxm) * rdmx1, dx2 = (Wxp - W0) * rdmx1p;
+            const R dy3 = (W0 - Wym) * rdmx2, dy4 = (Wyp - W0) * rdmx2p;
+            const R ds1 = (nU - U0) + R(0.5) * (nD - D0), ds2 = (nUx - Uxp) + R(0.5) * (nDx - Dxp);
+            const R dv3 = nV - V0, dv4 = nVy - Vyp, de3 = nE - E0, de4 = nEy - Eyp;
+            const R dt3 = dv3 + R(0.5) * de3, dt4 = dv4 + R(0.5) * de4;
+            const R s1 = (U0 + R(0.5) * D0) + cz * ds1, s2 = (Uxp + R(0.5) * Dxp) + cz * ds2;
+            const R t3 = (V0 + R(0.5) * E0) + cz * dt3, t4_ = (Vyp + R(0.5) * Eyp) + cz * dt4;
+            const R mu3 = mt.y, mu4 = muyz4;
+            const R vs = mt.x * (((dx2 - dx1) + (ds2 - ds1) * rdmx3) * rdx1) + (mu4 * (dy4 + dt4 * rdmx3) - mu3 * (dy3 + dt3 * rdmx3)) * rdx2 + R(2) * (H - H5) * rdmx3;
+            R rhs = R(2) * ih * vs - R(0.5) * ((s1 * dx1 + s2 * dx2) + (t3 * dy3 + t4_ * dy4) + (G5 + G));
+            rhs = rhs - p.Cmp * iR * (nP - P0) * rdmx3;
+            if (j == 1) {
+                const R v3 = V0 + cz * dv3, am = -(ih * rdx2 * mu3 + R(0.25) * v3) * rdmx2;
+                rhs = rhs + am * Wym + (R(0.5) * t3 - R(0.25) * v3) * dy3 + ih * rdx2 * mu3 * ((dv3 + de3) * rdmx3);
+                rhs = rhs + R(0.25) * v3 * rdmx2 * p.Wbt - R(0.25) * dy3 * p.Vbt + ih * rdx2 * mu3 * rdmx2p * p.Wbt;
+            }
+            if (j == g.N2) {
+                const R v4 = Vyp + cz * dv4, ap = (R(0.25) * v4 - ih * rdx2 * mu4) * rdmx2p;
+                rhs = rhs + ap * Wyp + (R(0.5) * t4_ - R(0.25) * v4) * dy4 - ih * rdx2 * mu4 * ((dv4 + de4) * rdmx3);
+                rhs = rhs - R(0.25) * v4 * rdmx2p * p.Wup - R(0.25) * dy4 * p.Vup + ih * rdx2 * mu4 * rdmx2 * p.Wup;
+            }
+            const R h3 = R(2) * ih * rdmx3;
+            const R am = (C5 - B5 - h3 * A5) * dt, ap = (B + C - h3 * A) * dt;
+            a = am; cc = ap; b = (1.0 - ((double)am + (double)ap)) + (double)(R(2) * (C5 + C) * dt);
+            d[0] = rhs * dt;
+            U0 = nU; Uxp = nUx; D0 = nD; Dxp = nDx; V0 = nV; Vyp = nVy; E0 = nE; Eyp = nEy; P0 = nP;
+        }
+    };
+    __device__ __forceinline__ void emit(int line, int by, int r, const double *x) const { f.scr[ix(g, 1 + line, 1 + by, r + 1)] = R(x[0]); }
 };
 
 // mu1..mu4 of solvedW's last stage-1 iteration (i = N1, j = N2, k = N3).
@@ -630,208 +767,27 @@ struct DWY {
     __device__ void emit(int l, int r, const R *x, const State &st) const { store_periodic(g, f.dW, li(l), r + 1, 1 + vby<ITEM>(), x[0]); }
 };
 
-// ---------------------------------------------------------------------------
-// solvedW's z sweep with its stencil inputs staged by TMA (FP64 form,
-// TCS_TUNE_Z_STAGING 2).  The same lines, rows, arithmetic and solve as the
-// DWZ line-solver launch (DWZ::build_with is shared, so the results are the
-// same bits); only where the stencil inputs come from differs.  A block of
-// 512 threads owns 8 lines (i0..i0+7) of one j; the rows are built in passes of
-// ZS_CH = 64 k-planes, one cell per thread per pass, from shared-memory boxes
-// of the six input arrays that the tensor memory accelerator copies one pass
-// ahead (two buffers):
-//   W       i0-1..i0+8 x j-1..j+1 x k-1..k+64      (x and y neighbours, k +-1)
-//   U, dU   i0-1..i0+8 x j        x k-1..k+63
-//   V, dV   i0-1..i0+8 x j..j+1   x k-1..k+63
-//   P       i0-1..i0+8 x j        x k-1..k+63
-// Every box starts at x = i0-1 = 8 bx, an even element, so its first byte is
-// 16-byte aligned as TMA requires, and is 10 doubles (80 bytes) wide.  It
-// requires N3 a multiple of ZS_CH and an even N1 (the row pitch a multiple of
-// 16 bytes); launch_solve_dw checks both.
-// ---------------------------------------------------------------------------
-constexpr int ZS_CH = 64, ZS_TL = 8, ZS_NT = 512;
-constexpr int ZS_WAIT = 1 << 22;   // polls of a bounded wait (each try_wait suspends briefly)
-__host__ __device__ constexpr int zs_rows(int a) { return a == 0 ? 3 : ((a == 2 || a == 4) ? 2 : 1); }
-__host__ __device__ constexpr int zs_planes(int a) { return a == 0 ? ZS_CH + 2 : ZS_CH + 1; }
-__host__ __device__ constexpr int zs_bytes(int a) { return 10 * zs_rows(a) * zs_planes(a) * 8; }
-__host__ __device__ constexpr int zs_off(int a) { return a == 0 ? 0 : zs_off(a - 1) + (zs_bytes(a - 1) + 127) / 128 * 128; }
-constexpr int ZS_BUF = zs_off(6);
-constexpr int ZS_TX = zs_bytes(0) + zs_bytes(1) + zs_bytes(2) + zs_bytes(3) + zs_bytes(4) + zs_bytes(5);
-
-struct alignas(64) DWZMaps {
-    CUtensorMap m[6];   // DWZ's A_W, A_U, A_V, A_DU, A_DV, A_P
-};
-
-// Dynamic shared memory: two box buffers, the rows (A, C, D), the row map, two mbarriers.
-inline size_t zs_smem(const LinePlan &lp)
+template <class R>
+static void launch_du_z(const Ctx<R> &cx, cudaStream_t s)
 {
-    const size_t rows = (size_t)3 * ZS_TL * lp.LS * sizeof(double) + (size_t)lp.n * sizeof(int);
-    return 2 * (size_t)ZS_BUF + ((rows + 15) & ~(size_t)15) + 2 * sizeof(uint64_t);
+    launch_march(cx, DUZ<R>{cx.g, cx.f}, cx.g.N3, true, cx.g.N1, cx.g.N2, s, K_DU_Z);
 }
-
-__global__ void __launch_bounds__(ZS_NT, 1) dwz_staged_kernel(const __grid_constant__ DWZ<double> prob,
-                                                              const __grid_constant__ DWZMaps maps, LinePlan lp)
+template <class R>
+static void launch_dv_z(const Ctx<R> &cx, cudaStream_t s)
 {
-    using P = DWZ<double>;
-    extern __shared__ __align__(128) unsigned char smraw[];
-    if (prob.skip()) return;
-    const P::State st = prob.prepare();
-    const int n = lp.n, LS = lp.LS, DS = ZS_TL * LS, nch = n / ZS_CH;
-    double *const sA = reinterpret_cast<double *>(smraw + 2 * ZS_BUF), *const sC = sA + DS, *const sD = sC + DS;
-    int *const spos = reinterpret_cast<int *>(sD + DS);
-    const size_t rows = (size_t)3 * DS * sizeof(double) + (size_t)n * sizeof(int);
-    uint64_t *const bar = reinterpret_cast<uint64_t *>(smraw + 2 * ZS_BUF + ((rows + 15) & ~(size_t)15));
-    const int x0 = ZS_TL * blockIdx.x, j = 1 + blockIdx.y;
-    if (smem_u32(smraw) & 127) {   // the boxes need 128-byte aligned destinations: record and stop, copy nothing
-        if (threadIdx.x == 0) {
-            atomicAdd(prob.g.scal + S_TIMEOUT, 1.0);
-            prob.g.scal[S_BLOWUP] = 1.0;
-        }
-        return;
-    }
-    if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_init_fence();
-    }
-    if (threadIdx.x < lp.P) {
-        const int p = threadIdx.x, m = lp.m0 + (p < lp.rem ? 1 : 0), start = p * lp.m0 + (p < lp.rem ? p : lp.rem);
-        for (int q = 0; q < m; q++) spos[start + q] = p * lp.PS + q;
-    }
-    __syncthreads();
-    auto issue = [&](int c) {   // thread 0: the boxes of pass c into buffer c & 1
-        uint64_t *b = &bar[c & 1];
-        unsigned char *dst = smraw + (c & 1) * ZS_BUF;
-        mbar_arrive_expect_tx(b, ZS_TX);
-#pragma unroll
-        for (int a = 0; a < 6; a++) tma_load_3d(dst + zs_off(a), &maps.m[a], b, x0, a == P::A_W ? j - 1 : j, c * ZS_CH);
-    };
-    if (threadIdx.x == 0) {
-        issue(0);
-        if (nch > 1) issue(1);
-    }
-    const int l = threadIdx.x & (ZS_TL - 1), rr = threadIdx.x >> 3;   // one cell per thread per pass
-    int c = 0;
-    bool ok = true;
-    for (; c < nch; c++) {
-        const bool got = mbar_wait(&bar[c & 1], (c >> 1) & 1, ZS_WAIT);
-        if (__syncthreads_or(!got)) { ok = false; break; }
-        const double *const t = reinterpret_cast<const double *>(smraw + (c & 1) * ZS_BUF);
-        // row r = c ZS_CH + rr is plane k = r + 1, plane k + dk of a box at z = rr + 1 + dk
-        auto val = [&](int a, int di, int dj, int dk) -> double {
-            int z = rr + 1 + dk, y = (a == P::A_W) ? 1 + dj : dj, x = l + 1 + di;
-            TCS_OOB(prob.g.scal, (unsigned)z >= (unsigned)zs_planes(a) || (unsigned)y >= (unsigned)zs_rows(a) || (unsigned)x >= 10u,
-                    (z = 0, y = 0, x = 0));
-            return t[zs_off(a) / 8 + (z * zs_rows(a) + y) * 10 + x];
-        };
-        const int r = c * ZS_CH + rr;
-        Coef<double, 1> cf;
-        if (prob.line_ok(l)) {
-            cf = prob.build_with(val, l, r, st);
-        } else {
-            cf.a = 0.0; cf.b = 1.0; cf.c = 0.0; cf.d[0] = 0.0;
-        }
-        const double rb = rcp_of<FastRcp<P>::on>(cf.b);
-        const int pos = l * LS + spos[r];
-        sA[pos] = cf.a * rb; sC[pos] = cf.c * rb; sD[pos] = cf.d[0] * rb;
-        __syncthreads();   // every thread is done with this buffer
-        if (threadIdx.x == 0 && c + 2 < nch) {
-            fence_proxy_async();
-            issue(c + 2);
-        }
-    }
-    if (!ok) {
-        // a copy did not arrive in time: record it, stop the step, and wait
-        // (bounded) for this block's copies still in flight before leaving
-        if (threadIdx.x == 0) {
-            atomicAdd(prob.g.scal + S_TIMEOUT, 1.0);
-            prob.g.scal[S_BLOWUP] = 1.0;
-            for (int d = c; d < c + 2 && d < nch; d++) mbar_wait(&bar[d & 1], (d >> 1) & 1, ZS_WAIT);
-        }
-        return;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int ll = warp; ll < ZS_TL; ll += ZS_NT / 32)
-        solve_line<double, 1, P::MREG, false, FastRcp<P>::on>(sA + ll * LS, sC + ll * LS, sD + ll * LS, DS, lp, lane);
-    __syncthreads();
-    if (prob.line_ok(l))
-        for (int r = rr; r < n; r += ZS_NT / ZS_TL) {
-            const double x = sD[l * LS + spos[r]];
-            prob.emit(l, r, &x, st);
-        }
+    launch_march(cx, DVZ<R>{cx.g, cx.f}, cx.g.N3, true, cx.g.N1, cx.g.N2 - 1, s, K_DV_Z);
 }
-
-// The tensor maps of the staged z sweep: one 3-D map (x = i, y = j, z = k over
-// the padded array) per input array with that array's box.
-typedef CUresult (*PfnTensorMapEncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                            const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                            CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static PfnTensorMapEncodeTiled tensor_map_encoder()
+template <class R>
+static void launch_dw_z(const Ctx<R> &cx, cudaStream_t s)
 {
-    static PfnTensorMapEncodeTiled fn = [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess) {
-            cudaGetLastError();
-            f = nullptr;
-        }
-        return (PfnTensorMapEncodeTiled)f;
-    }();
-    return fn;
-}
-
-static bool dwz_maps(const Ctx<double> &cx, DWZMaps &mp)
-{
-    const GridT<double> &g = cx.g;
-    PfnTensorMapEncodeTiled enc = tensor_map_encoder();
-    if (!enc) return false;
-    const double *src[6] = {cx.f.W, cx.f.U, cx.f.V, cx.f.dU, cx.f.dV, cx.f.P};
-    const cuuint64_t dims[3] = {(cuuint64_t)g.P1, (cuuint64_t)g.P2, (cuuint64_t)g.N3 + 2};
-    const cuuint64_t strides[2] = {(cuuint64_t)g.P1 * 8, (cuuint64_t)g.P1 * g.P2 * 8};
-    const cuuint32_t es[3] = {1, 1, 1};
-    for (int a = 0; a < 6; a++) {
-        const cuuint32_t box[3] = {10, (cuuint32_t)zs_rows(a), (cuuint32_t)zs_planes(a)};
-        if (enc(&mp.m[a], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, (void *)src[a], dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return false;
-    }
-    return true;
-}
-
-// Whether the staged form can run this case (shape, shared memory, tensor-map encoder).
-bool dwz_staging_possible(const Ctx<double> &cx)
-{
-    const GridT<double> &g = cx.g;
-    if (g.N3 % ZS_CH || (g.P1 * 8) % 16) return false;
-    if (zs_smem(make_line_plan(g.N3, true, ZS_TL, cx.lanes)) > 227 * 1024) return false;
-    DWZMaps mp;
-    return dwz_maps(cx, mp);
-}
-
-// Launches the staged form if the knob asks for it and the shape allows it.
-static bool launch_dwz_staged(const Ctx<double> &cx, cudaStream_t s)
-{
-    const GridT<double> &g = cx.g;
-    if (cx.z_staging != 2 || g.N3 % ZS_CH || (g.P1 * 8) % 16) return false;
-    const LinePlan lp = make_line_plan(g.N3, true, ZS_TL, cx.lanes);
-    const size_t sm = zs_smem(lp);
-    if (sm > 227 * 1024) return false;
-    DWZMaps mp;
-    if (!dwz_maps(cx, mp)) return false;
-    static size_t conf[64] = {};
-    smem_opt_in((const void *)dwz_staged_kernel, sm, conf);
-    probe_begin(cx, K_DW_Z, s);
-    dwz_staged_kernel<<<dim3((g.N1 + ZS_TL - 1) / ZS_TL, g.N2), ZS_NT, sm, s>>>(DWZ<double>{g, cx.f, ZS_TL}, mp, lp);
-    probe_end(cx, K_DW_Z, s);
-    record_launch_error(kernel_name(K_DW_Z));
-    return true;
+    launch_march(cx, DWZ<R>{cx.g, cx.f}, cx.g.N3, true, cx.g.N1, cx.g.N2, s, K_DW_Z);
 }
 
 template <class R>
 void launch_solve_du(const Ctx<R> &cx, cudaStream_t s)
 {
     const GridT<R> &g = cx.g;
-    launch_z<DUZ<R>>(cx, g.N3, g.N1, g.N2, [&](int tl) { return DUZ<R>{g, cx.f, tl}; }, s, K_DU_Z);
+    launch_du_z(cx, s);
     launch_x<DUX>(cx, g.N2, s, K_DU_X);
     launch_y<DUY<R>>(cx, g.N2, g.N1, g.N3, [&](int tl) { return DUY<R>{g, cx.f, tl}; }, s, K_DU_Y);
 }
@@ -840,7 +796,7 @@ template <class R>
 void launch_solve_dv(const Ctx<R> &cx, cudaStream_t s)
 {
     const GridT<R> &g = cx.g;
-    launch_z<DVZ<R>>(cx, g.N3, g.N1, g.N2 - 1, [&](int tl) { return DVZ<R>{g, cx.f, tl}; }, s, K_DV_Z);
+    launch_dv_z(cx, s);
     launch_x<DVX>(cx, g.N2 - 1, s, K_DV_X);
     launch_y<DVY<R>>(cx, g.N2 - 1, g.N1, g.N3, [&](int tl) { return DVY<R>{g, cx.f, tl}; }, s, K_DV_Y);
 }
@@ -849,9 +805,7 @@ template <class R>
 void launch_solve_dw(const Ctx<R> &cx, cudaStream_t s)
 {
     const GridT<R> &g = cx.g;
-    bool staged = false;
-    if constexpr (std::is_same<R, double>::value) staged = launch_dwz_staged(cx, s);
-    if (!staged) launch_z<DWZ<R>>(cx, g.N3, g.N1, g.N2, [&](int tl) { return DWZ<R>{g, cx.f, tl}; }, s, K_DW_Z);
+    launch_dw_z(cx, s);
     launch_x<DWX>(cx, g.N2, s, K_DW_X);
     launch_y<DWY<R>>(cx, g.N2, g.N1, g.N3, [&](int tl) { return DWY<R>{g, cx.f, tl}; }, s, K_DW_Y);
 }
@@ -1011,20 +965,17 @@ void launch_pseudo_update(const Ctx<R> &cx, cudaStream_t s)
 template <class R>
 void launch_momentum_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s)
 {
-    auto z = [](int ny) {
-        return [ny](const Ctx<R> &x) { return StageShape{x.g.N3, true, x.tl_strided, x.g.N1, x.g.N2 - ny}; };
-    };
     auto y = [](int ny) {
         return [ny](const Ctx<R> &x) { return StageShape{x.g.N2 - ny, false, x.tl_strided, x.g.N1, x.g.N3}; };
     };
     auto lines = [](int ny) { return [ny](const Ctx<R> &x) { return x.g.N2 - ny; }; };
-    multi_stage<DUZ<R, 1>>(cs, A, s, "du_z", z(0), [](const Ctx<R> &x, int tl) { return DUZ<R, 1>{x.g, x.f, tl}; });
+    march_stage(cs, A, s, launch_du_z<R>);
     multi_x<DUX>(cs, A, s, "du_x", lines(0));
     multi_stage<DUY<R, 1>>(cs, A, s, "du_y", y(0), [](const Ctx<R> &x, int tl) { return DUY<R, 1>{x.g, x.f, tl}; });
-    multi_stage<DVZ<R, 1>>(cs, A, s, "dv_z", z(1), [](const Ctx<R> &x, int tl) { return DVZ<R, 1>{x.g, x.f, tl}; });
+    march_stage(cs, A, s, launch_dv_z<R>);
     multi_x<DVX>(cs, A, s, "dv_x", lines(1));
     multi_stage<DVY<R, 1>>(cs, A, s, "dv_y", y(1), [](const Ctx<R> &x, int tl) { return DVY<R, 1>{x.g, x.f, tl}; });
-    multi_stage<DWZ<R, 1>>(cs, A, s, "dw_z", z(0), [](const Ctx<R> &x, int tl) { return DWZ<R, 1>{x.g, x.f, tl}; });
+    march_stage(cs, A, s, launch_dw_z<R>);
     multi_x<DWX>(cs, A, s, "dw_x", lines(0));
     multi_stage<DWY<R, 1>>(cs, A, s, "dw_y", y(0), [](const Ctx<R> &x, int tl) { return DWY<R, 1>{x.g, x.f, tl}; });
 }

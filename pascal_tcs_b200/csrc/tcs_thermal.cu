@@ -13,106 +13,143 @@
 
 namespace tcs {
 
-template <class R, int ITEM = 0>
+template <class R>
 struct ThermalZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = true;    // measured faster with qrcp
-    static constexpr int MINB = LineOcc<R>::z;
-    static constexpr int MREG = LineOcc<Real>::reg_z;
-    static constexpr int NT = LineOcc<Real>::nt_z;
-    static constexpr bool CONTIG = false;
-    static constexpr bool PAIR = LineOcc<Real>::pair_z;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr bool AHEAD = std::is_same<R, float>::value;   // FP64 inputs of two rows do not fit the registers
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt; };
-    __device__ State prepare() const { return State{R(g.scal[S_DT])}; }
-    __device__ int li(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return li(l) <= g.N1; }
+    __device__ int lines() const { return g.N1; }
+    // the rows of i that a plane needs in the column form
+    static constexpr int NROW = 7, J0 = 1;
+    static constexpr bool TABLES = false;
+    __device__ static constexpr int row_dj(int q) { constexpr int v[] = {0, -1, 1, 0, 0, 1, 0}; return v[q]; }
+    __device__ static constexpr int row_dk(int q) { constexpr int v[] = {1, 0, 0, 0, 0, 0, 1}; return v[q]; }
+    __device__ __forceinline__ const R *row_src(int q) const
+    {
+        switch (q) {
+        case 0: return f.T;
+        case 1: return f.T;
+        case 2: return f.T;
+        case 3: return f.U;
+        case 4: return f.V;
+        case 5: return f.V;
+        default: return f.W;
+        }
+    }
     // The right-hand side of :236-361 is the explicit operator minus the three
     // implicit operators applied to T.  Expanded, per direction d with faces
     // -/+ (kPP the face conductivity, ded the face gradient, u the face
     // velocity), the dK/dT products (e dkPP ded) of the explicit operator and
     // of the implicit one cancel, and so do the two dh Tc dv terms, leaving
     //   2 h rdx_d (kPP+ ded+ - kPP- ded-) - (u- ded- + u+ ded+) / 2.
-    // This build evaluates that reduced form (the same value in exact
-    // arithmetic, about half the arithmetic), except for the y direction on the
-    // two wall-adjacent planes (j = 1, N2), where the jC_BC masks and the wall
-    // terms keep the reference's full expression.  The z rows (am, ac, ap) are
-    // the reference's, dK/dT terms included.
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
-    {
-        const int i = li(l), j = 1 + vby<ITEM>(), k = r + 1;
-        const int im = i - 1, ip = i + 1, jm = j - 1, jp = j + 1, km = k - 1, kp = k + 1;
-        const PhysT<R> &p = g.ph;
-        const bool d2 = g.kdeg2 != 0;
-        const R *dx1 = g.m1.dx, *dx2 = g.m2.dx, *dx3 = g.m3.dx;
-        const R *rdx1 = g.m1.rdx, *rdx2 = g.m2.rdx, *rdx3 = g.m3.rdx;
-        const R *rdmx1 = g.m1.rdmx, *rdmx2 = g.m2.rdmx, *rdmx3 = g.m3.rdmx;
-        const long long c = ix(g, i, j, k), sj = g.P1, sk = (long long)g.P1 * g.P2;
-        const R *T = f.T;
-        const R Tc = ld(T + c), Txm = ld(T + c - 1), Txp = ld(T + c + 1);
-        const R Tym = ld(T + c - sj), Typ = ld(T + c + sj), Tzm = ld(T + c - sk), Tzp = ld(T + c + sk);
-        R Kc, dKc, Kzm, dKzm, Kzp, dKzp, irc, dirc;
-        kpp_eval(p, d2, Tc, Kc, dKc); kpp_eval(p, d2, Tzm, Kzm, dKzm); kpp_eval(p, d2, Tzp, Kzp, dKzp);
-        const R Kxm = kpp_only(p, d2, Txm), Kxp = kpp_only(p, d2, Txp);
-        rhocp_eval(p, Tc, irc, dirc);
-        const bool wall = j == 1 || j == g.N2;
-        const R Uc = ld(f.U + c), Uxp = ld(f.U + c + 1), Vc = ld(f.V + c), Vyp = ld(f.V + c + sj);
-        const R Wc = ld(f.W + c), Wzp = ld(f.W + c + sk);
-        const R h = R(0.5) * p.Ct * irc, dh = R(0.5) * p.Ct * dirc;
-        const R dedx1 = (Tc - Txm) * rdmx1[i], dedx2 = (Txp - Tc) * rdmx1[ip];
-        const R dedy3 = (Tc - Tym) * rdmx2[j], dedy4 = (Typ - Tc) * rdmx2[jp];
-        const R dedz5 = (Tc - Tzm) * rdmx3[k], dedz6 = (Tzp - Tc) * rdmx3[kp];
-        const R kPP1 = R(0.5) * rdmx1[i] * (dx1[i] * Kxm + dx1[im] * Kc), kPP2 = R(0.5) * rdmx1[ip] * (dx1[ip] * Kc + dx1[i] * Kxp);
-        const R kPP5 = R(0.5) * rdmx3[k] * (dx3[k] * Kzm + dx3[km] * Kc), kPP6 = R(0.5) * rdmx3[kp] * (dx3[kp] * Kc + dx3[k] * Kzp);
-        const R dkPP5 = R(0.5) * rdmx3[k] * (dx3[k] * dKzm + dx3[km] * dKc), dkPP6 = R(0.5) * rdmx3[kp] * (dx3[kp] * dKc + dx3[k] * dKzp);
-        const R fx = kPP2 * dedx2 - kPP1 * dedx1, fz = kPP6 * dedz6 - kPP5 * dedz5;
-        R rhs = R(2) * h * (fx * rdx1[i] + fz * rdx3[k]) - R(0.5) * (Uc * dedx1 + Uxp * dedx2) - R(0.5) * (Wc * dedz5 + Wzp * dedz6);
-        R fy;
-        if (!wall) {
-            const R Kym = kpp_only(p, d2, Tym), Kyp = kpp_only(p, d2, Typ);
-            const R kPP3 = R(0.5) * rdmx2[j] * (dx2[j] * Kym + dx2[jm] * Kc), kPP4 = R(0.5) * rdmx2[jp] * (dx2[jp] * Kc + dx2[j] * Kyp);
-            fy = kPP4 * dedy4 - kPP3 * dedy3;
-            rhs = rhs + R(2) * h * fy * rdx2[j] - R(0.5) * (Vc * dedy3 + Vyp * dedy4);
-        } else {
-            // the reference's y terms: convection, h ve2, the wall terms, minus the implicit y operator on T
-            R Kym, dKym, Kyp, dKyp;
-            kpp_eval(p, d2, Tym, Kym, dKym); kpp_eval(p, d2, Typ, Kyp, dKyp);
-            const R jem = (j == 1) ? R(0.0) : R(1.0), jep = (j == g.N2) ? R(0.0) : R(1.0);   // jC_BC(jm), jC_BC(jp)
-            const R e3 = (dx2[j] * Tym + dx2[jm] * Tc) * (R(0.5) * rdmx2[j]);
-            const R e4 = (dx2[jp] * Tc + dx2[j] * Typ) * (R(0.5) * rdmx2[jp]);
-            const R kPP3 = R(0.5) * rdmx2[j] * (dx2[j] * Kym + dx2[jm] * Kc), kPP4 = R(0.5) * rdmx2[jp] * (dx2[jp] * Kc + dx2[j] * Kyp);
-            const R dkPP3 = R(0.5) * rdmx2[j] * (dx2[j] * dKym + dx2[jm] * dKc), dkPP4 = R(0.5) * rdmx2[jp] * (dx2[jp] * dKc + dx2[j] * dKyp);
-            fy = kPP4 * dedy4 - kPP3 * dedy3;
-            const R ve2 = (kPP4 * dedy4 - kPP3 * dedy3 - e4 * dkPP4 * dedy4 + e3 * dkPP3 * dedy3) * rdx2[j];
-            R ebc_up = -R(0.25) * Vyp * rdmx2[jp] * p.Tup;
-            R ebc_dn = R(0.25) * Vc * rdmx2[j] * p.Tbt;
-            ebc_up = ebc_up + h * rdx2[j] * kPP4 * rdmx2[jp] * p.Tup + h * rdx2[j] * dkPP4 * dedy4 * p.Tup;
-            ebc_dn = ebc_dn + h * rdx2[j] * kPP3 * rdmx2[j] * p.Tbt - h * rdx2[j] * dkPP3 * dedy3 * p.Tbt;
-            const R eACJ = h * rdx2[j] * (kPP4 * rdmx2[jp] + kPP3 * rdmx2[j] - dx2[jp] * (R(0.5) * rdmx2[jp]) * dkPP4 * dedy4 * jep + dx2[jm] * (R(0.5) * rdmx2[j]) * dkPP3 * dedy3 * jem)
-                              + (R(0.25) * Vc * rdmx2[j] - R(0.25) * Vyp * rdmx2[jp]);
-            const R eAPJ = (-h * rdx2[j] * (kPP4 * rdmx2[jp] + dx2[j] * (R(0.5) * rdmx2[jp]) * dkPP4 * dedy4) + R(0.25) * Vyp * rdmx2[jp]) * jep;
-            const R eAMJ = (-h * rdx2[j] * (kPP3 * rdmx2[j] - dx2[j] * (R(0.5) * rdmx2[j]) * dkPP3 * dedy3) - R(0.25) * Vc * rdmx2[j]) * jem;
-            rhs = rhs - R(0.25) * (Vc * dedy3 + Vyp * dedy4) + h * ve2 + (R(1.0) - jem) * ebc_dn + (R(1.0) - jep) * ebc_up
-                  - (eAPJ * Typ + eACJ * Tc + eAMJ * Tym);
+    // On the two wall-adjacent planes (j = 1, N2) the jC_BC masks and the wall
+    // terms break that in y; the difference is added there.  The z rows (am,
+    // ac, ap) are the reference's, dK/dT terms included.
+    struct March {
+        R rdx1, rdx2, rdmx1, rdmx1p, rdmx2, rdmx2p, w1, w2, w3, w4, dt;   // w: weight of the neighbour at the x (1, 2) and y (3, 4) faces
+        R Tc, Kc, dKc, F, G, s, q, w, dx3m, dx3;     // the cell; the face below it
+        long long c;
+        int j;
+        __device__ __forceinline__ March(const ThermalZ &o, int line, int by, int r0)
+        {
+            const GridT<R> &g = o.g;
+            const int i = 1 + line, k = r0 + 1;
+            j = 1 + by;
+            const R d1 = ld(g.m1.dx + i), d2 = ld(g.m2.dx + j);
+            rdx1 = ld(g.m1.rdx + i); rdx2 = ld(g.m2.rdx + j);
+            rdmx1 = ld(g.m1.rdmx + i); rdmx1p = ld(g.m1.rdmx + i + 1);
+            rdmx2 = ld(g.m2.rdmx + j); rdmx2p = ld(g.m2.rdmx + j + 1);
+            w1 = R(0.5) * rdmx1 * d1; w2 = R(0.5) * rdmx1p * d1; w3 = R(0.5) * rdmx2 * d2; w4 = R(0.5) * rdmx2p * d2;
+            dt = R(g.scal[S_DT]);
+            c = ix(g, i, j, k);
+            dx3 = ld(g.m3.dx + k - 1);
+            Tc = ld(o.f.T + c - (long long)g.P1 * g.P2);
+            kpp_eval(g.ph, g.kdeg2 != 0, Tc, Kc, dKc);
+            face(o, ld(o.f.T + c), ld(o.f.W + c), ld(g.m3.dx + k), ld(g.m3.rdmx + k));
         }
-        const R dv = fx * rdx1[i] + fy * rdx2[j] + fz * rdx3[k];
-        const R eACK = h * rdx3[k] * (kPP6 * rdmx3[kp] + kPP5 * rdmx3[k] - dx3[kp] * (R(0.5) * rdmx3[kp]) * dkPP6 * dedz6 + dx3[km] * (R(0.5) * rdmx3[k]) * dkPP5 * dedz5)
-                          + (-R(0.25) * Wzp * rdmx3[kp] + R(0.25) * Wc * rdmx3[k]);
-        const R eAPK = -h * rdx3[k] * (kPP6 * rdmx3[kp] + dx3[k] * (R(0.5) * rdmx3[kp]) * dkPP6 * dedz6) + R(0.25) * Wzp * rdmx3[kp];
-        const R eAMK = -h * rdx3[k] * (kPP5 * rdmx3[k] - dx3[k] * (R(0.5) * rdmx3[k]) * dkPP5 * dedz5) - R(0.25) * Wc * rdmx3[k];
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = eACK * dt - R(0.5) * dh * dv * dt + R(1.0);
-        cf.c = eAPK * dt;
-        cf.a = eAMK * dt;
-        cf.d[0] = rhs * dt;
-        return cf;
-    }
-    __device__ void emit(int l, int r, const R *x, const State &st) const
+        // the z face between planes k-1 (Tc, Kc, dKc, dx3) and k, which becomes the current plane
+        __device__ __forceinline__ void face(const ThermalZ &o, R Tp, R Wp, R dz, R rdmx3)
+        {
+            const GridT<R> &g = o.g;
+            R Kp, dKp;
+            kpp_eval(g.ph, g.kdeg2 != 0, Tp, Kp, dKp);
+            dx3m = dx3;
+            dx3 = dz;
+            const R hm = R(0.5) * rdmx3, wm = hm * dx3m, de = (Tp - Tc) * rdmx3;
+            const R kPP = Kc + wm * (Kp - Kc), dkPP = dKc + wm * (dKp - dKc);
+            F = kPP * de;
+            G = Wp * de;
+            s = kPP * rdmx3;
+            q = hm * (dkPP * de);
+            w = R(0.25) * Wp * rdmx3;
+            Tc = Tp; Kc = Kp; dKc = dKp;
+        }
+        struct In { R Txm, Txp, Tym, Typ, Tzp, Uc, Uxp, Vc, Vyp, Wzp, rdx3, dx3, rdmx3; };
+        __device__ __forceinline__ void load(const ThermalZ &o, int r, In &n)
+        {
+            const GridT<R> &g = o.g;
+            const FieldsT<R> &f = o.f;
+            const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
+            n.Txm = ld(f.T + c - 1); n.Txp = ld(f.T + c + 1); n.Tym = ld(f.T + c - sj); n.Typ = ld(f.T + c + sj); n.Tzp = ld(f.T + c + sk);
+            n.Uc = ld(f.U + c); n.Uxp = ld(f.U + c + 1); n.Vc = ld(f.V + c); n.Vyp = ld(f.V + c + sj); n.Wzp = ld(f.W + c + sk);
+            n.rdx3 = ld(g.m3.rdx + r + 1); n.dx3 = ld(g.m3.dx + r + 2); n.rdmx3 = ld(g.m3.rdmx + r + 2);
+            c += sk;
+        }
+        // the same values from the ring: slot a holds plane k's rows, b the plane below's
+        __device__ __forceinline__ void fill(const ThermalZ &o, int r, In &n, const double *a, const double *b, int w, int l)
+        {
+            const GridT<R> &g = o.g;
+            const int s = w + 2;
+            a += l + 1; b += l + 1;
+            n.Txm = b[-1]; n.Txp = b[1]; n.Tzp = a[0]; n.Tym = a[s]; n.Typ = a[2 * s];
+            n.Uc = a[3 * s]; n.Uxp = a[3 * s + 1]; n.Vc = a[4 * s]; n.Vyp = a[5 * s]; n.Wzp = a[6 * s];
+            n.rdx3 = ld(g.m3.rdx + r + 1); n.dx3 = ld(g.m3.dx + r + 2); n.rdmx3 = ld(g.m3.rdmx + r + 2);
+        }
+        __device__ __forceinline__ void row(const ThermalZ &o, int r, const In &n, double &a, double &b, double &cc, double *d)
+        {
+            const GridT<R> &g = o.g;
+            const PhysT<R> &p = g.ph;
+            const bool d2 = g.kdeg2 != 0;
+            const R Txm = n.Txm, Txp = n.Txp, Tym = n.Tym, Typ = n.Typ, Tzp = n.Tzp, Uc = n.Uc, Uxp = n.Uxp, Vc = n.Vc, Vyp = n.Vyp, Wzp = n.Wzp;
+            const R rdx3 = n.rdx3;
+            const R T0 = Tc, K0 = Kc, dK0 = dKc, F5 = F, G5 = G, s5 = s, q5 = q, w5 = w, d3m = dx3m, d3 = dx3;
+            R irc, dirc;
+            rhocp_eval(p, T0, irc, dirc);
+            const R h = R(0.5) * p.Ct * irc, dh = R(0.5) * p.Ct * dirc;
+            face(o, Tzp, Wzp, n.dx3, n.rdmx3);
+            const R Kxm = kpp_only(p, d2, Txm), Kxp = kpp_only(p, d2, Txp);
+            R Kym, Kyp, dKym = R(0), dKyp = R(0);
+            const bool wall = j == 1 || j == g.N2;
+            if (wall) { kpp_eval(p, d2, Tym, Kym, dKym); kpp_eval(p, d2, Typ, Kyp, dKyp); }
+            else { Kym = kpp_only(p, d2, Tym); Kyp = kpp_only(p, d2, Typ); }
+            const R dx1 = (T0 - Txm) * rdmx1, dx2 = (Txp - T0) * rdmx1p, dy3 = (T0 - Tym) * rdmx2, dy4 = (Typ - T0) * rdmx2p;
+            const R kPP3 = K0 + w3 * (Kym - K0), kPP4 = K0 + w4 * (Kyp - K0);
+            const R fx = (K0 + w2 * (Kxp - K0)) * dx2 - (K0 + w1 * (Kxm - K0)) * dx1, fy = kPP4 * dy4 - kPP3 * dy3;
+            const R dv = fx * rdx1 + fy * rdx2 + (F - F5) * rdx3;
+            R rhs = R(2) * h * dv - R(0.5) * ((Uc * dx1 + Uxp * dx2) + (Vc * dy3 + Vyp * dy4) + (G5 + G));
+            if (wall) {
+                const R h2 = h * rdx2;
+                if (j == 1) {
+                    const R qd = (dK0 + w3 * (dKym - dK0)) * dy3, am = -h2 * (kPP3 * rdmx2 - w3 * qd) - R(0.25) * Vc * rdmx2;
+                    rhs = rhs + am * Tym + h2 * (R(1) - w3) * qd * T0 + (R(0.25) * Vc * rdmx2 + h2 * (kPP3 * rdmx2 - qd)) * p.Tbt;
+                }
+                if (j == g.N2) {
+                    const R qd = (dK0 + w4 * (dKyp - dK0)) * dy4, ap = -h2 * (kPP4 * rdmx2p + w4 * qd) + R(0.25) * Vyp * rdmx2p;
+                    rhs = rhs + ap * Typ - h2 * (R(1) - w4) * qd * T0 + (h2 * (kPP4 * rdmx2p + qd) - R(0.25) * Vyp * rdmx2p) * p.Tup;
+                }
+            }
+            const R h3 = h * rdx3;
+            a = (-h3 * (s5 - d3 * q5) - w5) * dt;
+            cc = (w - h3 * (s + d3 * q)) * dt;
+            b = 1.0 + (double)((h3 * (s + s5 - dx3 * q + d3m * q5) + (w5 - w) - R(0.5) * dh * dv) * dt);
+            d[0] = rhs * dt;
+        }
+    };
+    __device__ __forceinline__ void emit(int line, int by, int r, const double *x) const
     {
-        f.scr[ix(g, li(l), 1 + vby<ITEM>(), r + 1)] = x[0];
+        f.scr[ix(g, 1 + line, 1 + by, r + 1)] = R(x[0]);
     }
 };
 
@@ -243,10 +280,16 @@ struct ThermalY {
 };
 
 template <class R>
+static void launch_thermal_z(const Ctx<R> &cx, cudaStream_t s)
+{
+    launch_march(cx, ThermalZ<R>{cx.g, cx.f}, cx.g.N3, true, cx.g.N1, cx.g.N2, s, K_THERMAL_Z);
+}
+
+template <class R>
 void launch_thermal(const Ctx<R> &cx, cudaStream_t s)
 {
     const GridT<R> &g = cx.g;
-    launch_z<ThermalZ<R>>(cx, g.N3, g.N1, g.N2, [&](int tl) { return ThermalZ<R>{g, cx.f, tl}; }, s, K_THERMAL_Z);
+    launch_thermal_z(cx, s);
     launch_x<ThermalX>(cx, g.N2, s, K_THERMAL_X);
     launch_y<ThermalY<R>>(cx, g.N2, g.N1, g.N3, [&](int tl) { return ThermalY<R>{g, cx.f, tl}; }, s, K_THERMAL_Y);
 }
@@ -255,9 +298,7 @@ void launch_thermal(const Ctx<R> &cx, cudaStream_t s)
 template <class R>
 void launch_thermal_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s)
 {
-    multi_stage<ThermalZ<R, 1>>(cs, A, s, "thermal_z",
-        [](const Ctx<R> &x) { return StageShape{x.g.N3, true, x.tl_strided, x.g.N1, x.g.N2}; },
-        [](const Ctx<R> &x, int tl) { return ThermalZ<R, 1>{x.g, x.f, tl}; });
+    march_stage(cs, A, s, launch_thermal_z<R>);
     multi_x<ThermalX>(cs, A, s, "thermal_x", [](const Ctx<R> &x) { return x.g.N2; });
     multi_stage<ThermalY<R, 1>>(cs, A, s, "thermal_y",
         [](const Ctx<R> &x) { return StageShape{x.g.N2, false, x.tl_strided, x.g.N1, x.g.N3}; },

@@ -1,13 +1,11 @@
-// tcs_tma.cuh -- tensor-memory-accelerator (TMA) tile loads into shared
+// tcs_tma.cuh -- bulk asynchronous copies of this GPU's own memory into shared
 // memory for one thread block, with mbarrier completion, for sm_100a.
 //
-// Only plain tiled loads of this GPU's own memory are issued (one CTA, no
-// cluster multicast).  Every wait on an mbarrier is bounded: a wait that runs
-// out returns false, and the caller records the failure and leaves the kernel
-// after bounded waits for its other copies in flight.
+// Every wait on an mbarrier is bounded: a wait that runs out returns false, and
+// the caller records the failure and leaves the kernel after bounded waits for
+// its other copies in flight.
 #pragma once
 
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -20,11 +18,12 @@ __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 
-// Makes the initialised barriers visible to the asynchronous (TMA) proxy.
+// Makes the initialised barriers visible to the asynchronous proxy.
 __device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
-// Orders this thread's earlier shared-memory accesses before later
-// asynchronous-proxy accesses (a TMA write into a buffer the block has read).
+// Orders this thread's earlier shared-memory accesses (and, after a barrier,
+// the block's) before later asynchronous-proxy accesses: a bulk write into a
+// buffer the block has read.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes)
@@ -53,12 +52,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int li
     return false;
 }
 
-// A 3-D tiled load of the box at (x, y, z) of the tensor map into dst
-// (128-byte aligned shared memory); completion is counted on bar in bytes.
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y, int z)
+// Copies bytes (a multiple of 16) from src to dst (both 16-byte aligned);
+// completion is counted on bar in bytes.
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
 {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
 

@@ -1,0 +1,41 @@
+"""The marching solvers of the strided line sweeps at the edges of their shapes
+(needs a B200): few rows, lines of segments of unequal length, part-filled blocks,
+more than 32 segments, the column form of long FP64 lines and its fallback on an
+odd N1, against the oracle.  The diffusion number of the z rows is above 0.1 in
+the long cases, so a segment's coupling to its neighbour lives for tens of rows.
+
+Bars: FP64 the parity bar of the other oracle tests (1e-10); FP32-mixed storage
+keeps 6e-8 of each field per step, U, T and P within 1e-5 over two steps."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [
+    (4, 4, 4),        # one segment pair of 2 rows, 16-line blocks part-filled
+    (20, 7, 25),      # segments of 6 and 7 rows
+    (18, 9, 384),     # 32 segments of 12 rows
+    (36, 6, 400),     # the column form, block width 64 part-filled
+    (150, 5, 405),    # the column form, segments of 203 and 202 rows, a part-filled last block
+    (45, 6, 400),     # odd N1: rows of i are not 16-byte aligned, no column form
+    (45, 5, 640),     # 64 segments: reduced systems through shared memory
+]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", SHAPES)
+def test_strided_sweeps_match_oracle(n, precision):
+    import pascal_tcs_b200 as P
+    from oracle import oracle as O
+
+    cfg = dict(n1m=n[0], n2m=n[1], n3m=n[2], property_set=0, Pr=0.71, Ra=1e4, dtStart=2e-3, fixed_dt=1, seed=11,
+               noise_amp=0.05, gamma2=1.2)
+    g = P.Solver(precision=precision, **cfg)
+    o = O.Oracle(**{k: v for k, v in g.config.items() if k not in ("device", "precision")})
+    g.step(2)
+    o.step(2)
+    for f in ("T", "U", "V", "W", "P") if precision == 0 else ("T", "U", "P"):
+        a, b = g.get(f), o.get(f)
+        err = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300)
+        assert np.all(np.isfinite(a)) and err <= (1e-10 if precision == 0 else 1e-5), (f, err)
+    g.close()
