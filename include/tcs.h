@@ -232,42 +232,25 @@ const char *tcs_timer_name(int timer);
 int tcs_bounds_checked(void);
 int tcs_bounds_violations(tcs_ctx *ctx, double *count);
 int tcs_set_use_graph(tcs_ctx *ctx, int on);
-/* launch-shape knobs (powers of two): lines per thread block of the y lines,
- * the contiguous (x) and the modal line solvers and of the x and z FFTs, and
- * the most lanes (partitions) a tridiagonal line is split over (32: no bound for
- * the z sweeps, whose segments also follow the line's length).  A line-solver
+/* launch-shape knobs (powers of two): lines per thread block of the
+ * contiguous (x) and the modal line solvers and of the x and z FFTs, and the
+ * most lanes (partitions) a tridiagonal line is split over (32: no bound for
+ * the y and z sweeps, whose segments follow the line's length).  A line-solver
  * value is an upper bound: each launch runs the largest power of two up to it
  * whose blocks fit the SM's shared memory at the family's blocks per SM; a
- * value no single block could hold is refused (TCS_ERR_ARG).  The z sweeps
- * choose their own lines per block.
- * TCS_TUNE_LONG_LINES: 4 runs long y lines as one block per SM (the same
- * warps, lines fitted to 132 KiB of shared memory so that L1 keeps 124 KiB)
- * when the usual blocks would leave under 60 KiB of L1 or halve their lines; 1
- * and 2 (default) do not.
- * TCS_TUNE_Y_SOLVER picks the tridiagonal solver of the non-cyclic strided
- * lines: 1 the partitioned solver that every sweep uses (default: modified
- * Thomas per lane with a parallel reduced-system solve, pascal_tdma.f90:
- * 487-578; in the FP32-mixed form FP32 elimination with one FP64-residual
- * refinement pass); 2 the plain Thomas elimination with one line per thread
- * (tdmas.f90:27-50) in FP64 for the y sweeps (rows built in the field type);
- * 4 the same for the modal pressure solves too.  2 and 4 keep c' and d' in a
- * scratch buffer that setting the knob allocates ((1 + right-hand sides) x
- * rows x lines doubles: 2.1 GB for the y sweeps and 2.4 GB for the modal
- * solves at 512^3) and setting 1 frees.  Measured on B200: the one-line form
- * is faster for the y sweeps at 512^3 and slower at 256^3, where 65536 lines
- * leave the SMs short of threads; for the modal solves it is slower at both
- * sizes (its scratch traffic is 1.5x the spectrum's).
+ * value no single block could hold is refused (TCS_ERR_ARG).
+ * TCS_TUNE_TL_STRIDED, TCS_TUNE_LONG_LINES (1, 2, 4), TCS_TUNE_Y_SOLVER (1, 2,
+ * 4) and TCS_TUNE_Z_STAGING (1, 2) chose between forms of the y and z sweeps
+ * that one solver has replaced.  Their values are checked, kept and returned as
+ * before, without effect.
  * TCS_TUNE_IFFT_LINES_X: lines per block of the inverse x transform
  * (TCS_TUNE_FFT_LINES_X sets those of the pressure right-hand side and its
  * forward x transform).
  * TCS_TUNE_MIXED_ROWS (FP32-mixed form; no effect in the FP64 form): 1 the x
  * sweeps eliminate their FP32 rows in FP32 with one FP64-residual refinement
  * pass (default); 2, 4 and 8 they eliminate their FP32-built rows in FP64
- * instead (no refinement pass; the solution is rounded once to FP32).  The z
- * sweeps always eliminate in FP64.
- * TCS_TUNE_Z_STAGING: 1 or 2; kept for programs that set it, without effect
- * since the z sweeps have one staged form (2 is refused, TCS_ERR_ARG, unless the form is FP64, N3 a multiple of
- * 64 and N1 even). */
+ * instead (no refinement pass; the solution is rounded once to FP32).  The y
+ * and z sweeps always eliminate in FP64. */
 enum { TCS_TUNE_TL_STRIDED = 0, TCS_TUNE_TL_CONTIG, TCS_TUNE_TL_MODAL, TCS_TUNE_FFT_LINES_X, TCS_TUNE_FFT_LINES_Z,
        TCS_TUNE_LANES, TCS_TUNE_LONG_LINES, TCS_TUNE_Y_SOLVER, TCS_TUNE_IFFT_LINES_X, TCS_TUNE_MIXED_ROWS,
        TCS_TUNE_Z_STAGING, TCS_TUNE_COUNT };

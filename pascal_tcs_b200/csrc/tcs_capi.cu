@@ -567,7 +567,6 @@ int tcs_create(const tcs_config *cfg, tcs_ctx **out)
     c->cx.lanes = 32;
     c->cx.long_lines = 2;
     c->cx.y_solver = 1;
-    c->cx.thomas_scr = nullptr;
     c->cx.mixed_rows = 1;
     c->cx.z_staging = 1;
     c->cx.probe = &c->probe;
@@ -637,7 +636,6 @@ int tcs_destroy(tcs_ctx *c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (auto &ge : c->graphs) cudaGraphExecDestroy(ge.exec);
     for (void *p : c->allocs) cudaFree(p);
-    if (c->cx.thomas_scr) cudaFree(c->cx.thomas_scr);
     if (c->io_host) cudaFreeHost(c->io_host);
     for (auto &v : c->probe.rec) for (auto &pr : v) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
     for (cudaEvent_t e : c->probe.pool) cudaEventDestroy(e);
@@ -997,31 +995,11 @@ int tcs_set_tuning(tcs_ctx *c, int knob, int value)
         if (value < 2 || value > 32) return set_err(TCS_ERR_ARG, "lanes per line must be 2..32");
         x.lanes = value; break;
     case TCS_TUNE_LONG_LINES:
-        if (value > 4) return set_err(TCS_ERR_ARG, "long-line form: 1, 2 never, 4 the y sweeps");
+        if (value > 4) return set_err(TCS_ERR_ARG, "long lines: 1, 2 or 4");
         x.long_lines = value; break;
-    case TCS_TUNE_Y_SOLVER: {
-        if (value > 4) return set_err(TCS_ERR_ARG, "y solver: 1 partitioned, 2 one line per thread (y sweeps), 4 also the modal solves");
-        // c', d' of every line of the largest one-line-per-thread launch: the y
-        // sweeps (one right-hand side) and, with 4, the modal solves (two)
-        const size_t ny = value >= 2 ? thomas_words(g.N2, g.N1, g.N3, 1) : 0;
-        const size_t words = std::max(ny, value == 4 ? thomas_words(g.N2, x.h1p, g.N3, 2) : (size_t)0);
-        if (x.thomas_scr) {
-            cudaStreamSynchronize(c->stream);
-            cudaFree(x.thomas_scr);
-            x.thomas_scr = nullptr;
-        }
-        if (words) {
-            void *q = nullptr;
-            const cudaError_t ce = cudaMalloc(&q, words * sizeof(double));
-            if (ce != cudaSuccess) {
-                cudaGetLastError();
-                x.y_solver = 1;
-                sync_shapes(c);
-                return set_err(TCS_ERR_NOMEM, std::string("y solver scratch: ") + cudaGetErrorString(ce));
-            }
-            x.thomas_scr = (double *)q;
-        }
-        x.y_solver = value; break; }
+    case TCS_TUNE_Y_SOLVER:
+        if (value > 4) return set_err(TCS_ERR_ARG, "y solver: 1, 2 or 4");
+        x.y_solver = value; break;
     default: return set_err(TCS_ERR_ARG, "unknown tuning knob");
     }
     sync_shapes(c);
@@ -1717,6 +1695,8 @@ extern "C" int tcs_autotune(tcs_ctx *c, int trial_steps, const char *cache_path,
     if ((r = tune_trial(c, trial_steps, &best_ms))) return r;
     static const int cand[] = {1, 2, 4, 8, 16, 32};
     for (int k = 0; k < TCS_TUNE_COUNT; k++) {
+        if (k == TCS_TUNE_TL_STRIDED || k == TCS_TUNE_LONG_LINES || k == TCS_TUNE_Y_SOLVER || k == TCS_TUNE_Z_STAGING)
+            continue;                                                 // without effect: nothing to time
         for (int v : cand) {
             if (v == best[k]) continue;
             if (tcs_set_tuning(c, k, v) != TCS_OK) continue;          // not valid for this shape

@@ -706,25 +706,23 @@ struct Refine { static constexpr bool on = std::is_same<R, float>::value; };
 // Blocks per SM a line-solver family is compiled for (each Prob's MINB; the
 // register budget is 65536 / (NT MINB), and fit_tl sizes the lines per block
 // to the matching shared-memory share).  Measured on B200 at 256^3: the FP64 x
-// and y sweeps run fastest at 4 blocks (64 registers, no spills); the refined FP32
-// rows need 28 B each, so the FP32 y sweeps and the modal solves run best at 3
-// blocks of 256 threads and the FP32 x sweeps at 6 blocks of 128.
+// sweeps run fastest at 4 blocks (64 registers, no spills), the modal solves at 3
+// blocks of 256 threads and the FP32 x sweeps, whose refined rows need 28 B each,
+// at 6 blocks of 128.
 template <class R>
 struct LineOcc {
     static constexpr bool f32 = std::is_same<R, float>::value;
     static constexpr int x = f32 ? 6 : 4;
-    static constexpr int y = f32 ? 3 : 4;
     static constexpr int modal = 3;
     // rows per lane solved in registers (0: in shared memory), per family:
-    // wherever the registers allow it without spills (not the FP64 x/y sweeps
+    // wherever the registers allow it without spills (not the FP64 x sweeps
     // at 64 registers, nor the two-right-hand-side modal solves at 80)
     static constexpr int reg_x = f32 ? 8 : 0;
-    static constexpr int reg_y = f32 ? 8 : 0;
     static constexpr int reg_modal = 0;
     // threads per block, per family (the FP32 x sweeps run best as 128-thread
     // blocks of 4 lines: the refined rows fill shared memory, and smaller
     // blocks wait less at their barriers)
-    static constexpr int nt_x = f32 ? 128 : 256, nt_y = 256, nt_modal = 256;
+    static constexpr int nt_x = f32 ? 128 : 256, nt_modal = 256;
     // the x sweeps' wide shape, for lines too long to fit 4 per 128-thread block
     static constexpr int xw = f32 ? 3 : 4, nt_xw = 256, reg_xw = reg_x;
 };
@@ -885,72 +883,6 @@ template <class Prob>
 __global__ void __launch_bounds__(Prob::NT, Prob::MINB) line_solve_kernel(Prob prob, LinePlan lp)
 {
     line_block(prob, lp);
-}
-
-// Blocks per SM the one-line-per-thread kernel is compiled for
-// (Prob::THOMAS_MINB; default 8, i.e. 64 registers).  Measured on B200 at
-// 512^3: the y sweeps 4-18% faster at 64 registers than uncapped (80-96), and
-// slower at 48 (spills).
-template <class P, class = void>
-struct ThomasMinB { static constexpr int v = 8; };
-template <class P>
-struct ThomasMinB<P, std::void_t<decltype(P::THOMAS_MINB)>> { static constexpr int v = P::THOMAS_MINB; };
-
-// One line per thread: the plain Thomas elimination of a non-cyclic line in
-// FP64 (the sequential elimination of tdma_single and tdma_many,
-// PaScaL_TDMA/src/tdmas.f90:27-50 and 113-146), for the strided y lines and
-// the modal solves.  A block of THOMAS_TL threads takes THOMAS_TL consecutive
-// lines (the problem's TL is THOMAS_TL), thread l line l.  The forward sweep
-// builds each row with the problem's own build, keeps c' and d' of the current
-// row in registers and stores them for the back substitution in
-// scr[row][line] (consecutive threads, consecutive words: every store and load
-// of a warp is coalesced); the back substitution emits the rows from the last
-// to the first.  No shared memory and no barrier: the build's loads of the
-// next rows overlap the elimination of the current one.  scr holds
-// (1 + NRHS) x n x (all lines of the grid) doubles.  Rows built in FP32 (the
-// FP32-mixed form) are eliminated in FP64 and the solution rounded once when
-// it is emitted, which stands in for the FP32 elimination and its FP64-residual
-// refinement pass.
-template <class Prob>
-__global__ void __launch_bounds__(128, ThomasMinB<Prob>::v) thomas_line_kernel(Prob prob, int n, double *__restrict__ scr)
-{
-    using R = typename Prob::Real;
-    constexpr int NR = Prob::NRHS;
-    if (prob.skip()) return;
-    const int l = threadIdx.x;
-    if (!prob.line_ok(l)) return;
-    const typename Prob::State st = prob.prepare();
-    const long long nl = (long long)gridDim.x * gridDim.y * blockDim.x;
-    const long long me = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + l;
-    double *const sc = scr + me, *const sd = scr + nl * n + me;
-    double cp = 0.0, dp[NR];
-#pragma unroll
-    for (int q = 0; q < NR; q++) dp[q] = 0.0;
-#pragma unroll 2
-    for (int r = 0; r < n; r++) {
-        const Coef<R, NR> cf = prob.build(l, r, st);
-        const double a = r ? (double)cf.a : 0.0;
-        const double m = rcp_of<FastRcp<Prob>::on>((double)cf.b - a * cp);
-        cp = (double)cf.c * m;
-#pragma unroll
-        for (int q = 0; q < NR; q++) dp[q] = ((double)cf.d[q] - a * dp[q]) * m;
-        if (r < n - 1) {
-            sc[(long long)r * nl] = cp;
-#pragma unroll
-            for (int q = 0; q < NR; q++) sd[((long long)r * NR + q) * nl] = dp[q];
-        }
-    }
-    double x[NR];
-    R xr[NR];
-#pragma unroll
-    for (int q = 0; q < NR; q++) { x[q] = dp[q]; xr[q] = R(x[q]); }
-    prob.emit(l, n - 1, xr, st);
-    for (int r = n - 2; r >= 0; r--) {
-        const double c = sc[(long long)r * nl];
-#pragma unroll
-        for (int q = 0; q < NR; q++) { x[q] = sd[((long long)r * NR + q) * nl] - c * x[q]; xr[q] = R(x[q]); }
-        prob.emit(l, r, xr, st);
-    }
 }
 
 // The parameters of a multi-case line launch: the problems and plans of up to

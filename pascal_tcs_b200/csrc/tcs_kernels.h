@@ -77,11 +77,9 @@ struct Shapes {
     int fft_lines_x, fft_lines_z;
     int ifft_lines_x;                            // lines per block of the inverse x transform
     int lanes;                                   // at most this many partitions (lanes) per line
-    int long_lines;                              // one-block-per-SM form of long y lines: 4; 1, 2 never
-    int y_solver;                                // y lines: 1 partitioned (line_block), 2 one line per thread for the y sweeps, 4 also the modal solves
-    double *thomas_scr;                          // c', d' of the one-line-per-thread solver (null unless y_solver asks for it)
+    int long_lines, y_solver;                    // accepted and kept; one solver runs the strided lines
     int mixed_rows;                              // FP32-mixed form: 1 FP32 elimination + refinement in the x sweeps, 2, 4, 8 FP64 rows there
-    int z_staging;                               // 1 or 2 (FP64, N3 a multiple of 64, even N1): accepted, no effect
+    int z_staging;                               // likewise
     FFTPlan fp1, fp3;
     FFTPlan fp1u;                                // N1 with radices up to 8 (the inverse x transform's one-radix form)
     int h1p;
@@ -110,7 +108,7 @@ inline size_t line_smem(const LinePlan &lp)
 }
 
 // The plan of a line problem: make_line_plan's partitions, and for the
-// non-cyclic strided problems (the y sweeps and the modal solves) a
+// non-cyclic strided problems (the modal solves) a
 // line stride LS chosen for the build and the emission, where one warp
 // touches TL lines x 32/TL rows: LS = banks/TL (mod banks), banks = 32
 // four-byte words (FP32 rows) or 16 eight-byte words per half-warp (FP64
@@ -130,21 +128,13 @@ inline LinePlan plan_for(int n, bool cyclic, int tl, int pmax)
     return lp;
 }
 
-// The shared memory (KiB) a line family lets its blocks take per SM: all of
-// it (228 KiB) by default, less for the one-block-per-SM form of long lines
-// (LongLines), whose stencil builds need the L1 that the rest leaves.
-template <class P, class = void>
-struct SmemKiB { static constexpr int v = 228; };
-template <class P>
-struct SmemKiB<P, std::void_t<decltype(P::SMEM_KIB)>> { static constexpr int v = P::SMEM_KIB; };
-
 // Lines per block: the requested count, halved until MINB blocks fit in the
-// family's share of the SM's shared memory (1 KB reserved per block);
-// extra: static shared memory the kernel adds per block.
+// SM's shared memory (228 KiB, 1 KB reserved per block); extra: static shared
+// memory the kernel adds per block.
 template <class Prob>
 inline int fit_tl(int n, bool cyclic, int want, int pmax, size_t extra = 0)
 {
-    const size_t budget = (size_t)SmemKiB<Prob>::v * 1024 / Prob::MINB - 1024 - extra;
+    const size_t budget = (size_t)228 * 1024 / Prob::MINB - 1024 - extra;
     int tl = want;
     while (tl > 1 && line_smem<Prob>(plan_for<Prob>(n, cyclic, tl, pmax)) > budget) tl /= 2;
     return tl;
@@ -176,48 +166,6 @@ inline void launch_lines(const Prob &p, const LinePlan &lp, dim3 grid, cudaStrea
     record_launch_error(kernel_name(kid));
 }
 
-// The SM's unified L1/shared-memory configurations: the shared-memory share
-// (KiB) the driver picks for a given demand per SM; the L1 keeps the rest of
-// the 256 KiB.
-inline int smem_config_kib(size_t per_sm_bytes)
-{
-    static const int cfg[] = {0, 8, 16, 32, 64, 100, 132, 164, 196, 228};
-    for (int c : cfg)
-        if ((size_t)c * 1024 >= per_sm_bytes) return c;
-    return 228;
-}
-
-// A line family in one block per SM: the same warps per SM (NT x MINB threads
-// in one block, so the same registers per thread) with its lines per block
-// fitted to 132 KiB of shared memory, which leaves the SM 124 KiB of L1.
-template <class P>
-struct LongLines : P {
-    static constexpr int NT = P::NT * P::MINB;
-    static constexpr int MINB = 1;
-    static constexpr int SMEM_KIB = 132;
-};
-
-// A strided line sweep (y lines: TL consecutive i per block, gy block rows).  With allow_long, the one-block-per-SM form runs instead where the
-// usual form would leave less than 60 KiB of L1 or would have to halve its
-// lines per block.  make(tl) builds the problem for tl lines per block.
-template <class P, class Make>
-inline void launch_strided(const Shapes &cx, int n, bool cyclic, int nlines, int gy, Make make, cudaStream_t s, int kid,
-                           bool allow_long)
-{
-    const LinePlan a = plan_for<P>(n, cyclic, fit_tl<P>(n, cyclic, cx.tl_strided, cx.lanes), cx.lanes);
-    if (allow_long) {
-        using L = LongLines<P>;
-        const LinePlan b = plan_for<L>(n, cyclic, fit_tl<L>(n, cyclic, cx.tl_strided, cx.lanes), cx.lanes);
-        const size_t per_sm = (size_t)P::MINB * (line_smem<P>(a) + 1024);
-        const int l1_kib = 256 - smem_config_kib(per_sm);
-        if (b.TL > a.TL || l1_kib < 60) {
-            launch_lines(L{make(b.TL)}, b, dim3((nlines + b.TL - 1) / b.TL, gy), s, kid, cx);
-            return;
-        }
-    }
-    launch_lines(make(a.TL), a, dim3((nlines + a.TL - 1) / a.TL, gy), s, kid, cx);
-}
-
 // An FP32 x sweep whose rows are eliminated in FP64 (Shapes::mixed_rows): the
 // problem's own build in the field type, its coefficients widened to FP64 in
 // shared memory, the partitioned solve in FP64 without the refinement pass
@@ -247,43 +195,27 @@ struct FP64Rows : P {
     }
 };
 
-// Lines per block of the one-line-per-thread solver (thomas_line_kernel).
-constexpr int THOMAS_TL = 128;
-
-// Doubles of c', d' scratch the one-line-per-thread solver needs for nlines
-// lines of n rows in gy block rows with nrhs right-hand sides.
-inline size_t thomas_words(int n, int nlines, int gy, int nrhs)
-{
-    return (size_t)(1 + nrhs) * n * ((size_t)(nlines + THOMAS_TL - 1) / THOMAS_TL) * THOMAS_TL * gy;
-}
-
-template <class P, class Make>
-inline void launch_thomas(const Shapes &cx, int n, int nlines, int gy, Make make, cudaStream_t s, int kid)
-{
-    probe_begin(cx, kid, s);
-    thomas_line_kernel<P><<<dim3((nlines + THOMAS_TL - 1) / THOMAS_TL, gy), THOMAS_TL, 0, s>>>(make(THOMAS_TL), n, cx.thomas_scr);
-    probe_end(cx, kid, s);
-    record_launch_error(kernel_name(kid));
-}
-
 // The shape of a marching sweep (march_block) of `lines` lines in all: TI lines
 // and NS segments of every line per block.  Rows per segment, m = n / NS: at
-// most 12, because the parked rows (24 B each, 512 threads per SM) then leave L1
-// room for the stencil's x neighbours and tables (measured in FP64, ps per cell
-// of dw_z: m = 16 at 256^3 36, m = 8 24; m = 12 at 192^3 24, m = 6 28), and at least
-// 4, because every segment loads its first plane twice; with few lines, short
-// segments fill the SMs.  Lines too long for 16 of them at 12 rows a segment keep
-// 512 threads and take more rows.
-inline MarchPlan march_plan(int n, bool cyclic, int nrhs, int lanes, long long lines)
+// most P::ROWS, and at least 4, because every segment loads its first plane
+// twice; with few lines, short segments fill the SMs.  P::ROWS is 12 for the z
+// sweeps: the parked rows (24 B each, 512 threads per SM) then leave L1 room for
+// the stencil's x neighbours and tables (measured in FP64, ps per cell of dw_z:
+// m = 16 at 256^3 36, m = 8 22; m = 12 at 192^3 23, m = 6 28).  The y sweeps read
+// little through L1 and run best with 16 rows in two blocks per SM (256^3, ps per
+// cell of du_y: m = 16 12.0, m = 8 14.2; FP32-mixed 9.7 and 13.0).  Lines too long
+// for 16 of them to fit keep 512 threads and take more rows.
+template <class P>
+inline MarchPlan march_plan(int n, bool cyclic, int lanes, long long lines)
 {
     MarchPlan mp;
     mp.n = n; mp.cyclic = cyclic ? 1 : 0;
     mp.lgNS = 1;
     const int cap = lanes < 32 ? lanes : 256;
     auto more = [&]() { return (2 << mp.lgNS) <= cap && (n >> (mp.lgNS + 1)) >= 4; };
-    while (more() && mp.lgNS < 5 && (n > (12 << mp.lgNS) || (lines << mp.lgNS) < 131072)) mp.lgNS++;
+    while (more() && mp.lgNS < 5 && (n > (P::ROWS << mp.lgNS) || (lines << mp.lgNS) < 131072)) mp.lgNS++;
     mp.lgTI = 4;
-    auto words = [&]() { return march_words(n, 1 << mp.lgNS, 1 << mp.lgTI, nrhs) * sizeof(double); };
+    auto words = [&]() { return march_words(n, 1 << mp.lgNS, 1 << mp.lgTI, P::NRHS) * sizeof(double); };
     while (mp.lgTI > 0 && words() > 227 * 1024) {
         mp.lgTI--;
         if (more() && mp.lgNS + mp.lgTI < 9) mp.lgNS++;
@@ -338,25 +270,11 @@ inline bool launch_column(const Shapes &cx, const P &prob, int n, int nlines, in
 template <class P>
 inline void launch_march(const Shapes &cx, const P &prob, int n, bool cyclic, int nlines, int gy, cudaStream_t s, int kid)
 {
-    if constexpr (std::is_same<typename P::Real, double>::value)
-        if (cyclic && launch_column(cx, prob, n, nlines, gy, s, kid)) return;
-    const MarchPlan mp = march_plan(n, cyclic, P::NRHS, cx.lanes, (long long)nlines * gy);
+    if constexpr (Streams<P>::on)
+        if (launch_column(cx, prob, n, nlines, gy, s, kid)) return;
+    const MarchPlan mp = march_plan<P>(n, cyclic, cx.lanes, (long long)nlines * gy);
     if (mp.lgTI + mp.lgNS > 8) launch_march_nt<512>(cx, prob, mp, nlines, gy, s, kid);
     else launch_march_nt<256>(cx, prob, mp, nlines, gy, s, kid);
-}
-
-// A y sweep (non-cyclic strided lines, nlines x gy of n rows): the
-// one-line-per-thread solver when the knob asks for it (y_solver 2 or 4,
-// scratch allocated), else the partitioned line solver, in the
-// one-block-per-SM form where long_lines asks for it for the y sweeps.
-template <class P, class Make>
-inline void launch_y(const Shapes &cx, int n, int nlines, int gy, Make make, cudaStream_t s, int kid)
-{
-    if (cx.y_solver >= 2 && cx.thomas_scr) {
-        launch_thomas<P>(cx, n, nlines, gy, make, s, kid);
-        return;
-    }
-    launch_strided<P>(cx, n, false, nlines, gy, make, s, kid, cx.long_lines >= 4);
 }
 
 // ---------------------------------------------------------------------------

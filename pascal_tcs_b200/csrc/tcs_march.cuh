@@ -137,19 +137,47 @@ __device__ __forceinline__ void march_reduce(double *red, int lgNS, int TP, bool
     __syncthreads();
 }
 
+// Stores of a line's rows from the last to the first: into the sweep scratch, ...
+template <class R>
+struct ScratchOut {
+    R *p;
+    long long step;
+    __device__ __forceinline__ ScratchOut(const GridT<R> &g, R *a, int i, int j, int k, long long st) : p(a + ix(g, i, j, k)), step(st) {}
+    __device__ __forceinline__ void put(R v) { *p = v; p -= step; }
+};
+// ... or into a field with its periodic images, along y (see store_periodic).
+template <class R>
+struct PeriodicOut {
+    R *p;
+    long long gi, gk, step;      // offsets of the x and z images, 0: none
+    __device__ __forceinline__ PeriodicOut(const GridT<R> &g, R *a, int i, int j, int k)
+        : p(a + ix(g, i, j, k)), gi(i == 1 ? g.N1 : (i == g.N1 ? -g.N1 : 0)),
+          gk((long long)g.P1 * g.P2 * (k == 1 ? g.N3 : (k == g.N3 ? -g.N3 : 0))), step(g.P1) {}
+    __device__ __forceinline__ void put(R v)
+    {
+        *p = v;
+        if (gi) p[gi] = v;
+        if (gk) {
+            p[gk] = v;
+            if (gi) p[gi + gk] = v;
+        }
+        p -= step;
+    }
+};
+
 // The problem supplies
-//   static constexpr int NRHS;  static constexpr bool AHEAD (load a row ahead)
+//   static constexpr int NRHS, AHEAD (rows whose inputs are loaded ahead)
 //   skip(), lines() (count of lines along i of the block row)
 //   struct March { March(const Prob &, int line, int by, int r0);               // line: clamped to a valid one
 //                  struct In;  void load(const Prob &, int r, In &);             // the inputs of row r, rows in order from r0
 //                  void row(const Prob &, int r, const In &, double &a, double &b, double &c, double d[NRHS]); }
-//   emit(int line, int by, int r, const double x[NRHS])
+//   struct Out { Out(const Prob &, int line, int by, int r);  void put(const Prob &, const double x[NRHS]); }   // row r, then r - 1, ...
 template <class Prob>
 __device__ __forceinline__ void march_block(const Prob &prob, const MarchPlan &mp, int bx, int by)
 {
     constexpr int NR = Prob::NRHS, W = 2 + NR;
     extern __shared__ __align__(16) double msm[];
-    if (prob.skip()) return;
+    const bool skip = prob.skip();   // tested before the stores: its load does not delay the others
     const int TI = 1 << mp.lgTI, NS = 1 << mp.lgNS, TP = TI + 1;
     const int l = threadIdx.x & (TI - 1), s = threadIdx.x >> mp.lgTI;
     const int line = (bx << mp.lgTI) + l, nl = prob.lines();
@@ -184,34 +212,32 @@ __device__ __forceinline__ void march_block(const Prob &prob, const MarchPlan &m
             p = -p * cp;
             w += W * TI;
         };
+        // AHEAD rows of inputs are on their way while a row is worked on (0: it waits for its own)
+        constexpr int D = Prob::AHEAD, NB = D + 1;
         const int last = r0 + m - 1;
-        int r = r0;
-        typename Prob::March::In in0;
-        st.load(prob, r, in0);
-        if constexpr (Prob::AHEAD) {                   // the next row's inputs are on their way while this one is worked on
-            typename Prob::March::In in1;
-            for (; r + 1 < last; r += 2) {
-                st.load(prob, r + 1, in1);
-                eliminate(r, in0);
-                park();
-                st.load(prob, r + 2, in0);
-                eliminate(r + 1, in1);
-                park();
-            }
-            if (r < last) {
-                st.load(prob, r + 1, in1);
-                eliminate(r, in0);
-                park();
-                in0 = in1;
-            }
-        } else {
+        typename Prob::March::In in[NB];
+#pragma unroll
+        for (int q = 0; q < (D ? D : 1); q++)
+            if (r0 + q <= last) st.load(prob, r0 + q, in[q]);
+        if constexpr (D == 0) {
+            int r = r0;
             while (r < last) {
-                eliminate(r, in0);
+                eliminate(r, in[0]);
                 park();
-                st.load(prob, ++r, in0);
+                st.load(prob, ++r, in[0]);
+            }
+            eliminate(last, in[0]);
+        } else {
+            for (int r = r0; r <= last; r += NB) {
+#pragma unroll
+                for (int q = 0; q < NB; q++) {
+                    if (r + q > last) break;
+                    if (r + q + D <= last) st.load(prob, r + q + D, in[(q + D) % NB]);
+                    eliminate(r + q, in[q]);
+                    if (r + q < last) park();
+                }
             }
         }
-        eliminate(last, in0);
         double *const o = red + s * TP + l;
         o[0] = e; o[RS] = cp; o[2 * RS] = se; o[3 * RS] = p;
 #pragma unroll
@@ -219,25 +245,44 @@ __device__ __forceinline__ void march_block(const Prob &prob, const MarchPlan &m
     }
     __syncthreads();
     march_reduce<NR>(red, mp.lgNS, TP, mp.cyclic != 0);
-    if (line < nl) {
+    if (line < nl && !skip) {
         double x[NR], xp[NR];
         const int sp = (s - 1) & (NS - 1);
 #pragma unroll
         for (int q = 0; q < NR; q++) { x[q] = red[q * RS + s * TP + l]; xp[q] = red[q * RS + sp * TP + l]; }
-        prob.emit(line, by, r0 + m - 1, x);
+        typename Prob::Out out(prob, line, by, r0 + m - 1);
+        out.put(prob, x);
         const double *w = row0 + (m - 2) * W * TI;
-        for (int r = r0 + m - 2; r >= r0; r--, w -= W * TI) {
+        int left = m - 1;
+        constexpr int B = 4;                           // parked rows read ahead of the substitution
+        for (; left >= B; left -= B, w -= B * W * TI) {
+            double c[B], y[B][NR];
+#pragma unroll
+            for (int t = 0; t < B; t++) {
+                c[t] = w[-t * W * TI];
+                const double e = w[-t * W * TI + TI];
+#pragma unroll
+                for (int q = 0; q < NR; q++) y[t][q] = fma(-e, xp[q], w[-t * W * TI + (2 + q) * TI]);
+            }
+#pragma unroll
+            for (int t = 0; t < B; t++) {
+#pragma unroll
+                for (int q = 0; q < NR; q++) x[q] = fma(-c[t], x[q], y[t][q]);
+                out.put(prob, x);
+            }
+        }
+        for (; left > 0; left--, w -= W * TI) {
             const double c = w[0], e = w[TI];
 #pragma unroll
             for (int q = 0; q < NR; q++) x[q] = fma(-c, x[q], fma(-e, xp[q], w[(2 + q) * TI]));
-            prob.emit(line, by, r, x);
+            out.put(prob, x);
         }
     }
 }
 
-// NT: the most threads per block; 512 threads per SM (128 registers).
+// NT: the most threads per block; Prob::TPS threads per SM.
 template <class Prob, int NT>
-__global__ void __launch_bounds__(NT, 512 / NT) march_kernel(const __grid_constant__ Prob prob, MarchPlan mp)
+__global__ void __launch_bounds__(NT, Prob::TPS / NT) march_kernel(const __grid_constant__ Prob prob, MarchPlan mp)
 {
     march_block(prob, mp, blockIdx.x, blockIdx.y);
 }
@@ -258,6 +303,12 @@ __global__ void __launch_bounds__(NT, 512 / NT) march_kernel(const __grid_consta
 constexpr int COL_SLOTS = 4;
 constexpr double COL_TINY = 7.8886090522101181e-31;   // 2^-100
 constexpr int COL_WAIT = 1 << 22;                     // polls of a bounded wait
+
+// FP64 problems that name their stream (Prob::NROW): the cyclic z sweeps.
+template <class P, class = void>
+struct Streams { static constexpr bool on = false; };
+template <class P>
+struct Streams<P, std::void_t<decltype(P::NROW)>> { static constexpr bool on = std::is_same<typename P::Real, double>::value; };
 
 // Words of one segment's plane: NROW rows of w + 2, then the table words of rows
 // j-1, j, j+1 (Mu) and j (iR).

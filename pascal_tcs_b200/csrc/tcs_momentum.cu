@@ -76,7 +76,7 @@ template <class R>
 struct DUZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool AHEAD = std::is_same<R, float>::value;   // FP64 inputs of two rows do not fit the registers
+    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12;   // FP64 inputs of two rows do not fit the registers
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -200,7 +200,10 @@ struct DUZ {
             d[0] = rhs * dt;
         }
     };
-    __device__ __forceinline__ void emit(int line, int by, int r, const double *x) const { f.scr[ix(g, 1 + line, 1 + by, r + 1)] = R(x[0]); }
+    struct Out : ScratchOut<R> {
+        __device__ __forceinline__ Out(const DUZ &q, int line, int by, int r) : ScratchOut<R>(q.g, q.f.scr, 1 + line, 1 + by, r + 1, (long long)q.g.P1 * q.g.P2) {}
+        __device__ __forceinline__ void put(const DUZ &, const double *x) { ScratchOut<R>::put(R(x[0])); }
+    };
 };
 
 template <class R, int WIDE = 0, int ITEM = 0>
@@ -241,48 +244,57 @@ struct DUX {
     __device__ void emit(int l, int r, const R *x, const State &st) const { f.scr[ix(g, r + 1, lj(l), 1 + vby<ITEM>())] = x[0]; }
 };
 
-template <class R, int ITEM = 0>
+template <class R>
 struct DUY {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = std::is_same<R, float>::value;   // measured faster in FP32 only
-    static constexpr int MINB = LineOcc<R>::y;
-    static constexpr int MREG = LineOcc<Real>::reg_y;
-    static constexpr int NT = LineOcc<Real>::nt_y;
-    static constexpr bool CONTIG = false;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr int AHEAD = 2, TPS = 512, ROWS = 16;
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt; };
-    __device__ State prepare() const { return State{R(g.scal[S_DT])}; }
-    __device__ int li(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return li(l) <= g.N1; }
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
-    {
-        const int i = li(l), j = r + 1, k = 1 + vby<ITEM>(), im = i - 1, jm = j - 1, jp = j + 1;
-        const PhysT<R> &p = g.ph;
-        const R *dx1 = g.m1.dx, *dx2 = g.m2.dx;
-        const R *rdx2 = g.m2.rdx, *rdmx1 = g.m1.rdmx, *rdmx2 = g.m2.rdmx;
-        const long long c = ix(g, i, j, k), sj = g.P1;
-        const R jum = (j == 1) ? R(0.0) : R(1.0), jup = (j == g.N2) ? R(0.0) : R(1.0);
-        const R v3 = R(0.5) * (dx1[im] * ld(f.V + c) + dx1[i] * ld(f.V + c - 1)) * rdmx1[i];
-        const R v4 = R(0.5) * (dx1[im] * ld(f.V + c + sj) + dx1[i] * ld(f.V + c - 1 + sj)) * rdmx1[i];
-        const R Mjk = MU(j, k), Mjmk = MU(jm, k), Mjpk = MU(jp, k), iRjk = IR(j, k);
-        const R mua = R(0.5) * (dx1[im] * Mjmk + dx1[i] * Mjmk) * rdmx1[i];
-        const R muc = R(0.5) * (dx1[im] * Mjk + dx1[i] * Mjk) * rdmx1[i];
-        const R mub = R(0.5) * (dx1[im] * Mjpk + dx1[i] * Mjpk) * rdmx1[i];
-        const R mu3 = R(0.5) * (dx2[jm] * muc + dx2[j] * mua) * rdmx2[j];
-        const R mu4 = R(0.5) * (dx2[jp] * muc + dx2[j] * mub) * rdmx2[jp];
-        const R invRhoc = R(0.5) * (dx1[im] * iRjk + dx1[i] * iRjk) * rdmx1[i];
-        const R ih = R(0.5) * p.Cmu * invRhoc;
-        const R mACJ = ih * rdx2[j] * (mu4 * rdmx2[jp] + mu3 * rdmx2[j]) + R(0.25) * (-v4 * rdmx2[jp] + v3 * rdmx2[j]);
-        const R mAPJ = (-ih * rdx2[j] * mu4 * rdmx2[jp] + R(0.25) * (v4 * rdmx2[jp])) * jup;
-        const R mAMJ = (-ih * rdx2[j] * mu3 * rdmx2[j] + R(0.25) * (-v3 * rdmx2[j])) * jum;
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = mACJ * dt + R(1.0); cf.c = mAPJ * dt; cf.a = mAMJ * dt; cf.d[0] = ld(f.scr + c);
-        return cf;
-    }
-    __device__ void emit(int l, int r, const R *x, const State &st) const { store_periodic(g, f.dU, li(l), r + 1, 1 + vby<ITEM>(), x[0]); }
+    __device__ int lines() const { return g.N1; }
+    struct March {
+        R cu, dt, m, w;                                 // m, w: stress and convection terms of the face below the row
+        long long c;
+        int t4;
+        __device__ __forceinline__ March(const DUY &q, int line, int by, int r0)
+        {
+            const GridT<R> &g = q.g;
+            const int i = 1 + line, j = r0 + 1, k = 1 + by;
+            cu = R(0.5) * ld(g.m1.dx + i - 1) * ld(g.m1.rdmx + i);
+            dt = R(g.scal[S_DT]);
+            c = ix(g, i, j, k);
+            t4 = 4 * ix2(g, j, k);
+            face(ld(q.f.V + c), ld(q.f.V + c - 1), ld(q.f.MuT + t4 + 1), ld(g.m2.rdmx + j));
+        }
+        __device__ __forceinline__ void face(R V, R Vxm, R mu, R rdmx2)
+        {
+            m = mu * rdmx2;
+            w = R(0.25) * (Vxm + cu * (V - Vxm)) * rdmx2;
+        }
+        struct In { R V, Vxm, mu, iR, rdx2, rdmx2, d; };
+        __device__ __forceinline__ void load(const DUY &q, int r, In &n)
+        {
+            const long long sj = q.g.P1;
+            n.V = ld(q.f.V + c + sj); n.Vxm = ld(q.f.V + c + sj - 1);
+            n.mu = ld(q.f.MuT + t4 + 5); n.iR = ld(q.f.iRT + t4);
+            n.rdx2 = ld(q.g.m2.rdx + r + 1); n.rdmx2 = ld(q.g.m2.rdmx + r + 2);
+            n.d = q.f.scr[c];
+            c += sj;
+            t4 += 4;
+        }
+        __device__ __forceinline__ void row(const DUY &q, int r, const In &n, double &a, double &b, double &cc, double *d)
+        {
+            const R m3 = m, w3 = w, h = R(0.5) * q.g.ph.Cmu * n.iR * n.rdx2;
+            face(n.V, n.Vxm, n.mu, n.rdmx2);
+            const R am = -(h * m3 + w3) * dt, ap = (w - h * m) * dt;
+            a = r == 0 ? R(0) : am; cc = r == q.g.N2 - 1 ? R(0) : ap; b = 1.0 - ((double)am + (double)ap);
+            d[0] = n.d;
+        }
+    };
+    struct Out : PeriodicOut<R> {
+        __device__ __forceinline__ Out(const DUY &q, int line, int by, int r) : PeriodicOut<R>(q.g, q.f.dU, 1 + line, r + 1, 1 + by) {}
+        __device__ __forceinline__ void put(const DUY &, const double *x) { PeriodicOut<R>::put(R(x[0])); }
+    };
 };
 
 // ---------------------------------------------------------------------------
@@ -294,7 +306,7 @@ template <class R>
 struct DVZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool AHEAD = std::is_same<R, float>::value;   // FP64 inputs of two rows do not fit the registers
+    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12;   // FP64 inputs of two rows do not fit the registers
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -419,7 +431,10 @@ struct DVZ {
             d[0] = rhs * dt;
         }
     };
-    __device__ __forceinline__ void emit(int line, int by, int r, const double *x) const { f.scr[ix(g, 1 + line, 2 + by, r + 1)] = R(x[0]); }
+    struct Out : ScratchOut<R> {
+        __device__ __forceinline__ Out(const DVZ &q, int line, int by, int r) : ScratchOut<R>(q.g, q.f.scr, 1 + line, 2 + by, r + 1, (long long)q.g.P1 * q.g.P2) {}
+        __device__ __forceinline__ void put(const DVZ &, const double *x) { ScratchOut<R>::put(R(x[0])); }
+    };
 };
 
 // mu1, mu2 of solvedV's last stage-1 iteration (i = N1, j = N2, k = N3).
@@ -476,43 +491,61 @@ struct DVX {
     __device__ void emit(int l, int r, const R *x, const State &st) const { f.scr[ix(g, r + 1, lj(l), 1 + vby<ITEM>())] = x[0]; }
 };
 
-template <class R, int ITEM = 0>
+template <class R>
 struct DVY {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = std::is_same<R, float>::value;   // measured faster in FP32 only
-    static constexpr int MINB = LineOcc<R>::y;
-    static constexpr int MREG = LineOcc<Real>::reg_y;
-    static constexpr int NT = LineOcc<Real>::nt_y;
-    static constexpr bool CONTIG = false;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr int AHEAD = 2, TPS = 512, ROWS = 16;
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt; };
-    __device__ State prepare() const { return State{R(g.scal[S_DT])}; }
-    __device__ int li(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return li(l) <= g.N1; }
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
-    {
-        const int i = li(l), j = r + 2, k = 1 + vby<ITEM>(), jm = j - 1, jp = j + 1;
-        const PhysT<R> &p = g.ph;
-        const R *dx2 = g.m2.dx, *rdx2 = g.m2.rdx, *rdmx2 = g.m2.rdmx;
-        const long long c = ix(g, i, j, k), sj = g.P1;
-        const R jvp = (jm >= 2) ? R(1.0) : R(0.0), jvm = (jp <= g.N2) ? R(1.0) : R(0.0);
-        const R Vc = ld(f.V + c), Vym = ld(f.V + c - sj), Vyp = ld(f.V + c + sj);
-        const R v3 = R(0.5) * (Vym + Vc), v4 = R(0.5) * (Vc + Vyp);
-        const R dvdy3 = (Vc - Vym) * rdx2[jm], dvdy4 = (Vyp - Vc) * rdx2[j];
-        const R Mjk = MU(j, k), Mjmk = MU(jm, k);
-        const R invRhoc = R(0.5) * (dx2[jm] * IR(j, k) + dx2[j] * IR(jm, k)) * rdmx2[j];
-        const R ih = R(0.5) * p.Cmu * invRhoc;
-        const R mACJ = ih * rdmx2[j] * (Mjk * rdx2[j] + Mjmk * rdx2[jm]) * R(2.0) + R(0.25) * (dvdy4 * R(0.5) + dvdy3 * R(0.5) - v4 * rdx2[j] + v3 * rdx2[jm]);
-        const R mAPJ = (-ih * rdmx2[j] * Mjk * rdx2[j] * R(2.0) + R(0.25) * (v4 * rdx2[j] + dvdy4 * R(0.5))) * jvp;
-        const R mAMJ = (-ih * rdmx2[j] * Mjmk * rdx2[jm] * R(2.0) + R(0.25) * (-v3 * rdx2[jm] + dvdy3 * R(0.5))) * jvm;
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = mACJ * dt + R(1.0); cf.c = mAPJ * dt; cf.a = mAMJ * dt; cf.d[0] = ld(f.scr + c);
-        return cf;
-    }
-    __device__ void emit(int l, int r, const R *x, const State &st) const { store_periodic(g, f.dV, li(l), r + 2, 1 + vby<ITEM>(), x[0]); }
+    __device__ int lines() const { return g.N1; }
+    struct March {
+        R dt, Vc, A, B, C;                              // the cell below the row
+        long long c;
+        int t4;
+        __device__ __forceinline__ March(const DVY &q, int line, int by, int r0)
+        {
+            const GridT<R> &g = q.g;
+            const int i = 1 + line, j = r0 + 2, k = 1 + by;
+            dt = R(g.scal[S_DT]);
+            c = ix(g, i, j, k);
+            t4 = 4 * ix2(g, j, k);
+            Vc = ld(q.f.V + c);
+            cell(ld(q.f.V + c - g.P1), Vc, ld(q.f.MuT + t4 - 4), ld(g.m2.rdx + j - 1));
+        }
+        __device__ __forceinline__ void cell(R Vm, R Vp, R mu, R rdx2)
+        {
+            A = mu * rdx2;
+            B = R(0.125) * (Vm + Vp) * rdx2;
+            C = R(0.125) * (Vp - Vm) * rdx2;
+        }
+        struct In { R V, mu, iR, rdx2, rdmx2, d; };
+        __device__ __forceinline__ void load(const DVY &q, int r, In &n)
+        {
+            const long long sj = q.g.P1;
+            n.V = ld(q.f.V + c + sj);
+            n.mu = ld(q.f.MuT + t4); n.iR = ld(q.f.iRT + t4 + 1);
+            n.rdx2 = ld(q.g.m2.rdx + r + 2); n.rdmx2 = ld(q.g.m2.rdmx + r + 2);
+            n.d = q.f.scr[c];
+            c += sj;
+            t4 += 4;
+        }
+        __device__ __forceinline__ void row(const DVY &q, int r, const In &n, double &a, double &b, double &cc, double *d)
+        {
+            const R A3 = A, B3 = B, C3 = C, h = q.g.ph.Cmu * n.iR * n.rdmx2, V0 = Vc;
+            Vc = n.V;
+            cell(V0, n.V, n.mu, n.rdx2);
+            const R am = (C3 - B3 - h * A3) * dt, ap = (B + C - h * A) * dt;
+            // the upper coefficient carries the mask of the row below, the lower one that of the row above (:864-889)
+            a = r == q.g.N2 - 2 ? R(0) : am; cc = r == 0 ? R(0) : ap;
+            b = (1.0 - ((double)am + (double)ap)) + (double)(R(2) * (C3 + C) * dt);
+            d[0] = n.d;
+        }
+    };
+    struct Out : PeriodicOut<R> {
+        __device__ __forceinline__ Out(const DVY &q, int line, int by, int r) : PeriodicOut<R>(q.g, q.f.dV, 1 + line, r + 2, 1 + by) {}
+        __device__ __forceinline__ void put(const DVY &, const double *x) { PeriodicOut<R>::put(R(x[0])); }
+    };
 };
 
 // ---------------------------------------------------------------------------
@@ -523,7 +556,7 @@ template <class R>
 struct DWZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool AHEAD = std::is_same<R, float>::value;   // FP64 inputs of two rows do not fit the registers
+    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12;   // FP64 inputs of two rows do not fit the registers
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -658,7 +691,10 @@ struct DWZ {
             U0 = nU; Uxp = nUx; D0 = nD; Dxp = nDx; V0 = nV; Vyp = nVy; E0 = nE; Eyp = nEy; P0 = nP;
         }
     };
-    __device__ __forceinline__ void emit(int line, int by, int r, const double *x) const { f.scr[ix(g, 1 + line, 1 + by, r + 1)] = R(x[0]); }
+    struct Out : ScratchOut<R> {
+        __device__ __forceinline__ Out(const DWZ &q, int line, int by, int r) : ScratchOut<R>(q.g, q.f.scr, 1 + line, 1 + by, r + 1, (long long)q.g.P1 * q.g.P2) {}
+        __device__ __forceinline__ void put(const DWZ &, const double *x) { ScratchOut<R>::put(R(x[0])); }
+    };
 };
 
 // mu1..mu4 of solvedW's last stage-1 iteration (i = N1, j = N2, k = N3).
@@ -721,50 +757,62 @@ struct DWX {
     __device__ void emit(int l, int r, const R *x, const State &st) const { f.scr[ix(g, r + 1, lj(l), 1 + vby<ITEM>())] = x[0]; }
 };
 
-template <class R, int ITEM = 0>
+template <class R>
 struct DWY {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = std::is_same<R, float>::value;   // measured faster in FP32 only
-    static constexpr int MINB = LineOcc<R>::y;
-    static constexpr int MREG = LineOcc<Real>::reg_y;
-    static constexpr int NT = LineOcc<Real>::nt_y;
-    static constexpr bool CONTIG = false;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr int AHEAD = 2, TPS = 512, ROWS = 16;
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt, mu1, mu2, mu3, mu4; };
-    __device__ State prepare() const
-    {
-        State s;
-        s.dt = g.scal[S_DT];
-        dw_stale_mu(g, f, s.mu1, s.mu2, s.mu3, s.mu4);
-        return s;
-    }
-    __device__ int li(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return li(l) <= g.N1; }
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
-    {
-        const int i = li(l), j = r + 1, k = 1 + vby<ITEM>(), jp = j + 1, km = g.N3 - 1;
-        const PhysT<R> &p = g.ph;
-        const R *dx3 = g.m3.dx, *rdx2 = g.m2.rdx, *rdmx2 = g.m2.rdmx, *rdmx3 = g.m3.rdmx;
-        const long long c = ix(g, i, j, k), sj = g.P1;
-        const R jwm = (j == 1) ? R(0.0) : R(1.0), jwp = (j == g.N2) ? R(0.0) : R(1.0);
-        const R mu1 = st.mu1, mu2 = st.mu2, mu3 = st.mu3, mu4 = st.mu4;
-        (void)mu1; (void)mu2; (void)mu3; (void)mu4;
-        const long long ckm = ix(g, i, j, km);
-        const R v3 = (dx3[km] * ld(f.V + c) + dx3[k] * ld(f.V + ckm)) * rdmx3[k] * R(0.5);
-        const R v4 = (dx3[km] * ld(f.V + c + sj) + dx3[k] * ld(f.V + ckm + sj)) * rdmx3[k] * R(0.5);
-        const R invRhoc = R(0.5) * (dx3[km] * IR(j, k) + dx3[k] * IR(j, km)) * rdmx3[k];
-        const R ih = R(0.5) * p.Cmu * invRhoc;
-        const R mACJ = ih * rdx2[j] * (mu4 * rdmx2[jp] + mu3 * rdmx2[j]) + R(0.25) * (-v4 * rdmx2[jp] + v3 * rdmx2[j]);
-        const R mAPJ = (-ih * rdx2[j] * mu4 * rdmx2[jp] + R(0.25) * (v4 * rdmx2[jp])) * jwp;
-        const R mAMJ = (-ih * rdx2[j] * mu3 * rdmx2[j] + R(0.25) * (-v3 * rdmx2[j])) * jwm;
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = mACJ * dt + R(1.0); cf.c = mAPJ * dt; cf.a = mAMJ * dt; cf.d[0] = ld(f.scr + c);
-        return cf;
-    }
-    __device__ void emit(int l, int r, const R *x, const State &st) const { store_periodic(g, f.dW, li(l), r + 1, 1 + vby<ITEM>(), x[0]); }
+    __device__ int lines() const { return g.N1; }
+    struct March {
+        R z0, z1, mu3, mu4, dt, w, rdmx2;               // z0, z1: weights of planes k and N3-1; w: convection at the face below the row
+        long long c, dk;
+        int t4, t4k;
+        __device__ __forceinline__ March(const DWY &q, int line, int by, int r0)
+        {
+            const GridT<R> &g = q.g;
+            const int i = 1 + line, j = r0 + 1, k = 1 + by, km = g.N3 - 1;
+            R mu1, mu2;
+            dw_stale_mu(g, q.f, mu1, mu2, mu3, mu4);
+            const R h = R(0.5) * ld(g.m3.rdmx + k);
+            z0 = h * ld(g.m3.dx + km); z1 = h * ld(g.m3.dx + k);
+            dt = R(g.scal[S_DT]);
+            c = ix(g, i, j, k);
+            dk = (long long)g.P1 * g.P2 * (km - k);
+            t4 = 4 * ix2(g, j, k);
+            t4k = 4 * g.P2 * (km - k);
+            face(ld(q.f.V + c), ld(q.f.V + c + dk), ld(g.m2.rdmx + j));
+        }
+        __device__ __forceinline__ void face(R V, R Vk, R rd)
+        {
+            rdmx2 = rd;
+            w = R(0.25) * (z0 * V + z1 * Vk) * rd;
+        }
+        struct In { R V, Vk, iR, iRk, rdx2, rdmx2, d; };
+        __device__ __forceinline__ void load(const DWY &q, int r, In &n)
+        {
+            const long long sj = q.g.P1;
+            n.V = ld(q.f.V + c + sj); n.Vk = ld(q.f.V + c + sj + dk);
+            n.iR = ld(q.f.iRT + t4); n.iRk = ld(q.f.iRT + t4 + t4k);
+            n.rdx2 = ld(q.g.m2.rdx + r + 1); n.rdmx2 = ld(q.g.m2.rdmx + r + 2);
+            n.d = q.f.scr[c];
+            c += sj;
+            t4 += 4;
+        }
+        __device__ __forceinline__ void row(const DWY &q, int r, const In &n, double &a, double &b, double &cc, double *d)
+        {
+            const R w3 = w, m3 = mu3 * rdmx2, h = R(0.5) * q.g.ph.Cmu * (z0 * n.iR + z1 * n.iRk) * n.rdx2;
+            face(n.V, n.Vk, n.rdmx2);
+            const R am = -(h * m3 + w3) * dt, ap = (w - h * (mu4 * rdmx2)) * dt;
+            a = r == 0 ? R(0) : am; cc = r == q.g.N2 - 1 ? R(0) : ap; b = 1.0 - ((double)am + (double)ap);
+            d[0] = n.d;
+        }
+    };
+    struct Out : PeriodicOut<R> {
+        __device__ __forceinline__ Out(const DWY &q, int line, int by, int r) : PeriodicOut<R>(q.g, q.f.dW, 1 + line, r + 1, 1 + by) {}
+        __device__ __forceinline__ void put(const DWY &, const double *x) { PeriodicOut<R>::put(R(x[0])); }
+    };
 };
 
 template <class R>
@@ -784,30 +832,45 @@ static void launch_dw_z(const Ctx<R> &cx, cudaStream_t s)
 }
 
 template <class R>
+static void launch_du_y(const Ctx<R> &cx, cudaStream_t s)
+{
+    launch_march(cx, DUY<R>{cx.g, cx.f}, cx.g.N2, false, cx.g.N1, cx.g.N3, s, K_DU_Y);
+}
+
+template <class R>
+static void launch_dv_y(const Ctx<R> &cx, cudaStream_t s)
+{
+    launch_march(cx, DVY<R>{cx.g, cx.f}, cx.g.N2 - 1, false, cx.g.N1, cx.g.N3, s, K_DV_Y);
+}
+
+template <class R>
+static void launch_dw_y(const Ctx<R> &cx, cudaStream_t s)
+{
+    launch_march(cx, DWY<R>{cx.g, cx.f}, cx.g.N2, false, cx.g.N1, cx.g.N3, s, K_DW_Y);
+}
+
+template <class R>
 void launch_solve_du(const Ctx<R> &cx, cudaStream_t s)
 {
-    const GridT<R> &g = cx.g;
     launch_du_z(cx, s);
-    launch_x<DUX>(cx, g.N2, s, K_DU_X);
-    launch_y<DUY<R>>(cx, g.N2, g.N1, g.N3, [&](int tl) { return DUY<R>{g, cx.f, tl}; }, s, K_DU_Y);
+    launch_x<DUX>(cx, cx.g.N2, s, K_DU_X);
+    launch_du_y(cx, s);
 }
 
 template <class R>
 void launch_solve_dv(const Ctx<R> &cx, cudaStream_t s)
 {
-    const GridT<R> &g = cx.g;
     launch_dv_z(cx, s);
-    launch_x<DVX>(cx, g.N2 - 1, s, K_DV_X);
-    launch_y<DVY<R>>(cx, g.N2 - 1, g.N1, g.N3, [&](int tl) { return DVY<R>{g, cx.f, tl}; }, s, K_DV_Y);
+    launch_x<DVX>(cx, cx.g.N2 - 1, s, K_DV_X);
+    launch_dv_y(cx, s);
 }
 
 template <class R>
 void launch_solve_dw(const Ctx<R> &cx, cudaStream_t s)
 {
-    const GridT<R> &g = cx.g;
     launch_dw_z(cx, s);
-    launch_x<DWX>(cx, g.N2, s, K_DW_X);
-    launch_y<DWY<R>>(cx, g.N2, g.N1, g.N3, [&](int tl) { return DWY<R>{g, cx.f, tl}; }, s, K_DW_Y);
+    launch_x<DWX>(cx, cx.g.N2, s, K_DW_X);
+    launch_dw_y(cx, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -965,19 +1028,16 @@ void launch_pseudo_update(const Ctx<R> &cx, cudaStream_t s)
 template <class R>
 void launch_momentum_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s)
 {
-    auto y = [](int ny) {
-        return [ny](const Ctx<R> &x) { return StageShape{x.g.N2 - ny, false, x.tl_strided, x.g.N1, x.g.N3}; };
-    };
     auto lines = [](int ny) { return [ny](const Ctx<R> &x) { return x.g.N2 - ny; }; };
     march_stage(cs, A, s, launch_du_z<R>);
     multi_x<DUX>(cs, A, s, "du_x", lines(0));
-    multi_stage<DUY<R, 1>>(cs, A, s, "du_y", y(0), [](const Ctx<R> &x, int tl) { return DUY<R, 1>{x.g, x.f, tl}; });
+    march_stage(cs, A, s, launch_du_y<R>);
     march_stage(cs, A, s, launch_dv_z<R>);
     multi_x<DVX>(cs, A, s, "dv_x", lines(1));
-    multi_stage<DVY<R, 1>>(cs, A, s, "dv_y", y(1), [](const Ctx<R> &x, int tl) { return DVY<R, 1>{x.g, x.f, tl}; });
+    march_stage(cs, A, s, launch_dv_y<R>);
     march_stage(cs, A, s, launch_dw_z<R>);
     multi_x<DWX>(cs, A, s, "dw_x", lines(0));
-    multi_stage<DWY<R, 1>>(cs, A, s, "dw_y", y(0), [](const Ctx<R> &x, int tl) { return DWY<R, 1>{x.g, x.f, tl}; });
+    march_stage(cs, A, s, launch_dw_y<R>);
 }
 
 template void launch_momentum_multi<double>(const std::vector<Ctx<double> *> &, MultiArena &, cudaStream_t);

@@ -17,7 +17,7 @@ template <class R>
 struct ThermalZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool AHEAD = std::is_same<R, float>::value;   // FP64 inputs of two rows do not fit the registers
+    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12;   // FP64 inputs of two rows do not fit the registers
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -147,10 +147,10 @@ struct ThermalZ {
             d[0] = rhs * dt;
         }
     };
-    __device__ __forceinline__ void emit(int line, int by, int r, const double *x) const
-    {
-        f.scr[ix(g, 1 + line, 1 + by, r + 1)] = R(x[0]);
-    }
+    struct Out : ScratchOut<R> {
+        __device__ __forceinline__ Out(const ThermalZ &q, int line, int by, int r) : ScratchOut<R>(q.g, q.f.scr, 1 + line, 1 + by, r + 1, (long long)q.g.P1 * q.g.P2) {}
+        __device__ __forceinline__ void put(const ThermalZ &, const double *x) { ScratchOut<R>::put(R(x[0])); }
+    };
 };
 
 // Stage 2 (:388-429): jm, jp, km, kp keep the values of the last stage-1
@@ -217,66 +217,93 @@ struct ThermalX {
 };
 
 // Stage 3 (:456-507): km, kp stale (N3-1, N3+1); T += solution (:518-524).
-template <class R, int ITEM = 0>
+template <class R>
 struct ThermalY {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = std::is_same<R, float>::value;   // measured faster in FP32 only
-    static constexpr int MINB = LineOcc<R>::y;
-    static constexpr int MREG = LineOcc<Real>::reg_y;
-    static constexpr int NT = LineOcc<Real>::nt_y;
-    static constexpr bool CONTIG = false;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr int AHEAD = 0, TPS = 512, ROWS = 16;
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt; };
-    __device__ State prepare() const { return State{R(g.scal[S_DT])}; }
-    __device__ int li(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return li(l) <= g.N1; }
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
-    {
-        const int i = li(l), j = r + 1, k = 1 + vby<ITEM>();
-        const int im = i - 1, ip = i + 1, jm = j - 1, jp = j + 1, km = g.N3 - 1, kp = g.N3 + 1;
-        const PhysT<R> &p = g.ph;
-        const bool d2 = g.kdeg2 != 0;
-        const R *dx1 = g.m1.dx, *dx2 = g.m2.dx, *dx3 = g.m3.dx;
-        const R *rdx1 = g.m1.rdx, *rdx2 = g.m2.rdx, *rdx3 = g.m3.rdx;
-        const R *rdmx1 = g.m1.rdmx, *rdmx2 = g.m2.rdmx, *rdmx3 = g.m3.rdmx;
-        const long long c = ix(g, i, j, k), sj = g.P1;
-        const R *T = f.T;
-        const R Tc = ld(T + c), Txm = ld(T + c - 1), Txp = ld(T + c + 1), Tym = ld(T + c - sj), Typ = ld(T + c + sj);
-        const R Tkm = ld(T + ix(g, i, j, km)), Tkp = ld(T + ix(g, i, j, kp));
-        R Kc, dKc, Kym, dKym, Kyp, dKyp, irc, dirc;
-        kpp_eval(p, d2, Tc, Kc, dKc); kpp_eval(p, d2, Tym, Kym, dKym); kpp_eval(p, d2, Typ, Kyp, dKyp);
-        const R Kxm = kpp_only(p, d2, Txm), Kxp = kpp_only(p, d2, Txp), Kkm = kpp_only(p, d2, Tkm), Kkp = kpp_only(p, d2, Tkp);
-        rhocp_eval(p, Tc, irc, dirc);
-        const R h = R(0.5) * p.Ct * irc;
-        const R jem = (j == 1) ? R(0.0) : R(1.0), jep = (j == g.N2) ? R(0.0) : R(1.0);
-        const R KPP1 = R(0.5) * rdmx1[i] * (dx1[i] * Kxm + dx1[im] * Kc), KPP2 = R(0.5) * rdmx1[ip] * (dx1[ip] * Kc + dx1[i] * Kxp);
-        const R kPP3 = R(0.5) * rdmx2[j] * (dx2[j] * Kym + dx2[jm] * Kc), kPP4 = R(0.5) * rdmx2[jp] * (dx2[jp] * Kc + dx2[j] * Kyp);
-        const R KPP5 = R(0.5) * rdmx3[k] * (dx3[k] * Kkm + dx3[km] * Kc), KPP6 = R(0.5) * rdmx3[kp] * (dx3[kp] * Kc + dx3[k] * Kkp);
-        const R dkPP3 = R(0.5) * rdmx2[j] * (dx2[j] * dKym + dx2[jm] * dKc), dkPP4 = R(0.5) * rdmx2[jp] * (dx2[jp] * dKc + dx2[j] * dKyp);
-        const R dedx1 = (Tc - Txm) * rdmx1[i], dedx2 = (Txp - Tc) * rdmx1[ip];
-        const R dedy3 = (Tc - Tym) * rdmx2[j], dedy4 = (Typ - Tc) * rdmx2[jp];
-        const R dedz5 = (Tc - Tkm) * rdmx3[k], dedz6 = (Tkp - Tc) * rdmx3[kp];
-        const R Vc = ld(f.V + c), Vyp = ld(f.V + c + sj);
-        const R eACJ = h * rdx2[j] * (kPP4 * rdmx2[jp] + kPP3 * rdmx2[j] - dx2[jp] * (R(0.5) * rdmx2[jp]) * dkPP4 * dedy4 * jep + dx2[jm] * (R(0.5) * rdmx2[j]) * dkPP3 * dedy3 * jem)
-                          + (R(0.25) * Vc * rdmx2[j] - R(0.25) * Vyp * rdmx2[jp])
-                          - R(0.5) * h * ((KPP2 * dedx2 - KPP1 * dedx1) * rdx1[i] + (kPP4 * dedy4 - kPP3 * dedy3) * rdx2[j] + (KPP6 * dedz6 - KPP5 * dedz5) * rdx3[k]);
-        const R eAPJ = (-h * rdx2[j] * (kPP4 * rdmx2[jp] + dx2[j] * (R(0.5) * rdmx2[jp]) * dkPP4 * dedy4) + R(0.25) * Vyp * rdmx2[jp]) * jep;
-        const R eAMJ = (-h * rdx2[j] * (kPP3 * rdmx2[j] - dx2[j] * (R(0.5) * rdmx2[j]) * dkPP3 * dedy3) - R(0.25) * Vc * rdmx2[j]) * jem;
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = eACJ * dt + R(1.0);
-        cf.c = eAPJ * dt;
-        cf.a = eAMJ * dt;
-        cf.d[0] = ld(f.scr + c);
-        return cf;
-    }
-    __device__ void emit(int l, int r, const R *x, const State &st) const
-    {
-        const int i = li(l), j = r + 1, k = 1 + vby<ITEM>();
-        store_periodic(g, f.Tn, i, j, k, ld(f.T + ix(g, i, j, k)) + x[0]);
-    }
+    __device__ int lines() const { return g.N1; }
+    struct March {
+        R rdx1, rdmx1, rdmx1p, w1, w2, rdx3, rdmx3, rdmx3p, z5m, z5c, z6c, z6p, dt;   // weights along x (see ThermalZ) and of the stale z faces
+        R Tc, Kc, dKc, F, s, q, w, dx2m, dx2;         // the cell; the face below it
+        long long c, dkm, dkp;
+        __device__ __forceinline__ March(const ThermalY &o, int line, int by, int r0)
+        {
+            const GridT<R> &g = o.g;
+            const int i = 1 + line, j = r0 + 1, k = 1 + by, km = g.N3 - 1, kp = g.N3 + 1;
+            const long long sk = (long long)g.P1 * g.P2;
+            rdx1 = ld(g.m1.rdx + i); rdmx1 = ld(g.m1.rdmx + i); rdmx1p = ld(g.m1.rdmx + i + 1);
+            w1 = R(0.5) * rdmx1 * ld(g.m1.dx + i); w2 = R(0.5) * rdmx1p * ld(g.m1.dx + i);
+            rdx3 = ld(g.m3.rdx + k); rdmx3 = ld(g.m3.rdmx + k); rdmx3p = ld(g.m3.rdmx + kp);
+            z5m = R(0.5) * rdmx3 * ld(g.m3.dx + k); z5c = R(0.5) * rdmx3 * ld(g.m3.dx + km);
+            z6c = R(0.5) * rdmx3p * ld(g.m3.dx + kp); z6p = R(0.5) * rdmx3p * ld(g.m3.dx + k);
+            dt = R(g.scal[S_DT]);
+            c = ix(g, i, j, k);
+            dkm = sk * (km - k); dkp = sk * (kp - k);
+            dx2 = ld(g.m2.dx + j - 1);
+            Tc = ld(o.f.T + c - g.P1);
+            kpp_eval(g.ph, g.kdeg2 != 0, Tc, Kc, dKc);
+            face(o, ld(o.f.T + c), ld(o.f.V + c), ld(g.m2.dx + j), ld(g.m2.rdmx + j));
+        }
+        // the y face between rows j-1 (Tc, Kc, dKc, dx2) and j, which becomes the current row
+        __device__ __forceinline__ void face(const ThermalY &o, R Tp, R Vp, R dy, R rdmx2)
+        {
+            R Kp, dKp;
+            kpp_eval(o.g.ph, o.g.kdeg2 != 0, Tp, Kp, dKp);
+            dx2m = dx2;
+            dx2 = dy;
+            const R hm = R(0.5) * rdmx2, wm = hm * dx2m, de = (Tp - Tc) * rdmx2;
+            const R kPP = Kc + wm * (Kp - Kc), dkPP = dKc + wm * (dKp - dKc);
+            F = kPP * de;
+            s = kPP * rdmx2;
+            q = hm * (dkPP * de);
+            w = R(0.25) * Vp * rdmx2;
+            Tc = Tp; Kc = Kp; dKc = dKp;
+        }
+        struct In { R Txm, Txp, Typ, Tkm, Tkp, V, rdx2, dx2, rdmx2, d; };
+        __device__ __forceinline__ void load(const ThermalY &o, int r, In &n)
+        {
+            const GridT<R> &g = o.g;
+            const R *const T = o.f.T;
+            n.Txm = ld(T + c - 1); n.Txp = ld(T + c + 1); n.Typ = ld(T + c + g.P1);
+            n.Tkm = ld(T + c + dkm); n.Tkp = ld(T + c + dkp);
+            n.V = ld(o.f.V + c + g.P1);
+            n.rdx2 = ld(g.m2.rdx + r + 1); n.dx2 = ld(g.m2.dx + r + 2); n.rdmx2 = ld(g.m2.rdmx + r + 2);
+            n.d = o.f.scr[c];
+            c += g.P1;
+        }
+        __device__ __forceinline__ void row(const ThermalY &o, int r, const In &n, double &a, double &b, double &cc, double *d)
+        {
+            const PhysT<R> &p = o.g.ph;
+            const bool d2 = o.g.kdeg2 != 0;
+            const R T0 = Tc, K0 = Kc, F3 = F, s3 = s, q3 = q, w3 = w, d2m = dx2m, d2c = dx2;
+            R irc, dirc;
+            rhocp_eval(p, T0, irc, dirc);
+            const R h = R(0.5) * p.Ct * irc, h2 = h * n.rdx2;
+            face(o, n.Typ, n.V, n.dx2, n.rdmx2);
+            const R Kxm = kpp_only(p, d2, n.Txm), Kxp = kpp_only(p, d2, n.Txp), Kkm = kpp_only(p, d2, n.Tkm), Kkp = kpp_only(p, d2, n.Tkp);
+            const R fx = (K0 + w2 * (Kxp - K0)) * ((n.Txp - T0) * rdmx1p) - (K0 + w1 * (Kxm - K0)) * ((T0 - n.Txm) * rdmx1);
+            const R fz = (z6c * K0 + z6p * Kkp) * ((n.Tkp - T0) * rdmx3p) - (z5m * Kkm + z5c * K0) * ((T0 - n.Tkm) * rdmx3);
+            const R jem = r == 0 ? R(0) : R(1), jep = r == o.g.N2 - 1 ? R(0) : R(1);
+            const R ac = h2 * (s + s3 - dx2 * q * jep + d2m * q3 * jem) + (w3 - w) - R(0.5) * h * (fx * rdx1 + (F - F3) * n.rdx2 + fz * rdx3);
+            a = (-h2 * (s3 - d2c * q3) - w3) * jem * dt;
+            cc = (w - h2 * (s + d2c * q)) * jep * dt;
+            b = 1.0 + (double)(ac * dt);
+            d[0] = n.d;
+        }
+    };
+    struct Out : PeriodicOut<R> {
+        const R *T;
+        __device__ __forceinline__ Out(const ThermalY &q, int line, int by, int r)
+            : PeriodicOut<R>(q.g, q.f.Tn, 1 + line, r + 1, 1 + by), T(q.f.T + ix(q.g, 1 + line, r + 1, 1 + by)) {}
+        __device__ __forceinline__ void put(const ThermalY &q, const double *x)
+        {
+            PeriodicOut<R>::put(ld(T) + R(x[0]));
+            T -= q.g.P1;
+        }
+    };
 };
 
 template <class R>
@@ -286,12 +313,17 @@ static void launch_thermal_z(const Ctx<R> &cx, cudaStream_t s)
 }
 
 template <class R>
+static void launch_thermal_y(const Ctx<R> &cx, cudaStream_t s)
+{
+    launch_march(cx, ThermalY<R>{cx.g, cx.f}, cx.g.N2, false, cx.g.N1, cx.g.N3, s, K_THERMAL_Y);
+}
+
+template <class R>
 void launch_thermal(const Ctx<R> &cx, cudaStream_t s)
 {
-    const GridT<R> &g = cx.g;
     launch_thermal_z(cx, s);
-    launch_x<ThermalX>(cx, g.N2, s, K_THERMAL_X);
-    launch_y<ThermalY<R>>(cx, g.N2, g.N1, g.N3, [&](int tl) { return ThermalY<R>{g, cx.f, tl}; }, s, K_THERMAL_Y);
+    launch_x<ThermalX>(cx, cx.g.N2, s, K_THERMAL_X);
+    launch_thermal_y(cx, s);
 }
 
 // The same three sweeps for many cases, one launch per sweep.
@@ -300,9 +332,7 @@ void launch_thermal_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaSt
 {
     march_stage(cs, A, s, launch_thermal_z<R>);
     multi_x<ThermalX>(cs, A, s, "thermal_x", [](const Ctx<R> &x) { return x.g.N2; });
-    multi_stage<ThermalY<R, 1>>(cs, A, s, "thermal_y",
-        [](const Ctx<R> &x) { return StageShape{x.g.N2, false, x.tl_strided, x.g.N1, x.g.N3}; },
-        [](const Ctx<R> &x, int tl) { return ThermalY<R, 1>{x.g, x.f, tl}; });
+    march_stage(cs, A, s, launch_thermal_y<R>);
 }
 
 // the two forms

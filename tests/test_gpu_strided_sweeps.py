@@ -19,6 +19,7 @@ SHAPES = [
     (150, 5, 405),    # the column form, segments of 203 and 202 rows, a part-filled last block
     (45, 6, 400),     # odd N1: rows of i are not 16-byte aligned, no column form
     (45, 5, 640),     # 64 segments: reduced systems through shared memory
+    (20, 643, 8),     # the same along y, segments of unequal length
 ]
 
 
@@ -28,7 +29,11 @@ def test_strided_sweeps_match_oracle(n, precision):
     import pascal_tcs_b200 as P
     from oracle import oracle as O
 
-    cfg = dict(n1m=n[0], n2m=n[1], n3m=n[2], property_set=0, Pr=0.71, Ra=1e4, dtStart=2e-3, fixed_dt=1, seed=11,
+    # (643 stretched rows at Ra = 1e4 and dt = 2e-3 are no test: the y rows of T lose
+    # their dominance there, max |T| is 8e4 after two steps, and two restatements in
+    # 64 bits differ by 3e-10)
+    ra, dt = (1e4, 2e-3) if n[1] < 100 else (1e6, 1e-4)
+    cfg = dict(n1m=n[0], n2m=n[1], n3m=n[2], property_set=0, Pr=0.71, Ra=ra, dtStart=dt, fixed_dt=1, seed=11,
                noise_amp=0.05, gamma2=1.2)
     g = P.Solver(precision=precision, **cfg)
     o = O.Oracle(**{k: v for k, v in g.config.items() if k not in ("device", "precision")})
