@@ -232,25 +232,21 @@ const char *tcs_timer_name(int timer);
 int tcs_bounds_checked(void);
 int tcs_bounds_violations(tcs_ctx *ctx, double *count);
 int tcs_set_use_graph(tcs_ctx *ctx, int on);
-/* launch-shape knobs (powers of two): lines per thread block of the
- * contiguous (x) and the modal line solvers and of the x and z FFTs, and the
- * most lanes (partitions) a tridiagonal line is split over (32: no bound for
- * the y and z sweeps, whose segments follow the line's length).  A line-solver
- * value is an upper bound: each launch runs the largest power of two up to it
- * whose blocks fit the SM's shared memory at the family's blocks per SM; a
- * value no single block could hold is refused (TCS_ERR_ARG).
- * TCS_TUNE_TL_STRIDED, TCS_TUNE_LONG_LINES (1, 2, 4), TCS_TUNE_Y_SOLVER (1, 2,
- * 4) and TCS_TUNE_Z_STAGING (1, 2) chose between forms of the y and z sweeps
- * that one solver has replaced.  Their values are checked, kept and returned as
- * before, without effect.
+/* launch-shape knobs (powers of two): lines per thread block of the modal line
+ * solver and of the x and z FFTs, and the most lanes (partitions) a tridiagonal
+ * line is split over (32: no bound for the x, y and z sweeps, whose segments
+ * follow the line's length).  A line-solver value is an upper bound: each
+ * launch runs the largest power of two up to it whose blocks fit the SM's
+ * shared memory at the family's blocks per SM; a value no single block could
+ * hold is refused (TCS_ERR_ARG).
+ * TCS_TUNE_TL_STRIDED, TCS_TUNE_TL_CONTIG, TCS_TUNE_LONG_LINES (1, 2, 4),
+ * TCS_TUNE_Y_SOLVER (1, 2, 4), TCS_TUNE_MIXED_ROWS (1, 2, 4, 8) and
+ * TCS_TUNE_Z_STAGING (1, 2) chose between forms of the x, y and z sweeps that one
+ * solver, with FP64 elimination, has replaced.  Their values are checked, kept
+ * and returned as before, without effect.
  * TCS_TUNE_IFFT_LINES_X: lines per block of the inverse x transform
  * (TCS_TUNE_FFT_LINES_X sets those of the pressure right-hand side and its
- * forward x transform).
- * TCS_TUNE_MIXED_ROWS (FP32-mixed form; no effect in the FP64 form): 1 the x
- * sweeps eliminate their FP32 rows in FP32 with one FP64-residual refinement
- * pass (default); 2, 4 and 8 they eliminate their FP32-built rows in FP64
- * instead (no refinement pass; the solution is rounded once to FP32).  The y
- * and z sweeps always eliminate in FP64. */
+ * forward x transform). */
 enum { TCS_TUNE_TL_STRIDED = 0, TCS_TUNE_TL_CONTIG, TCS_TUNE_TL_MODAL, TCS_TUNE_FFT_LINES_X, TCS_TUNE_FFT_LINES_Z,
        TCS_TUNE_LANES, TCS_TUNE_LONG_LINES, TCS_TUNE_Y_SOLVER, TCS_TUNE_IFFT_LINES_X, TCS_TUNE_MIXED_ROWS,
        TCS_TUNE_Z_STAGING, TCS_TUNE_COUNT };

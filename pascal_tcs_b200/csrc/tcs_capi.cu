@@ -984,7 +984,7 @@ int tcs_set_tuning(tcs_ctx *c, int knob, int value)
         if (!ifftx_form(x.fp1u, value)) return set_err(TCS_ERR_ARG, "too many lines for shared memory");
         x.ifft_lines_x = value; break;
     case TCS_TUNE_MIXED_ROWS:
-        if (value > 8) return set_err(TCS_ERR_ARG, "mixed rows: 1 FP32 elimination in the x sweeps, 2, 4, 8 FP64 rows");
+        if (value > 8) return set_err(TCS_ERR_ARG, "mixed rows: 1, 2, 4 or 8");
         x.mixed_rows = value; break;
     case TCS_TUNE_Z_STAGING:
         if (value > 2) return set_err(TCS_ERR_ARG, "z staging: 1 or 2");
@@ -1695,7 +1695,8 @@ extern "C" int tcs_autotune(tcs_ctx *c, int trial_steps, const char *cache_path,
     if ((r = tune_trial(c, trial_steps, &best_ms))) return r;
     static const int cand[] = {1, 2, 4, 8, 16, 32};
     for (int k = 0; k < TCS_TUNE_COUNT; k++) {
-        if (k == TCS_TUNE_TL_STRIDED || k == TCS_TUNE_LONG_LINES || k == TCS_TUNE_Y_SOLVER || k == TCS_TUNE_Z_STAGING)
+        if (k == TCS_TUNE_TL_STRIDED || k == TCS_TUNE_TL_CONTIG || k == TCS_TUNE_LONG_LINES || k == TCS_TUNE_Y_SOLVER ||
+            k == TCS_TUNE_MIXED_ROWS || k == TCS_TUNE_Z_STAGING)
             continue;                                                 // without effect: nothing to time
         for (int v : cand) {
             if (v == best[k]) continue;

@@ -78,7 +78,7 @@ struct Shapes {
     int ifft_lines_x;                            // lines per block of the inverse x transform
     int lanes;                                   // at most this many partitions (lanes) per line
     int long_lines, y_solver;                    // accepted and kept; one solver runs the strided lines
-    int mixed_rows;                              // FP32-mixed form: 1 FP32 elimination + refinement in the x sweeps, 2, 4, 8 FP64 rows there
+    int mixed_rows;                              // likewise
     int z_staging;                               // likewise
     FFTPlan fp1, fp3;
     FFTPlan fp1u;                                // N1 with radices up to 8 (the inverse x transform's one-radix form)
@@ -166,35 +166,6 @@ inline void launch_lines(const Prob &p, const LinePlan &lp, dim3 grid, cudaStrea
     record_launch_error(kernel_name(kid));
 }
 
-// An FP32 x sweep whose rows are eliminated in FP64 (Shapes::mixed_rows): the
-// problem's own build in the field type, its coefficients widened to FP64 in
-// shared memory, the partitioned solve in FP64 without the refinement pass
-// (Refine<double> is off), and the solution rounded once to the field type when
-// the problem emits it.  Launch shape of the FP64 x sweeps.
-template <class P>
-struct FP64Rows : P {
-    using Real = double;
-    static constexpr int MINB = LineOcc<double>::x;
-    static constexpr int MREG = LineOcc<double>::reg_x;
-    static constexpr int NT = LineOcc<double>::nt_x;
-    __device__ Coef<double, P::NRHS> build(int l, int r, const typename P::State &st) const
-    {
-        const auto c = P::build(l, r, st);
-        Coef<double, P::NRHS> d;
-        d.a = c.a; d.b = c.b; d.c = c.c;
-#pragma unroll
-        for (int q = 0; q < P::NRHS; q++) d.d[q] = c.d[q];
-        return d;
-    }
-    __device__ void emit(int l, int r, const double *x, const typename P::State &st) const
-    {
-        typename P::Real xr[P::NRHS];
-#pragma unroll
-        for (int q = 0; q < P::NRHS; q++) xr[q] = (typename P::Real)x[q];
-        P::emit(l, r, xr, st);
-    }
-};
-
 // The shape of a marching sweep (march_block) of `lines` lines in all: TI lines
 // and NS segments of every line per block.  Rows per segment, m = n / NS: at
 // most P::ROWS, and at least 4, because every segment loads its first plane
@@ -275,6 +246,38 @@ inline void launch_march(const Shapes &cx, const P &prob, int n, bool cyclic, in
     const MarchPlan mp = march_plan<P>(n, cyclic, cx.lanes, (long long)nlines * gy);
     if (mp.lgTI + mp.lgNS > 8) launch_march_nt<512>(cx, prob, mp, nlines, gy, s, kid);
     else launch_march_nt<256>(cx, prob, mp, nlines, gy, s, kid);
+}
+
+// The shape of an x sweep: as many lines as two blocks per SM hold, segments for
+// 256 threads.
+template <class P>
+inline MarchPlan xmarch_plan(int n, int lanes)
+{
+    MarchPlan mp;
+    mp.n = n; mp.cyclic = 1;
+    const int cap = lanes < 32 ? lanes : 256;
+    for (mp.lgTI = 4;; mp.lgTI--) {
+        mp.lgNS = 1;
+        while (mp.lgNS + mp.lgTI < 8 && (2 << mp.lgNS) <= cap && (n >> (mp.lgNS + 1)) >= 4) mp.lgNS++;
+        while (mp.lgNS + mp.lgTI < 5) mp.lgNS++;          // whole warps
+        if (mp.lgTI == 0 || xmarch_words(n, 1 << mp.lgNS, 1 << mp.lgTI, P::WORDS) * sizeof(double) <= 113 * 1024) break;
+    }
+    mp.m0 = n >> mp.lgNS; mp.rem = n & ((1 << mp.lgNS) - 1);
+    return mp;
+}
+
+template <class P>
+inline void launch_xmarch(const Shapes &cx, const P &prob, int n, int nlines, int gy, cudaStream_t s, int kid)
+{
+    const MarchPlan mp = xmarch_plan<P>(n, cx.lanes);
+    const int TI = 1 << mp.lgTI;
+    const size_t smem = xmarch_words(n, 1 << mp.lgNS, TI, P::WORDS) * sizeof(double);
+    static size_t conf[64] = {};
+    smem_opt_in((const void *)xmarch_kernel<P>, smem, conf);
+    probe_begin(cx, kid, s);
+    xmarch_kernel<P><<<dim3((nlines + TI - 1) / TI, gy), TI << mp.lgNS, smem, s>>>(prob, mp);
+    probe_end(cx, kid, s);
+    record_launch_error(kernel_name(kid));
 }
 
 // ---------------------------------------------------------------------------
@@ -396,53 +399,6 @@ inline void march_stage(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStre
         cudaEventRecord(A.join[i], A.aux[i]);
         cudaStreamWaitEvent(s, A.join[i], 0);
     }
-}
-
-// Whether a case runs its x sweeps in the wide shape (the rule of launch_x).
-template <template <class, int, int> class X, class R>
-inline bool x_is_wide(const Ctx<R> &cx)
-{
-    if constexpr (LineOcc<R>::f32) return fit_tl<X<R, 0, 0>>(cx.g.N1, true, cx.tl_contig, cx.lanes) < 4;
-    return false;
-}
-
-// A multi-case x sweep: the cases split by shape, one launch per shape.
-template <template <class, int, int> class X, class R, class Lines>
-inline void multi_x(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s, const char *what, Lines lines)
-{
-    std::vector<Ctx<R> *> narrow, wide;
-    for (Ctx<R> *c : cs) (x_is_wide<X>(*c) ? wide : narrow).push_back(c);
-    auto shape = [&](const Ctx<R> &x) { return StageShape{x.g.N1, true, x.tl_contig, lines(x), x.g.N3}; };
-    multi_stage<X<R, 0, 1>>(narrow, A, s, what, shape, [](const Ctx<R> &x, int tl) { return X<R, 0, 1>{x.g, x.f, tl}; });
-    if constexpr (LineOcc<R>::f32)
-        multi_stage<X<R, 1, 1>>(wide, A, s, what, shape, [](const Ctx<R> &x, int tl) { return X<R, 1, 1>{x.g, x.f, tl}; });
-}
-
-// An x sweep: lines along i, one block row per (j-range, k).  FP32 runs the
-// 128-thread shape when at least 4 lines fit a block, else the wide shape;
-// with mixed_rows >= 2 the FP32-built rows are eliminated in FP64 instead.
-template <template <class, int, int> class X, class R>
-inline void launch_x(const Ctx<R> &cx, int nlines, cudaStream_t s, int kid)
-{
-    const GridT<R> &g = cx.g;
-    if constexpr (LineOcc<R>::f32) {
-        if (cx.mixed_rows >= 2) {   // FP32-built rows eliminated in FP64
-            using P = FP64Rows<X<R, 0, 0>>;
-            const LinePlan p = make_line_plan(g.N1, true, fit_tl<P>(g.N1, true, cx.tl_contig, cx.lanes), cx.lanes);
-            launch_lines(P{X<R, 0, 0>{g, cx.f, p.TL}}, p, dim3((nlines + p.TL - 1) / p.TL, g.N3), s, kid, cx);
-            return;
-        }
-    }
-    const int tl = fit_tl<X<R, 0, 0>>(g.N1, true, cx.tl_contig, cx.lanes);
-    if constexpr (LineOcc<R>::f32) {
-        if (tl < 4) {
-            const LinePlan p = make_line_plan(g.N1, true, fit_tl<X<R, 1, 0>>(g.N1, true, cx.tl_contig, cx.lanes), cx.lanes);
-            launch_lines(X<R, 1, 0>{g, cx.f, p.TL}, p, dim3((nlines + p.TL - 1) / p.TL, g.N3), s, kid, cx);
-            return;
-        }
-    }
-    const LinePlan p = make_line_plan(g.N1, true, tl, cx.lanes);
-    launch_lines(X<R, 0, 0>{g, cx.f, p.TL}, p, dim3((nlines + p.TL - 1) / p.TL, g.N3), s, kid, cx);
 }
 
 // Stage launchers (one per reference routine or fused group), instantiated

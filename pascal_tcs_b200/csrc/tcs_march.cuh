@@ -288,6 +288,104 @@ __global__ void __launch_bounds__(NT, Prob::TPS / NT) march_kernel(const __grid_
 }
 
 // ---------------------------------------------------------------------------
+// The x sweeps (lines contiguous in memory): the same march over lines held in
+// shared memory.  A block stages the inputs of TI lines (consecutive j at one k)
+// word plane by word plane, a warp per line with consecutive i in consecutive
+// lanes; thread (line l, segment s) marches over its rows there, parks d, c and e
+// in the places of the words it has used (planes 0, 1, 2), and the solution
+// leaves plane 0 as it came, a warp per line.  The line stride is odd, so the
+// TI lines of a warp's march sit on distinct banks.
+// The problem supplies
+//   static constexpr int WORDS;                                             // planes staged: 0 the right-hand side, 1.. the stencil
+//   struct Stage { Stage(const Prob &, int line, int by);  void put(const Prob &, int r, double *w, int PL); }   // row r of the line, words PL apart
+//   struct March { March(const Prob &, int line, int by, int r0, int m, int n, const double *w, int PL);  // reads across segment edges
+//                  void row(const Prob &, int r, bool last, const double *w, int PL, double &a, double &b, double &c, double &d); }
+//   lines(), out(line, by)                                                   // the row of the sweep scratch (i = 1)
+// ---------------------------------------------------------------------------
+__host__ __device__ __forceinline__ int xmarch_stride(int n) { return n | 1; }
+__host__ __device__ __forceinline__ size_t xmarch_words(int n, int NS, int TI, int words)
+{
+    return (size_t)words * TI * xmarch_stride(n) + (size_t)6 * NS * (TI + 1);
+}
+
+template <class Prob>
+__global__ void __launch_bounds__(256, 2) xmarch_kernel(const __grid_constant__ Prob prob, MarchPlan mp)
+{
+    using R = typename Prob::Real;
+    extern __shared__ __align__(16) double xsm[];
+    const bool skip = prob.skip();
+    const int n = mp.n, TI = 1 << mp.lgTI, NS = 1 << mp.lgNS, TP = TI + 1, LS = xmarch_stride(n), PL = TI * LS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, by = blockIdx.y;
+    const int line0 = blockIdx.x << mp.lgTI, nl = prob.lines();
+    double *const red = xsm + (size_t)Prob::WORDS * PL;
+    const int RS = NS * TP;
+    // a warp per line, or, with fewer lines than warps, nw / TI warps side by side on one
+    const int share = nw > TI ? nw >> mp.lgTI : 1;
+    auto stage = [&](int l, int first, int step) {
+        const typename Prob::Stage st(prob, min(line0 + l, nl - 1), by);
+        double *const w = xsm + l * LS;
+#pragma unroll Prob::UNROLL
+        for (int r = first; r < n; r += step) st.put(prob, r, w + r, PL);
+    };
+    if (share == 1)
+        for (int l = warp; l < TI; l += nw) stage(l, lane, 32);
+    else
+        stage(warp / share, lane + 32 * (warp % share), 32 * share);
+    __syncthreads();
+    const int l = threadIdx.x & (TI - 1), s = threadIdx.x >> mp.lgTI;
+    const int m = mp.m0 + (s < mp.rem ? 1 : 0), r0 = s * mp.m0 + min(s, mp.rem);
+    double *const w = xsm + l * LS;
+    {
+        typename Prob::March st(prob, min(line0 + l, nl - 1), by, r0, m, n, w, PL);
+        __syncthreads();                               // the words across segment edges have been read
+        double cp = 0.0, e = -1.0, p = 1.0, se = 0.0, dp = 0.0, sd = 0.0;
+        const int last = r0 + m - 1;
+        for (int r = r0; r <= last; r++) {
+            double a, b, c, d;
+            st.row(prob, r, r == last, w, PL, a, b, c, d);
+            const double rr = qrcp(fma(-a, cp, b));
+            e = -(a * rr) * e;
+            dp = fma(-a, dp, d) * rr;
+            cp = c * rr;
+            if (r < last) {
+                w[r] = dp; w[PL + r] = cp; w[2 * PL + r] = e;
+                sd = fma(p, dp, sd);
+                se = fma(p, e, se);
+                p = -p * cp;
+            }
+        }
+        double *const o = red + s * TP + l;
+        o[0] = e; o[RS] = cp; o[2 * RS] = se; o[3 * RS] = p; o[4 * RS] = dp; o[5 * RS] = sd;
+    }
+    __syncthreads();
+    march_reduce<1>(red, mp.lgNS, TP, true);
+    {
+        double x = red[s * TP + l];
+        const double xp = red[((s - 1) & (NS - 1)) * TP + l];
+        int r = r0 + m - 1;
+        w[r] = x;
+        for (r--; r - 3 >= r0; r -= 4) {
+            double c[4], y[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) { c[t] = w[PL + r - t]; y[t] = fma(-w[2 * PL + r - t], xp, w[r - t]); }
+#pragma unroll
+            for (int t = 0; t < 4; t++) { x = fma(-c[t], x, y[t]); w[r - t] = x; }
+        }
+        for (; r >= r0; r--) {
+            x = fma(-w[PL + r], x, fma(-w[2 * PL + r], xp, w[r]));
+            w[r] = x;
+        }
+    }
+    __syncthreads();
+    if (skip) return;
+    for (int q = warp / share; q < TI && line0 + q < nl; q += nw / share) {
+        R *const o = prob.out(line0 + q, by);
+        const double *const v = xsm + q * LS;
+        for (int r = lane + 32 * (warp % share); r < n; r += 32 * share) o[r] = R(v[r]);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // The column form (FP64, z lines): a block of w consecutive i marches up NS
 // segments of the lines together (w NS threads; NS = 1 where there are lines
 // enough).  The rows of i that a plane needs (the problem's stream: its arrays

@@ -206,42 +206,77 @@ struct DUZ {
     };
 };
 
-template <class R, int WIDE = 0, int ITEM = 0>
+template <class R>
 struct DUX {
     using Real = R;
-    static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = true;    // measured faster with qrcp
-    static constexpr int MINB = WIDE ? LineOcc<R>::xw : LineOcc<R>::x;
-    static constexpr int MREG = WIDE ? LineOcc<Real>::reg_xw : LineOcc<Real>::reg_x;
-    static constexpr int NT = WIDE ? LineOcc<Real>::nt_xw : LineOcc<Real>::nt_x;
-    static constexpr bool CONTIG = true;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr int WORDS = 3, UNROLL = 4;
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt; };
-    __device__ State prepare() const { return State{R(g.scal[S_DT])}; }
-    __device__ int lj(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return lj(l) <= g.N2; }
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
+    __device__ int lines() const { return g.N2; }
+    __device__ R *out(int line, int by) const { return f.scr + ix(g, 1, 1 + line, 1 + by); }
+    struct Stage {
+        long long c;
+        __device__ __forceinline__ Stage(const DUX &q, int line, int by) : c(ix(q.g, 1, 1 + line, 1 + by)) {}
+        __device__ __forceinline__ void put(const DUX &q, int r, double *w, int PL) const
+        {
+            w[0] = (double)q.f.scr[c + r];
+            w[PL] = (double)ld(q.f.U + c + r);
+        }
+    };
+    struct March {
+        R mu, h, dt, Uc, Un, A, B, C;                   // Un: U beyond the segment; A, B, C: the cell below the row
+        __device__ __forceinline__ March(const DUX &q, int line, int by, int r0, int m, int n, const double *w, int PL)
+        {
+            const int t4 = 4 * ix2(q.g, 1 + line, 1 + by);
+            mu = ld(q.f.MuT + t4);
+            h = q.g.ph.Cmu * ld(q.f.iRT + t4);
+            dt = R(q.g.scal[S_DT]);
+            Uc = R(w[PL + r0]);
+            Un = R(w[PL + (r0 + m < n ? r0 + m : 0)]);
+            cell(R(w[PL + (r0 ? r0 - 1 : n - 1)]), Uc, ld(q.g.m1.rdx + r0));
+        }
+        __device__ __forceinline__ void cell(R Um, R Up, R rdx1)
+        {
+            A = mu * rdx1;
+            B = R(0.125) * (Um + Up) * rdx1;
+            C = R(0.125) * (Up - Um) * rdx1;
+        }
+        __device__ __forceinline__ void row(const DUX &q, int r, bool last, const double *w, int PL, double &a, double &b, double &c, double &d)
+        {
+            const R rdx1 = ld(q.g.m1.rdx + r + 1), hd = h * ld(q.g.m1.rdmx + r + 1);
+            const R Up = last ? Un : R(w[PL + r + 1]);
+            const R A1 = A, B1 = B, C1 = C, U0 = Uc;
+            Uc = Up;
+            cell(U0, Up, rdx1);
+            const R am = (C1 - B1 - hd * A1) * dt, ap = (B + C - hd * A) * dt;
+            a = am; c = ap; b = (1.0 - ((double)am + (double)ap)) + (double)(R(2) * (C1 + C) * dt);
+            d = w[r];
+        }
+    };
+};
+
+// The rows along x of V and W: face velocities U averaged to the line (word 1)
+// and one pair of viscosities, the mu1 and mu2 left by the last cell of stage 1.
+template <class R>
+struct FaceRows {
+    R mu1, mu2, h, dt, un, w1, rdm;                     // un: the face velocity beyond the segment; w1, rdm: the face below the row
+    __device__ __forceinline__ void begin(const GridT<R> &g, R ih, int r0, int m, int n, const double *w, int PL)
     {
-        const int i = r + 1, j = lj(l), k = 1 + vby<ITEM>(), im = i - 1;
-        const PhysT<R> &p = g.ph;
-        const R *dx1 = g.m1.dx, *rdx1 = g.m1.rdx, *rdmx1 = g.m1.rdmx;
-        const long long c = ix(g, i, j, k);
-        const R Uc = ld(f.U + c), Uxm = ld(f.U + c - 1), Uxp = ld(f.U + c + 1);
-        const R Mjk = MU(j, k), iRjk = IR(j, k);
-        const R u1 = R(0.5) * (Uxm + Uc), u2 = R(0.5) * (Uxp + Uc);
-        const R dudx1 = (Uc - Uxm) * rdx1[im], dudx2 = (Uxp - Uc) * rdx1[i];
-        const R invRhoc = R(0.5) * (dx1[im] * iRjk + dx1[i] * iRjk) * rdmx1[i];
-        const R ih = R(0.5) * p.Cmu * invRhoc;
-        const R mACI = ih * rdmx1[i] * (Mjk * rdx1[i] + Mjk * rdx1[im]) * R(2.0) + R(0.25) * (dudx2 * R(0.5) + dudx1 * R(0.5) - u2 * rdx1[i] + u1 * rdx1[im]);
-        const R mAPI = -ih * rdmx1[i] * Mjk * rdx1[i] * R(2.0) + R(0.25) * (u2 * rdx1[i] + dudx2 * R(0.5));
-        const R mAMI = -ih * rdmx1[i] * Mjk * rdx1[im] * R(2.0) + R(0.25) * (-u1 * rdx1[im] + dudx1 * R(0.5));
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = mACI * dt + R(1.0); cf.c = mAPI * dt; cf.a = mAMI * dt; cf.d[0] = ld(f.scr + c);
-        return cf;
+        h = ih;
+        dt = R(g.scal[S_DT]);
+        un = R(w[PL + (r0 + m < n ? r0 + m : 0)]);
+        rdm = ld(g.m1.rdmx + r0 + 1);
+        w1 = R(0.25) * R(w[PL + r0]) * rdm;
     }
-    __device__ void emit(int l, int r, const R *x, const State &st) const { f.scr[ix(g, r + 1, lj(l), 1 + vby<ITEM>())] = x[0]; }
+    __device__ __forceinline__ void rows(const GridT<R> &g, int r, bool last, const double *w, int PL, double &a, double &b, double &c, double &d)
+    {
+        const R rdp = ld(g.m1.rdmx + r + 2), hd = h * ld(g.m1.rdx + r + 1);
+        const R w2 = R(0.25) * (last ? un : R(w[PL + r + 1])) * rdp;
+        const R am = -(hd * (mu1 * rdm) + w1) * dt, ap = (w2 - hd * (mu2 * rdp)) * dt;
+        a = am; c = ap; b = 1.0 - ((double)am + (double)ap);
+        d = w[r];
+        w1 = w2; rdm = rdp;
+    }
 };
 
 template <class R>
@@ -448,47 +483,37 @@ __device__ __forceinline__ void dv_stale_mu12(const GridT<R> &g, const FieldsT<R
     mu2 = R(0.5) * (dx1[ip] * mxy + dx1[i] * mxy) * rdmx1[ip];
 }
 
-template <class R, int WIDE = 0, int ITEM = 0>
+template <class R>
 struct DVX {
     using Real = R;
-    static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = true;    // measured faster with qrcp
-    static constexpr int MINB = WIDE ? LineOcc<R>::xw : LineOcc<R>::x;
-    static constexpr int MREG = WIDE ? LineOcc<Real>::reg_xw : LineOcc<Real>::reg_x;
-    static constexpr int NT = WIDE ? LineOcc<Real>::nt_xw : LineOcc<Real>::nt_x;
-    static constexpr bool CONTIG = true;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr int WORDS = 3, UNROLL = 4;
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt, mu1, mu2; };
-    __device__ State prepare() const
-    {
-        State s;
-        s.dt = g.scal[S_DT];
-        dv_stale_mu12(g, f, s.mu1, s.mu2);
-        return s;
-    }
-    __device__ int lj(int l) const { return 2 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return lj(l) <= g.N2; }
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
-    {
-        const int i = r + 1, j = lj(l), k = 1 + vby<ITEM>(), ip = i + 1, jm = j - 1;
-        const PhysT<R> &p = g.ph;
-        const R *dx2 = g.m2.dx, *rdx1 = g.m1.rdx, *rdmx1 = g.m1.rdmx, *rdmx2 = g.m2.rdmx;
-        const long long c = ix(g, i, j, k), sj = g.P1;
-        const R mu1 = st.mu1, mu2 = st.mu2;
-        const R u1 = (dx2[jm] * ld(f.U + c) + dx2[j] * ld(f.U + c - sj)) * rdmx2[j] * R(0.5);
-        const R u2 = (dx2[jm] * ld(f.U + c + 1) + dx2[j] * ld(f.U + c + 1 - sj)) * rdmx2[j] * R(0.5);
-        const R invRhoc = R(0.5) * (dx2[jm] * IR(j, k) + dx2[j] * IR(jm, k)) * rdmx2[j];
-        const R ih = R(0.5) * p.Cmu * invRhoc;
-        const R mACI = ih * rdx1[i] * (mu2 * rdmx1[ip] + mu1 * rdmx1[i]) + R(0.25) * (-u2 * rdmx1[ip] + u1 * rdmx1[i]);
-        const R mAPI = -ih * rdx1[i] * mu2 * rdmx1[ip] + R(0.25) * (u2 * rdmx1[ip]);
-        const R mAMI = -ih * rdx1[i] * mu1 * rdmx1[i] + R(0.25) * (-u1 * rdmx1[i]);
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = mACI * dt + R(1.0); cf.c = mAPI * dt; cf.a = mAMI * dt; cf.d[0] = ld(f.scr + c);
-        return cf;
-    }
-    __device__ void emit(int l, int r, const R *x, const State &st) const { f.scr[ix(g, r + 1, lj(l), 1 + vby<ITEM>())] = x[0]; }
+    __device__ int lines() const { return g.N2 - 1; }
+    __device__ R *out(int line, int by) const { return f.scr + ix(g, 1, 2 + line, 1 + by); }
+    struct Stage {
+        long long c;
+        R cy;
+        __device__ __forceinline__ Stage(const DVX &q, int line, int by)
+            : c(ix(q.g, 1, 2 + line, 1 + by)), cy(R(0.5) * ld(q.g.m2.dx + 1 + line) * ld(q.g.m2.rdmx + 2 + line)) {}
+        __device__ __forceinline__ void put(const DVX &q, int r, double *w, int PL) const
+        {
+            w[0] = (double)q.f.scr[c + r];
+            const R U0 = ld(q.f.U + c + r), Um = ld(q.f.U + c + r - q.g.P1);
+            w[PL] = (double)(Um + cy * (U0 - Um));
+        }
+    };
+    struct March : FaceRows<R> {
+        __device__ __forceinline__ March(const DVX &q, int line, int by, int r0, int m, int n, const double *w, int PL)
+        {
+            dv_stale_mu12(q.g, q.f, this->mu1, this->mu2);
+            this->begin(q.g, R(0.5) * q.g.ph.Cmu * ld(q.f.iRT + 4 * ix2(q.g, 2 + line, 1 + by) + 1), r0, m, n, w, PL);
+        }
+        __device__ __forceinline__ void row(const DVX &q, int r, bool last, const double *w, int PL, double &a, double &b, double &c, double &d)
+        {
+            this->rows(q.g, r, last, w, PL, a, b, c, d);
+        }
+    };
 };
 
 template <class R>
@@ -713,48 +738,38 @@ __device__ __forceinline__ void dw_stale_mu(const GridT<R> &g, const FieldsT<R> 
     mu4 = R(0.5) * (dx2[jp] * mxz + dx2[j] * mub) * rdmx2[jp];
 }
 
-template <class R, int WIDE = 0, int ITEM = 0>
+template <class R>
 struct DWX {
     using Real = R;
-    static constexpr int NRHS = 1;
-    static constexpr bool FAST_RCP = true;    // measured faster with qrcp
-    static constexpr int MINB = WIDE ? LineOcc<R>::xw : LineOcc<R>::x;
-    static constexpr int MREG = WIDE ? LineOcc<Real>::reg_xw : LineOcc<Real>::reg_x;
-    static constexpr int NT = WIDE ? LineOcc<Real>::nt_xw : LineOcc<Real>::nt_x;
-    static constexpr bool CONTIG = true;
-    GridT<R> g; FieldsT<R> f; int TL;
+    static constexpr int WORDS = 3, UNROLL = 4;
+    GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
-    struct State { R dt, mu1, mu2, mu3, mu4; };
-    __device__ State prepare() const
-    {
-        State s;
-        s.dt = g.scal[S_DT];
-        dw_stale_mu(g, f, s.mu1, s.mu2, s.mu3, s.mu4);
-        return s;
-    }
-    __device__ int lj(int l) const { return 1 + vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return lj(l) <= g.N2; }
-    __device__ Coef<R, 1> build(int l, int r, const State &st) const
-    {
-        const int i = r + 1, j = lj(l), k = 1 + vby<ITEM>(), ip = i + 1, km = k - 1;
-        const PhysT<R> &p = g.ph;
-        const R *dx3 = g.m3.dx, *rdx1 = g.m1.rdx, *rdmx1 = g.m1.rdmx, *rdmx3 = g.m3.rdmx;
-        const long long c = ix(g, i, j, k), sk = (long long)g.P1 * g.P2;
-        const R mu1 = st.mu1, mu2 = st.mu2, mu3 = st.mu3, mu4 = st.mu4;
-        (void)mu1; (void)mu2; (void)mu3; (void)mu4;
-        const R u1 = (dx3[km] * ld(f.U + c) + dx3[k] * ld(f.U + c - sk)) * rdmx3[k] * R(0.5);
-        const R u2 = (dx3[km] * ld(f.U + c + 1) + dx3[k] * ld(f.U + c + 1 - sk)) * rdmx3[k] * R(0.5);
-        const R invRhoc = R(0.5) * (dx3[km] * IR(j, k) + dx3[k] * IR(j, km)) * rdmx3[k];
-        const R ih = R(0.5) * p.Cmu * invRhoc;
-        const R mACI = ih * rdx1[i] * (mu2 * rdmx1[ip] + mu1 * rdmx1[i]) + R(0.25) * (-u2 * rdmx1[ip] + u1 * rdmx1[i]);
-        const R mAPI = -ih * rdx1[i] * mu2 * rdmx1[ip] + R(0.25) * (u2 * rdmx1[ip]);
-        const R mAMI = -ih * rdx1[i] * mu1 * rdmx1[i] + R(0.25) * (-u1 * rdmx1[i]);
-        const R dt = st.dt;
-        Coef<R, 1> cf;
-        cf.b = mACI * dt + R(1.0); cf.c = mAPI * dt; cf.a = mAMI * dt; cf.d[0] = ld(f.scr + c);
-        return cf;
-    }
-    __device__ void emit(int l, int r, const R *x, const State &st) const { f.scr[ix(g, r + 1, lj(l), 1 + vby<ITEM>())] = x[0]; }
+    __device__ int lines() const { return g.N2; }
+    __device__ R *out(int line, int by) const { return f.scr + ix(g, 1, 1 + line, 1 + by); }
+    struct Stage {
+        long long c, sk;
+        R cz;
+        __device__ __forceinline__ Stage(const DWX &q, int line, int by)
+            : c(ix(q.g, 1, 1 + line, 1 + by)), sk((long long)q.g.P1 * q.g.P2), cz(R(0.5) * ld(q.g.m3.dx + by) * ld(q.g.m3.rdmx + 1 + by)) {}
+        __device__ __forceinline__ void put(const DWX &q, int r, double *w, int PL) const
+        {
+            w[0] = (double)q.f.scr[c + r];
+            const R U0 = ld(q.f.U + c + r), Um = ld(q.f.U + c + r - sk);
+            w[PL] = (double)(Um + cz * (U0 - Um));
+        }
+    };
+    struct March : FaceRows<R> {
+        __device__ __forceinline__ March(const DWX &q, int line, int by, int r0, int m, int n, const double *w, int PL)
+        {
+            R mu3, mu4;
+            dw_stale_mu(q.g, q.f, this->mu1, this->mu2, mu3, mu4);
+            this->begin(q.g, R(0.5) * q.g.ph.Cmu * ld(q.f.iRT + 4 * ix2(q.g, 1 + line, 1 + by) + 2), r0, m, n, w, PL);
+        }
+        __device__ __forceinline__ void row(const DWX &q, int r, bool last, const double *w, int PL, double &a, double &b, double &c, double &d)
+        {
+            this->rows(q.g, r, last, w, PL, a, b, c, d);
+        }
+    };
 };
 
 template <class R>
@@ -850,10 +865,28 @@ static void launch_dw_y(const Ctx<R> &cx, cudaStream_t s)
 }
 
 template <class R>
+static void launch_du_x(const Ctx<R> &cx, cudaStream_t s)
+{
+    launch_xmarch(cx, DUX<R>{cx.g, cx.f}, cx.g.N1, cx.g.N2, cx.g.N3, s, K_DU_X);
+}
+
+template <class R>
+static void launch_dv_x(const Ctx<R> &cx, cudaStream_t s)
+{
+    launch_xmarch(cx, DVX<R>{cx.g, cx.f}, cx.g.N1, cx.g.N2 - 1, cx.g.N3, s, K_DV_X);
+}
+
+template <class R>
+static void launch_dw_x(const Ctx<R> &cx, cudaStream_t s)
+{
+    launch_xmarch(cx, DWX<R>{cx.g, cx.f}, cx.g.N1, cx.g.N2, cx.g.N3, s, K_DW_X);
+}
+
+template <class R>
 void launch_solve_du(const Ctx<R> &cx, cudaStream_t s)
 {
     launch_du_z(cx, s);
-    launch_x<DUX>(cx, cx.g.N2, s, K_DU_X);
+    launch_du_x(cx, s);
     launch_du_y(cx, s);
 }
 
@@ -861,7 +894,7 @@ template <class R>
 void launch_solve_dv(const Ctx<R> &cx, cudaStream_t s)
 {
     launch_dv_z(cx, s);
-    launch_x<DVX>(cx, cx.g.N2 - 1, s, K_DV_X);
+    launch_dv_x(cx, s);
     launch_dv_y(cx, s);
 }
 
@@ -869,7 +902,7 @@ template <class R>
 void launch_solve_dw(const Ctx<R> &cx, cudaStream_t s)
 {
     launch_dw_z(cx, s);
-    launch_x<DWX>(cx, cx.g.N2, s, K_DW_X);
+    launch_dw_x(cx, s);
     launch_dw_y(cx, s);
 }
 
@@ -1028,15 +1061,14 @@ void launch_pseudo_update(const Ctx<R> &cx, cudaStream_t s)
 template <class R>
 void launch_momentum_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s)
 {
-    auto lines = [](int ny) { return [ny](const Ctx<R> &x) { return x.g.N2 - ny; }; };
     march_stage(cs, A, s, launch_du_z<R>);
-    multi_x<DUX>(cs, A, s, "du_x", lines(0));
+    march_stage(cs, A, s, launch_du_x<R>);
     march_stage(cs, A, s, launch_du_y<R>);
     march_stage(cs, A, s, launch_dv_z<R>);
-    multi_x<DVX>(cs, A, s, "dv_x", lines(1));
+    march_stage(cs, A, s, launch_dv_x<R>);
     march_stage(cs, A, s, launch_dv_y<R>);
     march_stage(cs, A, s, launch_dw_z<R>);
-    multi_x<DWX>(cs, A, s, "dw_x", lines(0));
+    march_stage(cs, A, s, launch_dw_x<R>);
     march_stage(cs, A, s, launch_dw_y<R>);
 }
 
