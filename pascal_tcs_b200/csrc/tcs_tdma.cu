@@ -23,9 +23,23 @@ namespace tcs {
 #define ADD(a, b) __dadd_rn((a), (b))
 #define DIV(a, b) __ddiv_rn((a), (b))
 
-__global__ void tdma_many_kernel(double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C,
-                                 double *__restrict__ D, int n_sys, int n_row, int cyclic)
+// 1 / x correctly rounded: the same bits as the division.
+#define RCP(x) __drcp_rn(x)
+
+// One system per thread, three marches over its rows (17 passes over an array in
+// all).  Every row's loads are independent of the recurrences, so the first two
+// marches keep the next NB rows on their way while they work on NB; the last has
+// no recurrence at all.  Measured on B200, from a thread that waited for each
+// row's loads: 65536 systems of 256 rows 856 -> 351 us (2.7 -> 6.5 TB/s of those
+// passes), 30000 of 333 rows 1038 -> 264 us, 4096 of 64 rows 71 -> 31 us; NB = 4
+// 351, 301, 31 us; NB = 8 spills at the 128 registers that eight blocks leave.
+// 64 threads per block: 65536 systems are 6.9 blocks per SM.
+constexpr int TDMA_NT = 64, TDMA_NB = 6;
+
+__global__ void __launch_bounds__(TDMA_NT, 8) tdma_many_kernel(double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C,
+                                                            double *__restrict__ D, int n_sys, int n_row, int cyclic)
 {
+    constexpr int NB = TDMA_NB;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_sys) return;
     const size_t s = (size_t)n_sys;
@@ -34,31 +48,65 @@ __global__ void tdma_many_kernel(double *__restrict__ A, const double *__restric
 #define c(j) C[(size_t)i + s * (size_t)(j)]
 #define d(j) D[(size_t)i + s * (size_t)(j)]
     double r;
-    a(0) = DIV(a(0), b(0)); d(0) = DIV(d(0), b(0)); c(0) = DIV(c(0), b(0));
-    a(1) = DIV(a(1), b(1)); d(1) = DIV(d(1), b(1)); c(1) = DIV(c(1), b(1));
-    double am1 = a(1), cm1 = c(1), dm1 = d(1);
-    for (int j = 2; j < n_row; j++) {
-        const double aj = a(j);
-        r = DIV(1.0, SUB(b(j), MUL(aj, cm1)));
-        dm1 = MUL(r, SUB(d(j), MUL(aj, dm1))); d(j) = dm1;
-        cm1 = MUL(r, c(j)); c(j) = cm1;
-        am1 = MUL(MUL(-r, aj), am1); a(j) = am1;
+    double va[NB], vb[NB], vc[NB], vd[NB];
+    auto load = [&](int j) {                           // rows j, j + 1, .. below n_row
+#pragma unroll
+        for (int q = 0; q < NB; q++)
+            if (j + q < n_row) { va[q] = a(j + q); vb[q] = b(j + q); vc[q] = c(j + q); vd[q] = d(j + q); }
+    };
+    load(2);
+    const double a0 = DIV(a(0), b(0)), d0 = DIV(d(0), b(0)), c0 = DIV(c(0), b(0));
+    double am1 = DIV(a(1), b(1)), dm1 = DIV(d(1), b(1)), cm1 = DIV(c(1), b(1));
+    a(0) = a0; d(0) = d0; c(0) = c0;
+    a(1) = am1; d(1) = dm1; c(1) = cm1;
+    for (int j = 2; j < n_row; j += NB) {
+        double ua[NB], ub[NB], uc[NB], ud[NB];
+#pragma unroll
+        for (int q = 0; q < NB; q++) { ua[q] = va[q]; ub[q] = vb[q]; uc[q] = vc[q]; ud[q] = vd[q]; }
+        load(j + NB);
+#pragma unroll
+        for (int q = 0; q < NB; q++)
+            if (j + q < n_row) {
+                const double aj = ua[q];
+                r = RCP(SUB(ub[q], MUL(aj, cm1)));
+                dm1 = MUL(r, SUB(ud[q], MUL(aj, dm1))); d(j + q) = dm1;
+                cm1 = MUL(r, uc[q]); c(j + q) = cm1;
+                am1 = MUL(MUL(-r, aj), am1); a(j + q) = am1;
+            }
     }
+    auto load_down = [&](int j) {                      // rows j, j - 1, .. above 0
+#pragma unroll
+        for (int q = 0; q < NB; q++)
+            if (j - q >= 1) { va[q] = a(j - q); vc[q] = c(j - q); vd[q] = d(j - q); }
+    };
+    double a1 = a(1), c1 = c(1), d1 = d(1);            // row 1 as the closure needs it
     if (n_row >= 3) {
         double ap1 = a(n_row - 2), cp1 = c(n_row - 2), dp1 = d(n_row - 2);
-        for (int j = n_row - 3; j >= 1; j--) {
-            const double cj = c(j);
-            dp1 = SUB(d(j), MUL(cj, dp1)); d(j) = dp1;
-            ap1 = SUB(a(j), MUL(cj, ap1)); a(j) = ap1;
-            cp1 = MUL(-cj, cp1); c(j) = cp1;
+        load_down(n_row - 3);
+        for (int j = n_row - 3; j >= 1; j -= NB) {
+            double ua[NB], uc[NB], ud[NB];
+#pragma unroll
+            for (int q = 0; q < NB; q++) { ua[q] = va[q]; uc[q] = vc[q]; ud[q] = vd[q]; }
+            load_down(j - NB);
+#pragma unroll
+            for (int q = 0; q < NB; q++)
+                if (j - q >= 1) {
+                    const double cj = uc[q];
+                    dp1 = SUB(ud[q], MUL(cj, dp1)); d(j - q) = dp1;
+                    ap1 = SUB(ua[q], MUL(cj, ap1)); a(j - q) = ap1;
+                    cp1 = MUL(-cj, cp1); c(j - q) = cp1;
+                }
         }
+        a1 = ap1; c1 = cp1; d1 = dp1;
     }
-    r = DIV(1.0, SUB(1.0, MUL(a(1), c(0))));
-    d(0) = MUL(r, SUB(d(0), MUL(c(0), d(1))));
-    a(0) = MUL(r, a(0));
-    c(0) = MUL(MUL(-r, c(0)), c(1));
-    const double A1 = a(0), C1 = c(0), D1 = d(0);
     const double A2 = a(n_row - 1), C2 = c(n_row - 1), D2 = d(n_row - 1);
+    if (n_row == 2) { a1 = A2; c1 = C2; d1 = D2; }
+    r = DIV(1.0, SUB(1.0, MUL(a1, c0)));
+    const double D1 = MUL(r, SUB(d0, MUL(c0, d1)));
+    const double A1 = MUL(r, a0);
+    const double C1 = MUL(MUL(-r, c0), c1);
+    a(0) = A1;
+    c(0) = C1;
     double x1, x2;
     if (cyclic) {
         const double e2 = -C2;
@@ -71,13 +119,21 @@ __global__ void tdma_many_kernel(double *__restrict__ A, const double *__restric
     }
     d(0) = x1;
     d(n_row - 1) = x2;
-    for (int j = 1; j < n_row - 1; j++) d(j) = SUB(SUB(d(j), MUL(a(j), x1)), MUL(c(j), x2));
+    for (int j = 1; j < n_row - 1; j += NB) {
+#pragma unroll
+        for (int q = 0; q < NB; q++)
+            if (j + q < n_row - 1) { va[q] = a(j + q); vc[q] = c(j + q); vd[q] = d(j + q); }
+#pragma unroll
+        for (int q = 0; q < NB; q++)
+            if (j + q < n_row - 1) d(j + q) = SUB(SUB(vd[q], MUL(va[q], x1)), MUL(vc[q], x2));
+    }
 #undef a
 #undef b
 #undef c
 #undef d
 }
 
+#undef RCP
 #undef MUL
 #undef SUB
 #undef ADD
@@ -85,7 +141,7 @@ __global__ void tdma_many_kernel(double *__restrict__ A, const double *__restric
 
 void launch_tdma_many(double *A, const double *B, double *C, double *D, int n_sys, int n_row, int cyclic, cudaStream_t s)
 {
-    tdma_many_kernel<<<(n_sys + 127) / 128, 128, 0, s>>>(A, B, C, D, n_sys, n_row, cyclic);
+    tdma_many_kernel<<<(n_sys + TDMA_NT - 1) / TDMA_NT, TDMA_NT, 0, s>>>(A, B, C, D, n_sys, n_row, cyclic);
     record_launch_error("tdma_many");
 }
 
@@ -189,7 +245,7 @@ extern "C" int tcs_tdma_many_solve_noalloc(double *A, double *B, double *C, doub
         (e = cudaMemcpy(dC, C, bytes, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(dD, D, bytes, cudaMemcpyHostToDevice)) != cudaSuccess)
         return set_error(TCS_ERR_CUDA, std::string("cudaMemcpy to the static scratch: ") + cudaGetErrorString(e));
-    tdma_many_kernel<<<(n_sys + 127) / 128, 128, 0, 0>>>(dA, dB, dC, dD, n_sys, n_row, cyclic ? 1 : 0);
+    tdma_many_kernel<<<(n_sys + TDMA_NT - 1) / TDMA_NT, TDMA_NT, 0, 0>>>(dA, dB, dC, dD, n_sys, n_row, cyclic ? 1 : 0);
     if ((e = cudaGetLastError()) != cudaSuccess) return set_error(TCS_ERR_CUDA, std::string("tdma_many launch: ") + cudaGetErrorString(e));
     if ((e = cudaMemcpy(A, dA, bytes, cudaMemcpyDeviceToHost)) != cudaSuccess ||
         (e = cudaMemcpy(C, dC, bytes, cudaMemcpyDeviceToHost)) != cudaSuccess ||

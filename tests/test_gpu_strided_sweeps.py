@@ -44,3 +44,20 @@ def test_strided_sweeps_match_oracle(n, precision):
         err = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300)
         assert np.all(np.isfinite(a)) and err <= (1e-10 if precision == 0 else 1e-5), (f, err)
     g.close()
+
+
+@pytest.mark.parametrize("cyclic", [False, True])
+@pytest.mark.parametrize("n_sys,n_row", [(1, 2), (63, 3), (64, 4), (65, 7), (200, 8), (129, 9), (70, 14), (130, 15), (66, 61)])
+def test_tdma_many_bits_at_the_edges_of_its_prefetch(n_sys, n_row, cyclic):
+    # rows around multiples of the rows loaded ahead, systems around a block: the bits of the strict evaluation
+    import pascal_tcs_b200 as P
+    from oracle import oracle as O
+
+    rng = np.random.default_rng(100 * n_sys + n_row)
+    A, C, D = (rng.uniform(-0.4, 0.4, (n_row, n_sys)) for _ in range(3))
+    B = 1.0 + rng.uniform(0.0, 1.0, (n_row, n_sys))
+    ref = O.tdma_many(A, B, C, D, cyclic=cyclic)
+    Ag, Bg, Cg, Dg = A.copy(), B.copy(), C.copy(), D.copy()
+    plan = P.TdmaPlan(n_sys)
+    (plan.many_solve_cycle if cyclic else plan.many_solve)(Ag, Bg, Cg, Dg, n_sys, n_row)
+    np.testing.assert_array_equal(Dg, ref)
