@@ -52,10 +52,9 @@ typedef struct tcs_config {
 } tcs_config;
 
 /* numerical forms (tcs_config.precision).  FP32_MIXED stores the fields in FP32
- * and runs stencils, ADI sweeps and FFTs in FP32 with one FP64-residual
- * refinement pass per tridiagonal system; the modal pressure solves, the
- * pressure right-hand side, the projection and every reduction compute in
- * FP64.  The host interface moves FP64 arrays in both forms. */
+ * and builds the ADI rows in FP32; their elimination, the FFTs, the modal
+ * pressure solves, the pressure right-hand side, the projection and every
+ * reduction compute in FP64.  The host interface moves FP64 arrays in both forms. */
 enum { TCS_PREC_FP64 = 0, TCS_PREC_FP32_MIXED = 1 };
 
 /* field identifiers */
@@ -181,10 +180,9 @@ int tcs_extract_plane(tcs_ctx *ctx, int axis, int index, int nfields, const int 
 /* Ensembles (no counterpart in the reference, which runs one case per MPI job):
  * independent cases on one device advanced together.  Every tcs_ensemble_step
  * replays one CUDA graph per step, in one of two forms:
- *   batched (1): each line sweep (thermal, solvedU/V/W, the modal Poisson
- *     solves) is ONE launch over all cases (up to a parameter block's worth of
- *     cases per launch), a persistent grid whose blocks pull (case, block)
- *     work items; the kernels between the sweeps run as one branch per case;
+ *   batched (1): stage by stage, the line sweeps (thermal, solvedU/V/W, the
+ *     modal Poisson solves) of all cases side by side, joined after each
+ *     sweep; the kernels between the sweeps run as one branch per case;
  *   branch per case (0): every case's whole step is its own graph branch.
  * Both give results bit-identical to stepping each case alone.  The default,
  * auto (-1), runs the first 8 steps (real steps) 4 in each form, times the
@@ -232,18 +230,15 @@ const char *tcs_timer_name(int timer);
 int tcs_bounds_checked(void);
 int tcs_bounds_violations(tcs_ctx *ctx, double *count);
 int tcs_set_use_graph(tcs_ctx *ctx, int on);
-/* launch-shape knobs (powers of two): lines per thread block of the modal line
- * solver and of the x and z FFTs, and the most lanes (partitions) a tridiagonal
- * line is split over (32: no bound for the x, y and z sweeps, whose segments
- * follow the line's length).  A line-solver value is an upper bound: each
- * launch runs the largest power of two up to it whose blocks fit the SM's
- * shared memory at the family's blocks per SM; a value no single block could
- * hold is refused (TCS_ERR_ARG).
- * TCS_TUNE_TL_STRIDED, TCS_TUNE_TL_CONTIG, TCS_TUNE_LONG_LINES (1, 2, 4),
- * TCS_TUNE_Y_SOLVER (1, 2, 4), TCS_TUNE_MIXED_ROWS (1, 2, 4, 8) and
- * TCS_TUNE_Z_STAGING (1, 2) chose between forms of the x, y and z sweeps that one
- * solver, with FP64 elimination, has replaced.  Their values are checked, kept
- * and returned as before, without effect.
+/* launch-shape knobs (powers of two): lines per thread block of the x and z
+ * FFTs, and the most partitions a tridiagonal line is split over (TCS_TUNE_LANES;
+ * 32: no bound, a line's length decides).
+ * TCS_TUNE_TL_STRIDED, TCS_TUNE_TL_CONTIG, TCS_TUNE_TL_MODAL, TCS_TUNE_LONG_LINES
+ * (1, 2, 4), TCS_TUNE_Y_SOLVER (1, 2, 4), TCS_TUNE_MIXED_ROWS (1, 2, 4, 8) and
+ * TCS_TUNE_Z_STAGING (1, 2) chose between forms and shapes of the line solvers
+ * that one solver, with FP64 elimination and shapes of its own, has replaced.
+ * Their values are checked (TCS_ERR_ARG), kept and returned as before, without
+ * effect.
  * TCS_TUNE_IFFT_LINES_X: lines per block of the inverse x transform
  * (TCS_TUNE_FFT_LINES_X sets those of the pressure right-hand side and its
  * forward x transform). */

@@ -569,6 +569,7 @@ int tcs_create(const tcs_config *cfg, tcs_ctx **out)
     c->cx.y_solver = 1;
     c->cx.mixed_rows = 1;
     c->cx.z_staging = 1;
+    c->cx.spec_live = false;
     c->cx.probe = &c->probe;
     sync_shapes(c);
     {   // the FP32 context shares the grid, constants, scalars, tables and history
@@ -855,6 +856,7 @@ int tcs_pressure_RHS(tcs_ctx *c)
         ensure_ghosts(c, TCS_F_U); ensure_ghosts(c, TCS_F_V); ensure_ghosts(c, TCS_F_W);
         on_ctx(c, [&](auto &x) { launch_pseudo_prhs_fftx(x, c->stream, false); });
     }
+    c->cx.spec_live = true;
     return take_launch_error();
 }
 
@@ -863,8 +865,9 @@ int tcs_pressure_Poisson_FFT2(tcs_ctx *c)
     ENTER(c);
     int r = flush_pending(c);
     if (r) return r;
-    on_ctx(c, [&](auto &x) { launch_poisson_rest(x, c->stream); });
+    on_ctx(c, [&](auto &x) { launch_poisson_rest(x, c->stream, true); });
     c->ghost_ok |= (1u << TCS_F_DP);
+    c->cx.spec_live = false;
     return take_launch_error();
 }
 
@@ -882,7 +885,7 @@ int tcs_pressure_Projection(tcs_ctx *c)
     int r = flush_pending(c);
     if (r) return r;
     ensure_ghosts(c, TCS_F_DPHAT);
-    on_ctx(c, [&](auto &x) { launch_projection(x, c->stream); swap_phat(x); });
+    on_ctx(c, [&](auto &x) { launch_projection(x, c->stream, true); swap_phat(x); });
     c->ghost_ok |= (1u << TCS_F_U) | (1u << TCS_F_V) | (1u << TCS_F_W) | (1u << TCS_F_P) | (1u << TCS_F_DPHAT);
     return take_launch_error();
 }
@@ -892,7 +895,7 @@ int tcs_post_div(tcs_ctx *c, double *maxDivU)
     ENTER(c);
     int r = flush_pending(c);
     if (r) return r;
-    on_ctx(c, [&](auto &x) { launch_post(x, c->stream, 1); });
+    on_ctx(c, [&](auto &x) { launch_post(x, c->stream, 1, false); });
     if ((r = take_launch_error())) return r;
     double sc[S_NSCAL];
     CK(cudaMemcpyAsync(sc, c->cx.g.scal, sizeof(sc), cudaMemcpyDeviceToHost, c->stream));
@@ -927,10 +930,10 @@ static void launch_step_t(Ctx<R> &cx, cudaStream_t s)
     launch_blockld_u(cx, s);
     launch_pseudo_prhs_fftx(cx, s, true);
     swap_UVW(cx);
-    launch_poisson_rest(cx, s);
-    launch_projection(cx, s);
+    launch_poisson_rest(cx, s, false);
+    launch_projection(cx, s, false);
     swap_phat(cx);
-    launch_post(cx, s, 1);
+    launch_post(cx, s, 1, true);
 }
 
 static void launch_step(tcs_ctx *c)
@@ -1044,6 +1047,7 @@ int tcs_step(tcs_ctx *c, int nsteps, int *done)
     if (nsteps < 0) return set_err(TCS_ERR_ARG, "nsteps < 0");
     int r = flush_pending(c);
     if (r) return r;
+    c->cx.spec_live = false;   // the step writes the spectrum anew
     const int fl[] = {TCS_F_T, TCS_F_U, TCS_F_V, TCS_F_W, TCS_F_P, TCS_F_DPHAT};
     for (int f : fl) ensure_ghosts(c, f);
     if ((r = take_launch_error())) return r;
@@ -1325,7 +1329,7 @@ struct tcs_ensemble {
     cudaStream_t root = nullptr;
     cudaEvent_t fork = nullptr, fork2 = nullptr;
     std::vector<cudaEvent_t> join, join2;
-    // the form of a step: 1 = batched (a line sweep is one multi-case launch),
+    // the form of a step: 1 = batched (stage by stage over all cases),
     // 0 = one graph branch per case, -1 = auto (measure both, keep the faster)
     int mode = -1;
     int chosen = -1;          // auto: the form picked, -1 while measuring
@@ -1337,29 +1341,21 @@ struct tcs_ensemble {
         bool batched;
         cudaGraphExec_t exec;
         unsigned long long kernels;
-        void *arena;
     };
     std::vector<Entry> graphs;
 };
 
 static void ensemble_drop_graphs(tcs_ensemble *e)
 {
-    for (auto &g : e->graphs) {
-        cudaGraphExecDestroy(g.exec);
-        if (g.arena) cudaFree(g.arena);
-    }
+    for (auto &g : e->graphs) cudaGraphExecDestroy(g.exec);
     e->graphs.clear();
 }
 
-// One step of every case in the batched form.  The line sweeps (thermal,
-// solvedU/V/W, the modal Poisson solves) run as one line_solve_multi launch
-// per sweep on the root stream; the kernels between them run as one branch
-// per case (forked from and joined back to the root).  In planning mode
-// nothing is launched: the multi-case launches append their work lists to
-// the arena and the host-side buffer swaps are applied as the step makes them.
+// One step of every case in the batched form: stage by stage, a stage's launches
+// of all cases side by side (march_stage), and the kernels between the line
+// stages as one branch per case (forked from and joined back to the root).
 static void ensemble_sequence(tcs_ensemble *e, MultiArena &A)
 {
-    const bool plan = A.planning;
     std::vector<Ctx<double> *> d;
     std::vector<Ctx<float> *> f;
     for (tcs_ctx *c : e->cases) {
@@ -1367,63 +1363,47 @@ static void ensemble_sequence(tcs_ensemble *e, MultiArena &A)
         else d.push_back(&c->cx);
     }
     auto branches = [&](auto &&body) {
-        if (!plan) cudaEventRecord(e->fork, e->root);
+        cudaEventRecord(e->fork, e->root);
         for (size_t i = 0; i < e->cases.size(); i++) {
             tcs_ctx *c = e->cases[i];
-            if (!plan) cudaStreamWaitEvent(c->stream, e->fork, 0);
+            cudaStreamWaitEvent(c->stream, e->fork, 0);
             on_ctx(c, [&](auto &x) { body(x, c->stream); });
-            if (!plan) {
-                cudaEventRecord(e->join[i], c->stream);
-                cudaStreamWaitEvent(e->root, e->join[i], 0);
-            }
+            cudaEventRecord(e->join[i], c->stream);
+            cudaStreamWaitEvent(e->root, e->join[i], 0);
         }
     };
     launch_thermal_multi(d, A, e->root);
     launch_thermal_multi(f, A, e->root);
     branches([&](auto &x, cudaStream_t s) {
         swap_T(x);
-        if (!plan) launch_momentum_coeffi(x, s);
+        launch_momentum_coeffi(x, s);
     });
     launch_momentum_multi(d, A, e->root);
     launch_momentum_multi(f, A, e->root);
     branches([&](auto &x, cudaStream_t s) {
-        if (!plan) {
-            launch_blockld_v(x, s);
-            launch_blockld_u(x, s);
-            launch_pseudo_prhs_fftx(x, s, true);
-        }
+        launch_blockld_v(x, s);
+        launch_blockld_u(x, s);
+        launch_pseudo_prhs_fftx(x, s, true);
         swap_UVW(x);
-        if (!plan) launch_poisson_fwd(x, s);
+        launch_poisson_fwd(x, s);
     });
     launch_modal_multi(d, A, e->root);
     launch_modal_multi(f, A, e->root);
     branches([&](auto &x, cudaStream_t s) {
-        if (!plan) {
-            launch_poisson_back(x, s);
-            launch_projection(x, s);
-        }
+        launch_poisson_back(x, s, false);
+        launch_projection(x, s, false);
         swap_phat(x);
-        if (!plan) launch_post(x, s, 1);
+        launch_post(x, s, 1, true);
     });
 }
 
 // Capture one step of every case into a graph (the buffers swap as the step
-// swaps them).  Batched: plan the multi-case launches, put the buffer state
-// back, upload the work lists once, then capture; the graph keeps the upload.
-static int ensemble_capture(tcs_ensemble *e, bool batched, cudaGraphExec_t *exec, unsigned long long *nk, void **arena)
+// swaps them).
+static int ensemble_capture(tcs_ensemble *e, bool batched, cudaGraphExec_t *exec, unsigned long long *nk)
 {
     *exec = nullptr;
-    *arena = nullptr;
     MultiArena A;
-    if (batched) {
-        ensemble_sequence(e, A);
-        for (tcs_ctx *c : e->cases) on_ctx(c, [&](auto &x) { swap_T(x); swap_UVW(x); swap_phat(x); });
-        CK(cudaMalloc(&A.dev, std::max<size_t>(A.host.size(), 16)));
-        *arena = A.dev;
-        CK(cudaMemcpy(A.dev, A.host.data(), A.host.size(), cudaMemcpyHostToDevice));
-        A.planning = false;
-        A.cursor = 0;
-        // a stage's later launches run on the case streams (idle while the root runs a stage)
+    if (batched) {   // a stage's launches run on the case streams (idle while the root runs a stage)
         A.fork = e->fork2;
         for (size_t i = 0; i < e->cases.size(); i++) {
             A.aux.push_back(e->cases[i]->stream);
@@ -1450,10 +1430,6 @@ static int ensemble_capture(tcs_ensemble *e, bool batched, cudaGraphExec_t *exec
     cudaError_t ec = cudaStreamEndCapture(e->root, &gr);
     if (ec != cudaSuccess || take_launch_error())
         return set_err(TCS_ERR_CUDA, std::string("ensemble graph capture: ") + cudaGetErrorString(ec));
-    if (batched && A.cursor != A.host.size()) {
-        cudaGraphDestroy(gr);
-        return set_err(TCS_ERR_CUDA, "ensemble work lists do not match the captured step");
-    }
     ec = cudaGraphInstantiate(exec, gr, 0);
     cudaGraphDestroy(gr);
     if (ec != cudaSuccess) return set_err(TCS_ERR_CUDA, std::string("ensemble graph: ") + cudaGetErrorString(ec));
@@ -1530,6 +1506,7 @@ int tcs_ensemble_step(tcs_ensemble *e, int nsteps, int *nblown)
     int r;
     const int fl[] = {TCS_F_T, TCS_F_U, TCS_F_V, TCS_F_W, TCS_F_P, TCS_F_DPHAT};
     for (tcs_ctx *c : e->cases) {
+        c->cx.spec_live = false;
         if ((r = flush_pending(c))) return r;
         for (int f : fl) ensure_ghosts(c, f);
         if ((r = take_launch_error())) return r;
@@ -1551,13 +1528,9 @@ int tcs_ensemble_step(tcs_ensemble *e, int nsteps, int *nblown)
         for (auto &g : e->graphs)
             if (g.key == key && g.batched == form) { exec = g.exec; kernels = g.kernels; break; }
         if (!exec) {
-            void *arena = nullptr;
-            const int rc = ensemble_capture(e, form, &exec, &kernels, &arena);
-            if (rc) {
-                if (arena) cudaFree(arena);
-                return rc;
-            }
-            e->graphs.push_back({key, form, exec, kernels, arena});
+            const int rc = ensemble_capture(e, form, &exec, &kernels);
+            if (rc) return rc;
+            e->graphs.push_back({key, form, exec, kernels});
             // the capture swapped every case's buffers already
         } else {
             for (tcs_ctx *c : e->cases) on_ctx(c, [&](auto &x) { swap_T(x); swap_UVW(x); swap_phat(x); });
@@ -1695,7 +1668,7 @@ extern "C" int tcs_autotune(tcs_ctx *c, int trial_steps, const char *cache_path,
     if ((r = tune_trial(c, trial_steps, &best_ms))) return r;
     static const int cand[] = {1, 2, 4, 8, 16, 32};
     for (int k = 0; k < TCS_TUNE_COUNT; k++) {
-        if (k == TCS_TUNE_TL_STRIDED || k == TCS_TUNE_TL_CONTIG || k == TCS_TUNE_LONG_LINES || k == TCS_TUNE_Y_SOLVER ||
+        if (k == TCS_TUNE_TL_STRIDED || k == TCS_TUNE_TL_CONTIG || k == TCS_TUNE_TL_MODAL || k == TCS_TUNE_LONG_LINES || k == TCS_TUNE_Y_SOLVER ||
             k == TCS_TUNE_MIXED_ROWS || k == TCS_TUNE_Z_STAGING)
             continue;                                                 // without effect: nothing to time
         for (int v : cand) {

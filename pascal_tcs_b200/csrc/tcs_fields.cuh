@@ -63,6 +63,27 @@ template <class R> struct HasLo { static constexpr bool on = std::is_same<R, flo
 __device__ __forceinline__ double2 ld2(const double *p) { return __ldg(reinterpret_cast<const double2 *>(p)); }
 __device__ __forceinline__ float2 ld2(const float *p) { return __ldg(reinterpret_cast<const float2 *>(p)); }
 
+// Weights of the wall extrapolations (Pbc_a and Pbc_b of the lower and upper wall).
+struct WallRows { double ab, bb, at, bt; };
+
+// dP wall extrapolation (module_solve_pressure.f90:719-736) on every (i,k)
+// including ghost columns, which is what the extrapolation followed by
+// ghost(dP) produces.
+template <class R>
+__device__ __forceinline__ void dp_wall_cell(const GridT<R> &g, R *dP, int i, int k, const WallRows &w)
+{
+    dP[ix(g, i, 0, k)] = R(w.ab * (double)dP[ix(g, i, 1, k)] - w.bb * (double)dP[ix(g, i, 2, k)]);
+    dP[ix(g, i, g.N2 + 1, k)] = R(w.at * (double)dP[ix(g, i, g.N2, k)] - w.bt * (double)dP[ix(g, i, g.N2 - 1, k)]);
+}
+// P(i,0,k) = Pbc_a P(i,1,k) - Pbc_b P(i,2,k) and the top-wall counterpart
+// (:853-869), then ghost(P).
+template <class R>
+__device__ __forceinline__ void p_wall_cell(const GridT<R> &g, R *P, int i, int k, const WallRows &w)
+{
+    store_periodic(g, P, i, 0, k, R(w.ab * (double)P[ix(g, i, 1, k)] - w.bb * (double)P[ix(g, i, 2, k)]));
+    store_periodic(g, P, i, g.N2 + 1, k, R(w.at * (double)P[ix(g, i, g.N2, k)] - w.bt * (double)P[ix(g, i, g.N2 - 1, k)]));
+}
+
 // v = hi + lo in FP64, and its split back into an FP32 pair.
 __device__ __forceinline__ double join(float hi, float lo) { return (double)hi + (double)lo; }
 __device__ __forceinline__ void split(double v, float &hi, float &lo)

@@ -80,6 +80,7 @@ struct Shapes {
     int long_lines, y_solver;                    // accepted and kept; one solver runs the strided lines
     int mixed_rows;                              // likewise
     int z_staging;                               // likewise
+    bool spec_live;                              // the spectrum holds a right-hand side that no Poisson solve has taken yet
     FFTPlan fp1, fp3;
     FFTPlan fp1u;                                // N1 with radices up to 8 (the inverse x transform's one-radix form)
     int h1p;
@@ -100,46 +101,6 @@ void probe_end(const Shapes &cx, int kid, cudaStream_t s);
 int record_launch_error(const char *what);
 int set_error(int code, const std::string &msg);
 
-// Dynamic shared memory of a line-solver launch.
-template <class Prob>
-inline size_t line_smem(const LinePlan &lp)
-{
-    return (size_t)line_words<Prob>() * lp.TL * lp.LS * sizeof(typename Prob::Real) + (size_t)lp.n * sizeof(int);
-}
-
-// The plan of a line problem: make_line_plan's partitions, and for the
-// non-cyclic strided problems (the modal solves) a
-// line stride LS chosen for the build and the emission, where one warp
-// touches TL lines x 32/TL rows: LS = banks/TL (mod banks), banks = 32
-// four-byte words (FP32 rows) or 16 eight-byte words per half-warp (FP64
-// rows), puts those accesses on distinct banks.  The solve (one line per
-// warp) only uses the odd partition stride PS.  Measured at 256^3: the y
-// sweeps 2-5% and the modal solves 3-4% faster in both forms.
-template <class Prob>
-inline LinePlan plan_for(int n, bool cyclic, int tl, int pmax)
-{
-    LinePlan lp = make_line_plan(n, cyclic, tl, pmax);
-    if (!Prob::CONTIG && !cyclic && tl > 1) {
-        const int banks = sizeof(typename Prob::Real) == 4 ? 32 : 16;
-        const int want = tl < banks ? banks / tl : 1;
-        const int ls = lp.P * lp.PS;
-        lp.LS = ls + ((want - ls) % banks + banks) % banks;
-    }
-    return lp;
-}
-
-// Lines per block: the requested count, halved until MINB blocks fit in the
-// SM's shared memory (228 KiB, 1 KB reserved per block); extra: static shared
-// memory the kernel adds per block.
-template <class Prob>
-inline int fit_tl(int n, bool cyclic, int want, int pmax, size_t extra = 0)
-{
-    const size_t budget = (size_t)228 * 1024 / Prob::MINB - 1024 - extra;
-    int tl = want;
-    while (tl > 1 && line_smem<Prob>(plan_for<Prob>(n, cyclic, tl, pmax)) > budget) tl /= 2;
-    return tl;
-}
-
 // Opt a kernel in to smem bytes of dynamic shared memory on the current
 // device.  The attribute belongs to the function on each device, so the
 // largest size set so far is kept per device (cache: one entry per ordinal).
@@ -152,18 +113,6 @@ inline void smem_opt_in(const void *fn, size_t smem, size_t *cache)
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cache[dev] = smem;
     }
-}
-
-template <class Prob>
-inline void launch_lines(const Prob &p, const LinePlan &lp, dim3 grid, cudaStream_t s, int kid, const Shapes &cx)
-{
-    const size_t smem = line_smem<Prob>(lp);
-    static size_t configured[64] = {};
-    smem_opt_in((const void *)line_solve_kernel<Prob>, smem, configured);
-    probe_begin(cx, kid, s);
-    line_solve_kernel<Prob><<<grid, Prob::NT, smem, s>>>(p, lp);
-    probe_end(cx, kid, s);
-    record_launch_error(kernel_name(kid));
 }
 
 // The shape of a marching sweep (march_block) of `lines` lines in all: TI lines
@@ -185,7 +134,13 @@ inline MarchPlan march_plan(int n, bool cyclic, int lanes, long long lines)
     const int cap = lanes < 32 ? lanes : 256;
     auto more = [&]() { return (2 << mp.lgNS) <= cap && (n >> (mp.lgNS + 1)) >= 4; };
     while (more() && mp.lgNS < 5 && (n > (P::ROWS << mp.lgNS) || (lines << mp.lgNS) < 131072)) mp.lgNS++;
-    mp.lgTI = 4;
+    mp.lgTI = P::LGTI;
+    // FP64 z lines of more than 416 rows in too few lines for the column form: 64
+    // segments of 8 lines (64 x 64 x 512, ps per cell of dw_z: 33 against 45)
+    if (std::is_same<typename P::Real, double>::value && P::ROWS == 12 && mp.lgNS == 5 && n > 416 && cap >= 64) {
+        mp.lgNS = 6;
+        mp.lgTI = 3;
+    }
     auto words = [&]() { return march_words(n, 1 << mp.lgNS, 1 << mp.lgTI, P::NRHS) * sizeof(double); };
     while (mp.lgTI > 0 && words() > 227 * 1024) {
         mp.lgTI--;
@@ -212,8 +167,10 @@ inline void launch_march_nt(const Shapes &cx, const P &prob, const MarchPlan &mp
     record_launch_error(kernel_name(kid));
 }
 
-// The column form of a z sweep (column_kernel), in two segments per line: FP64
-// lines of more than 384 rows, with rows of i that start on 16 bytes.  Measured
+// The column form of a z sweep (column_kernel), in two segments per line: 24576
+// or more FP64 lines (a thread for each segment then half fills the SMs; with
+// 6240 lines of 400 rows the step took 1.2 times march_kernel's) of more than 384
+// rows, with rows of i that start on 16 bytes, while the spectrum is idle.  Measured
 // at 512^3 (ms, thermal_z, du_z, dv_z, dw_z): 3.17, 2.54, 2.81, 3.02 against 4.64,
 // 3.80, 4.85, 5.06 for march_kernel, whose parked rows then fill the shared
 // memory; at 384 rows the two are level, and below it march_kernel leads.
@@ -221,7 +178,7 @@ template <class P>
 inline bool launch_column(const Shapes &cx, const P &prob, int n, int nlines, int gy, cudaStream_t s, int kid)
 {
     constexpr int lgNS = 1;
-    if (n <= 384 || (prob.g.P1 & 1)) return false;
+    if (cx.spec_live || n <= 384 || (prob.g.P1 & 1) || (long long)nlines * gy < 24576) return false;
     int w = 0, best = 1 << 30;
     for (int c = 32; c <= (128 >> lgNS); c += 32) {       // the widest of the block widths that waste least
         const int waste = (nlines + c - 1) / c * c;
@@ -281,107 +238,14 @@ inline void launch_xmarch(const Shapes &cx, const P &prob, int n, int nlines, in
 }
 
 // ---------------------------------------------------------------------------
-// Ensemble launches: one line stage of many cases as line_solve_multi
-// launches of up to MultiParams::K cases each.  An ensemble builds each
-// step's launches twice in the same order: in planning mode every launch
-// reserves its item counter in the arena, then (after one upload of the
-// arena) in launch mode each launch takes its counter's device address.
-// The launches of one stage run concurrently on the aux streams (forked from
-// and joined back to the stage's stream).
+// Ensemble launches: the streams a stage's launches run on side by side (forked
+// from and joined back to the stage's stream).
 // ---------------------------------------------------------------------------
 struct MultiArena {
-    std::vector<unsigned char> host;
-    unsigned char *dev = nullptr;
-    size_t cursor = 0;
-    bool planning = true;
-    std::vector<cudaStream_t> aux;       // streams for a stage's second and later launches
+    std::vector<cudaStream_t> aux;
     std::vector<cudaEvent_t> join;       // one per aux stream
     cudaEvent_t fork = nullptr;
-    int *counter()
-    {
-        const size_t off = (cursor + 15) & ~(size_t)15;
-        cursor = off + 16;
-        if (planning) {
-            host.resize(cursor, 0);
-            return nullptr;
-        }
-        return (int *)(dev + off);
-    }
 };
-
-// One case's share of a multi-case line stage: the line length, cyclicity,
-// requested lines per block, and the block grid (lines / TL rounded up, gy).
-struct StageShape {
-    int n;
-    bool cyclic;
-    int want, lines, gy;
-};
-
-template <class Prob>
-inline void launch_lines_multi(MultiParams<Prob> &mp, int ncase, cudaStream_t s, const char *what)
-{
-    size_t smem = 0;
-    for (int c = 0; c < ncase; c++) smem = std::max(smem, line_smem<Prob>(mp.lp[c]));
-    static size_t conf[64] = {};
-    smem_opt_in((const void *)line_solve_multi<Prob>, smem, conf);
-    int dev = 0, sms = 148, occ = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, line_solve_multi<Prob>, Prob::NT, smem);
-    const int grid = (int)std::min<long long>(mp.nitems, (long long)std::max(occ, 1) * sms);
-    line_solve_multi<Prob><<<grid, Prob::NT, smem, s>>>(mp);
-    record_launch_error(what);
-}
-
-// A line stage for a group of same-precision cases: per case the same plan
-// and block grid as its one-case launch; the cases with the longest blocks
-// first (so the blocks that pull the last items finish close together),
-// MultiParams::K cases per launch.
-template <class P, class R, class Shape, class Make>
-inline void multi_stage(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s, const char *what, Shape shape,
-                        Make make)
-{
-    struct Entry { P prob; LinePlan lp; int gx, gy; long long cost; };
-    std::vector<Entry> es;
-    for (const Ctx<R> *xp : cs) {
-        const Ctx<R> &x = *xp;
-        const StageShape sh = shape(x);
-        const LinePlan lp = plan_for<P>(sh.n, sh.cyclic, fit_tl<P>(sh.n, sh.cyclic, sh.want, x.lanes, 64), x.lanes);
-        es.push_back({make(x, lp.TL), lp, (sh.lines + lp.TL - 1) / lp.TL, sh.gy, (long long)sh.n * lp.TL});
-    }
-    std::stable_sort(es.begin(), es.end(), [](const Entry &a, const Entry &b) { return a.cost > b.cost; });
-    constexpr int K = MultiParams<P>::K;
-    const int nl = (int)((es.size() + K - 1) / K);
-    const bool fan = !A.planning && nl > 1 && (int)A.aux.size() >= nl - 1;
-    if (fan) cudaEventRecord(A.fork, s);
-    for (int l = 0; l < nl; l++) {
-        const size_t c0 = (size_t)l * K;
-        const int nc = (int)std::min<size_t>(K, es.size() - c0);
-        int *ctr = A.counter();
-        if (A.planning) continue;
-        MultiParams<P> mp;
-        mp.start[0] = 0;
-        for (int c = 0; c < nc; c++) {
-            const Entry &e = es[c0 + c];
-            mp.p[c] = e.prob;
-            mp.lp[c] = e.lp;
-            mp.gx[c] = e.gx;
-            mp.start[c + 1] = mp.start[c] + e.gx * e.gy;
-        }
-        mp.nitems = mp.start[nc];
-        mp.ctr = ctr;
-        cudaStream_t ls = s;
-        if (fan && l > 0) {
-            ls = A.aux[l - 1];
-            cudaStreamWaitEvent(ls, A.fork, 0);
-        }
-        launch_lines_multi(mp, nc, ls, what);
-        if (fan && l > 0) {
-            cudaEventRecord(A.join[l - 1], ls);
-            cudaStreamWaitEvent(s, A.join[l - 1], 0);
-        }
-    }
-}
 
 // A marching sweep for a group of cases: one launch per case, side by side on
 // the aux streams.  (A persistent multi-case form of march_block was a second
@@ -390,7 +254,7 @@ inline void multi_stage(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStre
 template <class R, class Launch>
 inline void march_stage(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s, Launch launch)
 {
-    if (A.planning || cs.empty()) return;
+    if (cs.empty()) return;
     const size_t side = std::min(A.aux.size(), cs.size());
     if (side) cudaEventRecord(A.fork, s);
     for (size_t i = 0; i < side; i++) cudaStreamWaitEvent(A.aux[i], A.fork, 0);
@@ -412,14 +276,15 @@ template <class R> void launch_blockld_v(const Ctx<R> &cx, cudaStream_t s);
 template <class R> void launch_blockld_u(const Ctx<R> &cx, cudaStream_t s);
 template <class R> void launch_pseudo_update(const Ctx<R> &cx, cudaStream_t s);   // standalone (Un = U + dU, ...)
 template <class R> void launch_pseudo_prhs_fftx(const Ctx<R> &cx, cudaStream_t s, bool with_pseudo);
-template <class R> void launch_poisson_rest(const Ctx<R> &cx, cudaStream_t s);
+// walls: write the wall rows of dP (of P) too; a step leaves both to launch_post
+template <class R> void launch_poisson_rest(const Ctx<R> &cx, cudaStream_t s, bool walls);
 template <class R> void launch_modal(const Ctx<R> &cx, cudaStream_t s);
 template <class R> void launch_poisson_fwd(const Ctx<R> &cx, cudaStream_t s);   // z FFTs (forward)
-template <class R> void launch_poisson_back(const Ctx<R> &cx, cudaStream_t s);  // mean, z and x inverse FFTs, dP walls
-template <class R> void launch_projection(const Ctx<R> &cx, cudaStream_t s);
-template <class R> void launch_post(const Ctx<R> &cx, cudaStream_t s, int record_hist);
+template <class R> void launch_poisson_back(const Ctx<R> &cx, cudaStream_t s, bool walls);  // z and x inverse FFTs, dP walls
+template <class R> void launch_projection(const Ctx<R> &cx, cudaStream_t s, bool walls);
+template <class R> void launch_post(const Ctx<R> &cx, cudaStream_t s, int record_hist, bool walls);
 template <class R> void launch_ghost(const Ctx<R> &cx, R *a, cudaStream_t s);
-// the line stages of a step for a group of same-precision cases, one launch per stage
+// the line stages of a step for a group of same-precision cases
 template <class R> void launch_thermal_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s);
 template <class R> void launch_momentum_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s);
 template <class R> void launch_modal_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s);

@@ -137,6 +137,13 @@ __device__ __forceinline__ void march_reduce(double *red, int lgNS, int TP, bool
     __syncthreads();
 }
 
+// Problems that want the sum of line 0's solution in the first block row
+// (Out::total, set_total).
+template <class P, class = void>
+struct HasTotal { static constexpr bool on = false; };
+template <class P>
+struct HasTotal<P, std::void_t<decltype(P::TOTAL)>> { static constexpr bool on = true; };
+
 // Stores of a line's rows from the last to the first: into the sweep scratch, ...
 template <class R>
 struct ScratchOut {
@@ -166,7 +173,7 @@ struct PeriodicOut {
 };
 
 // The problem supplies
-//   static constexpr int NRHS, AHEAD (rows whose inputs are loaded ahead)
+//   static constexpr int NRHS, AHEAD (rows whose inputs are loaded ahead), ROWS, LGTI (most rows per segment, most lines per block), TPS
 //   skip(), lines() (count of lines along i of the block row)
 //   struct March { March(const Prob &, int line, int by, int r0);               // line: clamped to a valid one
 //                  struct In;  void load(const Prob &, int r, In &);             // the inputs of row r, rows in order from r0
@@ -276,6 +283,19 @@ __device__ __forceinline__ void march_block(const Prob &prob, const MarchPlan &m
 #pragma unroll
             for (int q = 0; q < NR; q++) x[q] = fma(-c, x[q], fma(-e, xp[q], w[(2 + q) * TI]));
             out.put(prob, x);
+        }
+        if constexpr (HasTotal<Prob>::on)
+            if (bx == 0 && by == 0 && l == 0) msm[r0 * W * TI] = out.total;   // over a row that this thread has used
+    }
+    if constexpr (HasTotal<Prob>::on) {
+        // the total of line 0 of the first block row, segment by segment
+        if (bx == 0 && by == 0 && !skip) {
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                double t = 0.0;
+                for (int q = 0; q < NS; q++) t += msm[(q * mp.m0 + min(q, mp.rem)) * W * TI];
+                prob.set_total(t);
+            }
         }
     }
 }

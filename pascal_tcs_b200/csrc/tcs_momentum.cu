@@ -1,8 +1,7 @@
 // tcs_momentum.cu -- momentum increments: mpi_momentum_coeffi, solvedU/V/W,
 // blockLdV/U and the standalone pseudo-update (module_solve_momentum.f90).
 //
-// Each solved* routine is three fused kernels (z, x, y sweeps) on the shared
-// line solver; the y sweep writes the increment with its periodic ghosts, which
+// Each solved* routine is three fused kernels (z, x, y sweeps, tcs_march.cuh); the y sweep writes the increment with its periodic ghosts, which
 // is the ghost update the driver performs right after (main.f90:151-169).
 //
 // Mu and invRho are the 2-D (j,k) tables of mpi_momentum_coeffi: the
@@ -76,7 +75,7 @@ template <class R>
 struct DUZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12;   // FP64 inputs of two rows do not fit the registers
+    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12, LGTI = 4;   // FP64 inputs of two rows do not fit the registers
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -283,7 +282,7 @@ template <class R>
 struct DUY {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr int AHEAD = 2, TPS = 512, ROWS = 16;
+    static constexpr int AHEAD = 2, TPS = 512, ROWS = 16, LGTI = 4;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -341,7 +340,7 @@ template <class R>
 struct DVZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12;   // FP64 inputs of two rows do not fit the registers
+    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12, LGTI = 4;   // FP64 inputs of two rows do not fit the registers
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -520,7 +519,7 @@ template <class R>
 struct DVY {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr int AHEAD = 2, TPS = 512, ROWS = 16;
+    static constexpr int AHEAD = 2, TPS = 512, ROWS = 16, LGTI = 4;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -581,7 +580,7 @@ template <class R>
 struct DWZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12;   // FP64 inputs of two rows do not fit the registers
+    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12, LGTI = 4;   // FP64 inputs of two rows do not fit the registers
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -776,7 +775,7 @@ template <class R>
 struct DWY {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr int AHEAD = 2, TPS = 512, ROWS = 16;
+    static constexpr int AHEAD = 2, TPS = 512, ROWS = 16, LGTI = 4;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }

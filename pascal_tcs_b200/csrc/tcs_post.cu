@@ -1,8 +1,10 @@
 // tcs_post.cu -- per-step diagnostics: mpi_Post_Div and mpi_Post_CFL
 // (module_post.f90:100-158, 168-230) with the adaptive time step, the
 // blow-up test of main.f90:208-212, and the Nusselt / kinetic-energy series.
-// Two kernels: block partials in a fixed order, then one block that combines
-// them and updates dt, time and CFL on the device (deterministic).  Both forms
+// One kernel: block partials in a fixed order; the last block to finish combines
+// them and updates dt, time and CFL on the device (deterministic).  Inside a step
+// it also writes the wall rows of dP and P, which nothing reads before (three
+// launches fewer per step: 19 us of 64^3's 203).  Both forms
 // reduce in FP64 from their fields, and the per-thread sums are compensated
 // (Neumaier), so the diagnostics keep FP64 accuracy over 512^3 cells.
 #include "tcs_kernels.h"
@@ -12,7 +14,7 @@
 namespace tcs {
 
 enum { PT_DIV = 0, PT_CFL, PT_KE, PT_NUB, PT_NUT, PT_N };
-static const int POST_BLOCKS = 592;   // 4 x 148 SMs
+static const int POST_BLOCKS = 592;   // 4 x 148 SMs: all resident in FP64 (64 registers; the FP32 form, with twice the loads, runs faster uncapped)
 
 // s + e carries a sum and its running rounding error (Neumaier's variant of
 // Kahan summation).
@@ -23,67 +25,16 @@ __device__ __forceinline__ void csum(double &s, double &e, double v)
     s = t;
 }
 
+// The last block's part: the partials of all blocks, then dt, time, CFL, the
+// series and the blow-up test.
 template <class R>
-__global__ void __launch_bounds__(256) post_kernel(GridT<R> g, FieldsT<R> f, FastDiv dn1, FastDiv dn2)
+__device__ __forceinline__ void finalize(const GridT<R> &g, const FieldsT<R> &f, double (*red)[256], int nblocks, int record_hist)
 {
-    __shared__ double red[PT_N][256];
-    if (blown(g)) return;
-    const long long n = (long long)g.N1 * g.N2 * g.N3;
-    double mdiv = -INFINITY, mcfl = -INFINITY, ke = 0.0, nub = 0.0, nut = 0.0, eke = 0.0, enb = 0.0, ent = 0.0;
-    const double *dx1 = g.d1.dx, *dx2 = g.d2.dx, *dx3 = g.d3.dx;
-    const double *rdx1 = g.d1.rdx, *rdx2 = g.d2.rdx, *rdx3 = g.d3.rdx;
-    const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
-    // two cells per pass keep twice the loads in flight (measured -21% at 256^3)
-#pragma unroll 2
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const unsigned q = dn1.div((unsigned)t), r = dn2.div(q);     // n < 2^31: 32-bit multiply-shift division
-        const int i = 1 + (int)((unsigned)t - q * (unsigned)g.N1);
-        const int j = 1 + (int)(q - r * (unsigned)g.N2), k = 1 + (int)r;
-        const long long c = ix(g, i, j, k);
-        double Uc, Vc, Wc, Ux, Vy, Wz;
-        if constexpr (HasLo<R>::on) {     // the FP32 form's velocity is its high + low pair
-            Uc = join(ld(f.U + c), ld(f.Ulo + c)); Vc = join(ld(f.V + c), ld(f.Vlo + c)); Wc = join(ld(f.W + c), ld(f.Wlo + c));
-            Ux = join(ld(f.U + c + 1), ld(f.Ulo + c + 1)); Vy = join(ld(f.V + c + sj), ld(f.Vlo + c + sj));
-            Wz = join(ld(f.W + c + sk), ld(f.Wlo + c + sk));
-        } else {
-            Uc = ld(f.U + c); Vc = ld(f.V + c); Wc = ld(f.W + c);
-            Ux = ld(f.U + c + 1); Vy = ld(f.V + c + sj); Wz = ld(f.W + c + sk);
-        }
-        const double dv = (Ux - Uc) * rdx1[i] + (Vy - Vc) * rdx2[j] + (Wz - Wc) * rdx3[k];
-        const double cf = (fabs(Ux + Uc) / 2.0) * rdx1[i] + (fabs(Vy + Vc) / 2.0) * rdx2[j] + (fabs(Wz + Wc) / 2.0) * rdx3[k];
-        mdiv = fmax(mdiv, dv);
-        mcfl = fmax(mcfl, cf);
-        csum(ke, eke, (Uc * Uc + Vc * Vc + Wc * Wc) * dx1[i] * dx2[j] * dx3[k]);
-        if (j == 1) csum(nub, enb, -((double)ld(f.T + c) - g.phd.Tbt) / g.d2.dmx[1]);
-        if (j == g.N2) csum(nut, ent, -(g.phd.Tup - (double)ld(f.T + c)) / g.d2.dmx[g.N2 + 1]);
-    }
-    ke += eke; nub += enb; nut += ent;
-    red[PT_DIV][threadIdx.x] = mdiv; red[PT_CFL][threadIdx.x] = mcfl;
-    red[PT_KE][threadIdx.x] = ke; red[PT_NUB][threadIdx.x] = nub; red[PT_NUT][threadIdx.x] = nut;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            red[PT_DIV][threadIdx.x] = fmax(red[PT_DIV][threadIdx.x], red[PT_DIV][threadIdx.x + w]);
-            red[PT_CFL][threadIdx.x] = fmax(red[PT_CFL][threadIdx.x], red[PT_CFL][threadIdx.x + w]);
-            red[PT_KE][threadIdx.x] += red[PT_KE][threadIdx.x + w];
-            red[PT_NUB][threadIdx.x] += red[PT_NUB][threadIdx.x + w];
-            red[PT_NUT][threadIdx.x] += red[PT_NUT][threadIdx.x + w];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x < PT_N) f.part[blockIdx.x * PT_N + threadIdx.x] = red[threadIdx.x][0];
-}
-
-template <class R>
-__global__ void __launch_bounds__(256) finalize_kernel(GridT<R> g, FieldsT<R> f, int nblocks, int record_hist)
-{
-    __shared__ double red[PT_N][256];
-    if (blown(g)) return;
     double mdiv = -INFINITY, mcfl = -INFINITY, ke = 0.0, nub = 0.0, nut = 0.0;
     for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
         const double *p = f.part + b * PT_N;
-        mdiv = fmax(mdiv, p[PT_DIV]); mcfl = fmax(mcfl, p[PT_CFL]);
-        ke += p[PT_KE]; nub += p[PT_NUB]; nut += p[PT_NUT];
+        mdiv = fmax(mdiv, __ldcg(p + PT_DIV)); mcfl = fmax(mcfl, __ldcg(p + PT_CFL));
+        ke += __ldcg(p + PT_KE); nub += __ldcg(p + PT_NUB); nut += __ldcg(p + PT_NUT);
     }
     red[PT_DIV][threadIdx.x] = mdiv; red[PT_CFL][threadIdx.x] = mcfl;
     red[PT_KE][threadIdx.x] = ke; red[PT_NUB][threadIdx.x] = nub; red[PT_NUT][threadIdx.x] = nut;
@@ -130,16 +81,83 @@ __global__ void __launch_bounds__(256) finalize_kernel(GridT<R> g, FieldsT<R> f,
 }
 
 template <class R>
-void launch_post(const Ctx<R> &cx, cudaStream_t s, int record_hist)
+__global__ void __launch_bounds__(256, HasLo<R>::on ? 1 : 4) post_kernel(GridT<R> g, FieldsT<R> f, FastDiv dn1, FastDiv dn2, int record_hist, int walls, WallRows wr)
 {
+    __shared__ double red[PT_N][256];
+    __shared__ int s_last;
+    if (blown(g)) return;
+    const long long n = (long long)g.N1 * g.N2 * g.N3;
+    double mdiv = -INFINITY, mcfl = -INFINITY, ke = 0.0, nub = 0.0, nut = 0.0, eke = 0.0, enb = 0.0, ent = 0.0;
+    const double *dx1 = g.d1.dx, *dx2 = g.d2.dx, *dx3 = g.d3.dx;
+    const double *rdx1 = g.d1.rdx, *rdx2 = g.d2.rdx, *rdx3 = g.d3.rdx;
+    const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
+    // two cells per pass keep twice the loads in flight (measured -21% at 256^3)
+#pragma unroll 2
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        const unsigned q = dn1.div((unsigned)t), r = dn2.div(q);     // n < 2^31: 32-bit multiply-shift division
+        const int i = 1 + (int)((unsigned)t - q * (unsigned)g.N1);
+        const int j = 1 + (int)(q - r * (unsigned)g.N2), k = 1 + (int)r;
+        const long long c = ix(g, i, j, k);
+        double Uc, Vc, Wc, Ux, Vy, Wz;
+        if constexpr (HasLo<R>::on) {     // the FP32 form's velocity is its high + low pair
+            Uc = join(ld(f.U + c), ld(f.Ulo + c)); Vc = join(ld(f.V + c), ld(f.Vlo + c)); Wc = join(ld(f.W + c), ld(f.Wlo + c));
+            Ux = join(ld(f.U + c + 1), ld(f.Ulo + c + 1)); Vy = join(ld(f.V + c + sj), ld(f.Vlo + c + sj));
+            Wz = join(ld(f.W + c + sk), ld(f.Wlo + c + sk));
+        } else {
+            Uc = ld(f.U + c); Vc = ld(f.V + c); Wc = ld(f.W + c);
+            Ux = ld(f.U + c + 1); Vy = ld(f.V + c + sj); Wz = ld(f.W + c + sk);
+        }
+        const double dv = (Ux - Uc) * rdx1[i] + (Vy - Vc) * rdx2[j] + (Wz - Wc) * rdx3[k];
+        const double cf = (fabs(Ux + Uc) / 2.0) * rdx1[i] + (fabs(Vy + Vc) / 2.0) * rdx2[j] + (fabs(Wz + Wc) / 2.0) * rdx3[k];
+        mdiv = fmax(mdiv, dv);
+        mcfl = fmax(mcfl, cf);
+        csum(ke, eke, (Uc * Uc + Vc * Vc + Wc * Wc) * dx1[i] * dx2[j] * dx3[k]);
+        if (j == 1) csum(nub, enb, -((double)ld(f.T + c) - g.phd.Tbt) / g.d2.dmx[1]);
+        if (j == g.N2) csum(nut, ent, -(g.phd.Tup - (double)ld(f.T + c)) / g.d2.dmx[g.N2 + 1]);
+    }
+    ke += eke; nub += enb; nut += ent;
+    red[PT_DIV][threadIdx.x] = mdiv; red[PT_CFL][threadIdx.x] = mcfl;
+    red[PT_KE][threadIdx.x] = ke; red[PT_NUB][threadIdx.x] = nub; red[PT_NUT][threadIdx.x] = nut;
+    __syncthreads();
+    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+        if (threadIdx.x < w) {
+            red[PT_DIV][threadIdx.x] = fmax(red[PT_DIV][threadIdx.x], red[PT_DIV][threadIdx.x + w]);
+            red[PT_CFL][threadIdx.x] = fmax(red[PT_CFL][threadIdx.x], red[PT_CFL][threadIdx.x + w]);
+            red[PT_KE][threadIdx.x] += red[PT_KE][threadIdx.x + w];
+            red[PT_NUB][threadIdx.x] += red[PT_NUB][threadIdx.x + w];
+            red[PT_NUT][threadIdx.x] += red[PT_NUT][threadIdx.x + w];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < PT_N) f.part[blockIdx.x * PT_N + threadIdx.x] = red[threadIdx.x][0];
+    if (walls) {
+        const int nx = g.N1 + 2, nw = nx * (g.N3 + 2);
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nw; t += gridDim.x * blockDim.x) {
+            const int k = t / nx, i = t - k * nx;
+            dp_wall_cell(g, f.dP, i, k, wr);
+            if (i >= 1 && i <= g.N1 && k >= 1 && k <= g.N3) p_wall_cell(g, f.P, i, k, wr);
+        }
+    }
+    __threadfence();                                   // the partials before the count
+    __syncthreads();
+    unsigned *const ctr = reinterpret_cast<unsigned *>(g.scal + S_CTR);
+    if (threadIdx.x == 0) s_last = atomicAdd(ctr, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x == 0) *ctr = 0;                    // the next launch counts from 0
+    finalize(g, f, red, gridDim.x, record_hist);
+}
+
+template <class R>
+void launch_post(const Ctx<R> &cx, cudaStream_t s, int record_hist, bool walls)
+{
+    const WallRows wr{cx.wall_ab, cx.wall_bb, cx.wall_at, cx.wall_bt};
     probe_begin(cx, K_POST, s);
-    post_kernel<<<POST_BLOCKS, 256, 0, s>>>(cx.g, cx.f, make_fastdiv((unsigned)cx.g.N1), make_fastdiv((unsigned)cx.g.N2));
+    post_kernel<<<POST_BLOCKS, 256, 0, s>>>(cx.g, cx.f, make_fastdiv((unsigned)cx.g.N1), make_fastdiv((unsigned)cx.g.N2), record_hist,
+                                            walls ? 1 : 0, wr);
     probe_end(cx, K_POST, s);
     record_launch_error("post");
-    probe_begin(cx, K_FINAL, s);
-    finalize_kernel<<<1, 256, 0, s>>>(cx.g, cx.f, POST_BLOCKS, record_hist);
-    probe_end(cx, K_FINAL, s);
-    record_launch_error("finalize");
 }
 
 int post_partial_count() { return POST_BLOCKS * PT_N; }
@@ -291,8 +309,8 @@ template void launch_plane<double>(const Ctx<double> &, const double *, const do
 template void launch_plane<float>(const Ctx<float> &, const float *, const float *, double *, int, int, cudaStream_t);
 
 // the two forms
-template void launch_post<double>(const Ctx<double> &, cudaStream_t, int);
-template void launch_post<float>(const Ctx<float> &, cudaStream_t, int);
+template void launch_post<double>(const Ctx<double> &, cudaStream_t, int, bool);
+template void launch_post<float>(const Ctx<float> &, cudaStream_t, int, bool);
 template void launch_ghost<double>(const Ctx<double> &, double *, cudaStream_t);
 template void launch_ghost<float>(const Ctx<float> &, float *, cudaStream_t);
 template void launch_convert<double>(const double *, double *, long long, cudaStream_t);

@@ -9,7 +9,7 @@
 //   prhs_fftx   pseudo-update (+ghosts) -> PRHS -> r2c along x   -> S
 //   fftz<-1>    c2c along z (FFTW_FORWARD)                        S -> S
 //   modal       y tridiagonal per (kx,kz), re and im together     S -> S
-//   mean        unweighted mean of the solution (from the (0,0) mode)
+//               and the unweighted mean of the solution (from the (0,0) mode)
 //   fftz<+1>    c2c along z (FFTW_BACKWARD)                       S -> S
 //   ifftx       c2r along x, /N1/N3, minus mean, periodic ghosts  S -> dP
 //   dp_wall     wall extrapolation of dP (:719-736)
@@ -597,62 +597,57 @@ __global__ void __launch_bounds__(1024, 1) fftz_uniform_kernel(GridT<R> g, Field
 // imaginary parts of (0,0) and (0,N3/2) are zeroed after the solve.  The
 // rows are FP64 in both forms: the zero and lowest wavenumbers are nearly
 // singular, and the FP32 form reads and writes its FP32 spectrum around them.
-template <class R, int ITEM = 0>
+// The unweighted mean of the solution (:703-710) leaves with them: the (i,k) sum
+// of the inverse transform of one j-plane is the real part of its (0,0)
+// coefficient, so the mean is the sum of line (0,0) over N1 N2 N3.
+template <class R>
 struct Modal {
     using Real = double;
     static constexpr int NRHS = 2;
-    static constexpr bool FAST_RCP = true;    // measured faster with qrcp
-    static constexpr int MINB = LineOcc<R>::modal;
-    static constexpr int MREG = LineOcc<Real>::reg_modal;
-    static constexpr int NT = LineOcc<Real>::nt_modal;
-    static constexpr bool CONTIG = false;
-    static constexpr bool LINE_PER_THREAD = true;   // measured faster in both forms
-    GridT<R> g; FieldsT<R> f; int TL; int h1p;
+    // 8 lines of 16 bytes a row; four rows ahead (256^3, ps per cell: 5.7; two ahead 6.1, 16 lines 8.3; the lane-per-
+    // partition solver before it 7.3)
+    static constexpr int AHEAD = 4, TPS = 512, ROWS = 16, LGTI = 3;
+    static constexpr bool TOTAL = true;
+    GridT<R> g; FieldsT<R> f; int h1p;
     __device__ bool skip() const { return blown(g); }
-    struct State { double dt; };
-    __device__ State prepare() const { return State{g.scal[S_DT]}; }
-    __device__ int lk(int l) const { return vbx<ITEM>() * TL + l; }
-    __device__ bool line_ok(int l) const { return lk(l) < h1p; }
-    __device__ Coef<double, 2> build(int l, int r, const State &st) const
-    {
-        const int kx = lk(l), kz = vby<ITEM>(), j = r + 1;
-        const double am = f.fam[j], ap = f.fap[j];
-        Coef<double, 2> cf;
-        const cplx_t<R> s = f.S[sidx(g, h1p, kx, j, kz)];
-        if (kx == 0 && kz == 0 && j == 1) {
-            cf.a = 0.0; cf.b = 1.0; cf.c = 0.0; cf.d[0] = 0.0; cf.d[1] = s.y;
-        } else {
-            cf.a = am; cf.c = ap;
-            cf.b = (-am - ap) - f.dxk2[kx] - f.dzk[kz];
-            cf.d[0] = s.x; cf.d[1] = s.y;
+    __device__ int lines() const { return h1p; }
+    __device__ void set_total(double t) const { g.scal[S_AVER] = t / (double)g.N1 / (double)g.N2 / (double)g.N3; }
+    struct March {
+        double kk;                                      // sum of the modified wavenumbers
+        bool pin;
+        const cplx_t<R> *p;
+        __device__ __forceinline__ March(const Modal &q, int line, int by, int r0)
+            : kk(ld(q.f.dxk2 + line) + ld(q.f.dzk + by)), pin(line == 0 && by == 0), p(q.f.S + sidx(q.g, q.h1p, line, r0 + 1, by)) {}
+        struct In { cplx_t<R> s; double am, ap; };
+        __device__ __forceinline__ void load(const Modal &q, int r, In &n)
+        {
+            n.s = *p;
+            n.am = ld(q.f.fam + r + 1); n.ap = ld(q.f.fap + r + 1);
+            p += q.h1p;
         }
-        return cf;
-    }
-    __device__ void emit(int l, int r, const double *x, const State &st) const
-    {
-        const int kx = lk(l), kz = vby<ITEM>(), j = r + 1;
-        const bool zi = (kx == 0) && (kz == 0 || kz == g.N3 / 2);
-        f.S[sidx(g, h1p, kx, j, kz)] = mkc<R>(R(x[0]), zi ? R(0) : R(x[1]));
-    }
+        __device__ __forceinline__ void row(const Modal &, int r, const In &n, double &a, double &b, double &c, double *d)
+        {
+            const bool fix = pin && r == 0;
+            a = fix ? 0.0 : n.am; c = fix ? 0.0 : n.ap;
+            b = fix ? 1.0 : -n.am - n.ap - kk;
+            d[0] = fix ? 0.0 : (double)n.s.x; d[1] = (double)n.s.y;
+        }
+    };
+    struct Out {
+        cplx_t<R> *p;
+        bool zi;
+        double total;
+        __device__ __forceinline__ Out(const Modal &q, int line, int by, int r)
+            : p(q.f.S + sidx(q.g, q.h1p, line, r + 1, by)), zi(line == 0 && (by == 0 || by == q.g.N3 / 2)), total(0.0) {}
+        __device__ __forceinline__ void put(const Modal &q, const double *x)
+        {
+            const R re = R(x[0]);
+            *p = mkc<R>(re, zi ? R(0) : R(x[1]));
+            total += (double)re;
+            p -= q.h1p;
+        }
+    };
 };
-
-// Unweighted mean of the solution (:703-710): the (i,k) sum of the inverse
-// transform of one j-plane is the real part of its (0,0) coefficient.
-template <class R>
-__global__ void mean_kernel(GridT<R> g, FieldsT<R> f, int h1p)
-{
-    __shared__ double red[256];
-    if (blown(g)) return;
-    double s = 0.0;
-    for (int j = 1 + threadIdx.x; j <= g.N2; j += blockDim.x) s += (double)f.S[sidx(g, h1p, 0, j, 0)].x;
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) g.scal[S_AVER] = red[0] / (double)g.N1 / (double)g.N2 / (double)g.N3;
-}
 
 // c2r along x (:681-683) with the scaling (:694-700), the mean removal
 // (:712-714) and the periodic ghosts of ghost(dP) (main.f90:189).
@@ -776,16 +771,12 @@ __global__ void __launch_bounds__(512) ifftx_uniform_kernel(GridT<R> g, FieldsT<
     }
 }
 
-// dP wall extrapolation (:719-736) on every (i,k) including ghost columns,
-// which is what the extrapolation followed by ghost(dP) produces.
 template <class R>
-__global__ void dp_wall_kernel(GridT<R> g, FieldsT<R> f, double ab, double bb, double at, double bt)
+__global__ void dp_wall_kernel(GridT<R> g, FieldsT<R> f, WallRows w)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y;
     if (i > g.N1 + 1 || blown(g)) return;
-    R *dP = f.dP;
-    dP[ix(g, i, 0, k)] = R(ab * (double)dP[ix(g, i, 1, k)] - bb * (double)dP[ix(g, i, 2, k)]);
-    dP[ix(g, i, g.N2 + 1, k)] = R(at * (double)dP[ix(g, i, g.N2, k)] - bt * (double)dP[ix(g, i, g.N2 - 1, k)]);
+    dp_wall_cell(g, f.dP, i, k, w);
 }
 
 // ---------------------------------------------------------------------------
@@ -854,16 +845,12 @@ __global__ void __launch_bounds__(256) projection_kernel(GridT<R> g, FieldsT<R> 
     f.dP0n[c] = dp0n;
 }
 
-// P(i,0,k) = Pbc_a P(i,1,k) - Pbc_b P(i,2,k) and the top-wall counterpart
-// (:853-869), then ghost(P).
 template <class R>
-__global__ void p_wall_kernel(GridT<R> g, FieldsT<R> f, double ab, double bb, double at, double bt)
+__global__ void p_wall_kernel(GridT<R> g, FieldsT<R> f, WallRows w)
 {
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, k = 1 + blockIdx.y;
     if (i > g.N1 || blown(g)) return;
-    const R *P = f.P;
-    store_periodic(g, f.P, i, 0, k, R(ab * (double)P[ix(g, i, 1, k)] - bb * (double)P[ix(g, i, 2, k)]));
-    store_periodic(g, f.P, i, g.N2 + 1, k, R(at * (double)P[ix(g, i, g.N2, k)] - bt * (double)P[ix(g, i, g.N2 - 1, k)]));
+    p_wall_cell(g, f.P, i, k, w);
 }
 
 template <class R>
@@ -948,19 +935,14 @@ template <class R>
 void launch_modal(const Ctx<R> &cx, cudaStream_t s)
 {
     const GridT<R> &g = cx.g;
-    LinePlan pm = plan_for<Modal<R>>(g.N2, false, fit_tl<Modal<R>>(g.N2, false, cx.tl_modal, cx.lanes), cx.lanes);
-    launch_lines(Modal<R>{g, cx.f, pm.TL, cx.h1p}, pm, dim3((cx.h1p + pm.TL - 1) / pm.TL, g.N3), s, K_MODAL, cx);
+    launch_march(cx, Modal<R>{g, cx.f, cx.h1p}, g.N2, false, cx.h1p, g.N3, s, K_MODAL);
 }
 
 template <class R>
-void launch_poisson_back(const Ctx<R> &cx, cudaStream_t s)
+void launch_poisson_back(const Ctx<R> &cx, cudaStream_t s, bool walls)
 {
     const GridT<R> &g = cx.g;
     const int h1p = cx.h1p, NLx = cx.ifft_lines_x, form = ifftx_form(cx.fp1u, NLx);
-    probe_begin(cx, K_MEAN, s);
-    mean_kernel<R><<<1, 256, 0, s>>>(g, cx.f, h1p);
-    probe_end(cx, K_MEAN, s);
-    record_launch_error("mean");
     launch_fftz<1>(cx, s, K_FFTZ_INV, "fftz_inv");
     probe_begin(cx, K_IFFTX, s);
     const dim3 gx((g.N2 + NLx - 1) / NLx, g.N3);
@@ -982,30 +964,32 @@ void launch_poisson_back(const Ctx<R> &cx, cudaStream_t s)
     }
     probe_end(cx, K_IFFTX, s);
     record_launch_error("ifftx");
+    if (!walls) return;
     probe_begin(cx, K_DP_WALL, s);
-    dp_wall_kernel<R><<<dim3((g.N1 + 2 + 127) / 128, g.N3 + 2), 128, 0, s>>>(g, cx.f, cx.wall_ab, cx.wall_bb, cx.wall_at, cx.wall_bt);
+    dp_wall_kernel<R><<<dim3((g.N1 + 2 + 127) / 128, g.N3 + 2), 128, 0, s>>>(g, cx.f, WallRows{cx.wall_ab, cx.wall_bb, cx.wall_at, cx.wall_bt});
     probe_end(cx, K_DP_WALL, s);
     record_launch_error("dp_wall");
 }
 
 template <class R>
-void launch_poisson_rest(const Ctx<R> &cx, cudaStream_t s)
+void launch_poisson_rest(const Ctx<R> &cx, cudaStream_t s, bool walls)
 {
     launch_poisson_fwd(cx, s);
     launch_modal(cx, s);
-    launch_poisson_back(cx, s);
+    launch_poisson_back(cx, s, walls);
 }
 
 template <class R>
-void launch_projection(const Ctx<R> &cx, cudaStream_t s)
+void launch_projection(const Ctx<R> &cx, cudaStream_t s, bool walls)
 {
     const GridT<R> &g = cx.g;
     probe_begin(cx, K_PROJECT, s);
     projection_kernel<R><<<dim3((g.N1 + 255) / 256, g.N2, g.N3), 256, 0, s>>>(g, cx.f);
     probe_end(cx, K_PROJECT, s);
     record_launch_error("projection");
+    if (!walls) return;
     probe_begin(cx, K_P_WALL, s);
-    p_wall_kernel<R><<<dim3((g.N1 + 127) / 128, g.N3), 128, 0, s>>>(g, cx.f, cx.wall_ab, cx.wall_bb, cx.wall_at, cx.wall_bt);
+    p_wall_kernel<R><<<dim3((g.N1 + 127) / 128, g.N3), 128, 0, s>>>(g, cx.f, WallRows{cx.wall_ab, cx.wall_bb, cx.wall_at, cx.wall_bt});
     probe_end(cx, K_P_WALL, s);
     record_launch_error("p_wall");
 }
@@ -1013,13 +997,11 @@ void launch_projection(const Ctx<R> &cx, cudaStream_t s)
 #undef IR
 
 // the two forms
-// The modal solves of many cases in one launch.
+// The modal solves of many cases.
 template <class R>
 void launch_modal_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s)
 {
-    multi_stage<Modal<R, 1>>(cs, A, s, "modal",
-        [](const Ctx<R> &x) { return StageShape{x.g.N2, false, x.tl_modal, x.h1p, x.g.N3}; },
-        [](const Ctx<R> &x, int tl) { return Modal<R, 1>{x.g, x.f, tl, x.h1p}; });
+    march_stage(cs, A, s, launch_modal<R>);
 }
 
 template void launch_modal_multi<double>(const std::vector<Ctx<double> *> &, MultiArena &, cudaStream_t);
@@ -1028,13 +1010,13 @@ template void launch_modal<double>(const Ctx<double> &, cudaStream_t);
 template void launch_modal<float>(const Ctx<float> &, cudaStream_t);
 template void launch_pseudo_prhs_fftx<double>(const Ctx<double> &, cudaStream_t, bool);
 template void launch_pseudo_prhs_fftx<float>(const Ctx<float> &, cudaStream_t, bool);
-template void launch_poisson_rest<double>(const Ctx<double> &, cudaStream_t);
-template void launch_poisson_rest<float>(const Ctx<float> &, cudaStream_t);
+template void launch_poisson_rest<double>(const Ctx<double> &, cudaStream_t, bool);
+template void launch_poisson_rest<float>(const Ctx<float> &, cudaStream_t, bool);
 template void launch_poisson_fwd<double>(const Ctx<double> &, cudaStream_t);
 template void launch_poisson_fwd<float>(const Ctx<float> &, cudaStream_t);
-template void launch_poisson_back<double>(const Ctx<double> &, cudaStream_t);
-template void launch_poisson_back<float>(const Ctx<float> &, cudaStream_t);
-template void launch_projection<double>(const Ctx<double> &, cudaStream_t);
-template void launch_projection<float>(const Ctx<float> &, cudaStream_t);
+template void launch_poisson_back<double>(const Ctx<double> &, cudaStream_t, bool);
+template void launch_poisson_back<float>(const Ctx<float> &, cudaStream_t, bool);
+template void launch_projection<double>(const Ctx<double> &, cudaStream_t, bool);
+template void launch_projection<float>(const Ctx<float> &, cudaStream_t, bool);
 
 } // namespace tcs

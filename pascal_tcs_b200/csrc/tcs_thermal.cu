@@ -1,8 +1,8 @@
 // tcs_thermal.cu -- energy equation: mpi_thermal_coeffi + mpi_thermal_solver
 // (module_solve_thermal.f90:116-532) as three fused kernels, one per ADI
-// sweep.  Each kernel evaluates the temperature-dependent properties at the
-// stencil points it needs, builds the tridiagonal rows straight into shared
-// memory and solves its lines there; only the sweep result goes to HBM.
+// sweep (tcs_march.cuh).  Each evaluates the temperature-dependent properties
+// at the stencil points it needs, builds the tridiagonal rows and solves its
+// lines; only the sweep result goes to HBM.
 //
 //   z sweep  (:236-366) lines (i,j), rows k, cyclic   -> R
 //   x sweep  (:388-434) lines (j,k), rows i, cyclic   R -> R
@@ -17,7 +17,7 @@ template <class R>
 struct ThermalZ {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12;   // FP64 inputs of two rows do not fit the registers
+    static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12, LGTI = 4;   // FP64 inputs of two rows do not fit the registers
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -225,7 +225,7 @@ template <class R>
 struct ThermalY {
     using Real = R;
     static constexpr int NRHS = 1;
-    static constexpr int AHEAD = 0, TPS = 512, ROWS = 16;
+    static constexpr int AHEAD = 0, TPS = 512, ROWS = 16, LGTI = 4;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }

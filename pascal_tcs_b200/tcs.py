@@ -71,7 +71,7 @@ class TcsConfig(ctypes.Structure):
 
 
 PREC_FP64 = 0          # the reference's arithmetic
-PREC_FP32_MIXED = 1    # FP32 fields/stencils/sweeps/FFTs, FP64 refinement, modal solves, projection, reductions
+PREC_FP32_MIXED = 1    # FP32 fields and stencils; FP64 eliminations, FFTs, modal solves, projection, reductions
 
 
 def default_config(**kw) -> dict:
@@ -458,9 +458,9 @@ def check_reciprocal(n: int = 1 << 16, fp32: bool = False) -> float:
 
 class Ensemble:
     """Independent cases on one GPU advanced together by one CUDA-graph launch
-    per step (tcs_ensemble_*).  batched: True = each line sweep is one launch
-    over all cases (blocks pull (case, block) work items); False = every
-    case's step is its own graph branch; None (default) = auto: the first 8
+    per step (tcs_ensemble_*).  batched: True = stage by stage, a stage's
+    launches of all cases side by side; False = every case's step is its own
+    graph branch; None (default) = auto: the first 8
     steps measure both forms, then the faster one is kept."""
 
     def __init__(self, solvers, batched=None):
