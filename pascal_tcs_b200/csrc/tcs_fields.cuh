@@ -39,6 +39,7 @@ struct FieldsT {
     // the same properties with their face averages, four words per (j,k) entry
     // (momentum_coeffi): Mu, Mu_y, Mu_z, Mu_yz and invRho, invRho_y, invRho_z, 0
     R *MuT, *iRT;
+    double *iRTd;            // the invRho words in FP64 (the same array in the FP64 form)
     // Poisson spectral work array: (h1p, N2, N3) complex, kx fastest
     cplx_t<R> *S;
     // modified wavenumbers and y coefficients of the modal solves (FP64 in both forms)

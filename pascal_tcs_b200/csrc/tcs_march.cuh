@@ -20,6 +20,13 @@
 //
 // Elimination, rows and solution are FP64 in both numerical forms; the
 // FP32-mixed form builds its rows in FP32 and rounds the solution once.
+//
+// What it bought (ms, from sweeps that built every row apart and solved in a
+// separate phase): dw_z at 256^3 0.51 -> 0.36, FP32-mixed 0.44 -> 0.30; at 180 x
+// 151 x 250 0.23 -> 0.17; at 512^3 (column form) 5.94 -> 3.07; du_y at 256^3
+// FP32-mixed 0.26 -> 0.17.  What bounds it now: load latency at the 16 warps per
+// SM that 128 registers allow (long-scoreboard stalls 4 to 5 per issue, issue
+// slots 40% busy, FP64 pipe 25 to 33%, DRAM 20 to 32%).
 #pragma once
 
 #include "tcs_fields.cuh"
@@ -314,7 +321,12 @@ __global__ void __launch_bounds__(NT, Prob::TPS / NT) march_kernel(const __grid_
 // lanes; thread (line l, segment s) marches over its rows there, parks d, c and e
 // in the places of the words it has used (planes 0, 1, 2), and the solution
 // leaves plane 0 as it came, a warp per line.  The line stride is odd, so the
-// TI lines of a warp's march sit on distinct banks.
+// TI lines of a warp's march sit on distinct banks.  Two blocks per SM: one
+// stages while the other marches.  Against the lane-per-partition solver that
+// was here before (ms): 256^3 FP64 du_x 0.195 -> 0.162, FP32-mixed 0.227 -> 0.148
+// and thermal_x 0.345 -> 0.251; 400 x 200 x 384 FP32-mixed du_x 0.56 -> 0.32; level
+// (within 10%) from 384 rows on in FP64.  It moves 3 or 4 arrays at 2.5 to 2.7
+// TB/s: latency at 16 warps per SM bounds it.
 // The problem supplies
 //   static constexpr int WORDS;                                             // planes staged: 0 the right-hand side, 1.. the stencil
 //   struct Stage { Stage(const Prob &, int line, int by);  void put(const Prob &, int r, double *w, int PL); }   // row r of the line, words PL apart

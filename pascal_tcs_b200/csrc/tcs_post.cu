@@ -4,8 +4,7 @@
 // One kernel: block partials in a fixed order; the last block to finish combines
 // them and updates dt, time and CFL on the device (deterministic).  Inside a step
 // it also writes the wall rows of dP and P, which nothing reads before (three
-// launches fewer per step: 19 us of 64^3's 203).  Both forms
-// reduce in FP64 from their fields, and the per-thread sums are compensated
+// launches fewer per step).  Both forms reduce in FP64 from their fields, and the per-thread sums are compensated
 // (Neumaier), so the diagnostics keep FP64 accuracy over 512^3 cells.
 #include "tcs_kernels.h"
 

@@ -31,6 +31,7 @@
 namespace tcs {
 
 #define IR(jj, kk) ld(f.iR2d + ix2(g, (jj), (kk)))   // FP64 invRho in both forms
+#define IRT(jj, kk, w) ld(f.iRTd + 4 * ix2(g, (jj), (kk)) + (w))   // and at the lower y (1) and z (2) faces
 
 template <class C> struct CReal;
 template <> struct CReal<double2> { using T = double; };
@@ -373,20 +374,19 @@ __global__ void __launch_bounds__(256) prhs_fftx_kernel(GridT<R> g, FieldsT<R> f
     }
 }
 
-// The split form of the same stage, for a one-radix plan of N1 (512 = 8^3,
-// 256 = 4^4): prhs_kernel forms the pseudo-update and the right-hand side one
-// cell per thread and stores the right-hand side in FP64 (padded layout, in
-// f.prhs); fftx_uniform_kernel transforms its x lines.  The fused kernel above
+// The split form of the same stage: prhs_kernel forms the pseudo-update and the
+// right-hand side one cell per thread and stores the right-hand side in FP64
+// (padded layout, in f.prhs); fftx_uniform_kernel (a one-radix plan of N1: 512 =
+// 8^3, 256 = 4^4) or fftx_kernel transforms its x lines.  The fused kernel above
 // keeps the right-hand side in shared memory, but its FFT's registers and
 // barriers hold its loads back (measured at 512^3: 3.55 ms FP64, 4.82 ms
 // FP32-mixed).  The new U at the x-upper neighbour (periodic) is formed again
-// from its inputs with the same arithmetic, so both forms give the same bits.
+// from its inputs with the same arithmetic as the neighbour's own.
 template <class R>
 __global__ void __launch_bounds__(256) prhs_kernel(GridT<R> g, FieldsT<R> f, int with_pseudo)
 {
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y, k = 1 + blockIdx.z;
     if (i > g.N1 || blown(g)) return;
-    const double *dx1 = g.d1.dx, *dx2 = g.d2.dx, *dx3 = g.d3.dx;
     const double *rdx1 = g.d1.rdx, *rdx2 = g.d2.rdx, *rdx3 = g.d3.rdx;
     const double *rdmx1 = g.d1.rdmx, *rdmx2 = g.d2.rdmx, *rdmx3 = g.d3.rdmx;
     const int sj = g.P1, sk = g.P1 * g.P2;   // 32-bit offsets (the padded grid is below 2^31 cells)
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(256) prhs_kernel(GridT<R> g, FieldsT<R> f, int
     const double dt = g.scal[S_DT], rdt = 1.0 / dt;
     const Phys &p = g.phd;
     const double rdtc = rdt / p.Cmp;
-    const int im = i - 1, ip = i + 1, jm = j - 1, jp = j + 1, km = k - 1, kp = k + 1;
+    const int ip = i + 1, jp = j + 1, kp = k + 1;
     const double DivUm = (Uxp - Uc) * rdx1[i] + (jvp * Vyp - jvm * Vc) * rdx2[j] + (Wzp - Wc) * rdx3[k];
     const double cbc = (1.0 - jvm) * p.Vbt * rdx2[j] - (1.0 - jvp) * p.Vup * rdx2[j];
     const R *dPh = f.dPhat;
@@ -440,16 +440,10 @@ __global__ void __launch_bounds__(256) prhs_kernel(GridT<R> g, FieldsT<R> f, int
     const double ddpdx1 = (Pc - (double)ld(dPh + (c - 1))) * rdmx1[i], ddpdx2 = ((double)ld(dPh + (c + 1)) - Pc) * rdmx1[ip];
     const double ddpdy3 = (Pc - (double)ld(dPh + (c - sj))) * rdmx2[j], ddpdy4 = ((double)ld(dPh + (c + sj)) - Pc) * rdmx2[jp];
     const double ddpdz5 = (Pc - (double)ld(dPh + (c - sk))) * rdmx3[k], ddpdz6 = ((double)ld(dPh + (c + sk)) - Pc) * rdmx3[kp];
-    const double iRjk = IR(j, k);
-    const double iR1 = 0.5 * rdmx1[i] * (dx1[im] * iRjk + dx1[i] * iRjk);
-    const double iR2_ = 0.5 * rdmx1[ip] * (dx1[ip] * iRjk + dx1[i] * iRjk);
-    const double iR3 = 0.5 * rdmx2[j] * (dx2[jm] * iRjk + dx2[j] * (double)IR(jm, k));
-    const double iR4 = 0.5 * rdmx2[jp] * (dx2[jp] * iRjk + dx2[j] * (double)IR(jp, k));
-    const double iR5 = 0.5 * rdmx3[k] * (dx3[km] * iRjk + dx3[k] * (double)IR(j, km));
-    const double iR6 = 0.5 * rdmx3[kp] * (dx3[kp] * iRjk + dx3[k] * (double)IR(j, kp));
-    const double Extra = ((1.0 - iR2_) * ddpdx2 - (1.0 - iR1) * ddpdx1) * rdx1[i]
-                       + ((1.0 - iR4) * ddpdy4 - (1.0 - iR3) * ddpdy3) * rdx2[j]
-                       + ((1.0 - iR6) * ddpdz6 - (1.0 - iR5) * ddpdz5) * rdx3[k];
+    // invRho is constant along i; its averages at the y and z faces are in the table
+    const double Extra = (1.0 - IRT(j, k, 0)) * (ddpdx2 - ddpdx1) * rdx1[i]
+                       + ((1.0 - IRT(jp, k, 1)) * ddpdy4 - (1.0 - IRT(j, k, 1)) * ddpdy3) * rdx2[j]
+                       + ((1.0 - IRT(j, kp, 2)) * ddpdz6 - (1.0 - IRT(j, k, 2)) * ddpdz5) * rdx3[k];
     f.prhs[c] = (DivUm - cbc) * rdtc + Extra;
 }
 
@@ -510,6 +504,35 @@ __global__ void __launch_bounds__(512) fftx_uniform_kernel(GridT<R> g, FieldsT<R
         const C v2 = (l & 1) ? make_double2(0.5 * (z.y + zr.y), 0.5 * (zr.x - z.x))
                              : make_double2(0.5 * (z.x + zr.x), 0.5 * (z.y - zr.y));
         f.S[sidx(g, h1p, kx, j, k - 1)] = mkc<R>(R(v2.x), R(v2.y));
+    }
+}
+
+// The same for any other plan of N1 (radices 2 to 5): two line-major buffers, 256 threads.
+template <class R>
+__global__ void __launch_bounds__(256) fftx_kernel(GridT<R> g, FieldsT<R> f, FFTPlan fp, int NL, int h1p)
+{
+    using C = double2;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    if (blown(g)) return;
+    const int N1 = g.N1, j0 = 1 + blockIdx.x * NL, k = 1 + blockIdx.y, nfl = (NL + 1) >> 1;
+    C *const b0 = reinterpret_cast<C *>(smraw), *const b1 = b0 + nfl * N1;
+    const double *const prhs = f.prhs;
+#pragma unroll 2
+    for (int t = threadIdx.x; t < nfl * N1; t += blockDim.x) {
+        const int p = (int)fp.dn.div(t), q = t - p * N1, ja = j0 + 2 * p;
+        const double re = (2 * p < NL && ja <= g.N2) ? ld(prhs + ix(g, q + 1, ja, k)) : 0.0;
+        const double im = (2 * p + 1 < NL && ja + 1 <= g.N2) ? ld(prhs + ix(g, q + 1, ja + 1, k)) : 0.0;
+        b0[t] = make_double2(re, im);
+    }
+    __syncthreads();
+    const C *res = block_fft_lm<-1>(b0, b1, nfl, N1, fp, f.tw1);
+    for (int t = threadIdx.x; t < NL * h1p; t += blockDim.x) {
+        const int l = (int)fp.dh.div(t), kx = t - l * h1p, j = j0 + l;
+        if (j > g.N2) continue;
+        const C z = res[(l >> 1) * N1 + kx], zr = res[(l >> 1) * N1 + (kx == 0 ? 0 : N1 - kx)];
+        const C v = (l & 1) ? make_double2(0.5 * (z.y + zr.y), 0.5 * (zr.x - z.x))
+                            : make_double2(0.5 * (z.x + zr.x), 0.5 * (z.y - zr.y));
+        f.S[sidx(g, h1p, kx, j, k - 1)] = mkc<R>(R(v.x), R(v.y));
     }
 }
 
@@ -853,6 +876,15 @@ __global__ void p_wall_kernel(GridT<R> g, FieldsT<R> f, WallRows w)
     p_wall_cell(g, f.P, i, k, w);
 }
 
+// Threads per block of the kernels with a thread per cell along i: the fewest
+// blocks of at most 256 that cover a row, in whole warps (180 cells: one block
+// of 192, not 256).
+static int rowt(int n)
+{
+    const int nb = (n + 255) / 256;
+    return ((n + nb - 1) / nb + 31) / 32 * 32;
+}
+
 template <class R>
 static size_t fftx_smem(const Ctx<R> &cx)
 {
@@ -865,15 +897,23 @@ void launch_pseudo_prhs_fftx(const Ctx<R> &cx, cudaStream_t s, bool with_pseudo)
 {
     const GridT<R> &g = cx.g;
     const int NL = cx.fft_lines_x;
-    if (cx.f.prhs && ifftx_form(cx.fp1u, NL) == 1) {   // the split form
-        const size_t sm = ifftx_smem(cx.fp1u, NL, 1);
+    const long long cells = (long long)g.N1 * g.N2 * g.N3;
+    const int form = ifftx_form(cx.fp1u, NL);
+    // the split form, but for small grids without a one-radix N1, where the second
+    // launch costs more than it frees (ps per cell, split and fused: 32^3 477 and
+    // 324; 96 x 77 x 90 46 and 50, FP32-mixed 49 and 59; 400 x 200 x 384 FP32-mixed 33 and 43)
+    if (form == 1 || cells >= 262144) {
+        const size_t sm = form == 1 ? ifftx_smem(cx.fp1u, NL, 1) : (size_t)((NL + 1) / 2) * g.N1 * 2 * sizeof(double2);
         const int nt = ((NL + 1) / 2) * (g.N1 / cx.fp1u.radix[0]);
         const dim3 gx((g.N2 + NL - 1) / NL, g.N3);
-        static size_t c8[64] = {}, c4[64] = {};
+        static size_t c8[64] = {}, c4[64] = {}, cg[64] = {};
         probe_begin(cx, K_PRHS_FFTX, s);
-        prhs_kernel<R><<<dim3((g.N1 + 255) / 256, g.N2, g.N3), 256, 0, s>>>(g, cx.f, with_pseudo ? 1 : 0);
+        prhs_kernel<R><<<dim3((g.N1 + rowt(g.N1) - 1) / rowt(g.N1), g.N2, g.N3), rowt(g.N1), 0, s>>>(g, cx.f, with_pseudo ? 1 : 0);
         record_launch_error("prhs");
-        if (cx.fp1u.radix[0] == 8) {
+        if (form != 1) {
+            smem_opt_in((const void *)fftx_kernel<R>, sm, cg);
+            fftx_kernel<R><<<gx, 256, sm, s>>>(g, cx.f, cx.fp1, NL, cx.h1p);
+        } else if (cx.fp1u.radix[0] == 8) {
             smem_opt_in((const void *)fftx_uniform_kernel<8, R>, sm, c8);
             fftx_uniform_kernel<8, R><<<gx, nt, sm, s>>>(g, cx.f, cx.fp1u, NL, cx.h1p);
         } else {
@@ -995,6 +1035,7 @@ void launch_projection(const Ctx<R> &cx, cudaStream_t s, bool walls)
 }
 
 #undef IR
+#undef IRT
 
 // the two forms
 // The modal solves of many cases.
