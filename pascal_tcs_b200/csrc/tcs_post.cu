@@ -79,8 +79,12 @@ __device__ __forceinline__ void finalize(const GridT<R> &g, const FieldsT<R> &f,
     sc[S_STEP] = step + 1;
 }
 
+// Bound by the latency of its loads, so by the blocks per SM: four of 256 threads at
+// 64 registers.  Without the bound the FP32 form, which reads two words per velocity,
+// takes 88 registers and two blocks: 0.220 against 0.170 ms at 256^3, 0.374 against
+// 0.294 ms at 400 x 200 x 384.  Neither form spills.
 template <class R>
-__global__ void __launch_bounds__(256, HasLo<R>::on ? 1 : 4) post_kernel(GridT<R> g, FieldsT<R> f, FastDiv dn1, FastDiv dn2, int record_hist, int walls, WallRows wr)
+__global__ void __launch_bounds__(256, 4) post_kernel(GridT<R> g, FieldsT<R> f, FastDiv dn1, FastDiv dn2, int record_hist, int walls, WallRows wr)
 {
     __shared__ double red[PT_N][256];
     __shared__ int s_last;
