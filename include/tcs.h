@@ -230,6 +230,12 @@ const char *tcs_timer_name(int timer);
 int tcs_bounds_checked(void);
 int tcs_bounds_violations(tcs_ctx *ctx, double *count);
 int tcs_set_use_graph(tcs_ctx *ctx, int on);
+/* The z sweeps of long FP64 lines wait for asynchronous copies, each wait bounded
+ * to `polls` polls (default 2^22).  If one runs out, the rest of the step is skipped
+ * and tcs_step, tcs_post_div, tcs_post_cfl and tcs_ensemble_step return
+ * TCS_ERR_CUDA; the fields are then undefined until tcs_restore.  0 makes every
+ * such wait run out at once, which is how the reporting is tested. */
+int tcs_set_copy_polls(tcs_ctx *ctx, int polls);
 /* launch-shape knobs (powers of two): lines per thread block of the x and z
  * FFTs, and the most partitions a tridiagonal line is split over (TCS_TUNE_LANES;
  * 32: no bound, a line's length decides).

@@ -571,6 +571,7 @@ int tcs_create(const tcs_config *cfg, tcs_ctx **out)
     c->cx.y_solver = 1;
     c->cx.mixed_rows = 1;
     c->cx.z_staging = 1;
+    c->cx.copy_polls = COL_WAIT;
     c->cx.spec_live = false;
     c->cx.probe = &c->probe;
     sync_shapes(c);
@@ -759,6 +760,25 @@ int tcs_set_dt(tcs_ctx *c, double dt)
     return TCS_OK;
 }
 
+// The scalar block with the words past the public ones, after the stream's work.
+static int read_scalars(tcs_ctx *c, double *sc)
+{
+    CK(cudaMemcpyAsync(sc, c->cx.g.scal, sizeof(double) * S_NALLOC, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return TCS_OK;
+}
+
+// What the scalars say about the step: a copy that did not arrive (the fields
+// are then undefined until tcs_restore), a blow-up, or nothing.
+static int stopped(const double *sc, const char *blown)
+{
+    if (sc[S_TIMEOUT] != 0.0)
+        return set_err(TCS_ERR_CUDA, "step " + std::to_string((long long)sc[S_BLOWUP]) + ": a bulk copy of a z sweep did not arrive within its bounded wait ("
+                                     + std::to_string((long long)sc[S_TIMEOUT]) + " blocks); the fields are undefined");
+    return sc[S_BLOWUP] != 0.0 ? set_err(TCS_ERR_BLOWUP, blown) : TCS_OK;
+}
+static const char *const k_blowup = "BLOW UP: max divergence >= 1e-3";
+
 // ---- stages ---------------------------------------------------------------
 #define ENTER(c)                                                   \
     if (!(c)) return set_err(TCS_ERR_ARG, "null context");        \
@@ -899,21 +919,21 @@ int tcs_post_div(tcs_ctx *c, double *maxDivU)
     if (r) return r;
     on_ctx(c, [&](auto &x) { launch_post(x, c->stream, 1, false); });
     if ((r = take_launch_error())) return r;
-    double sc[S_NSCAL];
-    CK(cudaMemcpyAsync(sc, c->cx.g.scal, sizeof(sc), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    double sc[S_NALLOC];
+    if ((r = read_scalars(c, sc))) return r;
     if (maxDivU) *maxDivU = sc[S_MAXDIV];
-    return sc[S_BLOWUP] != 0.0 ? set_err(TCS_ERR_BLOWUP, "BLOW UP: max divergence >= 1e-3") : TCS_OK;
+    return stopped(sc, k_blowup);
 }
 
 int tcs_post_cfl(tcs_ctx *c, double *CFL, double *dt)
 {
     ENTER(c);
-    double sc[S_NSCAL];
-    CK(cudaMemcpyAsync(sc, c->cx.g.scal, sizeof(sc), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    double sc[S_NALLOC];
+    const int r = read_scalars(c, sc);
+    if (r) return r;
     if (CFL) *CFL = sc[S_CFL];
     if (dt) *dt = sc[S_DT];
+    if (sc[S_TIMEOUT] != 0.0) return stopped(sc, k_blowup);
     return std::isfinite(sc[S_DT]) ? TCS_OK : set_err(TCS_ERR_NONFINITE, "dt is not finite");
 }
 
@@ -1035,6 +1055,17 @@ int tcs_get_tuning(tcs_ctx *c, int knob, int *value)
     return TCS_OK;
 }
 
+int tcs_set_copy_polls(tcs_ctx *c, int polls)
+{
+    ENTER(c);
+    if (polls < 0) return set_err(TCS_ERR_ARG, "polls < 0");
+    c->cx.copy_polls = polls;
+    sync_shapes(c);
+    for (auto &ge : c->graphs) cudaGraphExecDestroy(ge.exec);
+    c->graphs.clear();
+    return TCS_OK;
+}
+
 int tcs_set_use_graph(tcs_ctx *c, int on)
 {
     ENTER(c);
@@ -1053,10 +1084,8 @@ int tcs_step(tcs_ctx *c, int nsteps, int *done)
     const int fl[] = {TCS_F_T, TCS_F_U, TCS_F_V, TCS_F_W, TCS_F_P, TCS_F_DPHAT};
     for (int f : fl) ensure_ghosts(c, f);
     if ((r = take_launch_error())) return r;
-    double sc0[S_NSCAL];
-    CK(cudaMemcpyAsync(sc0, c->cx.g.scal, sizeof(sc0), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (sc0[S_BLOWUP] != 0.0) return set_err(TCS_ERR_BLOWUP, "the case has already blown up");
+    double sc0[S_NALLOC];
+    if ((r = read_scalars(c, sc0)) || (r = stopped(sc0, "the case has already blown up"))) return r;
     const bool graph = c->use_graph && c->probe.mask == 0;
     for (int n = 0; n < nsteps; n++) {
         if (!graph) {
@@ -1088,14 +1117,12 @@ int tcs_step(tcs_ctx *c, int nsteps, int *done)
         CK(cudaGraphLaunch(exec, c->stream));
         g_launches += kernels_this;
     }
-    double sc[S_NSCAL];
-    CK(cudaMemcpyAsync(sc, c->cx.g.scal, sizeof(sc), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    double sc[S_NALLOC];
+    if ((r = read_scalars(c, sc))) return r;
     c->ghost_ok |= (1u << TCS_F_T) | (1u << TCS_F_U) | (1u << TCS_F_V) | (1u << TCS_F_W) | (1u << TCS_F_P) | (1u << TCS_F_DPHAT) | (1u << TCS_F_DP);
     const int steps_now = (int)sc[S_STEP] - (int)sc0[S_STEP];
     if (done) *done = steps_now;
-    if (sc[S_BLOWUP] != 0.0) return set_err(TCS_ERR_BLOWUP, "BLOW UP: max divergence >= 1e-3");
-    return TCS_OK;
+    return stopped(sc, k_blowup);
 }
 
 // The buffers a snapshot holds: T, U, V, W, P, dPhat, dP0 and, in the FP32
@@ -1143,6 +1170,7 @@ int tcs_restore(tcs_ctx *c)
     for (int q = 0; q < n; q++)
         CK(cudaMemcpyAsync(dst[q], c->snap[q], bytes, cudaMemcpyDeviceToDevice, c->stream));
     CK(cudaMemcpyAsync(c->cx.g.scal, c->snap_scal, sizeof(c->snap_scal), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemsetAsync(c->cx.g.scal + S_TIMEOUT, 0, sizeof(double), c->stream));
     c->ghost_ok |= (1u << TCS_F_T) | (1u << TCS_F_U) | (1u << TCS_F_V) | (1u << TCS_F_W) | (1u << TCS_F_P) | (1u << TCS_F_DPHAT);
     return TCS_OK;
 }
@@ -1551,16 +1579,17 @@ int tcs_ensemble_step(tcs_ensemble *e, int nsteps, int *nblown)
         }
     }
     CK(cudaStreamSynchronize(e->root));
-    int blown = 0;
+    int blown = 0, failed = TCS_OK;
     for (tcs_ctx *c : e->cases) {
-        double sc[S_NSCAL];
+        double sc[S_NALLOC];
         CK(cudaMemcpy(sc, c->cx.g.scal, sizeof(sc), cudaMemcpyDeviceToHost));
-        if (sc[S_BLOWUP] != 0.0) blown++;
+        if (sc[S_TIMEOUT] != 0.0) failed = stopped(sc, k_blowup);
+        else if (sc[S_BLOWUP] != 0.0) blown++;
         c->ghost_ok |= (1u << TCS_F_T) | (1u << TCS_F_U) | (1u << TCS_F_V) | (1u << TCS_F_W) | (1u << TCS_F_P) |
                        (1u << TCS_F_DPHAT) | (1u << TCS_F_DP);
     }
     if (nblown) *nblown = blown;
-    return TCS_OK;
+    return failed;
 }
 
 int tcs_ensemble_size(const tcs_ensemble *e) { return e ? (int)e->cases.size() : 0; }

@@ -72,8 +72,9 @@ enum : int {
 // -DTCS_BOUNDS_CHECK, the number of out-of-range indices the kernels met
 // (each one recorded here and its access redirected to a valid cell instead of
 // made; the stand-in for a memory checker; 0 in the normal build); S_TIMEOUT,
-// the number of bounded waits on asynchronous copies that ran out (a kernel
-// that records one also sets S_BLOWUP, so the step stops and reports); S_CTR,
+// the number of blocks whose bounded wait on an asynchronous copy ran out (a
+// kernel that records one also sets S_BLOWUP, so that the rest of the step is
+// skipped, and the host reports TCS_ERR_CUDA, not a blow-up); S_CTR,
 // the count of diagnostics blocks done (an unsigned in the double's place).
 enum : int { S_OOB = S_NSCAL, S_TIMEOUT, S_CTR, S_NALLOC };
 

@@ -80,6 +80,7 @@ struct Shapes {
     int long_lines, y_solver;                    // accepted and kept; one solver runs the strided lines
     int mixed_rows;                              // likewise
     int z_staging;                               // likewise
+    int copy_polls;                              // polls of the column form's waits for its copies
     bool spec_live;                              // the spectrum holds a right-hand side that no Poisson solve has taken yet
     FFTPlan fp1, fp3;
     FFTPlan fp1u;                                // N1 with radices up to 8 (the inverse x transform's one-radix form)
@@ -188,7 +189,8 @@ inline bool launch_column(const Shapes &cx, const P &prob, int n, int nlines, in
     static size_t conf[64] = {};
     smem_opt_in((const void *)column_kernel<P>, smem, conf);
     probe_begin(cx, kid, s);
-    column_kernel<P><<<dim3((nlines + w - 1) / w, gy), w << lgNS, smem, s>>>(prob, n, w, lgNS, reinterpret_cast<double *>(prob.f.S), 2 * cx.h1p);
+    column_kernel<P><<<dim3((nlines + w - 1) / w, gy), w << lgNS, smem, s>>>(prob, n, w, lgNS, reinterpret_cast<double *>(prob.f.S), 2 * cx.h1p,
+                                                                              cx.copy_polls);
     probe_end(cx, kid, s);
     record_launch_error(kernel_name(kid));
     return true;

@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(256, 2) xmarch_kernel(const __grid_constant__ 
 // ---------------------------------------------------------------------------
 constexpr int COL_SLOTS = 4;
 constexpr double COL_TINY = 7.8886090522101181e-31;   // 2^-100
-constexpr int COL_WAIT = 1 << 22;                     // polls of a bounded wait
+constexpr int COL_WAIT = 1 << 22;                     // polls of a bounded wait (Shapes::copy_polls)
 
 // FP64 problems that name their stream (Prob::NROW): the cyclic z sweeps.
 template <class P, class = void>
@@ -448,11 +448,11 @@ template <class Prob>
 __host__ __device__ constexpr size_t col_smem(int w, int NS) { return ((size_t)COL_SLOTS * NS * col_slot_words<Prob>(w) + COL_SLOTS) * sizeof(double); }
 
 template <class Prob>
-__global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ Prob prob, int n, int w, int lgNS, double *cscr, int cpitch)
+__global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ Prob prob, int n, int w, int lgNS, double *cscr, int cpitch, int polls)
 {
     using March = typename Prob::March;
     extern __shared__ __align__(16) double csm[];
-    if (prob.skip()) return;
+    if (__syncthreads_or(prob.skip())) return;                       // as one block: another block's failed wait may set the flag now
     const GridT<double> &g = prob.g;
     const int NS = 1 << lgNS, s = threadIdx.x / w, l = threadIdx.x - s * w, by = blockIdx.y, x0 = w * blockIdx.x;
     const int SW = col_slot_words<Prob>(w) * NS;                     // words of a ring slot
@@ -500,9 +500,9 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
         March st(prob, sline, by, r0);
         double a, b, c, d;
         int r = 0;
-        bool ok = true, got = mbar_wait(&bar[0], 0, COL_WAIT);
+        bool ok = true, got = mbar_wait(&bar[0], 0, polls);
         for (; r < mmax; r++) {
-            got = mbar_wait(&bar[(r + 1) % COL_SLOTS], ((r + 1) / COL_SLOTS) & 1, COL_WAIT) && got;
+            got = mbar_wait(&bar[(r + 1) % COL_SLOTS], ((r + 1) / COL_SLOTS) & 1, polls) && got;
             if (got && r < m) {
                 typename March::In in;
                 st.fill(prob, r0 + r, in, mine + ((r + 1) % COL_SLOTS) * SW, mine + (r % COL_SLOTS) * SW, w, sline - x0);
@@ -530,11 +530,12 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
         }
         if (!ok) {
             // a copy did not arrive in time: record it, stop the step, and wait
-            // (bounded) for this block's copies still in flight before leaving
+            // (bounded) for this block's copies still in flight before leaving: the
+            // planes of rows r - 1 (the first row may not have got it) to r + COL_SLOTS - 2
             if (threadIdx.x == 0) {
                 atomicAdd(g.scal + S_TIMEOUT, 1.0);
-                g.scal[S_BLOWUP] = 1.0;
-                for (int q = r + 1; q < r + COL_SLOTS && q <= mmax; q++) mbar_wait(&bar[q % COL_SLOTS], (q / COL_SLOTS) & 1, COL_WAIT);
+                g.scal[S_BLOWUP] = g.scal[S_STEP] + 1.0;
+                for (int q = r; q < r + COL_SLOTS && q <= mmax; q++) mbar_wait(&bar[q % COL_SLOTS], (q / COL_SLOTS) & 1, COL_WAIT);
             }
             __syncthreads();
             return;

@@ -43,7 +43,7 @@ EXPORTS = [
     "tcs_tdma_plan_many_create", "tcs_tdma_plan_many_destroy", "tcs_tdma_many_solve",
     "tcs_tdma_many_solve_cycle", "tcs_tdma_many_solve_noalloc", "tcs_kernel_count", "tcs_launch_count", "tcs_measure_fp64_peak", "tcs_check_reciprocal", "tcs_kernel_name", "tcs_timer_of_kernel", "tcs_timer_name", "tcs_bounds_checked",
     "tcs_bounds_violations", "tcs_probe_enable",
-    "tcs_probe_read", "tcs_probe_reset", "tcs_set_use_graph", "tcs_set_tuning", "tcs_get_tuning",
+    "tcs_probe_read", "tcs_probe_reset", "tcs_set_use_graph", "tcs_set_copy_polls", "tcs_set_tuning", "tcs_get_tuning",
     "tcs_last_error", "tcs_precision", "tcs_ensemble_create", "tcs_ensemble_destroy", "tcs_ensemble_step",
     "tcs_ensemble_size", "tcs_ensemble_set_batched", "tcs_ensemble_form", "tcs_autotune", "tcs_write_continue", "tcs_read_continue", "tcs_extract_plane",
     "tcs_tdma_plan_single_create", "tcs_tdma_plan_single_destroy", "tcs_tdma_single_solve",
@@ -134,6 +134,7 @@ def load() -> ctypes.CDLL:
         "tcs_probe_read": ([vp, ip, dp, ctypes.POINTER(ip)], ip),
         "tcs_probe_reset": ([vp], ip),
         "tcs_set_use_graph": ([vp, ip], ip),
+        "tcs_set_copy_polls": ([vp, ip], ip),
         "tcs_set_tuning": ([vp, ip, ip], ip),
         "tcs_get_tuning": ([vp, ip, ctypes.POINTER(ip)], ip),
         "tcs_last_error": ([], ctypes.c_char_p),
@@ -422,6 +423,10 @@ class Solver:
 
     def use_graph(self, on: bool) -> None:
         _check(load().tcs_set_use_graph(self._h, int(bool(on))), "use_graph")
+
+    def set_copy_polls(self, polls: int) -> None:
+        """Bound of the waits for asynchronous copies (tcs_set_copy_polls); 0 makes each run out at once."""
+        _check(load().tcs_set_copy_polls(self._h, int(polls)), "set_copy_polls")
 
     # -- measurement ----------------------------------------------------------
     def probe(self, kernels) -> None:
