@@ -1080,12 +1080,12 @@ int tcs_step(tcs_ctx *c, int nsteps, int *done)
     if (nsteps < 0) return set_err(TCS_ERR_ARG, "nsteps < 0");
     int r = flush_pending(c);
     if (r) return r;
-    c->cx.spec_live = false;   // the step writes the spectrum anew
     const int fl[] = {TCS_F_T, TCS_F_U, TCS_F_V, TCS_F_W, TCS_F_P, TCS_F_DPHAT};
     for (int f : fl) ensure_ghosts(c, f);
     if ((r = take_launch_error())) return r;
     double sc0[S_NALLOC];
     if ((r = read_scalars(c, sc0)) || (r = stopped(sc0, "the case has already blown up"))) return r;
+    if (nsteps > 0) c->cx.spec_live = false;   // the step writes the spectrum anew
     const bool graph = c->use_graph && c->probe.mask == 0;
     for (int n = 0; n < nsteps; n++) {
         if (!graph) {
@@ -1536,7 +1536,7 @@ int tcs_ensemble_step(tcs_ensemble *e, int nsteps, int *nblown)
     int r;
     const int fl[] = {TCS_F_T, TCS_F_U, TCS_F_V, TCS_F_W, TCS_F_P, TCS_F_DPHAT};
     for (tcs_ctx *c : e->cases) {
-        c->cx.spec_live = false;
+        if (nsteps > 0) c->cx.spec_live = false;
         if ((r = flush_pending(c))) return r;
         for (int f : fl) ensure_ghosts(c, f);
         if ((r = take_launch_error())) return r;

@@ -49,3 +49,29 @@ def test_a_copy_that_does_not_arrive_in_time_is_not_a_blow_up(tcs):
     assert g.step(2) == 2
     for n in FIELDS:
         np.testing.assert_array_equal(g.get(n), ref.get(n), err_msg=n)
+
+
+def test_no_steps_leave_a_pending_right_hand_side_alone(tcs):
+    # the column form keeps its coefficients in the spectrum: after tcs_pressure_RHS it
+    # must not run before the Poisson solve has taken the right-hand side, and a call for
+    # no steps changes nothing about that
+    a, b = tcs.Solver(**CFG), tcs.Solver(**CFG)
+    ens = tcs.Ensemble([b])
+    for s in (a, b):
+        s.step(1)
+        s.thermal_solver()
+        s.momentum_coeffi()
+        s.momentum_solvedU()
+        s.momentum_solvedV()
+        s.momentum_solvedW()
+        s.momentum_blockLdV()
+        s.momentum_blockLdU()
+        s.momentum_pseudoupdateUVW()
+        s.pressure_RHS()
+        if s is b:
+            s.step(0)
+            ens.step(0)
+            s.momentum_solvedU()
+        s.pressure_Poisson_FFT2()
+    np.testing.assert_array_equal(b.get("dP"), a.get("dP"))
+    ens.close()
