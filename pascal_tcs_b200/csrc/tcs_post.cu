@@ -1,10 +1,11 @@
 // tcs_post.cu -- per-step diagnostics: mpi_Post_Div and mpi_Post_CFL
 // (module_post.f90:100-158, 168-230) with the adaptive time step, the
 // blow-up test of main.f90:208-212, and the Nusselt / kinetic-energy series.
-// One kernel: block partials in a fixed order; the last block to finish combines
-// them and updates dt, time and CFL on the device (deterministic).  Inside a step
-// it also writes the wall rows of dP and P, which nothing reads before (three
-// launches fewer per step).  Both forms reduce in FP64 from their fields, and the per-thread sums are compensated
+// Block partials in a fixed order; the last block to finish combines them and
+// updates dt, time and CFL on the device (deterministic).  Inside a step the wall
+// rows of dP and P, which nothing reads before, are written on the way.  One kernel
+// does all three; for the FP32 form on large grids the last two have a launch of
+// their own (launch_post).  Both forms reduce in FP64 from their fields, and the per-thread sums are compensated
 // (Neumaier), so the diagnostics keep FP64 accuracy over 512^3 cells.
 #include "tcs_kernels.h"
 
@@ -13,7 +14,7 @@
 namespace tcs {
 
 enum { PT_DIV = 0, PT_CFL, PT_KE, PT_NUB, PT_NUT, PT_N };
-static const int POST_BLOCKS = 592;   // 4 x 148 SMs: all resident in FP64 (64 registers; the FP32 form, with twice the loads, runs faster uncapped)
+static const int POST_BLOCKS = 592;   // 4 x 148 SMs: all resident at 64 registers
 
 // s + e carries a sum and its running rounding error (Neumaier's variant of
 // Kahan summation).
@@ -79,15 +80,41 @@ __device__ __forceinline__ void finalize(const GridT<R> &g, const FieldsT<R> &f,
     sc[S_STEP] = step + 1;
 }
 
-// Bound by the latency of its loads, so by the blocks per SM: four of 256 threads at
-// 64 registers.  Without the bound the FP32 form, which reads two words per velocity,
-// takes 88 registers and two blocks: 0.220 against 0.170 ms at 256^3, 0.374 against
-// 0.294 ms at 400 x 200 x 384.  Neither form spills.
+// The wall rows (walls), then, in the last block to come here, the end of the step's
+// diagnostics from the nparts blocks' partials.  The blow-up flag is set when every
+// block is past its test of it.
 template <class R>
-__global__ void __launch_bounds__(256, 4) post_kernel(GridT<R> g, FieldsT<R> f, FastDiv dn1, FastDiv dn2, int record_hist, int walls, WallRows wr)
+__device__ __forceinline__ void walls_and_finalize(const GridT<R> &g, const FieldsT<R> &f, double (*red)[256], int nparts, int record_hist, int walls,
+                                                   const WallRows &wr)
+{
+    __shared__ int s_last;
+    if (walls) {
+        const int nx = g.N1 + 2, nw = nx * (g.N3 + 2);
+        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nw; t += gridDim.x * blockDim.x) {
+            const int k = t / nx, i = t - k * nx;
+            dp_wall_cell(g, f.dP, i, k, wr);
+            if (i >= 1 && i <= g.N1 && k >= 1 && k <= g.N3) p_wall_cell(g, f.P, i, k, wr);
+        }
+    }
+    __threadfence();                                   // the partials before the count
+    __syncthreads();
+    unsigned *const ctr = reinterpret_cast<unsigned *>(g.scal + S_CTR);
+    if (threadIdx.x == 0) s_last = atomicAdd(ctr, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x == 0) *ctr = 0;                    // the next launch counts from 0
+    finalize(g, f, red, nparts, record_hist);
+}
+
+// Bound by the latency of its loads, so by the blocks per SM: four of 256 threads at
+// 64 registers.  Without the bound the fused FP32 form takes 88 registers and two
+// blocks (256^3: 0.220 against 0.170 ms); the partials alone take 64 without one (0: the
+// compiler's choice).  Neither form spills.
+template <class R, bool FUSED>
+__global__ void __launch_bounds__(256, FUSED ? 4 : 0) post_kernel(GridT<R> g, FieldsT<R> f, FastDiv dn1, FastDiv dn2, int record_hist, int walls, WallRows wr)
 {
     __shared__ double red[PT_N][256];
-    __shared__ int s_last;
     if (blown(g)) return;
     const long long n = (long long)g.N1 * g.N2 * g.N3;
     double mdiv = -INFINITY, mcfl = -INFINITY, ke = 0.0, nub = 0.0, nut = 0.0, eke = 0.0, enb = 0.0, ent = 0.0;
@@ -133,32 +160,44 @@ __global__ void __launch_bounds__(256, 4) post_kernel(GridT<R> g, FieldsT<R> f, 
         __syncthreads();
     }
     if (threadIdx.x < PT_N) f.part[blockIdx.x * PT_N + threadIdx.x] = red[threadIdx.x][0];
-    if (walls) {
-        const int nx = g.N1 + 2, nw = nx * (g.N3 + 2);
-        for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nw; t += gridDim.x * blockDim.x) {
-            const int k = t / nx, i = t - k * nx;
-            dp_wall_cell(g, f.dP, i, k, wr);
-            if (i >= 1 && i <= g.N1 && k >= 1 && k <= g.N3) p_wall_cell(g, f.P, i, k, wr);
-        }
-    }
-    __threadfence();                                   // the partials before the count
-    __syncthreads();
-    unsigned *const ctr = reinterpret_cast<unsigned *>(g.scal + S_CTR);
-    if (threadIdx.x == 0) s_last = atomicAdd(ctr, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    if (threadIdx.x == 0) *ctr = 0;                    // the next launch counts from 0
-    finalize(g, f, red, gridDim.x, record_hist);
+    if constexpr (FUSED) walls_and_finalize(g, f, red, gridDim.x, record_hist, walls, wr);
 }
 
 template <class R>
+__global__ void __launch_bounds__(256) post_finish_kernel(GridT<R> g, FieldsT<R> f, int nparts, int record_hist, int walls, WallRows wr)
+{
+    __shared__ double red[PT_N][256];
+    if (blown(g)) return;
+    walls_and_finalize(g, f, red, nparts, record_hist, walls, wr);
+}
+
+// The code after the FP32 form's main loop, which reads two words per velocity, costs
+// the loop more than a second launch above about 2^22 cells (tcs_post_div, us, one
+// kernel and two: 64^3 42.1 and 45.4; 64 x 64 x 1024 95 and 96; 180 x 151 x 250 103 and
+// 100; 256^3 193 and 180; 400 x 200 x 384 313 and 284; 512^3 1250 and 1114).  In FP64 one
+// kernel leads at every size (256^3 145 and 165, 512^3 842 and 1088).
+template <class R>
 void launch_post(const Ctx<R> &cx, cudaStream_t s, int record_hist, bool walls)
 {
+    const GridT<R> &g = cx.g;
     const WallRows wr{cx.wall_ab, cx.wall_bb, cx.wall_at, cx.wall_bt};
+    const FastDiv d1 = make_fastdiv((unsigned)g.N1), d2 = make_fastdiv((unsigned)g.N2);
+    if constexpr (HasLo<R>::on) {
+        if ((long long)g.N1 * g.N2 * g.N3 >= (1 << 22)) {
+            const int blocks = walls ? std::min(POST_BLOCKS, ((g.N1 + 2) * (g.N3 + 2) + 255) / 256) : 1;
+            probe_begin(cx, K_POST, s);
+            post_kernel<R, false><<<POST_BLOCKS, 256, 0, s>>>(g, cx.f, d1, d2, record_hist, 0, wr);
+            probe_end(cx, K_POST, s);
+            record_launch_error("post");
+            probe_begin(cx, K_FINAL, s);
+            post_finish_kernel<<<blocks, 256, 0, s>>>(g, cx.f, POST_BLOCKS, record_hist, walls ? 1 : 0, wr);
+            probe_end(cx, K_FINAL, s);
+            record_launch_error("finalize");
+            return;
+        }
+    }
     probe_begin(cx, K_POST, s);
-    post_kernel<<<POST_BLOCKS, 256, 0, s>>>(cx.g, cx.f, make_fastdiv((unsigned)cx.g.N1), make_fastdiv((unsigned)cx.g.N2), record_hist,
-                                            walls ? 1 : 0, wr);
+    post_kernel<R, true><<<POST_BLOCKS, 256, 0, s>>>(g, cx.f, d1, d2, record_hist, walls ? 1 : 0, wr);
     probe_end(cx, K_POST, s);
     record_launch_error("post");
 }
