@@ -984,9 +984,14 @@ __device__ __forceinline__ R blockld_u_value(const GridT<R> &g, const FieldsT<R>
         - dt * (R(0.25) * (dwm6 * dudz6 + dwm5 * dudz5) - R(0.5) * Cmu * invRhoc * rdx3[k] * (mu6 * dwmdx6 - mu5 * dwmdx5));
 }
 
-// KZ planes per thread: every input of the KZ cells is loaded before the first store
+// KZ planes per thread: every input of the KZ cells is loaded before the first store.
+// Bound by its load latency, so by the warps per SM: with the face tables and no bound
+// the FP32 form took 40 registers (12 blocks) and ran slower than the kernel before the
+// tables, which formed the faces (us, before, unbounded, 16 blocks per SM: 256^3 160, 162,
+// 117; 400 x 200 x 384 306, 318, 220); in FP64 the compiler's own 48 registers left
+// loads waiting (256^3 216, 222 and, at up to 64, 195; 180 x 151 x 250 107, 111, 99).
 template <class R, int KZ>
-__global__ void blockld_u_kernel(GridT<R> g, FieldsT<R> f)
+__global__ void __launch_bounds__(128, HasLo<R>::on ? 16 : 8) blockld_u_kernel(GridT<R> g, FieldsT<R> f)
 {
     const int i = 1 + blockIdx.x * blockDim.x + threadIdx.x, j = 1 + blockIdx.y, k0 = 1 + KZ * blockIdx.z;
     if (i > g.N1 || blown(g)) return;
