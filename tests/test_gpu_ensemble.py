@@ -3,6 +3,8 @@ and precisions advanced together by one CUDA graph per step must give, case
 by case, exactly what each case gives when stepped alone, in both forms (the
 batched one: one multi-case launch per line sweep; one branch per case) and
 in the auto mode that measures both (needs a B200)."""
+import time
+
 import numpy as np
 import pytest
 
@@ -110,3 +112,32 @@ def test_ensemble_auto_picks_a_form(tcs):
     for a, b in zip(alone, grouped):
         for n in ("T", "U", "V", "W", "P"):
             np.testing.assert_array_equal(a.get(n), b.get(n), err_msg=n)
+
+
+def test_many_tiny_cases_share_streams_and_stay_exact(tcs):
+    # more cases than the graph has branches for: cases on one stream follow each other,
+    # uneven sizes and both precisions, every case exactly as alone; and the batched form's
+    # joins do not grow with the square of the cases (with an edge between every two cases
+    # at every stage it took 1.6 times the branch form's time)
+    cfgs = [dict(n1m=(16, 20, 32)[i % 3], n2m=12 + i % 5, n3m=(10, 12, 16, 18)[i % 4], property_set=i % 3, Pr=7.0, Ra=1e5,
+                 dtStart=2e-4, fixed_dt=1, seed=i, precision=i % 2) for i in range(160)]
+    alone = [tcs.Solver(**c) for c in cfgs]
+    grouped = [tcs.Solver(**c) for c in cfgs]
+    ens = tcs.Ensemble(grouped)
+    assert ens.step(9) == 0                      # four steps in each form, then the one kept
+    for s in alone:
+        s.step(9)
+    for a, b in zip(alone, grouped):
+        for n in ("T", "U", "V", "W", "P", "dPhat"):
+            np.testing.assert_array_equal(a.get(n), b.get(n), err_msg=n)
+    best = {}
+    for form in (False, True):
+        ens.set_batched(form)
+        ens.step(2)                              # captures the form's graphs
+        for _ in range(6):
+            t = time.perf_counter()
+            ens.step(2)
+            best[form] = min(best.get(form, 1.0), time.perf_counter() - t)
+    print({k: f"{v * 500:.3f} ms" for k, v in best.items()})
+    assert best[True] < 1.35 * best[False]
+    ens.close()
