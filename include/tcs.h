@@ -229,6 +229,9 @@ const char *tcs_timer_name(int timer);
  * returns the case's count so far (always 0 in the normal build). */
 int tcs_bounds_checked(void);
 int tcs_bounds_violations(tcs_ctx *ctx, double *count);
+/* The line sweeps step offsets and pointers from row to row; in that build each row
+ * is checked as it is read and as it is written.  The count of those checks so far. */
+int tcs_bounds_rows(tcs_ctx *ctx, double *count);
 int tcs_set_use_graph(tcs_ctx *ctx, int on);
 /* The z sweeps of long FP64 lines wait for asynchronous copies, each wait bounded
  * to `polls` polls (default 2^22).  If one runs out, the rest of the step is skipped

@@ -420,6 +420,15 @@ int tcs_bounds_violations(tcs_ctx *c, double *count)
     return TCS_OK;
 }
 
+int tcs_bounds_rows(tcs_ctx *c, double *count)
+{
+    if (!c || !count) return set_err(TCS_ERR_ARG, "null argument");
+    cudaSetDevice(c->cfg.device);
+    CK(cudaMemcpyAsync(count, c->cx.g.scal + S_ROWS, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return TCS_OK;
+}
+
 int tcs_timer_of_kernel(int kid) { return (kid >= 0 && kid < K_COUNT) ? k_timer_of[kid] : -1; }
 const char *tcs_timer_name(int timer) { return (timer >= 1 && timer <= 18) ? k_timer_names[timer] : nullptr; }
 

@@ -75,16 +75,24 @@ enum : int {
 // the number of blocks whose bounded wait on an asynchronous copy ran out (a
 // kernel that records one also sets S_BLOWUP, so that the rest of the step is
 // skipped, and the host reports TCS_ERR_CUDA, not a blow-up); S_CTR,
-// the count of diagnostics blocks done (an unsigned in the double's place).
-enum : int { S_OOB = S_NSCAL, S_TIMEOUT, S_CTR, S_NALLOC };
+// the count of diagnostics blocks done (an unsigned in the double's place); S_ROWS,
+// in the bounds-check build, the number of rows the line sweeps have checked.
+enum : int { S_OOB = S_NSCAL, S_TIMEOUT, S_CTR, S_ROWS, S_NALLOC };
 
 #if defined(TCS_BOUNDS_CHECK) && defined(__CUDA_ARCH__)
 #define TCS_OOB(scal, bad, fix)                          \
     do {                                                 \
         if (bad) { atomicAdd((scal) + S_OOB, 1.0); fix; } \
     } while (0)
+// one row of a line sweep, reached by stepping an offset or a pointer
+#define TCS_ROW(scal, bad, fix)                          \
+    do {                                                 \
+        atomicAdd((scal) + S_ROWS, 1.0);                 \
+        TCS_OOB(scal, bad, fix);                         \
+    } while (0)
 #else
 #define TCS_OOB(scal, bad, fix) do { } while (0)
+#define TCS_ROW(scal, bad, fix) do { } while (0)
 #endif
 
 template <class R>

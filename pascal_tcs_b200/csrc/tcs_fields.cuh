@@ -64,6 +64,34 @@ template <class R> struct HasLo { static constexpr bool on = std::is_same<R, flo
 __device__ __forceinline__ double2 ld2(const double *p) { return __ldg(reinterpret_cast<const double2 *>(p)); }
 __device__ __forceinline__ float2 ld2(const float *p) { return __ldg(reinterpret_cast<const float2 *>(p)); }
 
+// The line sweeps step offsets and pointers from row to row.  In the bounds-check
+// build every row is looked at as it is reached (elsewhere nothing happens).
+// The cell at offset c of a padded field is interior: its stencil stays inside the
+// padding.
+template <class R>
+__device__ __forceinline__ void row_cell(const GridT<R> &g, long long &c)
+{
+    TCS_ROW(g.scal, c < 0 || c >= g.NP || (unsigned)(c % g.P1 - 1) >= (unsigned)g.N1 || (unsigned)(c / g.P1 % g.P2 - 1) >= (unsigned)g.N2 ||
+            (unsigned)(c / g.P1 / g.P2 - 1) >= (unsigned)g.N3, c = ix(g, 1, 1, 1));
+}
+// ... and word t4 of the face tables starts the entry of that cell's (j, k).
+template <class R>
+__device__ __forceinline__ void row_cell(const GridT<R> &g, long long &c, int &t4)
+{
+    row_cell(g, c);
+    TCS_OOB(g.scal, t4 != 4 * (int)(c / g.P1), t4 = 4 * (int)(c / g.P1));
+}
+// p points at an interior cell of the padded field a.
+template <class R, class V>
+__device__ __forceinline__ void row_ptr(const GridT<R> &g, V *a, V *&p)
+{
+#if defined(TCS_BOUNDS_CHECK) && defined(__CUDA_ARCH__)
+    long long c = p - a;
+    row_cell(g, c);
+    p = a + c;
+#endif
+}
+
 // Weights of the wall extrapolations (Pbc_a and Pbc_b of the lower and upper wall).
 struct WallRows { double ab, bb, at, bt; };
 

@@ -157,7 +157,12 @@ struct ScratchOut {
     R *p;
     long long step;
     __device__ __forceinline__ ScratchOut(const GridT<R> &g, R *a, int i, int j, int k, long long st) : p(a + ix(g, i, j, k)), step(st) {}
-    __device__ __forceinline__ void put(R v) { *p = v; p -= step; }
+    __device__ __forceinline__ void put(const GridT<R> &g, R *a, R v)
+    {
+        row_ptr(g, a, p);
+        *p = v;
+        p -= step;
+    }
 };
 // ... or into a field with its periodic images, along y (see store_periodic).
 template <class R>
@@ -167,8 +172,9 @@ struct PeriodicOut {
     __device__ __forceinline__ PeriodicOut(const GridT<R> &g, R *a, int i, int j, int k)
         : p(a + ix(g, i, j, k)), gi(i == 1 ? g.N1 : (i == g.N1 ? -g.N1 : 0)),
           gk((long long)g.P1 * g.P2 * (k == 1 ? g.N3 : (k == g.N3 ? -g.N3 : 0))), step(g.P1) {}
-    __device__ __forceinline__ void put(R v)
+    __device__ __forceinline__ void put(const GridT<R> &g, R *a, R v)
     {
+        row_ptr(g, a, p);
         *p = v;
         if (gi) p[gi] = v;
         if (gk) {
@@ -199,6 +205,7 @@ __device__ __forceinline__ void march_block(const Prob &prob, const MarchPlan &m
     double *const row0 = msm + (size_t)r0 * W * TI + l;
     double *const red = msm + (size_t)mp.n * W * TI;   // e, c, d[NR], se, p, sd[NR] of the last rows: word q of (s, l) at q NS TP + s TP + l
     const int RS = NS * TP;
+    TCS_OOB(prob.g.scal, blockDim.x != NS * TI || mp.m0 < 1 || NS * mp.m0 + mp.rem != mp.n, return);   // the same for the whole block
     {
         typename Prob::March st(prob, min(line, nl - 1), by, r0);
         double cp = 0.0, e = -1.0, p = 1.0, se = 0.0, dp[NR], sd[NR];
@@ -219,6 +226,7 @@ __device__ __forceinline__ void march_block(const Prob &prob, const MarchPlan &m
             }
         };
         auto park = [&]() {
+            TCS_OOB(prob.g.scal, w < msm || w + (W - 1) * TI >= msm + (size_t)mp.n * W * TI, w = row0);
             w[0] = cp; w[TI] = e;
 #pragma unroll
             for (int q = 0; q < NR; q++) { w[(2 + q) * TI] = dp[q]; sd[q] = fma(p, dp[q], sd[q]); }
@@ -270,6 +278,7 @@ __device__ __forceinline__ void march_block(const Prob &prob, const MarchPlan &m
         int left = m - 1;
         constexpr int B = 4;                           // parked rows read ahead of the substitution
         for (; left >= B; left -= B, w -= B * W * TI) {
+            TCS_OOB(prob.g.scal, w - (B - 1) * W * TI < msm || w + (W - 1) * TI >= msm + (size_t)mp.n * W * TI, break);
             double c[B], y[B][NR];
 #pragma unroll
             for (int t = 0; t < B; t++) {
@@ -286,6 +295,7 @@ __device__ __forceinline__ void march_block(const Prob &prob, const MarchPlan &m
             }
         }
         for (; left > 0; left--, w -= W * TI) {
+            TCS_OOB(prob.g.scal, w < msm || w + (W - 1) * TI >= msm + (size_t)mp.n * W * TI, break);
             const double c = w[0], e = w[TI];
 #pragma unroll
             for (int q = 0; q < NR; q++) x[q] = fma(-c, x[q], fma(-e, xp[q], w[(2 + q) * TI]));
@@ -357,7 +367,10 @@ __global__ void __launch_bounds__(256, 2) xmarch_kernel(const __grid_constant__ 
         const typename Prob::Stage st(prob, min(line0 + l, nl - 1), by);
         double *const w = xsm + l * LS;
 #pragma unroll Prob::UNROLL
-        for (int r = first; r < n; r += step) st.put(prob, r, w + r, PL);
+        for (int r = first; r < n; r += step) {
+            TCS_ROW(prob.g.scal, r < 0 || l < 0 || l >= TI, break);
+            st.put(prob, r, w + r, PL);
+        }
     };
     if (share == 1)
         for (int l = warp; l < TI; l += nw) stage(l, lane, 32);
@@ -367,6 +380,7 @@ __global__ void __launch_bounds__(256, 2) xmarch_kernel(const __grid_constant__ 
     const int l = threadIdx.x & (TI - 1), s = threadIdx.x >> mp.lgTI;
     const int m = mp.m0 + (s < mp.rem ? 1 : 0), r0 = s * mp.m0 + min(s, mp.rem);
     double *const w = xsm + l * LS;
+    TCS_OOB(prob.g.scal, blockDim.x != NS * TI || mp.m0 < 1 || NS * mp.m0 + mp.rem != n, return);   // the same for the whole block
     {
         typename Prob::March st(prob, min(line0 + l, nl - 1), by, r0, m, n, w, PL);
         __syncthreads();                               // the words across segment edges have been read
@@ -379,6 +393,7 @@ __global__ void __launch_bounds__(256, 2) xmarch_kernel(const __grid_constant__ 
             e = -(a * rr) * e;
             dp = fma(-a, dp, d) * rr;
             cp = c * rr;
+            TCS_OOB(prob.g.scal, r < 0 || r >= n, break);
             if (r < last) {
                 w[r] = dp; w[PL + r] = cp; w[2 * PL + r] = e;
                 sd = fma(p, dp, sd);
@@ -397,6 +412,7 @@ __global__ void __launch_bounds__(256, 2) xmarch_kernel(const __grid_constant__ 
         int r = r0 + m - 1;
         w[r] = x;
         for (r--; r - 3 >= r0; r -= 4) {
+            TCS_OOB(prob.g.scal, r >= n || r - 3 < 0, break);
             double c[4], y[4];
 #pragma unroll
             for (int t = 0; t < 4; t++) { c[t] = w[PL + r - t]; y[t] = fma(-w[2 * PL + r - t], xp, w[r - t]); }
@@ -413,7 +429,10 @@ __global__ void __launch_bounds__(256, 2) xmarch_kernel(const __grid_constant__ 
     for (int q = warp / share; q < TI && line0 + q < nl; q += nw / share) {
         R *const o = prob.out(line0 + q, by);
         const double *const v = xsm + q * LS;
-        for (int r = lane + 32 * (warp % share); r < n; r += 32 * share) o[r] = R(v[r]);
+        for (int r = lane + 32 * (warp % share); r < n; r += 32 * share) {
+            TCS_ROW(prob.g.scal, r < 0 || r >= prob.g.N1, break);
+            o[r] = R(v[r]);
+        }
     }
 }
 
@@ -463,6 +482,7 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
     const int m0 = n >> lgNS, rem = n & (NS - 1), m = m0 + (s < rem), r0 = s * m0 + min(s, rem), mmax = m0 + (rem > 0);
     const long long sk = (long long)g.P1 * g.P2;
     const uint32_t rowb = (uint32_t)min(w + 2, g.P1 - x0) * 8u;
+    TCS_OOB(g.scal, blockDim.x != NS * w || m0 < 1 || n != g.N3 || cpitch < g.N1 || cpitch > 2 * (g.N1 / 2 + 1), return);   // the same for the whole block
     if (threadIdx.x == 0) {
         for (int q = 0; q < COL_SLOTS; q++) mbar_init(&bar[q], NS);
         mbar_init_fence();
@@ -480,13 +500,17 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
         mbar_arrive_expect_tx(&bar[sl], Prob::NROW * rowb + (Prob::TABLES ? 128u : 0u));
 #pragma unroll
         for (int q = 0; q < Prob::NROW; q++) {
-            const int jq = j + Prob::row_dj(q), kq = k + Prob::row_dk(q);
+            int jq = j + Prob::row_dj(q), kq = k + Prob::row_dk(q);
+            TCS_OOB(g.scal, (unsigned)jq > (unsigned)g.N2 + 1u || (unsigned)kq > (unsigned)g.N3 + 1u || (x0 & 1) || x0 < 0 || x0 + (int)(rowb / 8) > g.P1 ||
+                    (int)(rowb / 8) > w + 2, jq = kq = 1);
             bulk_load(dst + q * (w + 2), prob.row_src(q) + (x0 + (long long)g.P1 * (jq + (long long)g.P2 * kq)), rowb, &bar[sl]);
         }
         if (Prob::TABLES) {
             double *const t = dst + Prob::NROW * (w + 2);
-            bulk_load(t, prob.f.MuT + 4 * (j - 1 + g.P2 * (k + 1)), 96, &bar[sl]);
-            bulk_load(t + 12, prob.f.iRT + 4 * (j + g.P2 * (k + 1)), 32, &bar[sl]);
+            int jt = j, kt = k + 1;
+            TCS_OOB(g.scal, jt < 1 || jt > g.N2 || kt < 0 || kt > g.N3 + 1, jt = kt = 1);
+            bulk_load(t, prob.f.MuT + 4 * (jt - 1 + g.P2 * kt), 96, &bar[sl]);
+            bulk_load(t + 12, prob.f.iRT + 4 * (jt + g.P2 * kt), 32, &bar[sl]);
         }
     };
     if (l == 0)
@@ -512,7 +536,9 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
                 dp = fma(-a, dp, d) * rr;
                 cp = c * rr;
                 if (r < m - 1) {
-                    if (line < nl) {
+                    bool in = line < nl;
+                    TCS_ROW(g.scal, r0 + r >= n || i > g.N1 || j > g.N2, in = false);
+                    if (in) {
                         sc[r * ck] = cp;
                         sd_[r * sk] = dp;
                     }
@@ -565,11 +591,13 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
             const double rr = qrcp(fma(-a, c2, b));
             e2 = -(a * rr) * e2;
             c2 = c * rr;
+            TCS_OOB(g.scal, r >= m - 1, break);
             if (line < nl) sd_[r * sk] = fma(-e2, Xp, sd_[r * sk]);
         }
     }
     if (line >= nl) return;
     double x = X;
+    TCS_ROW(g.scal, r0 + m > n || i > g.N1 || j > g.N2, return);
     sd_[(m - 1) * sk] = x;
     int r = m - 2;
     for (; r >= 7; r -= 8) {

@@ -137,6 +137,7 @@ struct DUZ {
         struct In { R Uxm, Uxp, Uym, Uyp, Uzp, Vc, Vxm, Vyp, Vxmyp, Wzp, Wxmzp, Pc, Pxm, T0, Txm, muy4, muz6, iR, rdx3, rdmx3; cplx_t<R> mt; };
         __device__ __forceinline__ void load(const DUZ &q, int r, In &n)
         {
+            row_cell(q.g, c, t4);
             const GridT<R> &g = q.g;
             const FieldsT<R> &f = q.f;
             const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
@@ -203,7 +204,7 @@ struct DUZ {
     };
     struct Out : ScratchOut<R> {
         __device__ __forceinline__ Out(const DUZ &q, int line, int by, int r) : ScratchOut<R>(q.g, q.f.scr, 1 + line, 1 + by, r + 1, (long long)q.g.P1 * q.g.P2) {}
-        __device__ __forceinline__ void put(const DUZ &, const double *x) { ScratchOut<R>::put(R(x[0])); }
+        __device__ __forceinline__ void put(const DUZ &q, const double *x) { ScratchOut<R>::put(q.g, q.f.scr, R(x[0])); }
     };
 };
 
@@ -220,6 +221,7 @@ struct DUX {
         __device__ __forceinline__ Stage(const DUX &q, int line, int by) : c(ix(q.g, 1, 1 + line, 1 + by)) {}
         __device__ __forceinline__ void put(const DUX &q, int r, double *w, int PL) const
         {
+            TCS_OOB(q.g.scal, r < 0 || r >= q.g.N1, return);
             w[0] = (double)q.f.scr[c + r];
             w[PL] = (double)ld(q.f.U + c + r);
         }
@@ -310,6 +312,7 @@ struct DUY {
         struct In { R V, Vxm, mu, iR, rdx2, rdmx2, d; };
         __device__ __forceinline__ void load(const DUY &q, int r, In &n)
         {
+            row_cell(q.g, c, t4);
             const long long sj = q.g.P1;
             n.V = ld(q.f.V + c + sj); n.Vxm = ld(q.f.V + c + sj - 1);
             n.mu = ld(q.f.MuT + t4 + 5); n.iR = ld(q.f.iRT + t4);
@@ -329,7 +332,7 @@ struct DUY {
     };
     struct Out : PeriodicOut<R> {
         __device__ __forceinline__ Out(const DUY &q, int line, int by, int r) : PeriodicOut<R>(q.g, q.f.dU, 1 + line, r + 1, 1 + by) {}
-        __device__ __forceinline__ void put(const DUY &, const double *x) { PeriodicOut<R>::put(R(x[0])); }
+        __device__ __forceinline__ void put(const DUY &q, const double *x) { PeriodicOut<R>::put(q.g, q.f.dU, R(x[0])); }
     };
 };
 
@@ -402,6 +405,7 @@ struct DVZ {
         struct In { R Vxm, Vxp, Vym, Vyp, Vzp, U0, Uym, Uxp, Uxpym, D0, Dym, Dxp, Dxpym, Wzp, Wzpym, Pc, Pym, Mm, muz6, iR, rdx3, rdmx3; cplx_t<R> mt; };
         __device__ __forceinline__ void load(const DVZ &q, int r, In &n)
         {
+            row_cell(q.g, c, t4);
             const GridT<R> &g = q.g;
             const FieldsT<R> &f = q.f;
             const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
@@ -469,7 +473,7 @@ struct DVZ {
     };
     struct Out : ScratchOut<R> {
         __device__ __forceinline__ Out(const DVZ &q, int line, int by, int r) : ScratchOut<R>(q.g, q.f.scr, 1 + line, 2 + by, r + 1, (long long)q.g.P1 * q.g.P2) {}
-        __device__ __forceinline__ void put(const DVZ &, const double *x) { ScratchOut<R>::put(R(x[0])); }
+        __device__ __forceinline__ void put(const DVZ &q, const double *x) { ScratchOut<R>::put(q.g, q.f.scr, R(x[0])); }
     };
 };
 
@@ -499,6 +503,7 @@ struct DVX {
             : c(ix(q.g, 1, 2 + line, 1 + by)), cy(R(0.5) * ld(q.g.m2.dx + 1 + line) * ld(q.g.m2.rdmx + 2 + line)) {}
         __device__ __forceinline__ void put(const DVX &q, int r, double *w, int PL) const
         {
+            TCS_OOB(q.g.scal, r < 0 || r >= q.g.N1, return);
             w[0] = (double)q.f.scr[c + r];
             const R U0 = ld(q.f.U + c + r), Um = ld(q.f.U + c + r - q.g.P1);
             w[PL] = (double)(Um + cy * (U0 - Um));
@@ -548,6 +553,7 @@ struct DVY {
         struct In { R V, mu, iR, rdx2, rdmx2, d; };
         __device__ __forceinline__ void load(const DVY &q, int r, In &n)
         {
+            row_cell(q.g, c, t4);
             const long long sj = q.g.P1;
             n.V = ld(q.f.V + c + sj);
             n.mu = ld(q.f.MuT + t4); n.iR = ld(q.f.iRT + t4 + 1);
@@ -570,7 +576,7 @@ struct DVY {
     };
     struct Out : PeriodicOut<R> {
         __device__ __forceinline__ Out(const DVY &q, int line, int by, int r) : PeriodicOut<R>(q.g, q.f.dV, 1 + line, r + 2, 1 + by) {}
-        __device__ __forceinline__ void put(const DVY &, const double *x) { PeriodicOut<R>::put(R(x[0])); }
+        __device__ __forceinline__ void put(const DVY &q, const double *x) { PeriodicOut<R>::put(q.g, q.f.dV, R(x[0])); }
     };
 };
 
@@ -647,6 +653,7 @@ struct DWZ {
         struct In { R Wxm, Wxp, Wym, Wyp, Wzp, U, Ux, D, Dx, V, Vy, E, Ey, P, Mc, muyz4, iR, dx3, rdx3, rdmx3; cplx_t<R> mt; };
         __device__ __forceinline__ void load(const DWZ &q, int r, In &n)
         {
+            row_cell(q.g, c, t4);
             const GridT<R> &g = q.g;
             const FieldsT<R> &f = q.f;
             const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
@@ -719,7 +726,7 @@ struct DWZ {
     };
     struct Out : ScratchOut<R> {
         __device__ __forceinline__ Out(const DWZ &q, int line, int by, int r) : ScratchOut<R>(q.g, q.f.scr, 1 + line, 1 + by, r + 1, (long long)q.g.P1 * q.g.P2) {}
-        __device__ __forceinline__ void put(const DWZ &, const double *x) { ScratchOut<R>::put(R(x[0])); }
+        __device__ __forceinline__ void put(const DWZ &q, const double *x) { ScratchOut<R>::put(q.g, q.f.scr, R(x[0])); }
     };
 };
 
@@ -754,6 +761,7 @@ struct DWX {
             : c(ix(q.g, 1, 1 + line, 1 + by)), sk((long long)q.g.P1 * q.g.P2), cz(R(0.5) * ld(q.g.m3.dx + by) * ld(q.g.m3.rdmx + 1 + by)) {}
         __device__ __forceinline__ void put(const DWX &q, int r, double *w, int PL) const
         {
+            TCS_OOB(q.g.scal, r < 0 || r >= q.g.N1, return);
             w[0] = (double)q.f.scr[c + r];
             const R U0 = ld(q.f.U + c + r), Um = ld(q.f.U + c + r - sk);
             w[PL] = (double)(Um + cz * (U0 - Um));
@@ -808,7 +816,9 @@ struct DWY {
         struct In { R V, Vk, iR, iRk, rdx2, rdmx2, d; };
         __device__ __forceinline__ void load(const DWY &q, int r, In &n)
         {
+            row_cell(q.g, c, t4);
             const long long sj = q.g.P1;
+            TCS_OOB(q.g.scal, c + dk < 0 || c + sj + dk >= q.g.NP, (dk = 0, t4k = 0));
             n.V = ld(q.f.V + c + sj); n.Vk = ld(q.f.V + c + sj + dk);
             n.iR = ld(q.f.iRT + t4); n.iRk = ld(q.f.iRT + t4 + t4k);
             n.rdx2 = ld(q.g.m2.rdx + r + 1); n.rdmx2 = ld(q.g.m2.rdmx + r + 2);
@@ -827,7 +837,7 @@ struct DWY {
     };
     struct Out : PeriodicOut<R> {
         __device__ __forceinline__ Out(const DWY &q, int line, int by, int r) : PeriodicOut<R>(q.g, q.f.dW, 1 + line, r + 1, 1 + by) {}
-        __device__ __forceinline__ void put(const DWY &, const double *x) { PeriodicOut<R>::put(R(x[0])); }
+        __device__ __forceinline__ void put(const DWY &q, const double *x) { PeriodicOut<R>::put(q.g, q.f.dW, R(x[0])); }
     };
 };
 

@@ -644,6 +644,7 @@ struct Modal {
         struct In { cplx_t<R> s; double am, ap; };
         __device__ __forceinline__ void load(const Modal &q, int r, In &n)
         {
+            TCS_ROW(q.g.scal, p < q.f.S || p >= q.f.S + (long long)q.h1p * q.g.N2 * q.g.N3, p = q.f.S);
             n.s = *p;
             n.am = ld(q.f.fam + r + 1); n.ap = ld(q.f.fap + r + 1);
             p += q.h1p;
@@ -665,6 +666,7 @@ struct Modal {
         __device__ __forceinline__ void put(const Modal &q, const double *x)
         {
             const R re = R(x[0]);
+            TCS_ROW(q.g.scal, p < q.f.S || p >= q.f.S + (long long)q.h1p * q.g.N2 * q.g.N3, p = q.f.S);
             *p = mkc<R>(re, zi ? R(0) : R(x[1]));
             total += (double)re;
             p -= q.h1p;

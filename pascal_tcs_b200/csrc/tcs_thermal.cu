@@ -89,6 +89,7 @@ struct ThermalZ {
         struct In { R Txm, Txp, Tym, Typ, Tzp, Uc, Uxp, Vc, Vyp, Wzp, rdx3, dx3, rdmx3; };
         __device__ __forceinline__ void load(const ThermalZ &o, int r, In &n)
         {
+            row_cell(o.g, c);
             const GridT<R> &g = o.g;
             const FieldsT<R> &f = o.f;
             const long long sj = g.P1, sk = (long long)g.P1 * g.P2;
@@ -149,7 +150,7 @@ struct ThermalZ {
     };
     struct Out : ScratchOut<R> {
         __device__ __forceinline__ Out(const ThermalZ &q, int line, int by, int r) : ScratchOut<R>(q.g, q.f.scr, 1 + line, 1 + by, r + 1, (long long)q.g.P1 * q.g.P2) {}
-        __device__ __forceinline__ void put(const ThermalZ &, const double *x) { ScratchOut<R>::put(R(x[0])); }
+        __device__ __forceinline__ void put(const ThermalZ &q, const double *x) { ScratchOut<R>::put(q.g, q.f.scr, R(x[0])); }
     };
 };
 
@@ -184,6 +185,7 @@ struct ThermalX {
         }
         __device__ __forceinline__ void put(const ThermalX &o, int r, double *w, int PL) const
         {
+            TCS_OOB(o.g.scal, r < 0 || r >= o.g.N1, return);
             const GridT<R> &g = o.g;
             const PhysT<R> &p = g.ph;
             const bool d2 = g.kdeg2 != 0;
@@ -269,9 +271,11 @@ struct ThermalY {
         struct In { R Txm, Txp, Typ, Tkm, Tkp, V, rdx2, dx2, rdmx2, d; };
         __device__ __forceinline__ void load(const ThermalY &o, int r, In &n)
         {
+            row_cell(o.g, c);
             const GridT<R> &g = o.g;
             const R *const T = o.f.T;
             n.Txm = ld(T + c - 1); n.Txp = ld(T + c + 1); n.Typ = ld(T + c + g.P1);
+            TCS_OOB(g.scal, c + dkm < 0 || c + dkp >= g.NP, dkm = dkp = 0);
             n.Tkm = ld(T + c + dkm); n.Tkp = ld(T + c + dkp);
             n.V = ld(o.f.V + c + g.P1);
             n.rdx2 = ld(g.m2.rdx + r + 1); n.dx2 = ld(g.m2.dx + r + 2); n.rdmx2 = ld(g.m2.rdmx + r + 2);
@@ -304,7 +308,8 @@ struct ThermalY {
             : PeriodicOut<R>(q.g, q.f.Tn, 1 + line, r + 1, 1 + by), T(q.f.T + ix(q.g, 1 + line, r + 1, 1 + by)) {}
         __device__ __forceinline__ void put(const ThermalY &q, const double *x)
         {
-            PeriodicOut<R>::put(ld(T) + R(x[0]));
+            row_ptr(q.g, (const R *)q.f.T, T);
+            PeriodicOut<R>::put(q.g, q.f.Tn, ld(T) + R(x[0]));
             T -= q.g.P1;
         }
     };

@@ -42,7 +42,7 @@ EXPORTS = [
     "tcs_snapshot", "tcs_restore",
     "tcs_tdma_plan_many_create", "tcs_tdma_plan_many_destroy", "tcs_tdma_many_solve",
     "tcs_tdma_many_solve_cycle", "tcs_tdma_many_solve_noalloc", "tcs_kernel_count", "tcs_launch_count", "tcs_measure_fp64_peak", "tcs_check_reciprocal", "tcs_kernel_name", "tcs_timer_of_kernel", "tcs_timer_name", "tcs_bounds_checked",
-    "tcs_bounds_violations", "tcs_probe_enable",
+    "tcs_bounds_violations", "tcs_bounds_rows", "tcs_probe_enable",
     "tcs_probe_read", "tcs_probe_reset", "tcs_set_use_graph", "tcs_set_copy_polls", "tcs_set_tuning", "tcs_get_tuning",
     "tcs_last_error", "tcs_precision", "tcs_ensemble_create", "tcs_ensemble_destroy", "tcs_ensemble_step",
     "tcs_ensemble_size", "tcs_ensemble_set_batched", "tcs_ensemble_form", "tcs_autotune", "tcs_write_continue", "tcs_read_continue", "tcs_extract_plane",
@@ -130,6 +130,7 @@ def load() -> ctypes.CDLL:
         "tcs_timer_name": ([ip], ctypes.c_char_p),
         "tcs_bounds_checked": ([], ip),
         "tcs_bounds_violations": ([vp, dp], ip),
+        "tcs_bounds_rows": ([vp, dp], ip),
         "tcs_probe_enable": ([vp, ctypes.c_uint64], ip),
         "tcs_probe_read": ([vp, ip, dp, ctypes.POINTER(ip)], ip),
         "tcs_probe_reset": ([vp], ip),
@@ -283,6 +284,12 @@ class Solver:
         """Out-of-range indices the kernels met so far (bounds-check build; 0 otherwise)."""
         v = ctypes.c_double()
         _check(load().tcs_bounds_violations(self._h, ctypes.byref(v)), "tcs_bounds_violations")
+        return int(v.value)
+
+    def bounds_rows(self) -> int:
+        """Rows of the line sweeps checked so far, each read and each write (bounds-check build; 0 otherwise)."""
+        v = ctypes.c_double()
+        _check(load().tcs_bounds_rows(self._h, ctypes.byref(v)), "tcs_bounds_rows")
         return int(v.value)
 
     @property

@@ -34,12 +34,22 @@ SCRIPT = textwrap.dedent("""
              top_wall_mode=1),
         dict(n1m=48, n2m=20, n3m=40, property_set=0),
         dict(n1m=16, n2m=512, n3m=512, gamma2=2.0, property_set=1, Pr=7.0, Ra=1e7, dtStart=5e-5, seed=2),
+        # in FP64 the column form of every z sweep: rows of unequal segments, a part-filled last block
+        dict(n1m=150, n2m=166, n3m=405, property_set=1, Pr=7.0, Ra=1e6, dtStart=5e-5, fixed_dt=1, seed=3),
     ]
     for ci, cfg in enumerate(cases):
         for prec in (0, 1):
             g = P.Solver(precision=prec, **cfg)
             g.step(2)
             g.driver_step()
+            # every row of the 13 sweeps of these 3 steps has been checked as it was read and as it was written
+            n1, n2, n3 = (cfg[k] for k in ("n1m", "n2m", "n3m"))
+            cells, below = n1 * n2 * n3, n1 * (n2 - 1) * n3
+            want = 9 * cells + 3 * below + (n1 // 2 + 1) * n2 * n3
+            reads = want - (3 * cells + below if ci == 4 and prec == 0 else 0)   # the column form reads by copies, which have checks of their own
+            rows = g.bounds_rows()
+            print(ci, prec, rows, 3 * (want + reads))
+            assert rows >= 3 * (want + reads), (rows, want, reads)
             with tempfile.TemporaryDirectory() as d:
                 g.write_continue(d)
                 g.read_continue(d)
