@@ -246,8 +246,9 @@ int tcs_set_copy_polls(tcs_ctx *ctx, int polls);
  * (1, 2, 4), TCS_TUNE_Y_SOLVER (1, 2, 4), TCS_TUNE_MIXED_ROWS (1, 2, 4, 8) and
  * TCS_TUNE_Z_STAGING (1, 2) chose between forms and shapes of the line solvers
  * that one solver, with FP64 elimination and shapes of its own, has replaced.
- * Their values are checked (TCS_ERR_ARG), kept and returned as before, without
- * effect.
+ * Their values are checked against those ranges (the TL ones: 1..64; Z_STAGING 2 as
+ * before only in the FP64 form with N3 a multiple of 64 and an even N1), kept and
+ * returned, without effect.
  * TCS_TUNE_IFFT_LINES_X: lines per block of the inverse x transform
  * (TCS_TUNE_FFT_LINES_X sets those of the pressure right-hand side and its
  * forward x transform). */

@@ -128,37 +128,6 @@ void probe_end(const Shapes &cx, int kid, cudaStream_t s)
 // ---------------------------------------------------------------------------
 // plans
 // ---------------------------------------------------------------------------
-LinePlan make_line_plan(int n, bool cyclic, int TL, int pmax)
-{
-    LinePlan lp;
-    int P;
-    if (pmax > 32) pmax = 32;
-    if (cyclic) { P = 1; while (P * 2 <= pmax && n / (P * 2) >= 2) P *= 2; }
-    else { P = n / 2; if (P > pmax) P = pmax; if (P < 1) P = 1; }
-    lp.n = n; lp.P = P; lp.m0 = n / P; lp.rem = n % P;
-    const int mmax = lp.m0 + (lp.rem > 0 ? 1 : 0);
-    lp.PS = mmax | 1;
-    lp.LS = (P * lp.PS) | 1;
-    lp.TL = TL;
-    lp.cyclic = cyclic ? 1 : 0;
-    return lp;
-}
-
-// Shared-memory bytes per row of a line-solver block: A, C, D[nrhs] of the
-// row type, plus the kept rows A0, B0, C0, D0[nrhs] when FP32 rows are refined.
-static size_t row_bytes(int nrhs, bool fp32_refined)
-{
-    return fp32_refined ? (size_t)(5 + 2 * nrhs) * sizeof(float) : (size_t)(2 + nrhs) * sizeof(double);
-}
-
-static int choose_tl(int n, bool cyclic, size_t rowb, int want)
-{
-    LinePlan lp = make_line_plan(n, cyclic, want);
-    int tl = want;
-    while (tl > 2 && rowb * tl * lp.LS + (size_t)n * sizeof(int) > 112 * 1024) tl /= 2;
-    return tl;
-}
-
 bool make_fft_plan(int n, FFTPlan &fp, int maxr)
 {
     fp.n = n; fp.npass = 0;
@@ -561,13 +530,6 @@ int tcs_create(const tcs_config *cfg, tcs_ctx **out)
         c->cx.wall_bt = dmx2[n2sub] * dmx2[n2sub] / (s2 - dmx2[n2sub] * dmx2[n2sub]);
     }
     c->cx.fp1 = fp1; c->cx.fp3 = fp3; c->cx.fp1u = fp1u;
-    const size_t rb1 = row_bytes(1, c->fp32);
-    c->cx.tl_contig = choose_tl(N1, true, rb1, 8);
-    c->cx.tl_modal = choose_tl(N2, false, row_bytes(2, false), 8);   // modal rows are FP64 in both forms
-    {
-        const int tz = choose_tl(N3, true, rb1, 8), ty = choose_tl(N2, false, rb1, 8);
-        c->cx.tl_strided = tz < ty ? tz : ty;
-    }
     // measured on B200 at 256^3: 4 lines per block beats 1, 2, 8 and 16 for both FFT kernels
     c->cx.fft_lines_x = N1 <= 256 ? 4 : (N1 <= 512 ? 2 : 1);
     // z transforms: 16 lines in the one-radix form (256-byte rows), else 4 (2 or 1 for long lines)
@@ -576,6 +538,7 @@ int tcs_create(const tcs_config *cfg, tcs_ctx **out)
     // lines per block (64 or 128 threads; 256^3 and 512^3), the general form with 8
     c->cx.ifft_lines_x = ifftx_form(fp1u, 2) == 1 ? 2 : (ifftx_form(fp1u, 8) ? 8 : 1);
     c->cx.lanes = 32;
+    c->cx.tl_strided = c->cx.tl_contig = c->cx.tl_modal = 8;
     c->cx.long_lines = 2;
     c->cx.y_solver = 1;
     c->cx.mixed_rows = 1;
@@ -974,40 +937,19 @@ static void launch_step(tcs_ctx *c, cudaStream_t s)
 
 extern "C" {
 
-// Launch-shape knobs (lines per block of the line-solver families and of the
-// FFT kernels).  A line-solver value is the most lines per block: every
-// launch fits it down (fit_tl halves it until the family's blocks per SM fit
-// the SM's shared memory), so the value that runs is the largest power of two
-// up to it that fits.  Values are refused only where one block of the
-// family's largest row type could not hold them at all (227 KB per block);
-// the bound takes the bank-padded line stride of the non-cyclic strided
-// problems (at most one bank row, 32 words, above the odd stride).
-static bool lines_fit_one_block(size_t rowb, int value, int LS, int n)
-{
-    return rowb * (size_t)value * (size_t)(LS + 32) + (size_t)n * sizeof(int) <= (size_t)227 * 1024;
-}
-
+// Launch-shape knobs.  The FFT kernels' are refused where a block could not hold the
+// lines; the ones without effect (TL_*, LONG_LINES, Y_SOLVER, MIXED_ROWS, Z_STAGING) are
+// checked against their range, kept and returned.
 int tcs_set_tuning(tcs_ctx *c, int knob, int value)
 {
     ENTER(c);
     if (value < 1 || value > 64 || (value & (value - 1))) return set_err(TCS_ERR_ARG, "tuning value must be a power of two in 1..64");
     Ctx<double> &x = c->cx;
     const GridT<double> &g = x.g;
-    const size_t rb1 = row_bytes(1, c->fp32);
     switch (knob) {
-    case TCS_TUNE_TL_STRIDED: {
-        LinePlan a = make_line_plan(g.N3, true, value), b = make_line_plan(g.N2, false, value);
-        if (!lines_fit_one_block(rb1, value, std::max(a.LS, b.LS), std::max(g.N2, g.N3)))
-            return set_err(TCS_ERR_ARG, "too many lines for shared memory");
-        x.tl_strided = value; break; }
-    case TCS_TUNE_TL_CONTIG: {
-        LinePlan a = make_line_plan(g.N1, true, value);
-        if (!lines_fit_one_block(rb1, value, a.LS, g.N1)) return set_err(TCS_ERR_ARG, "too many lines for shared memory");
-        x.tl_contig = value; break; }
-    case TCS_TUNE_TL_MODAL: {
-        LinePlan a = make_line_plan(g.N2, false, value);
-        if (!lines_fit_one_block(row_bytes(2, false), value, a.LS, g.N2)) return set_err(TCS_ERR_ARG, "too many lines for shared memory");
-        x.tl_modal = value; break; }
+    case TCS_TUNE_TL_STRIDED: x.tl_strided = value; break;
+    case TCS_TUNE_TL_CONTIG: x.tl_contig = value; break;
+    case TCS_TUNE_TL_MODAL: x.tl_modal = value; break;
     case TCS_TUNE_FFT_LINES_X:
         if ((size_t)value * g.N1 * (32 + esize(c)) > 200 * 1024) return set_err(TCS_ERR_ARG, "too many lines for shared memory");
         x.fft_lines_x = value; break;

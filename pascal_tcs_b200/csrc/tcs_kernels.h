@@ -13,7 +13,10 @@
 
 namespace tcs {
 
-// Every kernel the time step launches, in launch order.
+// The probed kernels, in launch order.  A step launches neither K_PSEUDO (part of the
+// right-hand side) nor K_DP_WALL and K_P_WALL (part of K_POST); K_FINAL is launched where
+// the diagnostics end in a launch of their own.  K_MEAN (part of K_MODAL) and K_TDMA_API
+// have no launch; their ids are kept.
 enum KernelId : int {
     K_THERMAL_Z = 0, K_THERMAL_X, K_THERMAL_Y, K_MOM_COEFFI,
     K_DU_Z, K_DU_X, K_DU_Y, K_DV_Z, K_DV_X, K_DV_Y, K_DW_Z, K_DW_X, K_DW_Y,
@@ -73,13 +76,10 @@ struct ProbeState;   // CUDA-event probes (tcs_capi.cu)
 
 // Launch shapes shared by both forms.
 struct Shapes {
-    int tl_strided, tl_contig, tl_modal;
     int fft_lines_x, fft_lines_z;
     int ifft_lines_x;                            // lines per block of the inverse x transform
     int lanes;                                   // at most this many partitions (lanes) per line
-    int long_lines, y_solver;                    // accepted and kept; one solver runs the strided lines
-    int mixed_rows;                              // likewise
-    int z_staging;                               // likewise
+    int tl_strided, tl_contig, tl_modal, long_lines, y_solver, mixed_rows, z_staging;   // knobs without effect: kept and returned
     int copy_polls;                              // polls of the column form's waits for its copies
     bool spec_live;                              // the spectrum holds a right-hand side that no Poisson solve has taken yet
     FFTPlan fp1, fp3;
@@ -95,7 +95,6 @@ struct Ctx : Shapes {
     FieldsT<R> f;
 };
 
-LinePlan make_line_plan(int n, bool cyclic, int TL, int pmax = 32);
 bool make_fft_plan(int n, FFTPlan &fp, int maxr);   // radices 2, 3, 4, 5 and (maxr >= 8) 8
 void probe_begin(const Shapes &cx, int kid, cudaStream_t s);
 void probe_end(const Shapes &cx, int kid, cudaStream_t s);
@@ -136,9 +135,9 @@ inline MarchPlan march_plan(int n, bool cyclic, int lanes, long long lines)
     auto more = [&]() { return (2 << mp.lgNS) <= cap && (n >> (mp.lgNS + 1)) >= 4; };
     while (more() && mp.lgNS < 5 && (n > (P::ROWS << mp.lgNS) || (lines << mp.lgNS) < 131072)) mp.lgNS++;
     mp.lgTI = P::LGTI;
-    // FP64 z lines of more than 416 rows in too few lines for the column form: 64
-    // segments of 8 lines (64 x 64 x 512, ps per cell of dw_z: 33 against 45)
-    if (std::is_same<typename P::Real, double>::value && P::ROWS == 12 && mp.lgNS == 5 && n > 416 && cap >= 64) {
+    // FP64 z lines (P::LONG64) of more than 416 rows in too few lines for the column
+    // form: 64 segments of 8 lines (64 x 64 x 512, ps per cell of dw_z: 33 against 45)
+    if (P::LONG64 && mp.lgNS == 5 && n > 416 && cap >= 64) {
         mp.lgNS = 6;
         mp.lgTI = 3;
     }

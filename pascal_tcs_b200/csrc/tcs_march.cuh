@@ -187,6 +187,7 @@ struct PeriodicOut {
 
 // The problem supplies
 //   static constexpr int NRHS, AHEAD (rows whose inputs are loaded ahead), ROWS, LGTI (most rows per segment, most lines per block), TPS
+//   static constexpr bool LONG64 (long lines in 64 segments, march_plan)
 //   skip(), lines() (count of lines along i of the block row)
 //   struct March { March(const Prob &, int line, int by, int r0);               // line: clamped to a valid one
 //                  struct In;  void load(const Prob &, int r, In &);             // the inputs of row r, rows in order from r0
@@ -438,11 +439,10 @@ __global__ void __launch_bounds__(256, 2) xmarch_kernel(const __grid_constant__ 
 
 // ---------------------------------------------------------------------------
 // The column form (FP64, z lines): a block of w consecutive i marches up NS
-// segments of the lines together (w NS threads; NS = 1 where there are lines
-// enough).  The rows of i that a plane needs (the problem's stream: its arrays
-// at j-1, j, j+1) come one bulk copy each into a ring of COL_SLOTS planes, up
-// to three planes ahead of the one being worked on, so no load latency is left
-// on the march; c and d of the eliminated rows go to global scratch
+// segments of the lines together (w NS threads).  The rows of i that a plane needs
+// (the problem's stream: its arrays at j-1, j, j+1) come one bulk copy each into a
+// ring of COL_SLOTS planes, up to two (COL_SLOTS - 2) ahead of the one being worked
+// on, so no load latency is left on the march; c and d of the eliminated rows go to global scratch
 // (consecutive i: coalesced) and the second march substitutes back.  The
 // segment's coupling e_r to the unknown before it is not stored: it dies out
 // within a few rows of a diagonally dominant line, so the rows up to the last
@@ -567,19 +567,13 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
             return;
         }
     }
-    double X, Xp;
-    if (NS == 1) {
-        X = Xp = (dp - cp * sd) * qrcp((1.0 - cp * se) + (e + cp * p));
-    } else {
-        // the ring is idle now: it holds the reduced systems
-        const int TP = w + 1, RS = NS * TP;
-        double *const o = csm + s * TP + l;
-        o[0] = e; o[RS] = cp; o[2 * RS] = se; o[3 * RS] = p; o[4 * RS] = dp; o[5 * RS] = sd;
-        __syncthreads();
-        march_reduce<1>(csm, lgNS, TP, true);
-        X = o[0];
-        Xp = csm[((s - 1) & (NS - 1)) * TP + l];
-    }
+    // the ring is idle now: it holds the reduced systems
+    const int TP = w + 1, RS = NS * TP;
+    double *const o = csm + s * TP + l;
+    o[0] = e; o[RS] = cp; o[2 * RS] = se; o[3 * RS] = p; o[4 * RS] = dp; o[5 * RS] = sd;
+    __syncthreads();
+    march_reduce<1>(csm, lgNS, TP, true);
+    const double X = o[0], Xp = csm[((s - 1) & (NS - 1)) * TP + l];
     K = __reduce_max_sync(0xffffffffu, K);
     {
         March st(prob, sline, by, r0);

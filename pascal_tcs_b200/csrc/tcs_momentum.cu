@@ -12,7 +12,6 @@
 namespace tcs {
 
 #define MU(jj, kk) ld(f.Mu2 + ix2(g, (jj), (kk)))
-#define IR(jj, kk) ld(f.iR2 + ix2(g, (jj), (kk)))
 
 // ---------------------------------------------------------------------------
 // mpi_momentum_coeffi (:145-173) -> (j,k) tables from T(n1sub, j, k).
@@ -78,6 +77,7 @@ struct DUZ {
     using Real = R;
     static constexpr int NRHS = 1;
     static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12, LGTI = 4;   // FP64 inputs of two rows do not fit the registers
+    static constexpr bool LONG64 = std::is_same<R, double>::value;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -287,6 +287,7 @@ struct DUY {
     using Real = R;
     static constexpr int NRHS = 1;
     static constexpr int AHEAD = 2, TPS = 512, ROWS = 16, LGTI = 4;
+    static constexpr bool LONG64 = false;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -346,6 +347,7 @@ struct DVZ {
     using Real = R;
     static constexpr int NRHS = 1;
     static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12, LGTI = 4;   // FP64 inputs of two rows do not fit the registers
+    static constexpr bool LONG64 = std::is_same<R, double>::value;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -527,6 +529,7 @@ struct DVY {
     using Real = R;
     static constexpr int NRHS = 1;
     static constexpr int AHEAD = 2, TPS = 512, ROWS = 16, LGTI = 4;
+    static constexpr bool LONG64 = false;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -589,6 +592,7 @@ struct DWZ {
     using Real = R;
     static constexpr int NRHS = 1;
     static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12, LGTI = 4;   // FP64 inputs of two rows do not fit the registers
+    static constexpr bool LONG64 = std::is_same<R, double>::value;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -674,14 +678,13 @@ struct DWZ {
             const GridT<R> &g = q.g;
             const int s = w + 2;
             a += l + 1; b += l + 1;
-            const double *const ta = a - (l + 1) + NROW * s, *const tb = b - (l + 1) + NROW * s;   // table words of planes k + 1 and k
+            const double *const tb = b - (l + 1) + NROW * s;   // table words of plane k
             n.Wxm = b[-1]; n.Wxp = b[1]; n.Wzp = a[0]; n.Wym = a[s]; n.Wyp = a[2 * s];
             n.U = a[3 * s]; n.Ux = a[3 * s + 1]; n.D = a[4 * s]; n.Dx = a[4 * s + 1];
             n.V = a[5 * s]; n.Vy = a[6 * s]; n.E = a[7 * s]; n.Ey = a[8 * s];
             n.P = a[9 * s];
             n.Mc = tb[4]; n.mt.x = tb[6]; n.mt.y = tb[7]; n.muyz4 = tb[11]; n.iR = tb[14];
             n.dx3 = ld(g.m3.dx + r + 1); n.rdx3 = ld(g.m3.rdx + r + 1); n.rdmx3 = ld(g.m3.rdmx + r + 1);
-            (void)ta;
         }
         __device__ __forceinline__ void row(const DWZ &q, int r, const In &n, double &a, double &b, double &cc, double *d)
         {
@@ -786,6 +789,7 @@ struct DWY {
     using Real = R;
     static constexpr int NRHS = 1;
     static constexpr int AHEAD = 2, TPS = 512, ROWS = 16, LGTI = 4;
+    static constexpr bool LONG64 = false;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -1060,10 +1064,8 @@ void launch_pseudo_update(const Ctx<R> &cx, cudaStream_t s)
 }
 
 #undef MU
-#undef IR
 
-// the two forms
-// The nine sweeps of solvedU, solvedV and solvedW for many cases, one launch per sweep.
+// The nine sweeps of solvedU, solvedV and solvedW for many cases, sweep by sweep (march_stage).
 template <class R>
 void launch_momentum_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s)
 {
@@ -1078,6 +1080,7 @@ void launch_momentum_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaS
     march_stage(cs, A, s, launch_dw_y<R>);
 }
 
+// the two forms
 template void launch_momentum_multi<double>(const std::vector<Ctx<double> *> &, MultiArena &, cudaStream_t);
 template void launch_momentum_multi<float>(const std::vector<Ctx<float> *> &, MultiArena &, cudaStream_t);
 template void launch_momentum_coeffi<double>(const Ctx<double> &, cudaStream_t);

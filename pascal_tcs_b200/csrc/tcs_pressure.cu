@@ -630,6 +630,7 @@ struct Modal {
     // 8 lines of 16 bytes a row; four rows ahead (256^3, ps per cell: 5.7; two ahead 6.1, 16 lines 8.3; the lane-per-
     // partition solver before it 7.3)
     static constexpr int AHEAD = 4, TPS = 512, ROWS = 16, LGTI = 3;
+    static constexpr bool LONG64 = false;
     static constexpr bool TOTAL = true;
     GridT<R> g; FieldsT<R> f; int h1p;
     __device__ bool skip() const { return blown(g); }

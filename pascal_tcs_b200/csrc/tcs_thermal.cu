@@ -18,6 +18,7 @@ struct ThermalZ {
     using Real = R;
     static constexpr int NRHS = 1;
     static constexpr int AHEAD = std::is_same<R, float>::value ? 1 : 0, TPS = 512, ROWS = 12, LGTI = 4;   // FP64 inputs of two rows do not fit the registers
+    static constexpr bool LONG64 = std::is_same<R, double>::value;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -228,6 +229,7 @@ struct ThermalY {
     using Real = R;
     static constexpr int NRHS = 1;
     static constexpr int AHEAD = 0, TPS = 512, ROWS = 16, LGTI = 4;
+    static constexpr bool LONG64 = false;
     GridT<R> g; FieldsT<R> f;
     __device__ bool skip() const { return blown(g); }
     __device__ int lines() const { return g.N1; }
@@ -341,7 +343,7 @@ void launch_thermal(const Ctx<R> &cx, cudaStream_t s)
     launch_thermal_y(cx, s);
 }
 
-// The same three sweeps for many cases, one launch per sweep.
+// The same three sweeps for many cases, sweep by sweep (march_stage).
 template <class R>
 void launch_thermal_multi(const std::vector<Ctx<R> *> &cs, MultiArena &A, cudaStream_t s)
 {

@@ -1,14 +1,16 @@
 """The bounds-check build (libtcs_bc.so, compiled with -DTCS_BOUNDS_CHECK):
-every field, 2-D table, spectrum and shared-memory row index the kernels form
-is checked on the device; an out-of-range index is counted and its access
-redirected to a valid cell, never made.  It stands in for a memory checker
-(the reference's own debug builds use the compiler's array checks,
-Makefile.inc:6-11).  The test runs that build in a fresh process over uneven
-sizes, both precisions, stretched and uniform grids, long lines, every
-launch-shape knob family, the per-routine driver sequence, an ensemble in
-both forms and a 26-case batched ensemble whose sweeps split over two
-multi-case launches, the restart files and planes, and the PaScaL_TDMA interface, and
-requires zero recorded violations (needs a B200)."""
+every field, 2-D table and spectrum index that the kernels form, every row that
+the line sweeps step to (in a field, a table, the spectrum, shared memory or the
+column form's scratch) and the column form's copies are checked on the device; an
+index out of range is counted and its access redirected to a valid cell or left
+out, never made.  It stands in for a memory checker (the reference's own debug
+builds use the compiler's array checks, Makefile.inc:6-11).  The test runs that
+build in a fresh process over uneven sizes, both precisions, stretched and uniform
+grids, long lines, the column form, segments bounded to 4, the FFT shapes, the
+per-routine driver sequence, ensembles in both forms (26 cases on 24 streams among
+them), the restart files and planes, and the PaScaL_TDMA interface, and requires
+zero recorded violations and a check of every row read and written (needs a
+B200)."""
 import os
 import subprocess
 import sys
@@ -56,14 +58,19 @@ SCRIPT = textwrap.dedent("""
             g.plane(1, 3); g.plane(2, 1); g.plane(3, cfg["n3m"])
             counts[f"case{{ci}} prec{{prec}}"] = g.bounds_violations()
             g.close()
-    for knob, v in (("lanes", 4), ("tl_strided", 2), ("tl_contig", 1), ("tl_modal", 1), ("fft_lines_x", 1),
-                    ("fft_lines_z", 8), ("long_lines", 4), ("y_solver", 4), ("mixed_rows", 4), ("ifft_lines_x", 8)):
-        for prec in ((0, 1) if knob in ("y_solver", "mixed_rows") else (0,)):
-            g = P.Solver(n1m=150 if knob == "y_solver" else 48, n2m=32, n3m=40, property_set=1, Pr=7.0, Ra=1e6,
-                         dtStart=5e-4, precision=prec)
+    for knob, v in (("lanes", 4), ("fft_lines_x", 1), ("fft_lines_z", 8), ("ifft_lines_x", 8)):
+        for prec in (0, 1):
+            g = P.Solver(n1m=150, n2m=32, n3m=40, property_set=1, Pr=7.0, Ra=1e6, dtStart=5e-4, precision=prec)
             g.set_tuning(knob, v)
             g.step(2)
             counts[f"{{knob}}={{v}} prec{{prec}}"] = g.bounds_violations()
+            g.close()
+    # more than 32 segments along x and in the modal solves
+    for n in ((540, 6, 8), (4096, 4, 4), (16, 900, 6)):
+        for prec in (0, 1):
+            g = P.Solver(n1m=n[0], n2m=n[1], n3m=n[2], Ra=1e8, dtStart=1e-5, precision=prec)
+            g.step(1)
+            counts[f"{{n}} prec{{prec}}"] = g.bounds_violations()
             g.close()
     ens = [P.Solver(n1m=n1, n2m=n2, n3m=n3, property_set=1, Pr=7.0, Ra=1e6, dtStart=5e-4, precision=prec)
            for (n1, n2, n3, prec) in ((16, 24, 20, 0), (32, 16, 12, 0), (24, 20, 16, 1), (20, 12, 30, 1))]
@@ -73,13 +80,7 @@ SCRIPT = textwrap.dedent("""
         e.step(2)
     for k, s in enumerate(ens):
         counts[f"ensemble case {{k}}"] = s.bounds_violations()
-    # 24 uneven cases per precision: more than one multi-case launch's parameter
-    # block holds (21 FP64 or 24 FP32 problems), so each batched sweep is split
-    g = P.Solver(n1m=36, n2m=20, n3m=64, property_set=1, Pr=7.0, Ra=1e6, dtStart=5e-4)
-    g.set_tuning("z_staging", 2)
-    g.step(2)
-    counts["z_staging=2"] = g.bounds_violations()
-    g.close()
+    # more uneven cases than the ensemble has streams
     rng = np.random.default_rng(3)
     for prec in (0, 1):
         big = [P.Solver(n1m=int(rng.choice([16, 20, 24])), n2m=int(rng.choice([12, 16, 24])),

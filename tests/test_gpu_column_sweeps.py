@@ -1,5 +1,7 @@
 """The column form of the FP64 z sweeps (column_kernel: even N1, more than 384 rows,
-24576 lines or more) through its public calls (needs a B200)."""
+24576 lines or more) through its public calls (needs a B200): its results against
+the oracle at the edges of its shapes, against the marching form on one grid, its use
+of the spectrum, and the report of a copy that does not arrive."""
 import numpy as np
 import pytest
 
@@ -75,3 +77,69 @@ def test_no_steps_leave_a_pending_right_hand_side_alone(tcs):
         s.pressure_Poisson_FFT2()
     np.testing.assert_array_equal(b.get("dP"), a.get("dP"))
     ens.close()
+
+
+def _takes_the_column_form(g, sweep):
+    # with waits that run out at once, a sweep in the column form reports a late copy
+    g.set_copy_polls(0)
+    sweep()
+    try:
+        g.post_cfl()
+        late = False
+    except Exception as e:
+        assert e.code == 2
+        late = True
+    g.set_copy_polls(1 << 22)
+    g.restore()
+    return late
+
+
+@pytest.mark.parametrize("n,column", [
+    ((150, 180, 405), True),      # block width 32, a part-filled last block; segments of 203 and 202 rows
+    ((180, 144, 405), True),      # block width 64, a part-filled last block
+    ((64, 396, 486), True),       # full blocks; two segments of 243 rows
+    ((135, 190, 400), False),     # odd N1: rows of i are not 16-byte aligned
+    ((128, 200, 384), False),     # 384 rows: the marching form
+])
+def test_column_form_matches_oracle(tcs, oracle_mod, n, column):
+    # the diffusion number of the z rows is above 0.1: a segment's coupling to its
+    # neighbour lives for tens of rows, which the second march repairs
+    cfg = dict(n1m=n[0], n2m=n[1], n3m=n[2], property_set=1, Pr=7.0, Ra=1e4, DeltaT=10.0, dtStart=1e-3 if n[1] < 300 else 2e-4,
+               fixed_dt=1, seed=11, noise_amp=0.05, gamma2=1.2)
+    g = tcs.Solver(**cfg)
+    dz = g.metric("dx3")[1]
+    assert 0.5 * (7.0 / 1e4) ** 0.5 * cfg["dtStart"] / dz**2 > 0.1
+    g.momentum_coeffi()
+    g.snapshot()
+    for sweep in (g.thermal_solver, g.momentum_solvedU, g.momentum_solvedV, g.momentum_solvedW):
+        assert _takes_the_column_form(g, sweep) == column, sweep.__name__
+    o = oracle_mod.Oracle(**{k: v for k, v in g.config.items() if k not in ("device", "precision")})
+    g.step(2)
+    o.step(2)
+    for f in ("T", "U", "V", "W", "P"):
+        a, b = g.get(f), o.get(f)
+        err = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300)
+        print(f, f"{err:.2e}")
+        assert np.all(np.isfinite(a)) and err <= 1e-10, (f, err)
+    g.close()
+
+
+def test_column_form_agrees_with_the_marching_form(tcs):
+    # a pending right-hand side keeps the spectrum, so the same sweep then takes the
+    # marching form: the same rows eliminated in another order
+    g = tcs.Solver(**CFG)
+    g.step(2)
+    g.momentum_coeffi()
+    g.snapshot()
+    for sweep, field in ((g.momentum_solvedU, "dU"), (g.momentum_solvedV, "dV"), (g.momentum_solvedW, "dW"), (g.thermal_solver, "T")):
+        assert _takes_the_column_form(g, sweep)
+        sweep()
+        a = g.get(field)
+        g.restore()
+        g.pressure_RHS()
+        assert not _takes_the_column_form(g, sweep)
+        sweep()
+        b = g.get(field)
+        g.restore()
+        g.pressure_Poisson_FFT2()
+        assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b), field

@@ -1,7 +1,7 @@
 """Ensembles (tcs_ensemble_*): independent cases of uneven sizes, properties
 and precisions advanced together by one CUDA graph per step must give, case
 by case, exactly what each case gives when stepped alone, in both forms (the
-batched one: one multi-case launch per line sweep; one branch per case) and
+batched one: stage by stage over all cases; one branch per case) and
 in the auto mode that measures both (needs a B200)."""
 import time
 
@@ -62,17 +62,15 @@ def test_ensemble_rejects_repeated_case(tcs):
         tcs.Ensemble([s, s])
 
 
-def test_batched_ensemble_more_cases_than_one_launch_holds(tcs):
-    # 24 FP64 cases: more than one multi-case launch's parameter block holds,
-    # so every sweep is split over several launches; two sizes, so the items
-    # of the longer lines come first.
+def test_batched_ensemble_of_many_sizes(tcs):
+    # 24 FP64 cases, as many as the graph has branches for, of several sizes
     cfgs = [dict(n1m=16, n2m=12 + 4 * (i % 2), n3m=(10, 12, 16)[i % 3], property_set=1, Pr=7.0, Ra=1e6,
                  dtStart=5e-4, seed=10 + i) for i in range(24)]
     alone = [tcs.Solver(**c) for c in cfgs]
     grouped = [tcs.Solver(**c) for c in cfgs]
     for s in alone:
         s.step(3)
-    ens = tcs.Ensemble(grouped)
+    ens = tcs.Ensemble(grouped, batched=True)
     assert ens.step(3) == 0
     for a, b in zip(alone, grouped):
         for n in ("T", "U", "V", "W", "P"):

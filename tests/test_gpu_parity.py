@@ -119,25 +119,21 @@ def _run_compare(tcs, oracle_mod, steps, **cfg):
 
 
 def test_long_lines_match_oracle(tcs, oracle_mod):
-    # 512-row z and y lines (16 rows per lane; the z and y sweeps in their
-    # one-block-per-SM form), water properties: whole steps against the oracle
-    err, g, _ = _run_compare(tcs, oracle_mod, 3, n1m=16, n2m=512, n3m=512, gamma2=2.0, property_set=1, Pr=7.0,
+    # 512-row z and y lines (32 segments of 16 rows along y, 64 of 8 along z), water
+    # properties: whole steps against the oracle
+    err, _, _ = _run_compare(tcs, oracle_mod, 3, n1m=16, n2m=512, n3m=512, gamma2=2.0, property_set=1, Pr=7.0,
                              Ra=1e7, DeltaT=10.0, dtStart=5e-5, fixed_dt=1, seed=2)
     print({k: f"{v:.2e}" for k, v in err.items()})
     for k, v in err.items():
         assert v <= RUN_TOL, f"{k}: rel L2 {v:.3e}"
-    g.set_tuning("long_lines", 4)
-    assert g.tuning()["long_lines"] == 4
 
 
-def test_one_line_per_thread_y_solver_matches_oracle(tcs, oracle_mod):
-    # the FP64 y sweeps and the modal solves on the plain Thomas elimination
-    # with one line per thread (y_solver 4); 150 lines along x leave the last
-    # block of 128 lines part-filled, water properties
+def test_part_filled_blocks_match_oracle(tcs, oracle_mod):
+    # 150 lines along x and 76 along kx leave the last blocks of 16 and 8 lines
+    # part-filled, water properties
     cfg = dict(n1m=150, n2m=40, n3m=24, gamma2=1.5, property_set=1, Pr=7.0, Ra=1e7, DeltaT=10.0,
                dtStart=2e-4, fixed_dt=1, seed=5)
     g, o = _pair(tcs, oracle_mod, **cfg)
-    g.set_tuning("y_solver", 4)
     g.step(12)
     hd = o.step(12)
     hg = g.history(0, 12)

@@ -1,8 +1,9 @@
-"""The marching solvers of the strided line sweeps at the edges of their shapes
-(needs a B200): few rows, lines of segments of unequal length, part-filled blocks,
-more than 32 segments, the column form of long FP64 lines and its fallback on an
-odd N1, against the oracle.  The diffusion number of the z rows is above 0.1 in
-the long cases, so a segment's coupling to its neighbour lives for tens of rows.
+"""The marching solvers of the line sweeps at the edges of their shapes (needs a
+B200): few rows, lines of segments of unequal length, part-filled blocks, more than
+32 segments along each axis and in the modal solves, against the oracle.  The
+diffusion number of the z rows is above 0.1 in the long cases, so a segment's
+coupling to its neighbour lives for tens of rows.  (The column form of long FP64 z
+lines: test_gpu_column_sweeps.py.)
 
 Bars: FP64 the parity bar of the other oracle tests (1e-10); FP32-mixed storage
 keeps 6e-8 of each field per step, U, T and P within 1e-5 over two steps."""
@@ -15,11 +16,17 @@ SHAPES = [
     (4, 4, 4),        # one segment pair of 2 rows, 16-line blocks part-filled
     (20, 7, 25),      # segments of 6 and 7 rows
     (18, 9, 384),     # 32 segments of 12 rows
-    (36, 6, 400),     # the column form, block width 64 part-filled
-    (150, 5, 405),    # the column form, segments of 203 and 202 rows, a part-filled last block
-    (45, 6, 400),     # odd N1: rows of i are not 16-byte aligned, no column form
-    (45, 5, 640),     # 64 segments: reduced systems through shared memory
-    (20, 643, 8),     # the same along y, segments of unequal length
+    (36, 6, 400),     # 32 segments of 12 and 13 rows, three blocks of 16 lines
+    (150, 5, 405),    # segments of 12 and 13 rows, a part-filled last block
+    (45, 6, 400),     # odd N1: rows of i are not 16-byte aligned
+    (45, 5, 640),     # z: 64 segments, reduced systems through shared memory
+    (20, 643, 8),     # y: 64 segments of unequal length
+    (540, 6, 8),      # x: 64 segments (from 531 cells on), several warps staging one line
+    (2160, 5, 6),     # x: 128 segments
+    (4096, 4, 4),     # x: 256 segments, one line per block
+    (16, 900, 6),     # modal solves (two right-hand sides): 64 segments (from 837 rows on)
+    (8, 4096, 4),     # y and modal: the longest lines
+    (8, 6, 4096),     # z: the longest lines
 ]
 
 
@@ -31,8 +38,9 @@ def test_strided_sweeps_match_oracle(n, precision):
 
     # (643 stretched rows at Ra = 1e4 and dt = 2e-3 are no test: the y rows of T lose
     # their dominance there, max |T| is 8e4 after two steps, and two restatements in
-    # 64 bits differ by 3e-10)
-    ra, dt = (1e4, 2e-3) if n[1] < 100 else (1e6, 1e-4)
+    # 64 bits differ by 3e-10; likewise 2160 cells along x (max |T| 1e6), 4096 along z,
+    # and 4096 rows along y at Ra = 1e6 and dt = 1e-4 (2e4))
+    ra, dt = (1e4, 2e-3) if n[1] < 100 and max(n) < 1000 else ((1e6, 1e-4) if n[1] < 1000 else (1e8, 1e-5))
     cfg = dict(n1m=n[0], n2m=n[1], n3m=n[2], property_set=0, Pr=0.71, Ra=ra, dtStart=dt, fixed_dt=1, seed=11,
                noise_amp=0.05, gamma2=1.2)
     g = P.Solver(precision=precision, **cfg)
