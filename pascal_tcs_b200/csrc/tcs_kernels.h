@@ -118,7 +118,13 @@ inline void smem_opt_in(const void *fn, size_t smem, size_t *cache)
 // The shape of a marching sweep (march_block) of `lines` lines in all: TI lines
 // and NS segments of every line per block.  Rows per segment, m = n / NS: at
 // most P::ROWS, and at least 4, because every segment loads its first plane
-// twice; with few lines, short segments fill the SMs.  P::ROWS is 12 for the z
+// twice; with few lines, short segments fill the SMs.  Up to 8192 threads in all a
+// sweep is one chain of loads per segment, so segments of 2 rows are taken there
+// (x sweeps alike; not where 4 rows are on their way at once, P::AHEAD).  With 4 the
+// FP64 step at 12 x 10 x 12 took 143 us against 131 before the sweeps marched, with 2
+// 118; 24^3 141, 141 and 118.  Up to 65536 threads a 32^3 or 48^3 step would gain 8% too,
+// but 48 such cases side by side, which fill the SMs, lose 15% by the planes loaded
+// twice (2.65 -> 3.07 ms), and a case has one plan, alone or not.  P::ROWS is 12 for the z
 // sweeps: the parked rows (24 B each, 512 threads per SM) then leave L1 room for
 // the stencil's x neighbours and tables (measured in FP64, ps per cell of dw_z:
 // m = 16 at 256^3 36, m = 8 22; m = 12 at 192^3 23, m = 6 28).  The y sweeps read
@@ -132,8 +138,10 @@ inline MarchPlan march_plan(int n, bool cyclic, int lanes, long long lines)
     mp.n = n; mp.cyclic = cyclic ? 1 : 0;
     mp.lgNS = 1;
     const int cap = lanes < 32 ? lanes : 256;
-    auto more = [&]() { return (2 << mp.lgNS) <= cap && (n >> (mp.lgNS + 1)) >= 4; };
-    while (more() && mp.lgNS < 5 && (n > (P::ROWS << mp.lgNS) || (lines << mp.lgNS) < 131072)) mp.lgNS++;
+    auto more = [&](int rows) { return (2 << mp.lgNS) <= cap && (n >> (mp.lgNS + 1)) >= rows; };
+    while (more(4) && mp.lgNS < 5 && (n > (P::ROWS << mp.lgNS) || (lines << mp.lgNS) < 131072)) mp.lgNS++;
+    if (P::AHEAD < 4)
+        while (more(2) && mp.lgNS < 5 && (lines << (mp.lgNS + 1)) <= 8192) mp.lgNS++;
     mp.lgTI = P::LGTI;
     // FP64 z lines (P::LONG64) of more than 416 rows in too few lines for the column
     // form: 64 segments of 8 lines (64 x 64 x 512, ps per cell of dw_z: 33 against 45)
@@ -144,7 +152,7 @@ inline MarchPlan march_plan(int n, bool cyclic, int lanes, long long lines)
     auto words = [&]() { return march_words(n, 1 << mp.lgNS, 1 << mp.lgTI, P::NRHS) * sizeof(double); };
     while (mp.lgTI > 0 && words() > 227 * 1024) {
         mp.lgTI--;
-        if (more() && mp.lgNS + mp.lgTI < 9) mp.lgNS++;
+        if (more(4) && mp.lgNS + mp.lgTI < 9) mp.lgNS++;
     }
     while (words() > 227 * 1024 || mp.lgTI + mp.lgNS < 5) {   // fits, in whole warps
         if (words() > 227 * 1024) mp.lgTI--;
@@ -207,16 +215,16 @@ inline void launch_march(const Shapes &cx, const P &prob, int n, bool cyclic, in
 }
 
 // The shape of an x sweep: as many lines as two blocks per SM hold, segments for
-// 256 threads.
+// 256 threads, of at least 4 rows (2 on small grids, as above).
 template <class P>
-inline MarchPlan xmarch_plan(int n, int lanes)
+inline MarchPlan xmarch_plan(int n, int lanes, long long lines)
 {
     MarchPlan mp;
     mp.n = n; mp.cyclic = 1;
     const int cap = lanes < 32 ? lanes : 256;
     for (mp.lgTI = 4;; mp.lgTI--) {
         mp.lgNS = 1;
-        while (mp.lgNS + mp.lgTI < 8 && (2 << mp.lgNS) <= cap && (n >> (mp.lgNS + 1)) >= 4) mp.lgNS++;
+        while (mp.lgNS + mp.lgTI < 8 && (2 << mp.lgNS) <= cap && (n >> (mp.lgNS + 1)) >= ((lines << (mp.lgNS + 1)) <= 8192 ? 2 : 4)) mp.lgNS++;
         while (mp.lgNS + mp.lgTI < 5) mp.lgNS++;          // whole warps
         if (mp.lgTI == 0 || xmarch_words(n, 1 << mp.lgNS, 1 << mp.lgTI, P::WORDS) * sizeof(double) <= 113 * 1024) break;
     }
@@ -227,7 +235,7 @@ inline MarchPlan xmarch_plan(int n, int lanes)
 template <class P>
 inline void launch_xmarch(const Shapes &cx, const P &prob, int n, int nlines, int gy, cudaStream_t s, int kid)
 {
-    const MarchPlan mp = xmarch_plan<P>(n, cx.lanes);
+    const MarchPlan mp = xmarch_plan<P>(n, cx.lanes, (long long)nlines * gy);
     const int TI = 1 << mp.lgTI;
     const size_t smem = xmarch_words(n, 1 << mp.lgNS, TI, P::WORDS) * sizeof(double);
     static size_t conf[64] = {};

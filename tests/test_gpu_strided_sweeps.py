@@ -14,7 +14,10 @@ pytestmark = pytest.mark.gpu
 
 SHAPES = [
     (4, 4, 4),        # one segment pair of 2 rows, 16-line blocks part-filled
-    (20, 7, 25),      # segments of 6 and 7 rows
+    (5, 4, 6),        # segments of 3 rows along z, of 2 along y, of 1 and 2 in V's y sweep
+    (12, 10, 25),     # of 3 and 4 rows along z, of 2 and 3 along y
+    (20, 7, 25),      # segments of 3 and 4 rows
+    (24, 20, 24),     # 8 segments of 3 rows along x and z, of 2 and 3 along y
     (18, 9, 384),     # 32 segments of 12 rows
     (36, 6, 400),     # 32 segments of 12 and 13 rows, three blocks of 16 lines
     (150, 5, 405),    # segments of 12 and 13 rows, a part-filled last block
