@@ -58,7 +58,7 @@ __device__ __forceinline__ void finalize(const GridT<R> &g, const FieldsT<R> &f,
     sc[S_NUBOT] = red[PT_NUB][0] / cnt;
     sc[S_NUTOP] = red[PT_NUT][0] / cnt;
     sc[S_KE] = 0.5 * red[PT_KE][0] / (g.phd.L1 * g.phd.L2 * g.phd.L3);
-    if (maxdiv >= 1.0e-3 || maxdiv != maxdiv) {
+    if (maxdiv >= 1.0e-3 || sc[S_KE] != sc[S_KE]) {   // a maximum passes over NaN, the kinetic energy's sum does not
         sc[S_BLOWUP] = sc[S_STEP] + 1.0;          // the step (1-based) that blew up
         return;
     }

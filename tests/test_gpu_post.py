@@ -52,3 +52,23 @@ def test_diagnostics_and_wall_rows(n, precision):
             np.testing.assert_array_equal(a[:, wall, 0], a[:, wall, -2])
             np.testing.assert_array_equal(a[0, wall, :], a[-2, wall, :])
     g.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_fields_that_are_not_finite_are_reported(value, precision):
+    # the pressure solve spreads them over every cell, and a maximum of NaN divergences
+    # is none of them: the step reports a blow-up by the kinetic energy
+    import pascal_tcs_b200 as P
+
+    for n in ((16, 12, 10), (128, 256, 128)):
+        g = P.Solver(n1m=n[0], n2m=n[1], n3m=n[2], property_set=1, Pr=7.0, Ra=1e6, dtStart=5e-4, fixed_dt=1, precision=precision)
+        g.step(1)
+        T = g.get("T")
+        T[5, 5, 5] = value
+        g.set("T", T)
+        with pytest.raises(P.TcsError) as ei:
+            g.step(2)
+        assert ei.value.code == 4
+        assert g.scalars()["blowup"] == 2 and g.scalars()["step"] == 1
+        g.close()
