@@ -333,11 +333,12 @@ __global__ void __launch_bounds__(NT, Prob::TPS / NT) march_kernel(const __grid_
 // in the places of the words it has used (planes 0, 1, 2), and the solution
 // leaves plane 0 as it came, a warp per line.  The line stride is odd, so the
 // TI lines of a warp's march sit on distinct banks.  Two blocks per SM: one
-// stages while the other marches.  Against the lane-per-partition solver that
-// was here before (ms): 256^3 FP64 du_x 0.195 -> 0.162, FP32-mixed 0.227 -> 0.148
-// and thermal_x 0.345 -> 0.251; 400 x 200 x 384 FP32-mixed du_x 0.56 -> 0.32; level
-// (within 10%) from 384 rows on in FP64.  It moves 3 or 4 arrays at 2.5 to 2.7
-// TB/s: latency at 16 warps per SM bounds it.
+// stages while the other marches.  Against the lane-per-partition solver that was
+// here before (du_x, ps per cell, before and now): FP64 256 cells along x 19.6 and
+// 15.7, 400 14.2 and 13.1, 512 12.7 and 12.2, but slower from 540 on, where fewer lines
+// fit a block (540 13.6 and 14.9, 1024 16.7 and 19.4, 4096 37.2 and 51.2); FP32-mixed
+// faster at every length (256 23.8 and 14.3, 540 18.5 and 13.2, 4096 91.7 and 45.6).
+// It moves 3 or 4 arrays at 2.5 to 2.7 TB/s: latency at 16 warps per SM bounds it.
 // The problem supplies
 //   static constexpr int WORDS;                                             // planes staged: 0 the right-hand side, 1.. the stencil
 //   struct Stage { Stage(const Prob &, int line, int by);  void put(const Prob &, int r, double *w, int PL); }   // row r of the line, words PL apart

@@ -903,8 +903,9 @@ void launch_pseudo_prhs_fftx(const Ctx<R> &cx, cudaStream_t s, bool with_pseudo)
     const long long cells = (long long)g.N1 * g.N2 * g.N3;
     const int form = ifftx_form(cx.fp1u, NL);
     // the split form, but for small grids without a one-radix N1, where the second
-    // launch costs more than it frees (ps per cell, split and fused: 32^3 477 and
-    // 324; 96 x 77 x 90 46 and 50, FP32-mixed 49 and 59; 400 x 200 x 384 FP32-mixed 33 and 43)
+    // launch costs more than it frees (us per whole step, split and fused, FP64; FP32-
+    // mixed: 48^3 156.4, 154.8; 150.7, 150.3.  60^3 185.4, 185.0; 174.6, 176.2.
+    // 60 x 70 x 72 198.0, 199.7; 185.1, 186.4.  72 x 80 x 90 291.2, 293.6; 267.5, 276.6)
     if (form == 1 || cells >= 262144) {
         const size_t sm = form == 1 ? ifftx_smem(cx.fp1u, NL, 1) : (size_t)((NL + 1) / 2) * g.N1 * 2 * sizeof(double2);
         const int nt = ((NL + 1) / 2) * (g.N1 / cx.fp1u.radix[0]);
