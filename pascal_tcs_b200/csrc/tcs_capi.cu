@@ -184,7 +184,7 @@ struct tcs_ctx {
     ProbeState probe;
     int partials = 0;
     void *snap[10] = {};                 // on-device copy of T, U, V, W, P, dPhat, dP0 (+ U, V, W low words)
-    double snap_scal[S_NSCAL] = {};
+    double snap_scal[S_TIMEOUT + 1] = {};   // the scalars of the snapshot, and S_TIMEOUT cleared
     bool have_snap = false;
 };
 
@@ -1103,7 +1103,7 @@ int tcs_snapshot(tcs_ctx *c)
         c->snap[q] = sp;
         CK(cudaMemcpyAsync(c->snap[q], src[q], bytes, cudaMemcpyDeviceToDevice, c->stream));
     }
-    CK(cudaMemcpyAsync(c->snap_scal, c->cx.g.scal, sizeof(c->snap_scal), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(c->snap_scal, c->cx.g.scal, sizeof(double) * S_NSCAL, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     c->have_snap = true;
     return TCS_OK;
@@ -1121,7 +1121,6 @@ int tcs_restore(tcs_ctx *c)
     for (int q = 0; q < n; q++)
         CK(cudaMemcpyAsync(dst[q], c->snap[q], bytes, cudaMemcpyDeviceToDevice, c->stream));
     CK(cudaMemcpyAsync(c->cx.g.scal, c->snap_scal, sizeof(c->snap_scal), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemsetAsync(c->cx.g.scal + S_TIMEOUT, 0, sizeof(double), c->stream));
     c->ghost_ok |= (1u << TCS_F_T) | (1u << TCS_F_U) | (1u << TCS_F_V) | (1u << TCS_F_W) | (1u << TCS_F_P) | (1u << TCS_F_DPHAT);
     return TCS_OK;
 }

@@ -77,7 +77,7 @@ enum : int {
 // skipped, and the host reports TCS_ERR_CUDA, not a blow-up); S_CTR,
 // the count of diagnostics blocks done (an unsigned in the double's place); S_ROWS,
 // in the bounds-check build, the number of rows the line sweeps have checked.
-enum : int { S_OOB = S_NSCAL, S_TIMEOUT, S_CTR, S_ROWS, S_NALLOC };
+enum : int { S_TIMEOUT = S_NSCAL, S_OOB, S_CTR, S_ROWS, S_NALLOC };   // S_TIMEOUT next to the public ones: one copy restores them
 
 #if defined(TCS_BOUNDS_CHECK) && defined(__CUDA_ARCH__)
 #define TCS_OOB(scal, bad, fix)                          \
