@@ -233,11 +233,12 @@ int tcs_bounds_violations(tcs_ctx *ctx, double *count);
  * is checked as it is read and as it is written.  The count of those checks so far. */
 int tcs_bounds_rows(tcs_ctx *ctx, double *count);
 int tcs_set_use_graph(tcs_ctx *ctx, int on);
-/* The z sweeps of long FP64 lines wait for asynchronous copies, each wait bounded
- * to `polls` polls (default 2^22).  If one runs out, the rest of the step is skipped
- * and tcs_step, tcs_post_div, tcs_post_cfl and tcs_ensemble_step return
- * TCS_ERR_CUDA; the fields are then undefined until tcs_restore.  0 makes every
- * such wait run out at once, which is how the reporting is tested. */
+/* The z sweeps of long FP64 lines wait for asynchronous copies, each wait bounded to
+ * 2^22 polls, the first of each thread block to `polls` (default 2^22).  If one runs
+ * out, the rest of the step is skipped and tcs_step, tcs_post_div, tcs_post_cfl and
+ * tcs_ensemble_step return TCS_ERR_CUDA; the fields are then undefined until
+ * tcs_restore.  0 makes that first wait run out at once, which is how the reporting
+ * is tested. */
 int tcs_set_copy_polls(tcs_ctx *ctx, int polls);
 /* launch-shape knobs (powers of two): lines per thread block of the x and z
  * FFTs, and the most partitions a tridiagonal line is split over (TCS_TUNE_LANES;

@@ -80,7 +80,7 @@ struct Shapes {
     int ifft_lines_x;                            // lines per block of the inverse x transform
     int lanes;                                   // at most this many partitions (lanes) per line
     int tl_strided, tl_contig, tl_modal, long_lines, y_solver, mixed_rows, z_staging;   // knobs without effect: kept and returned
-    int copy_polls;                              // polls of the column form's waits for its copies
+    int copy_polls;                              // polls of a block's first wait for its copies in the column form
     bool spec_live;                              // the spectrum holds a right-hand side that no Poisson solve has taken yet
     FFTPlan fp1, fp3;
     FFTPlan fp1u;                                // N1 with radices up to 8 (the inverse x transform's one-radix form)

@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(256, 2) xmarch_kernel(const __grid_constant__ 
 // ---------------------------------------------------------------------------
 constexpr int COL_SLOTS = 4;
 constexpr double COL_TINY = 7.8886090522101181e-31;   // 2^-100
-constexpr int COL_WAIT = 1 << 22;                     // polls of a bounded wait (Shapes::copy_polls)
+constexpr int COL_WAIT = 1 << 22;                     // polls of a bounded wait (a block's first: Shapes::copy_polls)
 
 // FP64 problems that name their stream (Prob::NROW): the cyclic z sweeps.
 template <class P, class = void>
@@ -472,7 +472,6 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
 {
     using March = typename Prob::March;
     extern __shared__ __align__(16) double csm[];
-    if (__syncthreads_or(prob.skip())) return;                       // as one block: another block's failed wait may set the flag now
     const GridT<double> &g = prob.g;
     const int NS = 1 << lgNS, s = threadIdx.x / w, l = threadIdx.x - s * w, by = blockIdx.y, x0 = w * blockIdx.x;
     const int SW = col_slot_words<Prob>(w) * NS;                     // words of a ring slot
@@ -488,7 +487,7 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
         for (int q = 0; q < COL_SLOTS; q++) mbar_init(&bar[q], NS);
         mbar_init_fence();
     }
-    __syncthreads();
+    if (__syncthreads_or(prob.skip())) return;                       // as one block: another block's failed wait may set the flag now
     // one thread of each segment: plane k of the segment's row r (k = r0 + r + 1) into
     // slot (r + 1) mod COL_SLOTS (r = -1: what the first row needs of the plane below)
     auto issue = [&](int r) {
@@ -525,9 +524,9 @@ __global__ void __launch_bounds__(128, 4) column_kernel(const __grid_constant__ 
         March st(prob, sline, by, r0);
         double a, b, c, d;
         int r = 0;
-        bool ok = true, got = mbar_wait(&bar[0], 0, polls);
+        bool ok = true, got = mbar_wait(&bar[0], 0, polls);   // (one bound for every wait, kept through the march, spilled: dw_z at 512^3 2.98 -> 3.20 ms)
         for (; r < mmax; r++) {
-            got = mbar_wait(&bar[(r + 1) % COL_SLOTS], ((r + 1) / COL_SLOTS) & 1, polls) && got;
+            got = mbar_wait(&bar[(r + 1) % COL_SLOTS], ((r + 1) / COL_SLOTS) & 1, COL_WAIT) && got;
             if (got && r < m) {
                 typename March::In in;
                 st.fill(prob, r0 + r, in, mine + ((r + 1) % COL_SLOTS) * SW, mine + (r % COL_SLOTS) * SW, w, sline - x0);

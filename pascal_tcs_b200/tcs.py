@@ -432,7 +432,7 @@ class Solver:
         _check(load().tcs_set_use_graph(self._h, int(bool(on))), "use_graph")
 
     def set_copy_polls(self, polls: int) -> None:
-        """Bound of the waits for asynchronous copies (tcs_set_copy_polls); 0 makes each run out at once."""
+        """Bound of a block's first wait for asynchronous copies (tcs_set_copy_polls); 0 makes it run out at once."""
         _check(load().tcs_set_copy_polls(self._h, int(polls)), "set_copy_polls")
 
     # -- measurement ----------------------------------------------------------
