@@ -999,11 +999,12 @@ __device__ __forceinline__ R blockld_u_value(const GridT<R> &g, const FieldsT<R>
 }
 
 // KZ planes per thread: every input of the KZ cells is loaded before the first store.
-// Bound by its load latency, so by the warps per SM: with the face tables and no bound
-// the FP32 form took 40 registers (12 blocks) and ran slower than the kernel before the
-// tables, which formed the faces (us, before, unbounded, 16 blocks per SM: 256^3 160, 162,
-// 117; 400 x 200 x 384 306, 318, 220); in FP64 the compiler's own 48 registers left
-// loads waiting (256^3 216, 222 and, at up to 64, 195; 180 x 151 x 250 107, 111, 99).
+// Bound by its load latency.  With the face tables and no bound it ran slower than the
+// kernel before the tables, which formed the faces: the FP32 form at 40 registers and 45
+// warps per SM (us, before, unbounded, and with 16 blocks of 32 registers and 60 warps:
+// 256^3 160, 162, 117; 400 x 200 x 384 306, 318, 220), the FP64 form at 48, too few to
+// have a cell's loads on their way at once (256^3 216, 222 and, at up to 64, with 29 warps
+// instead of 38, 195; 180 x 151 x 250 107, 111, 99).
 template <class R, int KZ>
 __global__ void __launch_bounds__(128, HasLo<R>::on ? 16 : 8) blockld_u_kernel(GridT<R> g, FieldsT<R> f)
 {
