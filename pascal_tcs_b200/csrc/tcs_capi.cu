@@ -469,14 +469,12 @@ int tcs_create(const tcs_config *cfg, tcs_ctx **out)
                     &F.dU, &F.dV, &F.dW, &F.dP, &F.scr};
         for (R **p : fl) if (!r) r = dalloc(c, p, NP);
         if (!r) r = dalloc(c, &F.Mu2, (size_t)(N2 + 2) * (N3 + 2));
-        if (!r) r = dalloc(c, &F.iR2, (size_t)(N2 + 2) * (N3 + 2));
+        if (!r) r = dalloc(c, &F.iR2d, (size_t)(N2 + 2) * (N3 + 2));
         if (!r) r = dalloc(c, &F.MuT, (size_t)4 * (N2 + 2) * (N3 + 2));
         if (!r) r = dalloc(c, &F.iRT, (size_t)4 * (N2 + 2) * (N3 + 2));
         if (HasLo<R>::on) {
-            if (!r) r = dalloc(c, &F.iR2d, (size_t)(N2 + 2) * (N3 + 2));
             if (!r) r = dalloc(c, &F.iRTd, (size_t)4 * (N2 + 2) * (N3 + 2));
         } else {
-            F.iR2d = (double *)F.iR2;
             F.iRTd = (double *)F.iRT;
         }
         if (!r) r = dalloc(c, &F.S, (size_t)c->cx.h1p * N2 * N3);

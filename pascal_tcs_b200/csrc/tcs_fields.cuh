@@ -27,14 +27,13 @@ struct FieldsT {
     // FP64 form's scr, the FP32 form's FP64 staging array; null where the split
     // form does not run
     double *prhs;
-    // 2-D (j,k) property tables: Mu and invRho of mpi_momentum_coeffi, in the
-    // field type (read by the line sweeps), and invRho in FP64 (the same array
-    // in the FP64 form).  invRho differs from 1 by about 1e-3 for water, and
+    // 2-D (j,k) property tables: Mu of mpi_momentum_coeffi in the field type, invRho
+    // in FP64 in both forms (the sweeps read both from the face tables below).  invRho differs from 1 by about 1e-3 for water, and
     // the pressure right-hand side and the projection use 1 - invRho: from an
     // FP32 table those terms carried 6e-5 relative error, which left P 2-3e-5
     // off the FP64 form after 5-8 steps of the 256^3 and 512^3 water cases
     // (3-8e-6 with the FP64 table).
-    R *Mu2, *iR2;
+    R *Mu2;
     double *iR2d;
     // the same properties with their face averages, four words per (j,k) entry
     // (momentum_coeffi): Mu, Mu_y, Mu_z, Mu_yz and invRho, invRho_y, invRho_z, 0

@@ -16,8 +16,8 @@ namespace tcs {
 // ---------------------------------------------------------------------------
 // mpi_momentum_coeffi (:145-173) -> (j,k) tables from T(n1sub, j, k).
 // ---------------------------------------------------------------------------
-// Evaluated in FP64 in both forms; the FP32 form also keeps invRho in FP64
-// (FieldsT::iR2d) for the pressure right-hand side and the projection.
+// Evaluated in FP64 in both forms; invRho stays FP64 (FieldsT::iR2d, iRTd) for the
+// pressure right-hand side and the projection.
 template <class R>
 __global__ void momentum_coeffi_kernel(GridT<R> g, FieldsT<R> f)
 {
@@ -35,8 +35,7 @@ __global__ void momentum_coeffi_kernel(GridT<R> g, FieldsT<R> f)
     props(j, k, mu, ir);
     const int c = ix2(g, j, k);
     f.Mu2[c] = (R)mu;
-    f.iR2[c] = (R)ir;
-    if constexpr (HasLo<R>::on) f.iR2d[c] = ir;
+    f.iR2d[c] = ir;
     // the averages at the faces between row j-1 and j (y), plane k-1 and k (z)
     // and at the edge between them (yz), which the sweeps read instead of
     // forming them again at every i: Mu, Mu_y, Mu_z, Mu_yz and iR, iR_y, iR_z
